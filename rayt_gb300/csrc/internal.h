@@ -94,7 +94,7 @@ struct TraceParams {
   uint32_t* fault_bits;    // one bit per tree block
   int fault_bit_limit;     // number of tree blocks (bits in fault_bits)
   uint32_t* hit_bits;      // bit 2*cache_block + dup
-  int* n_words;            // number of non-NO_HIT words this pass
+  int* no_word;            // set to 1 when a ray produced no feedback word this pass
   unsigned long long* counters;  // optional: rays, link fetches, far fetches, iterations, hits, faults
   // served mode (zero in the per-frame path).  Client slot i owns the pixels
   // [client_base[i], client_base[i + 1]) of the image buffer.
@@ -104,9 +104,10 @@ struct TraceParams {
   unsigned long long finish_mask;  // continuation rays of these slots are finished, not traced
   int* client_faults;      // per slot: rays that faulted in this pass
   // persistent kernels
-  int* work;               // work counter, zero before the launch
+  int* work;               // persistent kernel: work counter, zero before the launch
   int refill;              // idle lanes that let a warp take new rays (< 32)
   int step_budget;         // iterations a warp runs between refill checks
+  int lanes;               // rays per warp (a power of two; see trace_lanes)
   ViewDesc views[kViewsPerLaunch];
 };
 
@@ -119,18 +120,19 @@ struct RayList {
   float* adv = nullptr;      // distance advanced over earlier passes (depth output only)
 };
 
-// first: rays come from the views' cameras (refill = 32: one thread per ray
-// over rays = total_tiles * 32 threads; refill < 32: the persistent
-// work-stealing kernel over `grid` CTAs, 0 = as many as are resident).
-// Otherwise the faulted rays of the input list, by a persistent kernel whose
-// warps take 32 rays at a time (the count is read on the device).
+// first: rays come from the views' cameras (refill = 32: one lane per ray of
+// the `rays` = total_tiles * 32; refill < 32: the persistent work-stealing
+// kernel over `grid` CTAs, 0 = as many as are resident).  Otherwise the `rays`
+// faulted rays of the input list, one lane each.
+// Rays per warp (TraceParams::lanes) for a launch over `rays` rays.
+int trace_lanes(bool first, int rays);
 cudaError_t launch_trace(const TraceParams& p, bool first, bool count, int rays, int grid, cudaStream_t s);
 // The same launch as a kernel node of a CUDA graph (args: room for one pointer;
 // p must stay valid until the node is added or updated).
 cudaError_t trace_node_params(const TraceParams* p, bool first, bool count, int rays, int grid, void** args,
                               cudaKernelNodeParams* kp);
 // Resident CTAs of the persistent traversal kernel on the current device.
-int trace_persistent_grid(bool first, bool count);
+int trace_persistent_grid(bool count);
 cudaError_t launch_finish(const TraceParams& p, int max_rays, cudaStream_t s);
 cudaError_t launch_fill_i32(int* p, int32_t v, size_t n, cudaStream_t s);
 // The reference's debug depth view (raytracer.cl) of views[0] into image.
@@ -142,7 +144,8 @@ struct UniqueFromBitsParams {
   int fault_words;
   const uint32_t* hit_bits;
   int hit_words;
-  const int* n_words;
+  const int* no_word;    // set: some ray of the pass produced no word
+  const int* n_in;       // later passes: rays traced (the other pixels have no word); null: all of them
   int total_pixels;
   int32_t* unique_out;   // room for fault bits + hit bits + 1
   const int* n_rays;     // rays the pass appended to its output list

@@ -66,7 +66,7 @@ class Renderer {
   cudaStream_t stream() const { return s_; }
 
  private:
-  static constexpr int kBlockInts = 16;  // pass block: {words, rays out, pad, pad, work counter per launch group}
+  static constexpr int kBlockInts = 16;  // pass block: {some ray without a word, rays out, pad, pad, work counter per launch group}
   Cache* cache_ = nullptr;
   int total_pixels_ = 0, padded_pixels_ = 0;
   cudaStream_t s_ = nullptr;
@@ -105,7 +105,7 @@ class Renderer {
   int* block(int k) const { return k ? d_state_ + kBlockInts + fault_words_ + hit_words_ : d_state_; }
   int SetViews(const float* m);
   TraceParams Params(int it) const;
-  int Grid(bool first, bool count) const;
+  int Grid(bool count) const;
   int Prepare(int it);
   int Trace(int it, bool count, int rays);
   UniqueFromBitsParams UniqueParams(int it) const;
@@ -123,7 +123,8 @@ class Renderer {
     std::vector<cudaGraphNode_t> trace_nodes;
     TraceParams key;  // the parameters (without views) it was built with
     int ctas = 0;     // and the persistent kernel's CTAs per SM
-    unsigned blocks = 0;  // later passes: the traversal node's grid now
+    unsigned blocks = 0;  // later passes: the traversal node's grid
+    int lanes = 0;        // and rays per warp now
   };
   Graph graphs_[3];
   void DropGraphs();
@@ -298,15 +299,16 @@ TraceParams Renderer::Params(int it) const {
   p.fault_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts);
   p.fault_bit_limit = (int)cache_->tree_blocks();
   p.hit_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts + fault_words_);
-  p.n_words = block(k);
+  p.no_word = block(k);
+  p.lanes = 32;
   p.work = block(k) + 4;
   p.refill = refill;
   p.step_budget = step_budget;
   return p;
 }
 
-int Renderer::Grid(bool first, bool count) const {
-  const int full = trace_persistent_grid(first, count);
+int Renderer::Grid(bool count) const {
+  const int full = trace_persistent_grid(count);
   if (ctas_per_sm <= 0) return full;
   int dev = 0, sms = 1;
   cudaGetDevice(&dev);
@@ -328,8 +330,9 @@ int Renderer::Prepare(int it) {
 int Renderer::Trace(int it, bool count, int rays) {
   TraceParams p = Params(it);
   if (count) p.counters = d_fetch_;
-  const int grid = refill < 32 ? Grid(it == 0, count) : 0;
+  const int grid = refill < 32 ? Grid(count) : 0;
   if (it > 0) {
+    p.lanes = trace_lanes(false, rays);
     RAYT_CUDA_TRY(launch_trace(p, false, count, rays, grid, s_));
     return RAYT_OK;
   }
@@ -339,6 +342,7 @@ int Renderer::Trace(int it, bool count, int rays) {
     std::memcpy(p.views, views_.data() + first, (size_t)p.n_views * sizeof(ViewDesc));
     p.total_tiles = group_tiles_[g];
     p.work = block(0) + 4 + g;
+    p.lanes = trace_lanes(true, p.total_tiles * 32);
     RAYT_CUDA_TRY(launch_trace(p, true, count, group_tiles_[g] * 32, grid, s_));
   }
   return RAYT_OK;
@@ -350,7 +354,8 @@ UniqueFromBitsParams Renderer::UniqueParams(int it) const {
   q.fault_words = fault_words_;
   q.hit_bits = reinterpret_cast<const uint32_t*>(d_state_ + kBlockInts + fault_words_);
   q.hit_words = hit_words_;
-  q.n_words = block(it & 1);
+  q.no_word = block(it & 1);
+  q.n_in = it > 0 ? block(1 - (it & 1)) + 1 : nullptr;
   q.n_rays = block(it & 1) + 1;
   q.total_pixels = total_pixels_;
   q.unique_out = d_unique_;
@@ -382,9 +387,12 @@ int Renderer::PassGraph(int kind, int it, int rays) {
       std::memcpy(p.views, views_.data() + v0, (size_t)p.n_views * sizeof(ViewDesc));
       p.total_tiles = group_tiles_[grp];
       p.work = block(0) + 4 + grp;
+      p.lanes = trace_lanes(true, p.total_tiles * 32);
     }
+  } else {
+    tp[0].lanes = trace_lanes(false, rays);
   }
-  const int grid = refill < 32 ? Grid(first, false) : 0;
+  const int grid = refill < 32 ? Grid(false) : 0;
   void* args[1];
   cudaKernelNodeParams kp;
   if (!g.exec) {
@@ -402,6 +410,7 @@ int Renderer::PassGraph(int kind, int it, int rays) {
     for (size_t i = 0; e == cudaSuccess && i < tp.size(); ++i) {
       trace_node_params(&tp[i], first, false, first ? group_tiles_[i] * 32 : rays, grid, args, &kp);
       g.blocks = kp.gridDim.x;
+      g.lanes = tp[i].lanes;
       e = cudaGraphAddKernelNode(&node, graph, &prev, 1, &kp);
       g.trace_nodes.push_back(node);
       prev = node;
@@ -431,11 +440,12 @@ int Renderer::PassGraph(int kind, int it, int rays) {
       RAYT_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g.exec, g.trace_nodes[i], &kp));
     }
   } else {
-    // a later pass's grid follows its ray count
+    // a later pass's grid and rays per warp follow its ray count
     trace_node_params(&tp[0], false, false, rays, grid, args, &kp);
-    if (kp.gridDim.x != g.blocks) {
+    if (kp.gridDim.x != g.blocks || tp[0].lanes != g.lanes) {
       RAYT_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g.exec, g.trace_nodes[0], &kp));
       g.blocks = kp.gridDim.x;
+      g.lanes = tp[0].lanes;
     }
   }
   RAYT_CUDA_TRY(cudaGraphLaunch(g.exec, s_));

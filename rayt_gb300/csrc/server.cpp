@@ -61,7 +61,7 @@ class Server {
   LibcRand rand;
 
  private:
-  static constexpr int kBlockInts = 16;  // {words, rays out, pad, pad, work: first pass, continuation}
+  static constexpr int kBlockInts = 16;  // {some ray without a word, rays out, pad}
   struct Client {
     bool live = false;
     int w = 0, h = 0;
@@ -338,7 +338,8 @@ TraceParams Server::Params(int k) const {
   p.fault_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts);
   p.fault_bit_limit = (int)cache_->tree_blocks();
   p.hit_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts + fault_words_);
-  p.n_words = block(k);
+  p.no_word = block(k);
+  p.lanes = 32;
   p.refill = 32;
   p.restart = 1;
   p.client_faults = d_client_faults_;
@@ -422,7 +423,7 @@ int Server::Step(int* finished) {
     }
     q.n_views = n;
     q.total_tiles = (int)tiles;
-    q.work = block(k) + 4 + (int)(g / kViewsPerLaunch) % 8;
+    q.lanes = trace_lanes(true, (int)tiles * 32);
     RAYT_CUDA_TRY(launch_trace(q, true, false, (int)tiles * 32, 0, s_));
     ++stats.kernel_launches;
   }
@@ -431,7 +432,7 @@ int Server::Step(int* finished) {
     TraceParams q = p;
     for (const Flight& f : flights_)
       if (!f.fresh && f.finishing) q.finish_mask |= 1ull << slot_of_client[f.client];
-    q.work = block(k) + 12;
+    q.lanes = trace_lanes(false, carried_);
     RAYT_CUDA_TRY(launch_trace(q, false, false, carried_, 0, s_));
     ++stats.kernel_launches;
   }
@@ -440,7 +441,7 @@ int Server::Step(int* finished) {
   u.fault_words = fault_words_;
   u.hit_bits = p.hit_bits;
   u.hit_words = hit_words_;
-  u.n_words = p.n_words;
+  u.no_word = p.no_word;
   u.n_rays = p.n_out;
   u.total_pixels = (int)std::min<int64_t>(rays_tick, 1 << 30);
   u.unique_out = d_unique_;

@@ -11,11 +11,11 @@
 //   block words     NodeToBlockKernel  (rayt/GPU_renderer/kernels/feedback_compression.cl:4-13)
 //
 // Kernels:
-//   trace_kernel             first pass, one thread per ray over the 32-pixel
+//   trace_kernel             one ray per lane: first passes over the 32-pixel
 //                            tiles of all views of the launch (4x8 by default;
-//                            lane i of a tile = pixel (i % tile_w, i / tile_w))
-//   trace_queue_kernel       later passes: persistent warps take 32 rays at a
-//                            time of the compacted list of rays that faulted
+//                            lane i of a tile = pixel (i % tile_w, i / tile_w)),
+//                            later passes over the compacted list of rays that
+//                            faulted; small launches give a warp fewer rays
 //   trace_persistent_kernel  first pass with work stealing: warps stop their
 //                            rays every step_budget iterations and refill idle
 //                            lanes (an autotuner candidate; slower on the
@@ -165,7 +165,9 @@ struct RayEnd {
 // are cast_begin + cast_run's; kept as a single loop with the reference's
 // shape because that form compiles to about 5% fewer warp instructions on
 // sm_103a than the resumable one.
-template <bool kCount>
+// kBias: the ray may have an LOD bias (origins that were advanced, the depth
+// view); first-pass rays start with a bias of zero.
+template <bool kCount, bool kBias>
 __device__ __forceinline__ RayEnd cast_ray(const TraceParams& p, float4 o, float4 d, uint32_t& fetches,
                                            uint32_t& far_fetches) {
   RayEnd r;
@@ -218,7 +220,14 @@ __device__ __forceinline__ RayEnd cast_ray(const TraceParams& p, float4 o, float
   // follows a pop; same value, one fewer test per iteration).  The counting
   // form keeps the reference's fetch points so its counts equal the oracle's.
   if (!kCount) desc = __ldg(p.links + parent);
-  while (scale < kSMax) {
+  // `child` holds 31 minus the mirrored child index (the reference's
+  // idx ^ octant, the child's flag in the descriptor): shifted left by it, a
+  // descriptor has that child's flag on top and only the flags below it under
+  // it, so one shift serves the test and the count of the children before it
+  // (1.5-2% off the first pass against a mask for each).
+  const int mirror = 31 ^ octant;
+  int child = mirror ^ idx;
+  for (;;) {  // left by a hit, a fault, the iteration limit or a pop past the root
     if (++iter > kIterLimit) {
       r.error = 1;
       break;
@@ -231,8 +240,8 @@ __device__ __forceinline__ RayEnd cast_ray(const TraceParams& p, float4 o, float
     const float ty_corner = py * ty_coef - ty_bias;
     const float tz_corner = pz * tz_coef - tz_bias;
     const float tc_max = fminf(fminf(tx_corner, ty_corner), tz_corner);
-    const uint32_t bit = 1u << (idx ^ octant);
-    if ((desc & bit) != 0 && t_min <= t_max) {
+    const uint32_t flags = desc << child;
+    if ((int)flags < 0 && t_min <= t_max) {
       if (desc & (1u << 8)) {  // children not loaded: fault
         r.node = (int)parent;
         r.t = t_min;
@@ -252,44 +261,52 @@ __device__ __forceinline__ RayEnd cast_ray(const TraceParams& p, float4 o, float
       } else {
         ofs = (desc >> 11) + parent - (1u << 20);
       }
-      ofs = min(ofs + __popc(desc & (bit - 1) & 255u), p.node_limit - 1u);
+      ofs = min(ofs + __popc(flags) - 1u, p.node_limit - 1u);
       desc = __ldg(p.links + ofs);
       if (kCount) ++fetches;
-      if (!(desc & 255u) || scale == 0 || tc_max * coef + bias >= scale_exp2) {
+      // without a bias the sum differs from the product in a zero's sign only
+      const float voxel = kBias ? tc_max * coef + bias : tc_max * coef;
+      if (!(desc & 255u) || scale == 0 || voxel >= scale_exp2) {
         r.t = t_min;
         r.node = (int)ofs;
         r.dup = (int)((desc >> 9) & 1u);
         break;
       }
+      // half is a power of two (at least 2^-24) and |coef| is about 1 or
+      // more, so half * coef is exact and the fused sum rounds as the
+      // reference's multiply and add do
       const float half = scale_exp2 * 0.5f;
-      const float tx_center = half * tx_coef + tx_corner;
-      const float ty_center = half * ty_coef + ty_corner;
-      const float tz_center = half * tz_coef + tz_corner;
+      const float tx_center = fmaf(half, tx_coef, tx_corner);
+      const float ty_center = fmaf(half, ty_coef, ty_corner);
+      const float tz_center = fmaf(half, tz_coef, tz_corner);
       if (tc_max < h) stack[scale] = make_uint4(parent, __float_as_uint(t_max), pdesc, 0u);
       h = tc_max;
       parent = ofs;
-      idx = 0;
       --scale;
       scale_exp2 = half;
-      if (tx_center > t_min) idx ^= 1, px = px + scale_exp2;
-      if (ty_center > t_min) idx ^= 2, py = py + scale_exp2;
-      if (tz_center > t_min) idx ^= 4, pz = pz + scale_exp2;
+      child = mirror;
+      if (tx_center > t_min) child ^= 1, px = px + half;
+      if (ty_center > t_min) child ^= 2, py = py + half;
+      if (tz_center > t_min) child ^= 4, pz = pz + half;
       t_max = tc_max;
       continue;
     }
-    int step = 0;
-    if (tx_corner <= tc_max) step ^= 1, px = px - scale_exp2;
-    if (ty_corner <= tc_max) step ^= 2, py = py - scale_exp2;
-    if (tz_corner <= tc_max) step ^= 4, pz = pz - scale_exp2;
+    const bool sx = tx_corner <= tc_max, sy = ty_corner <= tc_max, sz = tz_corner <= tc_max;
+    const int before = child;
+    if (sx) child ^= 1, px = px - scale_exp2;
+    if (sy) child ^= 2, py = py - scale_exp2;
+    if (sz) child ^= 4, pz = pz - scale_exp2;
     t_min = tc_max;
-    idx ^= step;
-    if ((idx & step) != 0) {
+    if (((child ^ mirror) & (child ^ before)) != 0) {  // idx & step: out of the parent
       uint32_t diff = 0;
-      if (step & 1) diff |= (uint32_t)(__float_as_int(px) ^ __float_as_int(px + scale_exp2));
-      if (step & 2) diff |= (uint32_t)(__float_as_int(py) ^ __float_as_int(py + scale_exp2));
-      if (step & 4) diff |= (uint32_t)(__float_as_int(pz) ^ __float_as_int(pz + scale_exp2));
-      scale = (__float_as_int((float)diff) >> 23) - 127;
-      if (scale >= kSMax) break;
+      if (sx) diff |= (uint32_t)(__float_as_int(px) ^ __float_as_int(px + scale_exp2));
+      if (sy) diff |= (uint32_t)(__float_as_int(py) ^ __float_as_int(py + scale_exp2));
+      if (sz) diff |= (uint32_t)(__float_as_int(pz) ^ __float_as_int(pz + scale_exp2));
+      scale = 31 - __clz((int)diff);  // the highest bit that changed
+      if (scale >= kSMax) {           // left the octree: a miss
+        r.node = -1;
+        break;
+      }
       scale_exp2 = __int_as_float((scale - kSMax + 127) << 23);
       const uint4 e = stack[scale];
       parent = e.x;
@@ -301,11 +318,10 @@ __device__ __forceinline__ RayEnd cast_ray(const TraceParams& p, float4 o, float
       px = __uint_as_float(shx << scale);
       py = __uint_as_float(shy << scale);
       pz = __uint_as_float(shz << scale);
-      idx = (int)((shx & 1u) | ((shy & 1u) << 1) | ((shz & 1u) << 2));
+      child = mirror ^ (int)((shx & 1u) | ((shy & 1u) << 1) | ((shz & 1u) << 2));
       h = 0.0f;
     }
   }
-  if (scale >= kSMax && !r.error && r.fault_block == -1) r.node = -1;  // left the octree: miss
   r.iter = iter;
   return r;
 }
@@ -502,24 +518,34 @@ __device__ __forceinline__ int warp_append(int* counter, bool pred) {
   return pred ? base + __popc(mask & ((1u << lane) - 1)) : -1;
 }
 
-// Sets bit `bit` (>= 0) of a bitmap, one atomic per distinct word in the warp.
+// Sets bit `bit` (>= 0) of a bitmap, one atomic per distinct word in the warp:
+// the lanes of a word OR their bits in one reduction, word by word (a tile's
+// hits lie in one or two words), then each word's first lane looks whether
+// they are all set already, all words at once.
 __device__ __forceinline__ void warp_set_bit(uint32_t* bits, int bit) {
   const unsigned active = __activemask();
-  const int word = bit >= 0 ? (bit >> 5) : -1;
-  const unsigned peers = __match_any_sync(active, word);
-  if (word < 0) return;
-  const unsigned m = 1u << (bit & 31);
-  unsigned acc = 0;
-  unsigned rest = peers;
-  while (rest) {
-    const int src = __ffs(rest) - 1;
-    acc |= __shfl_sync(peers, m, src);
-    rest &= rest - 1;
-  }
   const int lane = threadIdx.x & 31;
-  if (lane == __ffs(peers) - 1) {
-    if ((__ldcg(bits + word) & acc) != acc) atomicOr(bits + word, acc);
+  const int word = bit >> 5;  // negative: no bit
+  const unsigned m = 1u << (bit & 31);
+  unsigned todo = __ballot_sync(active, bit >= 0);
+  unsigned mine = 0;
+  while (todo) {
+    const int leader = __ffs(todo) - 1;
+    const bool same = word == __shfl_sync(active, word, leader);
+    const unsigned acc = __reduce_or_sync(active, same ? m : 0u);
+    if (lane == leader) mine = acc;
+    todo &= ~__ballot_sync(active, same);
   }
+  if (mine && (__ldcg(bits + word) & mine) != mine) atomicOr(bits + word, mine);
+}
+
+// Notes that a ray of the warp ended without a feedback word (the unique array
+// then ends with NO_HIT).  Only warps with such a ray touch the flag, and only
+// the first of them write it: a count of the words was one atomic per warp on
+// one address.
+__device__ __forceinline__ void mark_no_word(const TraceParams& p, bool none) {
+  const unsigned m = __ballot_sync(__activemask(), none);
+  if (m && (int)(threadIdx.x & 31) == __ffs(m) - 1 && __ldcg(p.no_word) == 0) *p.no_word = 1;
 }
 
 // View of the launch holding tile `tile` (tile_base is ascending).
@@ -645,11 +671,7 @@ __device__ __forceinline__ void end_ray(const TraceParams& p, const RayEnd& e, u
   }
   warp_set_bit(p.fault_bits, faulted && fault_block < p.fault_bit_limit ? fault_block : -1);
   warp_set_bit(p.hit_bits, hit ? (int)(2 * ((uint32_t)node / (uint32_t)p.nodes_in_block)) + dup : -1);
-  {
-    const unsigned active = __activemask();
-    const unsigned m = __ballot_sync(active, word != kNoHit);
-    if (m && lane == __ffs(m) - 1) atomicAdd(p.n_words, __popc(m));
-  }
+  mark_no_word(p, word == kNoHit);
   if (kCount) {
     const unsigned v[6] = {1u, fetches, far_fetches, (unsigned)e.iter, hit ? 1u : 0u, faulted ? 1u : 0u};
     const unsigned active = __activemask();
@@ -661,19 +683,30 @@ __device__ __forceinline__ void end_ray(const TraceParams& p, const RayEnd& e, u
   }
 }
 
-// One ray per thread over a grid that covers the launch's rays (a warp = one
-// 32-ray tile); the hardware hands CTAs to SMs as earlier ones retire.
+// One ray per lane, p.lanes of them per warp, over a grid that covers the
+// launch's rays: the first pass's 32-ray tiles, or (kFirst false) the rays
+// that faulted in the pass before.
 template <bool kFirst, bool kCount>
 __global__ void __launch_bounds__(kBlockThreads) trace_kernel(const __grid_constant__ TraceParams p) {
   const int total = kFirst ? p.total_tiles * 32 : *p.n_in;
-  const int r = blockIdx.x * kBlockThreads + threadIdx.x;
-  if (r >= total) return;
+  const int lane = threadIdx.x & 31;
+  const int r = (blockIdx.x * (kBlockThreads / 32) + (threadIdx.x >> 5)) * p.lanes + lane;
+  if (lane >= p.lanes || r >= total) return;
   uint32_t ray;
   float4 o, d;
   float adv;
   if (!ray_at<kFirst>(p, r, ray, o, d, adv)) return;
+  if (!kFirst && p.finish_mask && ((p.finish_mask >> slot_of(p, ray)) & 1ull)) {
+    // served mode: the request stops here; FinishTracingFrame's shading with
+    // the fault's parent node
+    const uchar4 col = (p.normals && p.colors) ? shade(p, (uint32_t)p.in_parent[r]) : make_uchar4(0, 0, 0, 0);
+    put_pixel(p, ray, finish(p, col));
+    if (p.depth) write_depth(p, ray, adv, p.in_parent[r]);
+    mark_no_word(p, true);
+    return;
+  }
   uint32_t fetches = 0, far_fetches = 0;
-  const RayEnd e = cast_ray<kCount>(p, o, d, fetches, far_fetches);
+  const RayEnd e = cast_ray<kCount, !kFirst>(p, o, d, fetches, far_fetches);
   end_ray<kCount>(p, e, ray, o, d, adv, fetches, far_fetches);
 }
 
@@ -739,39 +772,6 @@ __global__ void __launch_bounds__(kBlockThreads) trace_persistent_kernel(const _
   }
 }
 
-// Persistent form without lane refills, for the passes after the first: each
-// warp takes 32 rays at a time from the work counter and runs them to their
-// end.  Its grid does not depend on the ray count (read on the device), so the
-// pass can be replayed from a CUDA graph unchanged.
-template <bool kFirst, bool kCount>
-__global__ void __launch_bounds__(kBlockThreads) trace_queue_kernel(const __grid_constant__ TraceParams p) {
-  const int lane = threadIdx.x & 31;
-  const int total = kFirst ? p.total_tiles * 32 : *p.n_in;
-  for (;;) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(p.work, 32);
-    base = __shfl_sync(kFull, base, 0);
-    if (base >= total) break;
-    const int r = base + lane;
-    uint32_t ray;
-    float4 o, d;
-    float adv;
-    if (r < total && ray_at<kFirst>(p, r, ray, o, d, adv)) {
-      if (!kFirst && p.finish_mask && ((p.finish_mask >> slot_of(p, ray)) & 1ull)) {
-        // served mode: the request stops here; FinishTracingFrame's shading
-        // with the fault's parent node
-        const uchar4 col = (p.normals && p.colors) ? shade(p, (uint32_t)p.in_parent[r]) : make_uchar4(0, 0, 0, 0);
-        put_pixel(p, ray, finish(p, col));
-        if (p.depth) write_depth(p, ray, adv, p.in_parent[r]);
-      } else {
-        uint32_t fetches = 0, far_fetches = 0;
-        const RayEnd e = cast_ray<kCount>(p, o, d, fetches, far_fetches);
-        end_ray<kCount>(p, e, ray, o, d, adv, fetches, far_fetches);
-      }
-    }
-  }
-}
-
 // FinishTracingFrame for rays still faulted at the end of the frame: shade
 // with the fault's parent node as the cache holds it now.  Depth output: the
 // distance at which the ray stopped and that parent node.
@@ -816,7 +816,7 @@ __global__ void __launch_bounds__(kBlockThreads) depth_view_kernel(const __grid_
   const float bias = v.lod * dist(p1n, p2n);
   const float coef = bias < 1e-10f ? 0.0f : __fdiv_rn(v.lod * (dist(p1f, p2f) - dist(p1n, p2n)), dist(p1n, p1f));
   uint32_t fetches = 0, far_fetches = 0;
-  const RayEnd e = cast_ray<false>(p, make_float4(o[0], o[1], o[2], bias), make_float4(dx, dy, dz, coef), fetches,
+  const RayEnd e = cast_ray<false, true>(p, make_float4(o[0], o[1], o[2], bias), make_float4(dx, dy, dz, coef), fetches,
                                    far_fetches);
   uchar4 c;
   if (e.error || e.fault_block != -1) {
@@ -901,7 +901,7 @@ __global__ void __launch_bounds__(kUniqThreads) unique_from_bits_kernel(const Un
   __syncthreads();
   if (threadIdx.x == kUniqThreads - 1) {
     int n = pos;  // the last thread's end position = total set bits
-    if (*q.n_words < q.total_pixels) q.unique_out[n++] = kNoHit;
+    if (*q.no_word || (q.n_in && *q.n_in < q.total_pixels)) q.unique_out[n++] = kNoHit;
     q.counts_out[0] = n;
     q.counts_out[1] = fsum;
     q.counts_out[2] = q.n_rays ? *q.n_rays : 0;
@@ -917,44 +917,53 @@ int resident_grid(Kernel kernel) {
   return sms * (per_sm > 0 ? per_sm : 1);
 }
 
-template <bool kFirst, bool kCount>
-int persistent_grid() {
-  static const int grid = resident_grid(trace_persistent_kernel<kFirst, kCount>);
-  return grid;
-}
-
 template <bool kCount>
-int queue_grid() {
-  static const int grid = resident_grid(trace_queue_kernel<false, kCount>);
+int persistent_grid() {
+  static const int grid = resident_grid(trace_persistent_kernel<true, kCount>);
   return grid;
 }
 
 // The traversal launch for pass kind (first, count): function and grid.
 template <bool kFirst, bool kCount>
 void trace_launch_shape(const TraceParams& p, int rays, int grid, void** func, dim3* blocks) {
-  if (!kFirst) {
-    // persistent warps over the faulted rays; when the caller knows their
-    // count, no more CTAs than they fill (a later pass often traces a few
-    // hundred rays, and every idle warp of a full grid still launches and
-    // claims from the one work counter)
-    *func = reinterpret_cast<void*>(trace_queue_kernel<false, kCount>);
-    const int full = queue_grid<kCount>();
-    *blocks = dim3(rays > 0 ? std::min(full, (rays + kBlockThreads - 1) / kBlockThreads) : full);
-  } else if (p.refill < 32) {
+  if (kFirst && p.refill < 32) {
     *func = reinterpret_cast<void*>(trace_persistent_kernel<true, kCount>);
-    *blocks = dim3(grid > 0 ? grid : persistent_grid<true, kCount>());
+    *blocks = dim3(grid > 0 ? grid : persistent_grid<kCount>());
   } else {
-    *func = reinterpret_cast<void*>(trace_kernel<true, kCount>);
-    *blocks = dim3((rays + kBlockThreads - 1) / kBlockThreads);
+    *func = reinterpret_cast<void*>(trace_kernel<kFirst, kCount>);
+    const int per = kBlockThreads / 32 * p.lanes;
+    *blocks = dim3(std::max(1, (rays + per - 1) / per));
   }
 }
 
 }  // namespace
 
-int trace_persistent_grid(bool first, bool count) {
-  if (first) return count ? persistent_grid<true, true>() : persistent_grid<true, false>();
-  return count ? persistent_grid<false, true>() : persistent_grid<false, false>();
+// A warp of 32 rays runs both sides of most iterations (descents and
+// advances mix) and takes about 600 cycles for one; with 1 to 4 rays it is
+// 350 to 450.  That is what a launch waits for when its warps do not fill the
+// GPU and the longest ray decides, so such launches spread their rays over
+// more warps: first passes up to 48 warps per SM (one resident wave holds 40;
+// 128x96: 31.7 us with 32 rays per warp, 24.7 with 2; 200x150: 40.7 and 37.6
+// with 4; 400x300 the same with 32 and 16, slower with 8), later passes, whose
+// warps also end with a list append and feedback atomics each, up to 16
+// (1280x720 stream, 12 thousand rays per later pass: 0.199 ms of traversal per
+// frame with 32, 0.191 with 8 or 4, 0.196 with 2; 1919x1079, 27 thousand:
+// best with 32 or 16).  Larger launches are bound by instruction issue, where
+// half-empty warps cost 1.5 times the instructions.
+int trace_lanes(bool first, int rays) {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 1;
+  }();
+  const int warps = sms * (first ? 48 : 16);
+  int lanes = 32;
+  while (lanes > 1 && rays / (lanes / 2) <= warps) lanes /= 2;
+  return lanes;
 }
+
+int trace_persistent_grid(bool count) { return count ? persistent_grid<true>() : persistent_grid<false>(); }
 
 cudaError_t trace_node_params(const TraceParams* p, bool first, bool count, int rays, int grid, void** args,
                               cudaKernelNodeParams* kp) {

@@ -86,6 +86,31 @@ def test_resident_frame_vs_oracle(trees, size):
     assert rt.stats()["passes"] == ref[0]
 
 
+@pytest.mark.parametrize("size", [(60, 48), (97, 75), (121, 121), (171, 170), (241, 242), (342, 341), (484, 483)])
+@pytest.mark.parametrize("blocks", [0, 250])
+def test_rays_per_warp_vs_oracle(trees, size, blocks):
+    """Frame sizes on both sides of the ray counts where a launch gives its
+    warps fewer rays (1 to 32, 48 first-pass or 16 later-pass warps per SM),
+    resident and streamed: words of every pass and images."""
+    w, h = size
+    mats = [_matrix([a, -25.0, 0.0, 0.5 - 0.6 * np.sin(np.radians(a)), 0.7, 0.5 + 0.6 * np.cos(np.radians(a)), 60.0],
+                    w, h) for a in (20, 200)]
+    from oracle import oracle as O
+    sc = O.OracleScene(trees["terrain8s"], blocks, w, h)
+    sc.record(True)
+    libc_srand(3)
+    ld, cm, rt = _scene(trees["terrain8s"], blocks, w, h, seed=3)
+    rt.record_passes(True)
+    for m in mats:
+        passes, ref = sc.render(m)
+        rt.RenderFrame(m)
+        assert rt.stats()["passes"] == passes
+        for p in range(passes):
+            np.testing.assert_array_equal(rt.pass_words(p), sc.pass_words(p), err_msg="pass %d" % p)
+        np.testing.assert_array_equal(rt.read_image(), ref)
+    sc.close()
+
+
 EDGE_CAMERAS = {
     "looking_away": [225.0, 30.0, 0.0, -0.5, 1.5, 1.5, 60.0],       # every ray misses
     "inside_volume": [10.0, -5.0, 0.0, 0.5, 0.45, 0.5, 90.0],        # origin inside the octree
