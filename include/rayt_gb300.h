@@ -418,7 +418,7 @@ int rayt_feedback_unique(const int32_t* device_words, int n, int nodes_in_block,
  * All calls on a device share that array: calls whose GPU work overlaps race.
  * The library serialises its own calls: this entry point, rayt_sort_i32,
  * rayt_scan_i32 and rayt_feedback_unique take one lock and return after their
- * stream finished (they share a device error flag and look-back epoch).  The
+ * stream finished (they share the look-back epoch).  The
  * first call on a device looks up the array's address and zeroes the array on
  * `stream`; make it before any stream capture.
  * Returns after the result is on the device and *unique_count is set. */

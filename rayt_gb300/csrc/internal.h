@@ -155,43 +155,47 @@ cudaError_t launch_unique_from_bits(const UniqueFromBitsParams& p, cudaStream_t 
 cudaError_t unique_node_params(const UniqueFromBitsParams* q, void** args, cudaKernelNodeParams* kp);
 
 // ---- radix sort / scan / unique -------------------------------------------------
-struct SortScratch {
-  // sizes computed by sort_scratch_bytes
-  size_t bytes;
-};
+// Memory of a call: `scratch` (any contents), `status` (look-back words, zero or
+// left by earlier calls), `result` and `err` (device or mapped host memory the
+// host reads once the stream has finished).  `epoch` (27 bits, from
+// lookback_epoch_step) tags the call's look-back words.  err becomes 1 when a
+// bounded wait gave up.
 size_t feedback_scratch_bytes(int n);
-// Compaction (drop NO_HIT, NodeToBlock), radix sort, unique.  counts_dev[0]
-// receives the unique count (incl. NO_HIT); everything stays on device.
-cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t* unique_out,
-                                   int* counts_dev, void* scratch, size_t scratch_bytes, cudaStream_t s);
+size_t feedback_status_bytes(int n);
+// Compaction (drop NO_HIT, NodeToBlock) and sorted unique.  result[0] receives
+// the unique count (incl. NO_HIT), unless the keys span too wide a range for a
+// bitmap: feedback_unique_needs_radix(result) says so, and
+// feedback_unique_radix_device, on the same memory, then sorts them.
+cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t* unique_out, void* scratch,
+                                   unsigned long long* status, uint32_t epoch, int* result, int* err, cudaStream_t s);
+bool feedback_unique_needs_radix(const int* result);
+cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scratch, unsigned long long* status,
+                                         uint32_t epoch, int* result, int* err, cudaStream_t s);
 size_t sort_scratch_bytes(int n);
-cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, size_t scratch_bytes, cudaStream_t s);
-size_t scan_scratch_bytes(int n);
-cudaError_t scan_i32_device(int32_t* data, int n, void* scratch, size_t scratch_bytes, cudaStream_t s);
-// Device error flag set by bounded waits that gave up (decoupled look-back).
-int* device_error_flag();
-// The sort/unique look-back words carry the tag epoch * 8 + pass, where the
-// device-side epoch (27 bits) advances once per sort or unique call.  Sets
-// that epoch (stream-ordered on s).
-cudaError_t set_lookback_epoch(uint32_t epoch, cudaStream_t s);
+size_t sort_status_bytes(int n);
+cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch, int* err,
+                            cudaStream_t s);
+size_t scan_status_bytes(int n);
+cudaError_t scan_i32_device(int32_t* data, int n, unsigned long long* status, uint32_t epoch, int* err,
+                            cudaStream_t s);
 
 // ---- stand-alone primitives (prims.cpp) -------------------------------------------
 // Serialises every sort/scan/unique entry point on all devices: they share
-// the device error flag and the look-back epoch, and each one holds the lock
-// until its stream has finished its work.
+// scratch memory and the look-back epoch, and each one holds the lock until
+// its stream has finished its work.
 std::mutex& prims_mutex();
-// Called (with prims_mutex held) before each sort or unique call on the
-// current device: counts epochs, and before the epoch would repeat a tag
-// still present in a look-back table (after 2^27 - 1 calls), clears every
-// look-back table of the device on s and restarts the epoch at 0.
-int lookback_epoch_step(cudaStream_t s);
-// Registers a scratch area holding look-back tables on the current device
-// besides the library's growable scratch (the allocation-free entry point's
-// static array), so lookback_epoch_step clears it too.
+// Called (with prims_mutex held) before each call on the current device: its
+// epoch.  Before the epoch would repeat a tag still present in a look-back
+// table (after 2^27 - 1 calls), clears every look-back table of the device on
+// s and restarts at 1.
+int lookback_epoch_step(cudaStream_t s, uint32_t* epoch);
+// Registers a look-back table on the current device besides the library's own
+// (the allocation-free entry point's static array), so lookback_epoch_step
+// clears it too.
 void register_lookback_area(void* p, size_t bytes);
 // Runs one wait on a word nothing publishes, with a limit of limit_s seconds
-// (restored to 1 s after); the wait must give up and set the error flag.
-cudaError_t bounded_wait_probe(double limit_s, cudaStream_t s);
+// (restored to 1 s after); the wait must give up and set *err.
+cudaError_t bounded_wait_probe(double limit_s, int* err, cudaStream_t s);
 
 // ---- block upload --------------------------------------------------------------
 constexpr int kMaxChannels = 8;

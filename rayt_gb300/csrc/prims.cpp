@@ -1,28 +1,92 @@
 // C ABI of the stand-alone feedback primitives (GPUSort, GPUScan and the
-// feedback extractor's GetUnique).  Scratch memory is a per-device buffer the
+// feedback extractor's GetUnique).  Scratch memory is per-device buffers the
 // library grows on demand and keeps; calls are serialised by one mutex, so
 // concurrent host threads do not share it mid-operation.
+#include <algorithm>
 #include <mutex>
 #include "internal.h"
 
 namespace rayt {
 namespace {
-struct Scratch {
-  void* ptr = nullptr;
-  size_t bytes = 0;
+// Memory and bookkeeping of one device.  The look-back words have a buffer of
+// their own: they are recognised by their tag, so no other data may ever lie
+// where a later call looks for them.
+struct Device {
+  void* scratch = nullptr;
+  size_t scratch_bytes = 0;
+  unsigned long long* status = nullptr;
+  size_t status_bytes = 0;
+  void* area = nullptr;       // the allocation-free entry point's look-back words
+  size_t area_bytes = 0;
+  uint32_t epoch = 0;         // of the last call since the tables were cleared
+  int* host = nullptr;        // mapped pinned: [0] error flag, [1..2] result
+  int* host_dev = nullptr;
 };
-Scratch g_scratch[64];
-
-// Look-back epoch bookkeeping per device: calls since the tables were last
-// cleared (= the device epoch), and the static area of the allocation-free
-// entry point.
+Device g_devices[64];
 constexpr uint32_t kEpochLimit = (1u << 27) - 1;
-uint32_t g_epoch_calls[64];
-Scratch g_static_area[64];
 
-int current_device(int* dev) {
-  RAYT_CUDA_TRY(cudaGetDevice(dev));
-  if (*dev < 0 || *dev >= 64) return fail(RAYT_E_ARG, "device ordinal out of range");
+int current_device(Device** d) {
+  int dev = 0;
+  RAYT_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return fail(RAYT_E_ARG, "device ordinal out of range");
+  *d = &g_devices[dev];
+  return RAYT_OK;
+}
+
+// Clears the look-back tables on s.
+int clear_tables(Device& d, cudaStream_t s) {
+  if (d.status) RAYT_CUDA_TRY(cudaMemsetAsync(d.status, 0, d.status_bytes, s));
+  if (d.area) RAYT_CUDA_TRY(cudaMemsetAsync(d.area, 0, d.area_bytes, s));
+  d.epoch = 0;
+  return RAYT_OK;
+}
+
+template <typename T>
+int grow(T** p, size_t* have, size_t bytes) {
+  if (*have >= bytes) return RAYT_OK;
+  if (*p) {
+    RAYT_CUDA_TRY(cudaDeviceSynchronize());
+    cudaFree(*p);
+    *p = nullptr;
+    *have = 0;
+  }
+  if (cudaMalloc((void**)p, bytes) != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();
+    return fail(RAYT_E_OOM, "scratch allocation failed");
+  }
+  *have = bytes;
+  return RAYT_OK;
+}
+
+// The current device's memory for a call, and the call's epoch.
+int begin(size_t scratch_bytes, size_t status_bytes, cudaStream_t s, Device** out, uint32_t* epoch) {
+  int rc = current_device(out);
+  if (rc != RAYT_OK) return rc;
+  Device& d = **out;
+  if (!d.host) {
+    RAYT_CUDA_TRY(cudaHostAlloc(&d.host, 4 * sizeof(int), cudaHostAllocMapped));
+    for (int k = 0; k < 4; ++k) d.host[k] = 0;
+    RAYT_CUDA_TRY(cudaHostGetDevicePointer((void**)&d.host_dev, d.host, 0));
+  }
+  if ((rc = grow(&d.scratch, &d.scratch_bytes, scratch_bytes)) != RAYT_OK) return rc;
+  if (d.status_bytes < status_bytes) {
+    if ((rc = grow(&d.status, &d.status_bytes, status_bytes)) != RAYT_OK) return rc;
+    // look-back words are epoch-tagged, never cleared: start from zeros,
+    // ordered before the call's kernels on the caller's stream
+    RAYT_CUDA_TRY(cudaMemsetAsync(d.status, 0, d.status_bytes, s));
+  }
+  return lookback_epoch_step(s, epoch);
+}
+
+// Waits for the call's work and reads the error flag.
+int finish(Device& d, cudaStream_t s) {
+  RAYT_CUDA_TRY(cudaStreamSynchronize(s));
+  volatile int* flag = d.host;
+  if (*flag) {
+    *flag = 0;
+    return fail(RAYT_E_TIMEOUT, "a bounded device wait gave up (look-back did not complete)");
+  }
   return RAYT_OK;
 }
 }  // namespace
@@ -33,112 +97,22 @@ std::mutex& prims_mutex() {
 }
 
 void register_lookback_area(void* p, size_t bytes) {
-  int dev = 0;
-  if (current_device(&dev) != RAYT_OK) return;
-  g_static_area[dev].ptr = p;
-  g_static_area[dev].bytes = bytes;
+  Device* d = nullptr;
+  if (current_device(&d) != RAYT_OK) return;
+  d->area = p;
+  d->area_bytes = bytes;
 }
 
-int lookback_epoch_step(cudaStream_t s) {
-  int dev = 0;
-  int rc = current_device(&dev);
+int lookback_epoch_step(cudaStream_t s, uint32_t* epoch) {
+  Device* d = nullptr;
+  int rc = current_device(&d);
   if (rc != RAYT_OK) return rc;
-  if (g_epoch_calls[dev] >= kEpochLimit) {
-    // the next epoch would reuse a tag that old look-back words may still
-    // carry: zero every table (a zero word is never "published") and restart
-    for (const Scratch* a : {&g_scratch[dev], &g_static_area[dev]})
-      if (a->ptr) RAYT_CUDA_TRY(cudaMemsetAsync(a->ptr, 0, a->bytes, s));
-    RAYT_CUDA_TRY(set_lookback_epoch(0, s));
-    g_epoch_calls[dev] = 0;
-  }
-  ++g_epoch_calls[dev];
+  // the next epoch would reuse a tag that old look-back words may still carry:
+  // zero every table (a zero word is never "published") and restart
+  if (d->epoch >= kEpochLimit && (rc = clear_tables(*d, s)) != RAYT_OK) return rc;
+  *epoch = ++d->epoch;
   return RAYT_OK;
 }
-
-namespace {
-
-int get_scratch(size_t bytes, void** out, cudaStream_t stream) {
-  int dev = 0;
-  RAYT_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return fail(RAYT_E_ARG, "device ordinal out of range");
-  Scratch& s = g_scratch[dev];
-  if (s.bytes < bytes) {
-    if (s.ptr) {
-      RAYT_CUDA_TRY(cudaDeviceSynchronize());
-      cudaFree(s.ptr);
-      s.ptr = nullptr;
-      s.bytes = 0;
-    }
-    if (cudaMalloc(&s.ptr, bytes) != cudaSuccess) return fail(RAYT_E_OOM, "scratch allocation failed");
-    s.bytes = bytes;
-    // the sort's look-back words are epoch-tagged, never cleared: start from
-    // zeros, ordered before the call's kernels on the caller's stream
-    RAYT_CUDA_TRY(cudaMemsetAsync(s.ptr, 0, bytes, stream));
-  }
-  *out = s.ptr;
-  return RAYT_OK;
-}
-
-int check_device_error(cudaStream_t s) {
-  RAYT_CUDA_TRY(cudaStreamSynchronize(s));
-  int flag = 0;
-  RAYT_CUDA_TRY(cudaMemcpy(&flag, device_error_flag(), 4, cudaMemcpyDeviceToHost));
-  if (flag) {
-    int zero = 0;
-    cudaMemcpy(device_error_flag(), &zero, 4, cudaMemcpyHostToDevice);
-    return fail(RAYT_E_TIMEOUT, "a bounded device wait gave up (look-back did not complete)");
-  }
-  return RAYT_OK;
-}
-
-// rayt_feedback_unique's device work (4 memsets and 12 kernels, most of them
-// short or returning at once) as one CUDA graph, replayed while the call's
-// arguments repeat (a frame loop calls with the same buffers every frame):
-// one graph launch instead of 16 stream operations.  The count and the
-// device error flag come back in one copy into pinned memory.
-struct UniqueGraph {
-  const int32_t* words = nullptr;
-  int n = 0, nib = 0;
-  int32_t* out = nullptr;
-  void* scratch = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  cudaStream_t capture = nullptr;  // private stream the graph is captured on
-  int* host = nullptr;             // pinned: [0] unique count, [1] error flag
-};
-UniqueGraph g_unique[64];
-
-// Launches the device work of one call on s: the cached graph when the
-// arguments match, else a newly captured one; direct launches if capture
-// fails.  Then queues the read-back of the count and the error flag.
-int unique_launch(int dev, const int32_t* words, int n, int nib, int32_t* out, void* scratch, size_t bytes,
-                  int* counts, cudaStream_t s, int** host) {
-  UniqueGraph& g = g_unique[dev];
-  if (!g.host) RAYT_CUDA_TRY(cudaHostAlloc(&g.host, 2 * sizeof(int), cudaHostAllocDefault));
-  if (!g.capture) RAYT_CUDA_TRY(cudaStreamCreateWithFlags(&g.capture, cudaStreamNonBlocking));
-  const bool same = g.exec && g.words == words && g.n == n && g.nib == nib && g.out == out && g.scratch == scratch;
-  if (!same) {
-    if (g.exec) cudaGraphExecDestroy(g.exec);
-    g.exec = nullptr;
-    cudaGraph_t graph = nullptr;
-    if (cudaStreamBeginCapture(g.capture, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
-      const cudaError_t le = feedback_unique_device(words, n, nib, out, counts, scratch, bytes, g.capture);
-      const cudaError_t ce = cudaStreamEndCapture(g.capture, &graph);
-      if (le == cudaSuccess && ce == cudaSuccess && graph &&
-          cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess)
-        g.exec = nullptr;
-      if (graph) cudaGraphDestroy(graph);
-    }
-    cudaGetLastError();  // a failed capture leaves its error behind; the launches below report their own
-    g.words = words, g.n = n, g.nib = nib, g.out = out, g.scratch = scratch;
-  }
-  if (g.exec) RAYT_CUDA_TRY(cudaGraphLaunch(g.exec, s));
-  else RAYT_CUDA_TRY(feedback_unique_device(words, n, nib, out, counts, scratch, bytes, s));
-  RAYT_CUDA_TRY(cudaMemcpyAsync(g.host, counts, sizeof(int), cudaMemcpyDeviceToHost, s));
-  RAYT_CUDA_TRY(cudaMemcpyAsync(g.host + 1, device_error_flag(), sizeof(int), cudaMemcpyDeviceToHost, s));
-  *host = g.host;
-  return RAYT_OK;
-}
-}  // namespace
 }  // namespace rayt
 
 using rayt::fail;
@@ -151,13 +125,12 @@ int rayt_sort_i32(int32_t* data, int n, void* stream) {
   if (n <= 1) return RAYT_OK;
   std::lock_guard<std::mutex> lock(rayt::prims_mutex());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  void* scratch = nullptr;
-  const size_t bytes = rayt::sort_scratch_bytes(n);
-  int rc = rayt::get_scratch(bytes, &scratch, s);
+  rayt::Device* d = nullptr;
+  uint32_t epoch = 0;
+  const int rc = rayt::begin(rayt::sort_scratch_bytes(n), rayt::sort_status_bytes(n), s, &d, &epoch);
   if (rc != RAYT_OK) return rc;
-  if ((rc = rayt::lookback_epoch_step(s)) != RAYT_OK) return rc;
-  RAYT_CUDA_TRY(rayt::sort_i32_device(data, n, scratch, bytes, s));
-  return rayt::check_device_error(s);
+  RAYT_CUDA_TRY(rayt::sort_i32_device(data, n, d->scratch, d->status, epoch, d->host_dev, s));
+  return rayt::finish(*d, s);
 }
 
 int rayt_scan_i32(int32_t* data, int n, void* stream) {
@@ -166,23 +139,22 @@ int rayt_scan_i32(int32_t* data, int n, void* stream) {
   if (n == 0) return RAYT_OK;
   std::lock_guard<std::mutex> lock(rayt::prims_mutex());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  void* scratch = nullptr;
-  const size_t bytes = rayt::scan_scratch_bytes(n);
-  int rc = rayt::get_scratch(bytes, &scratch, s);
+  rayt::Device* d = nullptr;
+  uint32_t epoch = 0;
+  const int rc = rayt::begin(0, rayt::scan_status_bytes(n), s, &d, &epoch);
   if (rc != RAYT_OK) return rc;
-  RAYT_CUDA_TRY(rayt::scan_i32_device(data, n, scratch, bytes, s));
-  return rayt::check_device_error(s);
+  RAYT_CUDA_TRY(rayt::scan_i32_device(data, n, d->status, epoch, d->host_dev, s));
+  return rayt::finish(*d, s);
 }
 
 int rayt_testing_set_lookback_epoch(uint32_t calls) {
   if (calls >= (1u << 27)) return fail(RAYT_E_ARG, "rayt_testing_set_lookback_epoch: epoch out of range");
   std::lock_guard<std::mutex> lock(rayt::prims_mutex());
-  int dev = 0;
-  RAYT_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return fail(RAYT_E_ARG, "device ordinal out of range");
-  RAYT_CUDA_TRY(rayt::set_lookback_epoch(calls, nullptr));
+  rayt::Device* d = nullptr;
+  const int rc = rayt::current_device(&d);
+  if (rc != RAYT_OK) return rc;
   RAYT_CUDA_TRY(cudaDeviceSynchronize());
-  rayt::g_epoch_calls[dev] = calls;
+  d->epoch = calls;
   return RAYT_OK;
 }
 
@@ -190,8 +162,12 @@ int rayt_selftest_bounded_wait(double limit_s, void* stream) {
   if (!(limit_s > 0) || limit_s > 10) return fail(RAYT_E_ARG, "rayt_selftest_bounded_wait: limit out of range (0, 10] s");
   std::lock_guard<std::mutex> lock(rayt::prims_mutex());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  RAYT_CUDA_TRY(rayt::bounded_wait_probe(limit_s, s));
-  const int rc = rayt::check_device_error(s);
+  rayt::Device* d = nullptr;
+  uint32_t epoch = 0;
+  int rc = rayt::begin(0, 0, s, &d, &epoch);
+  if (rc != RAYT_OK) return rc;
+  RAYT_CUDA_TRY(rayt::bounded_wait_probe(limit_s, d->host_dev, s));
+  rc = rayt::finish(*d, s);
   if (rc == RAYT_E_TIMEOUT) return RAYT_OK;  // the wait gave up as it must
   return rc != RAYT_OK ? rc : fail(RAYT_E_STATE, "bounded wait did not give up");
 }
@@ -206,24 +182,18 @@ int rayt_feedback_unique(const int32_t* words, int n, int nib, int32_t* unique, 
   }
   std::lock_guard<std::mutex> lock(rayt::prims_mutex());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  void* scratch = nullptr;
-  const size_t bytes = rayt::feedback_scratch_bytes(n) + 256;
-  int rc = rayt::get_scratch(bytes, &scratch, s);
+  rayt::Device* d = nullptr;
+  uint32_t epoch = 0;
+  int rc = rayt::begin(rayt::feedback_scratch_bytes(n), rayt::feedback_status_bytes(n), s, &d, &epoch);
   if (rc != RAYT_OK) return rc;
-  int* counts = reinterpret_cast<int*>(static_cast<uint8_t*>(scratch) + (bytes - 256));
-  int dev = 0;
-  RAYT_CUDA_TRY(cudaGetDevice(&dev));
-  int* host = nullptr;
-  if ((rc = rayt::lookback_epoch_step(s)) != RAYT_OK) return rc;
-  rc = rayt::unique_launch(dev, words, n, nib, unique, scratch, bytes - 256, counts, s, &host);
-  if (rc != RAYT_OK) return rc;
-  RAYT_CUDA_TRY(cudaStreamSynchronize(s));
-  if (host[1]) {
-    const int zero = 0;
-    cudaMemcpy(rayt::device_error_flag(), &zero, 4, cudaMemcpyHostToDevice);
-    return fail(RAYT_E_TIMEOUT, "a bounded device wait gave up (look-back did not complete)");
+  int *err = d->host_dev, *result = d->host_dev + 1;
+  RAYT_CUDA_TRY(rayt::feedback_unique_device(words, n, nib, unique, d->scratch, d->status, epoch, result, err, s));
+  if ((rc = rayt::finish(*d, s)) != RAYT_OK) return rc;
+  if (rayt::feedback_unique_needs_radix(d->host + 1)) {
+    RAYT_CUDA_TRY(rayt::feedback_unique_radix_device(n, unique, d->scratch, d->status, epoch, result, err, s));
+    if ((rc = rayt::finish(*d, s)) != RAYT_OK) return rc;
   }
-  *unique_count = host[0];
+  *unique_count = d->host[1];
   return RAYT_OK;
 }
 

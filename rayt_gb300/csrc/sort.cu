@@ -1,36 +1,40 @@
-// Feedback primitives: stream compaction, LSD radix sort and unique of int32
-// feedback words, and an inclusive scan.
+// Feedback primitives: sorted unique of int32 feedback words, radix sort, and
+// an inclusive scan.
 //
 // The reference does this with a work-group merge sort plus log2(N/wg) global
 // merge passes (rayt/GPU algorithms/kernels/merge_sort.cl:2-73), an
 // adjacent-difference flag, a Hillis-Steele scan of log2(N) full passes
 // (rayt/GPU algorithms/kernels/scan.cl:2-12) and a scatter
 // (rayt/GPU_renderer/kernels/feedback_compression.cl:4-34).  Here:
+//
+// Feedback unique, up to kSmall words: small_unique_kernel, one CTA.  Above:
 //   compact_kernel   drops NO_HIT words, applies NodeToBlock, maps each word
 //                    to an unsigned key (x ^ 0x80000000 keeps signed order),
-//                    builds all four 8-bit digit histograms and the key range
-//                    in the same read,
-//   hist_offsets     digit offsets; for feedback unique, chooses the path:
-//   bitmap path      (the keys span at most 32 values per input word and at
+//                    drops most repeats through a per-CTA filter, finds the
+//                    key range; its last CTA chooses the path:
+//   bitmap           (the keys span at most 32 values per input word and at
 //                    most 2^26) a bitmap over [min, max], whose set bits read
-//                    in order are the sorted unique set: range_hist and
-//                    range_partition split the keys into 256 ranges
-//                    (unstable), bucket_bitmap builds each range's slice of the
-//                    bitmap in shared memory (so frequent keys cost no global
-//                    atomics), bitmap_unique writes the set bits in order,
-//   radix path       (wider ranges, and GPUSort) four stable digit_kernel
-//                    passes (persistent CTAs, tiles of 8192 keys brought into
-//                    shared memory by bulk async copies a tile ahead, ranking
-//                    through per-warp peer masks in shared memory, per-digit
-//                    decoupled look-back, scatter staged through shared
-//                    memory) and unique_kernel (run starts counted per tile
-//                    with a look-back prefix).
-// The kernels of the path not taken return at once.  Tiles are claimed in
-// order from an atomic counter, by one CTA per tile (the scan) or by
-// persistent CTAs until the device-side count runs out (the digit passes,
-// feedback unique), so a tile only waits on tiles claimed by running CTAs.
-// The sort's look-back words
-// are tagged with a per-call epoch and the pass, so its table is never
+//                    in order are the sorted unique set: set straight into
+//                    the global bitmap and written out (direct_bitmap: few
+//                    keys or a small bitmap), or range by range: range_hist and range_partition
+//                    split the keys into 256 ranges (unstable), bucket_bitmap
+//                    builds each range's slice in shared memory, emit writes
+//                    the set bits in order.
+//   radix            (wider ranges; launched once the host has read the
+//                    choice) digit_hist, the digit passes, unique_kernel.
+// Sort, up to kSmall keys: small_sort_kernel, one CTA.  Above: digit_hist (the
+// four digits' counts in one read) and four digit_kernel passes (persistent
+// CTAs, tiles of 8192 keys brought into shared memory by bulk async copies a
+// tile ahead, per-digit decoupled look-back, scatter staged through shared
+// memory); a pass whose digit is the same in every key is skipped.
+//
+// Scan: scan_kernel.
+//
+// The scan, direct_bitmap and emit kernels are cooperative launches (their CTAs
+// wait on one another).  Tiles of the digit and unique kernels are claimed in order from an atomic
+// counter by persistent CTAs until they run out, so a tile only waits on tiles
+// claimed by running CTAs.  Published words live in a table of their own
+// and are tagged with a per-call epoch and the pass, so the table is never
 // cleared.  Every wait is bounded and sets an error flag instead of hanging.
 #include <algorithm>
 
@@ -45,23 +49,27 @@ constexpr int kItems = 16;
 constexpr int kTile = kThreads * kItems;  // 4096 keys
 constexpr int kBuckets = 256;
 constexpr int kPasses = 4;
-// histogram rows: the four digits, then the range buckets' counts and offsets
-constexpr int kHistRows = kPasses + 2;
-constexpr int kRangeCounts = kPasses * kBuckets, kRangeOffsets = (kPasses + 1) * kBuckets;
 // the range partition's per-bucket cursors, one per 128-byte line, so that
 // claims on different buckets (every tile claims from most of them) never
 // contend for one line
 constexpr int kCursorStride = 32;
-// tile counters: digit passes 0-3, unique, bitmap unique, range histogram done
-// count, bucket items
-constexpr int kCtrUnique = 4, kCtrBitmapUnique = 5, kCtrRangeDone = 6, kCtrBuckets = 7;
 // the bitmap path keeps one range bucket's bitmap (span / 256 bits) in shared memory
 constexpr int kMaxSpanLog2 = 26;
+// Inputs of up to kDirectWords words put their keys straight into the bitmap
+// (the launches of the partition would cost more than they give).  Of larger
+// ones, those that kept up to kDirectKeys keys, or whose bitmap is built in
+// shared memory: scattered atomics on a wide one take 10 to 100 us per million
+// keys (30 million words, 1.5 million kept, 50 million bits: 196 us straight,
+// 160 us partitioned).
+constexpr int kDirectWords = 1 << 21;
+constexpr int kDirectKeys = 1 << 18;
+// A bitmap of up to this many words is built in shared memory.
+constexpr int kDirectSliceWords = 1 << 15;
 constexpr long long kSpinLimit = 1ll << 26;  // polls, a backstop to the time limit
 
-__device__ int g_error_flag;
 // Time limit of every wait on another CTA's result (ns): a correct wait ends in
-// microseconds, so one that lasts this long sets g_error_flag and gives up.
+// microseconds, so one that lasts this long sets the call's error flag and
+// gives up.
 __device__ unsigned long long g_wait_ns = 1000000000ull;
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -73,10 +81,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
 __device__ __forceinline__ bool wait_over(long long& spins, unsigned long long start) {
   return ++spins > kSpinLimit || ((spins & 63) == 0 && global_ns() - start > g_wait_ns);
 }
-// Call counter of the sort/unique kernels.  Their look-back words carry the
-// tag epoch * 8 + pass, so words left by earlier calls never look published
-// and the look-back table needs no clearing between passes or calls.
-__device__ uint32_t g_epoch;
+// Sets a call's error flag (device or mapped host memory).
+__device__ __forceinline__ void set_error(int* err) { *(volatile int*)err = 1; }
 
 __device__ __forceinline__ unsigned long long ld_volatile64(const unsigned long long* p) {
   return *(const volatile unsigned long long*)p;
@@ -85,7 +91,8 @@ __device__ __forceinline__ void st_volatile64(unsigned long long* p, unsigned lo
   *(volatile unsigned long long*)p = v;
 }
 
-// Look-back words: [63:34] tag, [33:32] 1 = tile aggregate, 2 = inclusive
+// Look-back words: [63:34] tag (the call's 27-bit epoch * 8 + the pass, so words
+// of earlier calls and passes never look published), [33:32] 1 = tile aggregate, 2 = inclusive
 // prefix, [31:0] value.
 __device__ __forceinline__ unsigned long long lb_word(uint32_t tag, uint32_t flag, uint32_t value) {
   return ((unsigned long long)tag << 34) | ((unsigned long long)flag << 32) | value;
@@ -100,7 +107,8 @@ constexpr int kLookAhead = 4;
 __device__ __forceinline__ bool lb_ready(unsigned long long w, uint32_t tag) {
   return (uint32_t)(w >> 34) == tag && ((w >> 32) & 3u) != 0;
 }
-__device__ uint32_t look_back(const unsigned long long* status, int tile, int stride, int lane, uint32_t tag) {
+__device__ uint32_t look_back(const unsigned long long* status, int tile, int stride, int lane, uint32_t tag,
+                              int* err) {
   uint32_t excl = 0;
   for (int j = tile - 1; j >= 0; j -= kLookAhead) {
     const int k = min(kLookAhead, j + 1);
@@ -115,7 +123,7 @@ __device__ uint32_t look_back(const unsigned long long* status, int tile, int st
       const unsigned long long start = lb_ready(w[i], tag) ? 0 : global_ns();
       while (!lb_ready(w[i], tag)) {
         if (wait_over(spins, start)) {
-          atomicExch(&g_error_flag, 1);
+          set_error(err);
           return excl;
         }
         __nanosleep(32);  // a polling warp yields its issue slots to the SM's other warps
@@ -134,7 +142,7 @@ __device__ uint32_t look_back(const unsigned long long* status, int tile, int st
 // inclusive prefix is summed; a round that meets an unpublished word first
 // consumes the ready lanes before it and polls again (bounded).  All 32 lanes
 // call it and get the same result.
-__device__ uint32_t warp_look_back(const unsigned long long* status, int tile, uint32_t tag) {
+__device__ uint32_t warp_look_back(const unsigned long long* status, int tile, uint32_t tag, int* err) {
   const int lane = threadIdx.x & 31;
   uint32_t excl = 0;
   int j = tile - 1;
@@ -159,7 +167,7 @@ __device__ uint32_t warp_look_back(const unsigned long long* status, int tile, u
     if (take == 0) {  // the nearest unpublished word: poll it
       if (start == 0) start = global_ns();
       if (wait_over(spins, start)) {
-        if (lane == 0) atomicExch(&g_error_flag, 1);
+        if (lane == 0) set_error(err);
         return excl;
       }
     } else {
@@ -170,67 +178,116 @@ __device__ uint32_t warp_look_back(const unsigned long long* status, int tile, u
   return excl;
 }
 
-// Called by one warp: turns the per-warp counts s_warp[0..kWarps) into
-// exclusive offsets (s_warp[kWarps] = the tile's total), publishes the tile's
-// aggregate, looks back, publishes the inclusive prefix and returns the
-// tile's exclusive prefix.
-__device__ uint32_t tile_prefix(uint32_t* s_warp, unsigned long long* status, int tile, uint32_t tag) {
+// Called by one warp: turns the per-warp counts s_warp[0..kW) into exclusive
+// offsets (s_warp[kW] = the tile's total), publishes the tile's aggregate,
+// looks back, publishes the inclusive prefix and returns the tile's exclusive
+// prefix.
+template <int kW>
+__device__ uint32_t tile_prefix(uint32_t* s_warp, unsigned long long* status, int tile, uint32_t tag, int* err) {
   const int lane = threadIdx.x & 31;
-  const uint32_t c = lane < kWarps ? s_warp[lane] : 0u;
+  const uint32_t c = lane < kW ? s_warp[lane] : 0u;
   uint32_t incl = c;
   for (int off = 1; off < 32; off <<= 1) {
     const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
     if (lane >= off) incl += t;
   }
   const uint32_t run = __shfl_sync(0xffffffffu, incl, 31);
-  __syncwarp();
-  if (lane < kWarps) s_warp[lane] = incl - c;
-  if (lane == 0) s_warp[kWarps] = run;
   unsigned long long* st = status + tile;
-  if (tile == 0) {
-    if (lane == 0) st_volatile64(st, lb_word(tag, 2u, run));
-    return 0;
-  }
-  if (lane == 0) st_volatile64(st, lb_word(tag, 1u, run));
-  const uint32_t excl = warp_look_back(status, tile, tag);
+  if (lane == 0) st_volatile64(st, lb_word(tag, tile == 0 ? 2u : 1u, run));
+  __syncwarp();
+  if (lane < kW) s_warp[lane] = incl - c;
+  if (lane == 0) s_warp[kW] = run;
+  if (tile == 0) return 0;
+  const uint32_t excl = warp_look_back(status, tile, tag, err);
   if (lane == 0) st_volatile64(st, lb_word(tag, 2u, excl + run));
   return excl;
 }
 
+// Control words of a call, zeroed by one memset before it.
+struct Control {
+  uint32_t hist[kPasses * kBuckets];  // digit counts
+  uint32_t range_counts[kBuckets];    // keys per range bucket
+  uint32_t range[2];                  // max of ~key (so the minimum), max key
+  int keys;                           // compacted keys
+  int no_hit;                         // 1: some input word was NO_HIT
+  int done[3];                        // CTAs finished: compaction, range histogram, digit histogram
+  int barrier[3];                     // CTAs at the barriers of the bitmap's cooperative kernels
+  int tiles[kPasses];                 // tile counters: digit passes
+  int unique_tiles, bucket_items;
+};
+// Words one kernel of a call leaves for the next; not cleared.
+struct Plan {
+  int path;               // feedback unique: kPath...
+  uint32_t bitmap_words, range_shift;
+  int skip[kPasses];      // digit pass not needed
+  int unstable[kPasses];  // first pass: equal digits may leave in any order
+  int src[kPasses], dst[kPasses], last;  // buffers of the passes, and where the keys end up
+  uint32_t offsets[kPasses * kBuckets];  // global start of each digit
+  uint32_t range_offsets[kBuckets];
+  uint32_t cursors[kBuckets * kCursorStride];
+  uint32_t segment_bits[1 << (kMaxSpanLog2 - 15)];  // set bits per 1024 words of the bitmap
+};
+constexpr int kPathEmpty = 0, kPathDirect = 1, kPathPartition = 2, kPathRadix = 3;
+
 struct SortScratchLayout {
   uint32_t* keys_a;
   uint32_t* keys_b;
-  uint32_t* hist;                 // kPasses * kBuckets counts, then turned into offsets
-  unsigned long long* status;     // tiles * kBuckets tagged look-back words
-  int* tile_counter;              // kPasses + 2 counters
-  int* count;                     // [0] compacted keys, [1] unique count
-  uint32_t* cursors;              // kBuckets range-partition cursors, kCursorStride words apart
-  uint32_t* range;                // [0] max of ~key, [1] max key, [2] path (kBitmapPath), [3] bitmap words,
-                                  // [4] range-bucket shift
-  size_t bitmap_bits;             // unique-by-bitmap capacity: the bitmap lives in keys_b
+  uint32_t* bitmap;
+  Control* control;
+  Plan* plan;
+  size_t bitmap_bits;  // unique-by-bitmap capacity
   size_t bytes;
 };
 
 SortScratchLayout layout(void* base, int n) {
-  const size_t tiles = ((size_t)n + kTile - 1) / kTile + 1;
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
   SortScratchLayout l{};
   size_t off = 0;
   uint8_t* b = static_cast<uint8_t*>(base);
+  l.control = reinterpret_cast<Control*>(b + off); off += up(sizeof(Control));
+  l.plan = reinterpret_cast<Plan*>(b + off); off += up(sizeof(Plan));
   l.keys_a = reinterpret_cast<uint32_t*>(b + off); off += up((size_t)n * 4 + 16);
   l.keys_b = reinterpret_cast<uint32_t*>(b + off); off += up((size_t)n * 4 + 16);
-  l.hist = reinterpret_cast<uint32_t*>(b + off); off += up(kHistRows * kBuckets * 4);
-  l.status = reinterpret_cast<unsigned long long*>(b + off); off += up(tiles * kBuckets * 8);
-  l.tile_counter = reinterpret_cast<int*>(b + off); off += up(16 * 4);
-  l.count = reinterpret_cast<int*>(b + off); off += up(4 * 4);
-  l.range = reinterpret_cast<uint32_t*>(b + off); off += up(8 * 4);
-  l.cursors = reinterpret_cast<uint32_t*>(b + off); off += up(kBuckets * kCursorStride * 4);
-  l.bitmap_bits = (((size_t)n * 4 + 16) / 16) * 16 * 8;  // whole 16-byte units of keys_b
+  l.bitmap_bits = std::min<size_t>((((size_t)n * 4 + 16) / 16) * 16 * 8, (size_t)1 << kMaxSpanLog2);
+  // the direct path leaves keys_b free; larger inputs may be partitioned into it
+  if (n <= kDirectWords) l.bitmap = l.keys_b;
+  else l.bitmap = reinterpret_cast<uint32_t*>(b + off), off += up(l.bitmap_bits / 8);
   l.bytes = off;
   return l;
 }
 
-// ---- compaction + histograms -------------------------------------------------
+// Exclusive scan of 256 values, 8 per lane, by one warp: row[i] becomes the sum
+// of the values before it; returns the total.
+__device__ __forceinline__ uint32_t warp_scan_256(const uint32_t* in, uint32_t* out) {
+  const int lane = threadIdx.x & 31;
+  uint32_t v[8], sum = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) { v[k] = in[lane * 8 + k]; sum += v[k]; }
+  uint32_t incl = sum;
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += t;
+  }
+  uint32_t run = incl - sum;
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 8; ++k) { out[lane * 8 + k] = run; run += v[k]; }
+  return __shfl_sync(0xffffffffu, incl, 31);
+}
+
+// True in every thread of the CTA that finishes last of `ctas` (no CTA waits);
+// what the other CTAs wrote before their call is visible to it.
+__device__ __forceinline__ bool last_cta(int* done, int ctas) {
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1) == ctas - 1;
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last;
+}
+
+// ---- compaction ---------------------------------------------------------------
 // NodeToBlock's division of a node index (0 <= x < 2^31) by nodes_in_block d
 // without a hardware divide: q = floor(x * M / 2^64) with M = ceil(2^64 / d).
 // For x < 2^31 and d < 2^32 the product's excess x * (M - 2^64/d) / 2^64 is
@@ -254,17 +311,26 @@ __device__ __forceinline__ uint32_t divide(uint32_t x, Divider v) {
 // (scalar loads otherwise, and for the last, partial tile).  The next tile's
 // loads are issued before the current tile is processed, so memory latency
 // overlaps the work.  The per-word loop only drops NO_HIT words: each warp
-// appends the words it keeps to its own 1024-word region of shared memory.
-// NodeToBlock, the key mapping and the four 8-bit digit histograms run when
-// the regions are flushed, on the kept words with every lane busy (at 10%
-// kept words, doing them per word cost three quarters of the instructions of
-// an issue-bound kernel).  The CTA flushes, claiming its output range with
-// one atomicAdd on `claim`, only when a region could not take another tile or
-// after its last tile; the regions go out coalesced.  Input words are read
-// once, with evict-first loads, so they do not push the compacted keys (read
-// again by the digit passes) out of L2.  Keys leave a warp in any order: only
-// sorted keys leave the sort.
-constexpr int kRegion = 1024;  // keys per warp region; a tile adds at most 512
+// appends the words it keeps to its own region of shared memory.
+// NodeToBlock, the key mapping and the filter run when the regions are
+// flushed, on the kept words with every lane busy (at 10% kept words, doing
+// them per word cost three quarters of the instructions of an issue-bound
+// kernel).  The filter is a direct-mapped table of keys the CTA has kept
+// before: a key found there is dropped.  Feedback repeats its frequent keys
+// (neighbouring pixels hit the same blocks), and every later kernel reads
+// what is kept here.  Warps race on the table without order; the worst that
+// does is keep a repeat.  The CTA flushes, claiming its output range with one
+// atomicAdd, only when a region could not take another tile or after its last
+// tile; the regions go out coalesced.  (Regions of 640 words and 4096 filter
+// entries leave 5 CTAs per SM; 1024 and 2048 took 403 us for the unique of
+// 2^28 words where these take 364.)  Input words are read once, with
+// evict-first loads, so they do not push the compacted keys out of L2.  Keys
+// leave in any order.  The CTAs also clear the bitmap (they are done before
+// the first kernel that sets bits), and the last one chooses the path.
+constexpr int kRegion = 640;  // words per warp region; a tile adds at most 512
+constexpr int kFilterLog2 = 12;
+constexpr int kFlush = 2;  // words in flight per lane of a flush
+constexpr uint32_t kNoKey = 0xffffffffu;  // NO_HIT's key: never kept
 
 template <bool kVec>
 __device__ __forceinline__ void load_words(int32_t (&w)[kItems], const int32_t* words, uint32_t n, uint32_t first) {
@@ -286,39 +352,47 @@ __device__ __forceinline__ void load_words(int32_t (&w)[kItems], const int32_t* 
   }
 }
 
-template <bool kCompact, bool kVec>
+template <bool kVec>
 __global__ void __launch_bounds__(kThreads) compact_kernel(const int32_t* words, int n_words, int nib, Divider div,
-                                                           uint32_t* keys, int* claim, uint32_t* hist,
-                                                           uint32_t* range) {
-  __shared__ uint32_t sh[kPasses][kBuckets];
+                                                           uint32_t* keys, Control* ctl, Plan* plan, uint4* bitmap,
+                                                           uint32_t bitmap_units, unsigned long long bitmap_bits,
+                                                           int32_t* out, int* result) {
   __shared__ uint32_t s_range[2];  // max of ~key (so the minimum), max key
   __shared__ uint32_t s_keys[kWarps * kRegion];
+  __shared__ uint32_t s_filter[1 << kFilterLog2];
   __shared__ uint32_t s_fill[2][kWarps];  // by tile parity: a warp may write the next tile's entry early
   __shared__ uint32_t s_base;
-  for (int i = threadIdx.x; i < kPasses * kBuckets; i += kThreads) (&sh[0][0])[i] = 0;
-  if (threadIdx.x < 2) s_range[threadIdx.x] = 0;
-  uint32_t not_min = 0, max_key = 0;
   const uint32_t n = (uint32_t)n_words;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1;
   const uint32_t mine = warp * (kItems * 32) + lane * 4;  // offset of the thread's first word in a tile
   uint32_t* region = s_keys + warp * kRegion;
+  volatile uint32_t* filter = s_filter;
   const uint32_t stride = gridDim.x * kTile;  // tiles of n < 2^31 words: base + stride stays below 2^32
   int32_t cur[kItems], nxt[kItems];
   uint32_t base = blockIdx.x * kTile;
   load_words<kVec>(cur, words, n, base + mine);
-  uint32_t fill = 0;  // keys in this warp's region
-  __syncthreads();    // histograms zeroed
+  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < bitmap_units; i += gridDim.x * kThreads)
+    bitmap[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = threadIdx.x; i < (1 << kFilterLog2); i += kThreads) s_filter[i] = kNoKey;
+  if (threadIdx.x < 2) s_range[threadIdx.x] = 0;
+  uint32_t not_min = 0, max_key = 0;
+  uint32_t fill = 0;  // words in this warp's region
+  bool dropped = false;
   for (int parity = 0; base < n; base += stride, parity ^= 1) {
     const uint32_t next = base + stride;
     load_words<kVec>(nxt, words, n, next + mine);
+    const uint32_t before = fill;
 #pragma unroll
     for (int q = 0; q < kItems; ++q) {
-      const bool keep = kCompact ? cur[q] != kNoHit  // words past the end were loaded as NO_HIT
-                                 : base + mine + (q >> 2) * 128 + (q & 3) < n;
+      const bool keep = cur[q] != kNoHit;  // words past the end were loaded as NO_HIT
       const unsigned mask = __ballot_sync(0xffffffffu, keep);
       if (keep) region[fill + __popc(mask & lt)] = (uint32_t)cur[q];
       fill += __popc(mask);
+    }
+    {
+      const uint32_t first = base + warp * (kItems * 32);
+      dropped = dropped || (first < n && fill - before < min(n - first, (uint32_t)kItems * 32));
     }
 #pragma unroll
     for (int q = 0; q < kItems; ++q) cur[q] = nxt[q];
@@ -328,91 +402,190 @@ __global__ void __launch_bounds__(kThreads) compact_kernel(const int32_t* words,
 #pragma unroll
     for (int k = 0; k < kWarps; ++k) flush = flush || s_fill[parity][k] > kRegion - kItems * 32;
     if (!flush) continue;
+    // words to keys, in place (a round writes at or below what it has read)
+    uint32_t kept = 0;
+    for (uint32_t j0 = 0; j0 < fill; j0 += 32 * kFlush) {
+      uint32_t key[kFlush];
+      bool keep[kFlush];
+#pragma unroll
+      for (int r = 0; r < kFlush; ++r) {
+        const uint32_t j = j0 + r * 32 + lane;
+        keep[r] = j < fill;
+        int32_t v = keep[r] ? (int32_t)region[j] : 0;
+        if (v > 0 && nib > 0) v = (int32_t)(((divide((uint32_t)((v >> 1) - 1), div) + 1) << 1) | (v & 1));
+        key[r] = (uint32_t)v ^ 0x80000000u;
+      }
+#pragma unroll
+      for (int r = 0; r < kFlush; ++r) {
+        const uint32_t h = (key[r] * 0x9e3779b1u) >> (32 - kFilterLog2);
+        if (keep[r]) {
+          if (filter[h] == key[r]) keep[r] = false;
+          else filter[h] = key[r];
+        }
+      }
+      __syncwarp();  // the round's words are read before keys overwrite them
+#pragma unroll
+      for (int r = 0; r < kFlush; ++r) {
+        const unsigned mask = __ballot_sync(0xffffffffu, keep[r]);
+        if (keep[r]) {
+          region[kept + __popc(mask & lt)] = key[r];
+          not_min = max(not_min, ~key[r]);
+          max_key = max(max_key, key[r]);
+        }
+        kept += __popc(mask);
+      }
+      __syncwarp();
+    }
+    __syncthreads();  // every warp has read this tile's fills
+    if (lane == 0) s_fill[parity][warp] = kept;
+    __syncthreads();
     if (threadIdx.x == 0) {
       uint32_t total = 0;
       for (int k = 0; k < kWarps; ++k) total += s_fill[parity][k];
-      s_base = (uint32_t)atomicAdd(claim, (int)total);
+      s_base = total ? (uint32_t)atomicAdd(&ctl->keys, (int)total) : 0u;
     }
     __syncthreads();
-    uint32_t out = s_base;
-    for (int k = 0; k < warp; ++k) out += s_fill[parity][k];
-    for (uint32_t j = lane; j < fill; j += 32) {
-      int32_t v = (int32_t)region[j];
-      if (kCompact && v > 0 && nib > 0) v = (int32_t)(((divide((uint32_t)((v >> 1) - 1), div) + 1) << 1) | (v & 1));
-      const uint32_t key = (uint32_t)v ^ 0x80000000u;
-#pragma unroll
-      for (int p = 0; p < kPasses; ++p) atomicAdd(&sh[p][(key >> (8 * p)) & 255u], 1u);
-      not_min = max(not_min, ~key);
-      max_key = max(max_key, key);
-      keys[out + j] = key;
-    }
+    uint32_t at = s_base;
+    for (int k = 0; k < warp; ++k) at += s_fill[parity][k];
+    for (uint32_t j = lane; j < kept; j += 32) keys[at + j] = region[j];
     fill = 0;
     __syncthreads();  // s_base is reused by the next flush
   }
-  if (range) {
-    not_min = __reduce_max_sync(0xffffffffu, not_min);
-    max_key = __reduce_max_sync(0xffffffffu, max_key);
-    if (lane == 0) {
-      atomicMax(&s_range[0], not_min);
-      atomicMax(&s_range[1], max_key);
-    }
+  not_min = __reduce_max_sync(0xffffffffu, not_min);
+  max_key = __reduce_max_sync(0xffffffffu, max_key);
+  __syncthreads();  // s_range zeroed
+  if (lane == 0) {
+    atomicMax(&s_range[0], not_min);
+    atomicMax(&s_range[1], max_key);
+    if (dropped) ctl->no_hit = 1;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < kPasses * kBuckets; i += kThreads) {
-    const uint32_t v = (&sh[0][0])[i];
-    if (v) atomicAdd(hist + i, v);
+  if (threadIdx.x < 2 && s_range[threadIdx.x]) atomicMax(&ctl->range[threadIdx.x], s_range[threadIdx.x]);
+  if (!last_cta(&ctl->done[0], gridDim.x) || threadIdx.x != 0) return;
+  // the path: a bitmap when it fits, straight or range by range
+  const volatile Control* c = ctl;
+  const int m = c->keys;
+  const uint32_t lo = ~c->range[0], hi = c->range[1];
+  const unsigned long long span = (unsigned long long)hi - (unsigned long long)lo + 1ull;
+  const bool direct = n_words <= kDirectWords || m <= kDirectKeys || span <= kDirectSliceWords * 32ull;
+  const int path = m == 0 ? kPathEmpty : span > bitmap_bits ? kPathRadix : direct ? kPathDirect : kPathPartition;
+  plan->path = path;
+  plan->bitmap_words = (uint32_t)((span + 31) / 32);
+  const int bits = span > 1 ? 64 - __clzll((long long)(span - 1)) : 0;  // bits of the largest key - min
+  plan->range_shift = bits > 8 ? (uint32_t)(bits - 8) : 0u;
+  if (path == kPathEmpty) {
+    if (c->no_hit) out[0] = kNoHit;
+    result[0] = c->no_hit ? 1 : 0;
   }
-  if (range && threadIdx.x < 2 && s_range[threadIdx.x]) atomicMax(range + threadIdx.x, s_range[threadIdx.x]);
+  result[1] = path;
 }
 
 // Compaction launch: 16-byte loads when `words` allows them.
-template <bool kCompact>
-cudaError_t launch_compact(int grid, const int32_t* words, int n, int nib, uint32_t* keys, int* claim,
-                           uint32_t* hist, uint32_t* range, cudaStream_t s) {
+cudaError_t launch_compact(int grid, const int32_t* words, int n, int nib, const SortScratchLayout& l, int32_t* out,
+                           int* result, cudaStream_t s) {
   const Divider div = make_divider((uint32_t)nib);
+  uint4* bitmap = reinterpret_cast<uint4*>(l.bitmap);
+  const uint32_t units = (uint32_t)(l.bitmap_bits / 128);
   if ((reinterpret_cast<uintptr_t>(words) & 15) == 0)
-    compact_kernel<kCompact, true><<<grid, kThreads, 0, s>>>(words, n, nib, div, keys, claim, hist, range);
+    compact_kernel<true><<<grid, kThreads, 0, s>>>(words, n, nib, div, l.keys_a, l.control, l.plan, bitmap, units,
+                                                  l.bitmap_bits, out, result);
   else
-    compact_kernel<kCompact, false><<<grid, kThreads, 0, s>>>(words, n, nib, div, keys, claim, hist, range);
+    compact_kernel<false><<<grid, kThreads, 0, s>>>(words, n, nib, div, l.keys_a, l.control, l.plan, bitmap, units,
+                                                   l.bitmap_bits, out, result);
   return cudaGetLastError();
 }
 
-// Unique-by-bitmap: when the kept keys span at most `bitmap_bits` values (and
-// at most 2^26), a bitmap over [min, max] read in order is the sorted unique
-// set, and the radix passes are skipped.  range[2] holds the choice.
-constexpr uint32_t kBitmapPath = 1;
-
-// hist counts -> exclusive offsets (one CTA of 256 threads); opens a new epoch
-// for the look-back words of this call.  With `range`, also chooses between
-// the radix passes and the bitmap.
-__global__ void hist_offsets_kernel(uint32_t* hist, const int* count, uint32_t* range,
-                                    unsigned long long bitmap_bits) {
-  if (range && threadIdx.x == 0) {
-    const int m = *count;
-    const unsigned long long span = (unsigned long long)range[1] - (unsigned long long)(~range[0]) + 1ull;
-    const bool bitmap = m > 0 && span <= bitmap_bits && span <= (1ull << kMaxSpanLog2);
-    range[2] = bitmap ? kBitmapPath : 0u;
-    range[3] = bitmap ? (uint32_t)((span + 31) / 32) : 0u;
-    const int bits = span > 1 ? 64 - __clzll((long long)(span - 1)) : 0;  // bits of the largest key - min
-    range[4] = bits > 8 ? (uint32_t)(bits - 8) : 0u;
-  }
-  // warp p scans digit row p: 8 counts per lane, then a warp scan
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < kPasses) {
-    uint32_t* row = hist + warp * kBuckets;
-    uint32_t v[8], sum = 0;
+// ---- digit histograms ----------------------------------------------------------
+// All four digits' counts in one read of the keys.  Random digits collide in
+// the banks of a 256-entry table (3 to 4 wavefronts per atomic: the counting
+// took 139 us on 2^26 keys with a copy of the keys beside it); here each lane
+// of a warp counts in its own bank, 256 x 32 counters per digit, so an atomic
+// is one wavefront whatever the digits are.  One CTA of 1024 threads per SM
+// holds the 128 KB of counters.  The last CTA turns the counts into offsets
+// and lays out the passes: a digit that is the same in every key needs none.
+constexpr int kHistThreads = 1024;
+constexpr int kHistSmemBytes = kPasses * kBuckets * 32 * 4;
+template <bool kVec>
+__global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint32_t* keys, int n, const int* count,
+                                                                    uint32_t flip, bool in_place, Control* ctl,
+                                                                    Plan* plan) {
+  extern __shared__ __align__(128) uint32_t s_hist[];
+  __shared__ uint32_t s_max[kPasses];
+  for (int i = threadIdx.x; i < kPasses * kBuckets * 32; i += kHistThreads) s_hist[i] = 0;
+  const uint32_t m = count ? (uint32_t)*count : (uint32_t)n;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  uint32_t* col = s_hist + lane;
+  auto add = [&](uint32_t k) {
+    k ^= flip;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) { v[k] = row[lane * 8 + k]; sum += v[k]; }
-    uint32_t incl = sum;
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += t;
+    for (int p = 0; p < kPasses; ++p) atomicAdd(col + (p * kBuckets + ((k >> (8 * p)) & 255u)) * 32, 1u);
+  };
+  if (kVec) {  // 16-byte units, four in flight per thread
+    const uint32_t units = m / 4, step = gridDim.x * kHistThreads;
+    const uint4* k4 = reinterpret_cast<const uint4*>(keys);
+    uint32_t i = blockIdx.x * kHistThreads + threadIdx.x;
+    for (; i + 3 * step < units; i += 4 * step) {  // below 2^28 + 4 * step
+      uint4 v[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) v[r] = __ldg(k4 + i + r * step);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) add(v[r].x), add(v[r].y), add(v[r].z), add(v[r].w);
     }
-    uint32_t run = incl - sum;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { row[lane * 8 + k] = run; run += v[k]; }
+    for (; i < units; i += step) {
+      const uint4 v = __ldg(k4 + i);
+      add(v.x), add(v.y), add(v.z), add(v.w);
+    }
+    if (blockIdx.x == 0 && threadIdx.x < (m & 3u)) add(keys[units * 4 + threadIdx.x]);
+  } else {
+    for (uint32_t i = blockIdx.x * kHistThreads + threadIdx.x; i < m; i += gridDim.x * kHistThreads)
+      add(__ldg(keys + i));
   }
-  if (threadIdx.x == 0) g_epoch = (g_epoch + 1) & ((1u << 27) - 1);
+  __syncthreads();
+  {  // thread t: digit value t of the 4 x 256, its 32 columns from its own bank on
+    uint32_t sum = 0;
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) sum += s_hist[threadIdx.x * 32 + ((lane + k) & 31)];
+    if (sum) atomicAdd(&ctl->hist[threadIdx.x], sum);
+  }
+  if (!last_cta(&ctl->done[2], gridDim.x)) return;
+  uint32_t* counts = s_hist;  // reused
+  __syncthreads();
+  counts[threadIdx.x] = *(volatile uint32_t*)&ctl->hist[threadIdx.x];
+  if (threadIdx.x < kPasses) s_max[threadIdx.x] = 0;
+  __syncthreads();
+  atomicMax(&s_max[threadIdx.x >> 8], counts[threadIdx.x]);
+  __syncthreads();
+  if (threadIdx.x < 32 * kPasses) {
+    const int p = threadIdx.x >> 5;
+    warp_scan_256(counts + p * kBuckets, plan->offsets + p * kBuckets);
+  }
+  if (threadIdx.x == 0) {
+    int active = 0;
+    bool skip[kPasses];
+    for (int p = 0; p < kPasses; ++p) active += !(skip[p] = s_max[p] == m);
+    // in place: buffer 0 is both where the keys come from and where they go,
+    // so one pass alone has nowhere to go and another one runs with it
+    if (in_place && active == 1) {
+      skip[skip[0] ? 0 : 1] = false;
+      active = 2;
+    }
+    int at = 0, j = 0;
+    for (int p = 0; p < kPasses; ++p) {
+      plan->skip[p] = skip[p];
+      if (skip[p]) continue;
+      plan->src[p] = at;
+      // in place: 0 -> 1 -> 2 -> 1 -> 0 for four passes; else 0 and 1 in turn
+      at = in_place ? (j == active - 1 ? 0 : (j & 1) ? 2 : 1) : 1 - at;
+      plan->dst[p] = at;
+      // the first pass may leave equal digits in any order (no earlier pass
+      // has ordered them): worth it where no digit is so frequent that its
+      // count is contended
+      plan->unstable[p] = j == 0 && s_max[p] <= m / 16;
+      ++j;
+    }
+    plan->last = at;
+  }
 }
 
 // ---- bulk async copies into shared memory ------------------------------------
@@ -439,13 +612,13 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, uint32_t 
 }
 // Waits for the phase of `bar` with parity `parity`; false (error flag set)
 // when the wait runs out.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t parity, int* err) {
   if (mbar_try_wait(bar, parity)) return true;
   long long spins = 0;
   const unsigned long long start = global_ns();
   while (!mbar_try_wait(bar, parity)) {
     if (wait_over(spins, start)) {
-      atomicExch(&g_error_flag, 1);
+      set_error(err);
       return false;
     }
   }
@@ -458,29 +631,33 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t pari
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, unsigned long long* bar) {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+  if (bytes == 0) return;  // the phase is complete already
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    smem_addr(dst)),
                "l"(src), "r"(bytes), "r"(smem_addr(bar))
                : "memory");
 }
 
-// ---- one stable counting pass over 8 bits ------------------------------------
+// ---- one counting pass over 8 bits ---------------------------------------------
 // Persistent CTAs of 512 threads claim tiles of 8192 keys in order from
-// tile_counter until the keys run out (the count is read on the device: for
-// feedback unique only the compaction knows it).  A CTA claims its next tile
-// when it starts the current one, and the next tile's keys come into the
-// other half of a double buffer by one bulk async copy while the current tile
-// is ranked, looked back and written out.  (A next tile is always above its
-// CTA's current one, so the lowest unfinished tile is always some CTA's
+// the pass's tile counter until the keys run out (the count is read on the
+// device: for feedback unique only the compaction knows it).  A CTA claims its
+// next tile when it starts the current one, and the next tile's keys come into
+// the other half of a double buffer by one bulk async copy while the current
+// tile is ranked, looked back and written out.  (A next tile is always above
+// its CTA's current one, so the lowest unfinished tile is always some CTA's
 // current tile and every look-back ends.)  Per tile:
-// - ranking (stable), a warp's 512 keys in 16 rounds of 32: the lanes of a
+// - ranking, stable: a warp's 512 keys in 16 rounds of 32: the lanes of a
 //   round holding the same digit find one another through a per-warp table of
 //   peer masks in shared memory (each lane ORs its bit into its digit's word;
 //   one shared atomic instead of eight ballots and the selects between them,
 //   which had made the pass issue-bound at 4.9 warp instructions per key); the
 //   group's first lane adds the group to the warp's count of that digit with
 //   one atomic, clears the mask word and shares the old count; ranks follow
-//   lane order inside the group, and rounds apply in order;
+//   lane order inside the group, and rounds apply in order.  The pass is bound
+//   by the shared-memory pipe, and these accesses by random digits are most of
+//   its wavefronts, so the first pass, which has no earlier order to keep,
+//   takes its ranks from one atomic per key on the CTA's counts instead;
 // - the per-digit counts over warps become offsets; the tile's count per digit
 //   is published at once (the look-back's aggregate); the 256 counts are
 //   scanned into the tile-local start of each digit run, which is added into
@@ -492,7 +669,7 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 // - each digit run goes out contiguously.
 // 8192-key tiles halve the look-back's walk per key twice over 4096-key ones:
 // half the tiles, and half as many tiles in flight behind a tile's
-// predecessors.  With `range` (feedback unique), skipped on the bitmap path.
+// predecessors.
 constexpr int kDigitThreads = 512;
 constexpr int kDigitWarps = kDigitThreads / 32;
 constexpr int kDigitTile = kDigitThreads * kItems;  // 8192 keys
@@ -500,23 +677,33 @@ constexpr int kDigitTile = kDigitThreads * kItems;  // 8192 keys
 // starts and offsets, 8 warp totals, two mbarriers and the next tile's index
 constexpr int kDigitSmemBytes = (2 * kDigitTile + 2 * kDigitWarps * kBuckets + 2 * kBuckets + 8) * 4 + 32;
 
-// Bytes copied for tile t of m keys: the partial last tile is rounded up to 16
-// bytes (the key buffers carry 16 bytes of padding).
+// Bytes copied for tile t of m keys: whole 16-byte units; the up to three keys
+// after them are read straight from memory when they are ranked.
 __device__ __forceinline__ uint32_t digit_tile_bytes(int t, int m) {
   const int valid = min(kDigitTile, m - t * kDigitTile);
-  return (uint32_t)((valid * 4 + 15) & ~15);
+  return (uint32_t)(valid / 4 * 16);
 }
 
-template <bool kFull>
-__device__ __forceinline__ void rank_tile(const uint32_t* s_tile_keys, uint32_t (&keys)[kItems],
-                                          uint32_t (&ranks)[kItems / 2], uint32_t* s_count, uint32_t* s_peers,
-                                          int shift, int valid, int w0, int lane) {
+// Key `li` of a partial tile of `valid` keys: in shared memory, or past the last
+// whole 16-byte unit in global memory.
+__device__ __forceinline__ uint32_t tail_key(const uint32_t* s_tile_keys, const uint32_t* tile_keys, int li,
+                                             int valid) {
+  return li < (valid & ~3) ? s_tile_keys[li] : li < valid ? tile_keys[li] : 0u;
+}
+
+// Ranks a warp's kRounds * 32 keys (positions w0 + r * 32 + lane of `src`, or
+// of the partial tile `tail`) among the warp's keys of the same digit, stable;
+// two 16-bit ranks per word.
+template <bool kFull, int kRounds>
+__device__ __forceinline__ void rank_keys(const uint32_t* src, const uint32_t* tail, uint32_t (&keys)[kRounds],
+                                          uint32_t (&ranks)[(kRounds + 1) / 2], uint32_t* s_count, uint32_t* s_peers,
+                                          int shift, uint32_t flip, int valid, int w0, int lane) {
 #pragma unroll
-  for (int r = 0; r < kItems; ++r) {
+  for (int r = 0; r < kRounds; ++r) {
     const int li = w0 + r * 32 + lane;
     const bool ok = kFull || li < valid;
-    keys[r] = s_tile_keys[li];  // past `valid` a stale word, not used
-    const uint32_t d = (keys[r] >> shift) & 255u;
+    keys[r] = kFull ? src[li] : tail_key(src, tail, li, valid);
+    const uint32_t d = ((keys[r] >> shift) & 255u) ^ flip;
     if (ok) atomicOr(&s_peers[d], 1u << lane);
     __syncwarp();
     const unsigned peers = ok ? s_peers[d] : (1u << lane);
@@ -530,14 +717,21 @@ __device__ __forceinline__ void rank_tile(const uint32_t* s_tile_keys, uint32_t 
     before = __shfl_sync(0xffffffffu, before, leader);
     __syncwarp();  // the cleared mask is in place before the next round's ORs
     const uint32_t rank = before + __popc(peers & ((1u << lane) - 1));
-    ranks[r / 2] = (r & 1) ? ranks[r / 2] | (rank << 16) : rank;  // two 16-bit ranks (< 512) per word
+    ranks[r / 2] = (r & 1) ? ranks[r / 2] | (rank << 16) : rank;
   }
 }
 
-__global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const uint32_t* in, uint32_t* out, const int* count,
-                                                              int shift, const uint32_t* digit_base,
-                                                              unsigned long long* status, int* tile_counter, int pass,
-                                                              bool last, int32_t* final_out, const uint32_t* range) {
+// Buffers of the passes by the plan's numbers: source 0 may be another memory
+// than destination 0 (an unaligned array is sorted from a copy).
+struct DigitBuffers {
+  const uint32_t* in0;
+  uint32_t *out0, *b1, *b2;
+};
+
+__global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const DigitBuffers bufs, int n, const int* count,
+                                                              int pass, uint32_t flip, const Plan* plan,
+                                                              unsigned long long* status, int* tile_counter,
+                                                              uint32_t tag, int* err) {
   extern __shared__ __align__(128) uint32_t smem[];
   uint32_t* s_warp = smem + 2 * kDigitTile;         // [warp][digit] counts, then offsets
   uint32_t* s_peers = s_warp + kDigitWarps * kBuckets;  // [warp][digit] peer masks of a round
@@ -546,11 +740,18 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const uint32_t*
   uint32_t* s_wsum = s_off + kBuckets;                  // per digit warp: its digits' counts summed
   unsigned long long* s_bar = reinterpret_cast<unsigned long long*>(s_wsum + 8);
   int* s_next = reinterpret_cast<int*>(s_bar + 2);
-  if (range && range[2] == kBitmapPath) return;
-  const int m = *count;
-  const uint32_t tag = g_epoch * 8u + (uint32_t)pass;
+  if (plan->skip[pass]) return;
+  const int m = count ? *count : n;
+  const int shift = 8 * pass;
+  const bool unstable = plan->unstable[pass] != 0;
+  const int src = plan->src[pass], dst = plan->dst[pass];
+  const uint32_t* in = src == 0 ? bufs.in0 : src == 1 ? bufs.b1 : bufs.b2;
+  uint32_t* out = dst == 0 ? bufs.out0 : dst == 1 ? bufs.b1 : bufs.b2;
+  const uint32_t* digit_base = plan->offsets + pass * kBuckets;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w0 = warp * (kItems * 32);  // warp `warp` ranks keys [w0, w0 + 512) of a tile
+  const int rows = unstable ? 1 : kDigitWarps;  // rows of counts in use
+  uint32_t* s_mine = unstable ? s_warp : s_warp + warp * kBuckets;  // this warp's row
   for (int i = threadIdx.x; i < 2 * kDigitWarps * kBuckets; i += kDigitThreads) s_warp[i] = 0;
   if (threadIdx.x == 0) {
     mbar_init(&s_bar[0]);
@@ -568,20 +769,31 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const uint32_t*
   while ((long long)tile * kDigitTile < m) {
     const int valid = min(kDigitTile, m - tile * kDigitTile);
     uint32_t* s_tile_keys = smem + b * kDigitTile;
+    const uint32_t* tile_keys = in + (size_t)tile * kDigitTile;
     if (threadIdx.x == 0) *s_next = atomicAdd(tile_counter, 1);  // read after (A)
-    const bool landed = mbar_wait(&s_bar[b], (phases >> b) & 1u);
+    const bool landed = mbar_wait(&s_bar[b], (phases >> b) & 1u, err);
     uint32_t keys[kItems], ranks[kItems / 2];
-    if (valid == kDigitTile)
-      rank_tile<true>(s_tile_keys, keys, ranks, s_warp + warp * kBuckets, s_peers + warp * kBuckets, shift, valid, w0,
+    if (unstable) {
+#pragma unroll
+      for (int r = 0; r < kItems; ++r) {
+        const int li = w0 + r * 32 + lane;
+        keys[r] = valid == kDigitTile ? s_tile_keys[li] : tail_key(s_tile_keys, tile_keys, li, valid);
+        uint32_t rank = 0;
+        if (li < valid) rank = atomicAdd(&s_warp[((keys[r] >> shift) & 255u) ^ flip], 1u);
+        ranks[r / 2] = (r & 1) ? ranks[r / 2] | (rank << 16) : rank;
+      }
+    } else if (valid == kDigitTile) {
+      rank_keys<true>(s_tile_keys, nullptr, keys, ranks, s_mine, s_peers + warp * kBuckets, shift, flip, valid, w0,
                       lane);
-    else
-      rank_tile<false>(s_tile_keys, keys, ranks, s_warp + warp * kBuckets, s_peers + warp * kBuckets, shift, valid,
-                       w0, lane);
+    } else {
+      rank_keys<false>(s_tile_keys, tile_keys, keys, ranks, s_mine, s_peers + warp * kBuckets, shift, flip, valid, w0,
+                       lane);
+    }
     // (A) every read of this buffer is done.  A wait that ran out (error flag
     // set) ends the CTA, after its copy has landed (bounded), so that nothing
     // lands in shared memory after the CTA has left.
     if (!__syncthreads_and(landed)) {
-      if (threadIdx.x == 0) mbar_wait(&s_bar[b], (phases >> b) & 1u);
+      if (threadIdx.x == 0) mbar_wait(&s_bar[b], (phases >> b) & 1u, err);
       return;
     }
     phases ^= 1u << b;
@@ -596,11 +808,15 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const uint32_t*
     if (threadIdx.x < kBuckets) {
       const int d = threadIdx.x;
       uint32_t run = 0;
+      if (unstable) {
+        run = s_warp[d];
+      } else {
 #pragma unroll
-      for (int w = 0; w < kDigitWarps; ++w) {
-        const uint32_t v = s_warp[w * kBuckets + d];
-        s_warp[w * kBuckets + d] = run;
-        run += v;
+        for (int w = 0; w < kDigitWarps; ++w) {
+          const uint32_t v = s_warp[w * kBuckets + d];
+          s_warp[w * kBuckets + d] = run;
+          run += v;
+        }
       }
       tile_count = run;
       st_volatile64(status + (size_t)tile * kBuckets + d, lb_word(tag, tile == 0 ? 2u : 1u, run));
@@ -620,20 +836,22 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const uint32_t*
       uint32_t start = incl - tile_count;
       for (int k = 0; k < warp; ++k) start += s_wsum[k];
       s_start[d] = start;
+      if (unstable) {
+        s_warp[d] = start;
+      } else {
 #pragma unroll
-      for (int w = 0; w < kDigitWarps; ++w) s_warp[w * kBuckets + d] += start;
+        for (int w = 0; w < kDigitWarps; ++w) s_warp[w * kBuckets + d] += start;
+      }
     }
     __syncthreads();  // (C)
-    {  // stage keys in tile-local sorted order, in place: every read of the buffer finished before (A)
-      const uint32_t* s_pos = s_warp + warp * kBuckets;
+    // stage keys in tile-local sorted order, in place: every read of the buffer finished before (A)
 #pragma unroll
-      for (int r = 0; r < kItems; ++r) {
-        const int li = w0 + r * 32 + lane;
-        if (valid == kDigitTile || li < valid) {
-          const uint32_t k = keys[r];
-          const uint32_t rank = (r & 1) ? ranks[r / 2] >> 16 : ranks[r / 2] & 0xffffu;
-          s_tile_keys[s_pos[(k >> shift) & 255u] + rank] = k;
-        }
+    for (int r = 0; r < kItems; ++r) {
+      const int li = w0 + r * 32 + lane;
+      if (valid == kDigitTile || li < valid) {
+        const uint32_t k = keys[r];
+        const uint32_t rank = (r & 1) ? ranks[r / 2] >> 16 : ranks[r / 2] & 0xffffu;
+        s_tile_keys[s_mine[((k >> shift) & 255u) ^ flip] + rank] = k;
       }
     }
     // global position of each digit run: look-back over earlier tiles
@@ -641,7 +859,7 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const uint32_t*
       const int d = threadIdx.x;
       uint32_t excl = 0;
       if (tile != 0) {
-        excl = look_back(status, tile, kBuckets, d, tag);
+        excl = look_back(status, tile, kBuckets, d, tag, err);
         st_volatile64(status + (size_t)tile * kBuckets + d, lb_word(tag, 2u, excl + tile_count));
       }
       s_off[d] = digit_base[d] + excl - s_start[d];
@@ -649,24 +867,20 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const uint32_t*
     __syncthreads();  // (D)
     // contiguous write-out of each digit run; the counts are cleared for the
     // next tile on the way (the write-out does not read them)
-    for (int i = threadIdx.x; i < kDigitWarps * kBuckets; i += kDigitThreads) s_warp[i] = 0;
+    for (int i = threadIdx.x; i < rows * kBuckets; i += kDigitThreads) s_warp[i] = 0;
     if (valid == kDigitTile) {
 #pragma unroll
       for (int k = 0; k < kItems; ++k) {
         const int i = threadIdx.x + k * kDigitThreads;
         const uint32_t key = s_tile_keys[i];
-        const uint32_t pos = s_off[(key >> shift) & 255u] + (uint32_t)i;
-        if (pos >= (uint32_t)m) continue;  // only after a look-back gave up (error flag set)
-        if (last && final_out) final_out[pos] = (int32_t)(key ^ 0x80000000u);
-        else out[pos] = key;
+        const uint32_t pos = s_off[((key >> shift) & 255u) ^ flip] + (uint32_t)i;
+        if (pos < (uint32_t)m) out[pos] = key;  // past m only after a look-back gave up (error flag set)
       }
     } else {
       for (int i = threadIdx.x; i < valid; i += kDigitThreads) {
         const uint32_t key = s_tile_keys[i];
-        const uint32_t pos = s_off[(key >> shift) & 255u] + (uint32_t)i;
-        if (pos >= (uint32_t)m) continue;
-        if (last && final_out) final_out[pos] = (int32_t)(key ^ 0x80000000u);
-        else out[pos] = key;
+        const uint32_t pos = s_off[((key >> shift) & 255u) ^ flip] + (uint32_t)i;
+        if (pos < (uint32_t)m) out[pos] = key;
       }
     }
     __syncthreads();  // (E) the buffer, the run starts and offsets and the counts are reused
@@ -675,30 +889,191 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const uint32_t*
   }
 }
 
+// ---- one CTA --------------------------------------------------------------------
+// Up to kSmall keys stay in one CTA: a chain of launches costs 40 to 80 us
+// whatever the size (2013 keys: 45 us in 7 kernels, and the copy of the error
+// flag).  The keys are reduced by their minimum, so only the 8-bit digits that
+// their range needs are passed over (one for the reference test's 201
+// values), each with the digit pass's ranking; the keys live in shared memory
+// between passes.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmall = 8192;
+template <int kRounds>
+constexpr int small_smem_bytes() {
+  return (kSmallThreads * kRounds + 2 * kSmallWarps * kBuckets + kBuckets) * 4;
+}
+
+// Sorts the kSmallThreads * kRounds keys in s_keys by their low `bits` bits,
+// in place.  All threads of the CTA call it.
+template <int kRounds>
+__device__ void cta_sort(uint32_t* s_keys, int bits) {
+  uint32_t* s_warp = s_keys + kSmallThreads * kRounds;       // [warp][digit] counts, then offsets
+  uint32_t* s_peers = s_warp + kSmallWarps * kBuckets;       // [warp][digit] peer masks
+  uint32_t* s_count = s_peers + kSmallWarps * kBuckets;      // per digit
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < 2 * kSmallWarps * kBuckets; i += kSmallThreads) s_warp[i] = 0;
+  __syncthreads();
+  for (int shift = 0; shift < bits; shift += 8) {
+    uint32_t keys[kRounds], ranks[(kRounds + 1) / 2];
+    rank_keys<true>(s_keys, nullptr, keys, ranks, s_warp + warp * kBuckets, s_peers + warp * kBuckets, shift, 0u, 0,
+                    warp * kRounds * 32, lane);
+    __syncthreads();
+    // four threads per digit sum 8 warps each, then the digit's offsets
+    const int d = threadIdx.x >> 2, part = threadIdx.x & 3;
+    uint32_t* col = s_warp + part * (kSmallWarps / 4) * kBuckets + d;
+    uint32_t v[kSmallWarps / 4], sum = 0;
+#pragma unroll
+    for (int w = 0; w < kSmallWarps / 4; ++w) {
+      v[w] = col[w * kBuckets];
+      sum += v[w];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int off = 1; off < 4; off <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+      if (part >= off) incl += t;
+    }
+    if (part == 3) s_count[d] = incl;
+    __syncthreads();
+    if (warp == 0) warp_scan_256(s_count, s_count);
+    __syncthreads();
+    uint32_t run = s_count[d] + incl - sum;
+#pragma unroll
+    for (int w = 0; w < kSmallWarps / 4; ++w) {
+      col[w * kBuckets] = run;
+      run += v[w];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const uint32_t rank = (r & 1) ? ranks[r / 2] >> 16 : ranks[r / 2] & 0xffffu;
+      s_keys[s_warp[warp * kBuckets + ((keys[r] >> shift) & 255u)] + rank] = keys[r];
+    }
+    __syncthreads();
+    if (shift + 8 < bits) {
+      for (int i = threadIdx.x; i < kSmallWarps * kBuckets; i += kSmallThreads) s_warp[i] = 0;
+      __syncthreads();
+    }
+  }
+}
+
+// Minimum and maximum over the CTA of (lo, hi); all threads get both.
+__device__ __forceinline__ void cta_range(uint32_t& lo, uint32_t& hi) {
+  __shared__ uint32_t s_lo[kSmallWarps], s_hi[kSmallWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) s_lo[warp] = lo, s_hi[warp] = hi;
+  __syncthreads();
+  lo = __reduce_min_sync(0xffffffffu, s_lo[lane]);
+  hi = __reduce_max_sync(0xffffffffu, s_hi[lane]);
+}
+
+template <int kRounds>
+__global__ void __launch_bounds__(kSmallThreads, 1) small_sort_kernel(int32_t* data, int n) {
+  extern __shared__ __align__(128) uint32_t smem[];
+  uint32_t k[kRounds], lo = 0xffffffffu, hi = 0;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const int i = r * kSmallThreads + threadIdx.x;
+    if (i < n) {
+      k[r] = (uint32_t)data[i] ^ 0x80000000u;
+      lo = min(lo, k[r]);
+      hi = max(hi, k[r]);
+    }
+  }
+  cta_range(lo, hi);
+  // the places past n hold the largest key: they sort to the end
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const int i = r * kSmallThreads + threadIdx.x;
+    smem[i] = (i < n ? k[r] : hi) - lo;
+  }
+  cta_sort<kRounds>(smem, 32 - __clz((int)(hi - lo)));
+  for (int i = threadIdx.x; i < n; i += kSmallThreads) data[i] = (int32_t)((smem[i] + lo) ^ 0x80000000u);
+}
+
+// Feedback unique of up to kSmall words: NO_HIT words (and the places past n)
+// become a key above every other.  result[0] = the unique count.
+template <int kRounds>
+__global__ void __launch_bounds__(kSmallThreads, 1) small_unique_kernel(const int32_t* words, int n, int nib,
+                                                                       Divider div, int32_t* out, int* result) {
+  extern __shared__ __align__(128) uint32_t smem[];
+  __shared__ uint32_t s_warp[kSmallWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t k[kRounds], lo = 0xffffffffu, hi = 0;
+  bool none = false;  // a NO_HIT word
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const int i = r * kSmallThreads + threadIdx.x;
+    int32_t v = i < n ? words[i] : kNoHit;
+    none = none || (i < n && v == kNoHit);
+    if (v > 0 && v != kNoHit && nib > 0) v = (int32_t)(((divide((uint32_t)((v >> 1) - 1), div) + 1) << 1) | (v & 1));
+    k[r] = (uint32_t)v ^ 0x80000000u;
+    if (k[r] != kNoKey) {
+      lo = min(lo, k[r]);
+      hi = max(hi, k[r]);
+    }
+  }
+  cta_range(lo, hi);
+  none = __syncthreads_or(none);
+  const bool any = lo <= hi;
+  const uint32_t top = any ? hi - lo + 1 : 0;  // the dropped words' key; hi < kNoKey, so it does not wrap
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) smem[r * kSmallThreads + threadIdx.x] = k[r] == kNoKey ? top : k[r] - lo;
+  cta_sort<kRounds>(smem, 32 - __clz((int)top));
+  __syncthreads();
+  // run starts of the kept keys, kRounds consecutive keys per thread
+  uint32_t starts = 0, cnt = 0;
+  const int first = threadIdx.x * kRounds;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const uint32_t v = smem[first + r];
+    const bool start = v != top && (first + r == 0 || smem[first + r - 1] != v);
+    starts |= (uint32_t)start << r;
+    cnt += start;
+  }
+  uint32_t incl = cnt;
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += t;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  uint32_t pos = incl - cnt, total = 0;
+  {
+    const uint32_t w = s_warp[lane];
+    pos += __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u);
+    total = __reduce_add_sync(0xffffffffu, w);
+  }
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r)
+    if ((starts >> r) & 1u) out[pos++] = (int32_t)((smem[first + r] + lo) ^ 0x80000000u);
+  if (threadIdx.x == 0) {
+    if (none) out[total++] = kNoHit;
+    result[0] = (int)total;
+    result[1] = kPathEmpty;
+  }
+}
+
 // ---- unique of sorted keys -----------------------------------------------------
 // Persistent like digit_kernel, and pipelined the same way: a tile's run-start
 // keys are compacted into shared memory (each warp into its own range), the
 // next tile (claimed at the start of this one) is loaded, and only then does
 // the tile's look-back for its output position run.
-__global__ void __launch_bounds__(kThreads) unique_kernel(const uint32_t* keys, const int* count, int n_total,
-                                                          int32_t* out, unsigned long long* status,
-                                                          int* tile_counter, int* result, const uint32_t* range) {
+__global__ void __launch_bounds__(kThreads) unique_kernel(const uint32_t* keys_a, const uint32_t* keys_b,
+                                                          Control* ctl, const Plan* plan, int32_t* out,
+                                                          unsigned long long* status, int* result, uint32_t tag,
+                                                          int* err) {
   __shared__ int s_tile;
   __shared__ uint32_t s_warp[kWarps + 1];
   __shared__ uint32_t s_excl;
   __shared__ uint32_t s_starts[kTile];
-  if (range[2] == kBitmapPath) return;
-  const int m = *count;
-  const uint32_t tag = g_epoch * 8u + 4u;
+  const uint32_t* keys = plan->last == 0 ? keys_a : keys_b;
+  int* tile_counter = &ctl->unique_tiles;
+  const int m = ctl->keys;  // at least one
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (m == 0) {  // nothing but sentinels (or nothing at all)
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      int u = 0;
-      if (n_total > 0) out[u++] = kNoHit;
-      *result = u;
-    }
-    return;
-  }
   // warp `warp` owns keys [w0, w0 + 512) of a tile, 32 per round (coalesced);
   // a key starts a run when it differs from the key before it
   const int w0 = warp * (kItems * 32);
@@ -743,11 +1118,11 @@ __global__ void __launch_bounds__(kThreads) unique_kernel(const uint32_t* keys, 
       prev_last = lane == 0 && b > 0 && b < m ? __ldg(keys + b - 1) : 0u;
     }
     if (warp == 0) {
-      const uint32_t excl = tile_prefix(s_warp, status, tile, tag);
+      const uint32_t excl = tile_prefix<kWarps>(s_warp, status, tile, tag, err);
       if (lane == 0 && base + valid == m) {  // last tile: totals and the NO_HIT sentinel
         int u = min((int)(excl + s_warp[kWarps]), m);
-        if (m < n_total) out[u++] = kNoHit;
-        *result = u;
+        if (ctl->no_hit) out[u++] = kNoHit;
+        result[0] = u;
       }
       if (lane == 0) s_excl = excl;
     }
@@ -762,26 +1137,264 @@ __global__ void __launch_bounds__(kThreads) unique_kernel(const uint32_t* keys, 
 }
 
 // ---- unique by bitmap ------------------------------------------------------------
-// Bit b of the bitmap stands for key min + b.  All three kernels return at once
-// on the radix path.
-__global__ void __launch_bounds__(kThreads) bitmap_clear_kernel(const uint32_t* range, uint4* bitmap) {
-  if (range[2] != kBitmapPath) return;
-  const size_t n4 = ((size_t)range[3] + 3) / 4;
-  for (size_t i = blockIdx.x * (size_t)kThreads + threadIdx.x; i < n4; i += (size_t)gridDim.x * kThreads)
-    bitmap[i] = make_uint4(0u, 0u, 0u, 0u);
+// Bit b of the bitmap stands for key min + b.  Each kernel returns at once on
+// the paths that do not need it.
+
+// ---- writing a bitmap's values -------------------------------------------------
+// By cooperative kernels of 1024-thread CTAs: each CTA writes the values of some
+// of the words, and what it needs to know of the words before is their bit
+// count.  (Tiles claimed in order with a look-back for the position took
+// 35 us on 1.5 million words, and 10 us on 3 thousand.)
+constexpr int kShareThreads = 1024;
+constexpr int kShareWarps = kShareThreads / 32;
+
+// Waits until `ctas` CTAs have come here; false in every thread when the wait
+// runs out.  What they wrote before is visible after it.
+__device__ __forceinline__ bool grid_barrier(int* counter, int ctas, int* err) {
+  __threadfence();
+  __syncthreads();
+  bool ok = true;
+  if (threadIdx.x == 0) {
+    atomicAdd(counter, 1);
+    long long spins = 0;
+    const unsigned long long start = global_ns();
+    while (*(volatile int*)counter < ctas) {
+      if (wait_over(spins, start)) {
+        set_error(err);
+        ok = false;
+        break;
+      }
+    }
+    __threadfence();
+  }
+  return __syncthreads_and(ok) != 0;
 }
 
-// Histogram of the range buckets (top 8 bits of key - min) of the kept keys;
-// the last CTA to finish turns the counts into offsets (no CTA waits).
-__global__ void __launch_bounds__(kThreads) range_hist_kernel(const uint32_t* keys, const int* count,
-                                                              const uint32_t* range, uint32_t* hist, int* done,
-                                                              uint32_t* cursors) {
-  __shared__ uint32_t sh[kBuckets];
-  __shared__ bool s_last;
-  if (range[2] != kBitmapPath) return;
-  const uint32_t m = (uint32_t)*count, lo = ~range[0];
-  const int shift = (int)range[4];
-  sh[threadIdx.x] = 0;
+// Sum of v over the CTA's threads, in all of them.
+__device__ __forceinline__ uint32_t share_sum(uint32_t v, uint32_t* s_warp) {
+  const uint32_t sum = __reduce_add_sync(0xffffffffu, v);
+  __syncthreads();  // an earlier use of s_warp is over
+  if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  return __reduce_add_sync(0xffffffffu, s_warp[threadIdx.x & 31]);
+}
+
+// Set bits of words [w0, w1), w0 a multiple of 4, over the CTA's threads.
+__device__ __forceinline__ uint32_t count_bits(const uint32_t* bitmap, int w0, int w1, uint32_t* s_warp) {
+  uint32_t bits = 0;
+  for (int i = w0 / 4 + threadIdx.x; i < w1 / 4; i += kShareThreads) {
+    const uint4 q = __ldcg(reinterpret_cast<const uint4*>(bitmap) + i);
+    bits += __popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w);
+  }
+  const int i = max(w0, w1 & ~3) + (int)threadIdx.x;
+  if (i < w1) bits += __popc(__ldcg(bitmap + i));
+  return share_sum(bits, s_warp);
+}
+
+// A warp's bitmap words (one per lane, the lane's first output position `pos`)
+// as signed words.  Dense words go word by word, a lane per bit (one coalesced
+// store per word); else each lane walks its own word's bits into the warp's
+// stage, which is then written in order (stored as they are found, every value
+// is a sector of its own, which bound the kernel).
+constexpr int kStage = 512;  // values per warp
+__device__ __forceinline__ void emit_words(uint32_t w, uint32_t key0, uint32_t pos, uint32_t* stage, int32_t* out) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t first = __shfl_sync(0xffffffffu, pos, 0);
+  const uint32_t total = __shfl_sync(0xffffffffu, pos + __popc(w), 31) - first;
+  if (total > kStage) {
+    unsigned nonempty = __ballot_sync(0xffffffffu, w != 0);
+    while (nonempty) {
+      const int src = __ffs(nonempty) - 1;
+      nonempty &= nonempty - 1;
+      const uint32_t v = __shfl_sync(0xffffffffu, w, src);
+      const uint32_t k = __shfl_sync(0xffffffffu, key0, src);
+      const uint32_t at = __shfl_sync(0xffffffffu, pos, src) + __popc(v & ((1u << lane) - 1));
+      if ((v >> lane) & 1u) out[at] = (int32_t)((k + (uint32_t)lane) ^ 0x80000000u);
+    }
+  } else {
+    uint32_t at = pos - first;
+    while (w) {
+      const int b = __ffs(w) - 1;
+      w &= w - 1;
+      stage[at++] = (key0 + (uint32_t)b) ^ 0x80000000u;
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < total; i += 32) out[first + i] = (int32_t)stage[i];
+    __syncwarp();
+  }
+}
+
+// Positions of one word per thread over the CTA: `run` plus the bits of the
+// threads before; run becomes the total.
+__device__ __forceinline__ uint32_t word_positions(uint32_t w, uint32_t& run, uint32_t* s_warp) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t bits = __popc(w);
+  uint32_t incl = bits;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += t;
+  }
+  __syncthreads();  // an earlier use of s_warp is over
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  const uint32_t c = s_warp[lane];
+  const uint32_t pos = run + __reduce_add_sync(0xffffffffu, lane < warp ? c : 0u) + incl - bits;
+  run += __reduce_add_sync(0xffffffffu, c);
+  return pos;
+}
+
+// Writes the bitmap's values, complete in global memory; s_words: kEmitSmemBytes
+// of shared memory.  A small bitmap is cut into one share
+// per CTA, and every CTA counts the bits of the words before its own.  A large
+// one is cut into segments of 1024 words, dealt to the CTAs in turn (feedback's
+// low block numbers set whole stretches of bits; shares of neighbouring words
+// left most CTAs waiting for a few, 97 us instead of 35), which count them,
+// meet at a barrier and read each other's counts.  The CTA with the last words
+// writes the count and the NO_HIT sentinel when any word was NO_HIT.
+constexpr int kCountAllWords = 1 << 15;
+constexpr int kEmitSmemBytes = (2 * kShareThreads + kShareWarps * kStage) * 4;
+static_assert((1 << kMaxSpanLog2) / 32 / kShareThreads <= 2 * kShareThreads, "two segment counts per thread");
+__device__ __forceinline__ void emit_bitmap(const uint32_t* bitmap, Control* ctl, Plan* plan, int ctas,
+                                            uint32_t* s_words, uint32_t* s_warp, int32_t* out, int* result, int* err) {
+  const uint32_t lo = ~ctl->range[0];
+  const int words = (int)plan->bitmap_words;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t* stage = s_words + 2 * kShareThreads + warp * kStage;
+  uint32_t run = 0;
+  bool last;
+  if (words <= kCountAllWords) {
+    const int share = ((words + ctas - 1) / ctas + 3) & ~3;  // whole 16-byte units
+    const int w0 = min(words, (int)blockIdx.x * share), w1 = min(words, w0 + share);
+    last = w0 < w1 && w1 == words;
+    run = count_bits(bitmap, 0, w0, s_warp);
+    for (int r0 = w0; r0 < w1; r0 += kShareThreads) {
+      const int k = r0 + threadIdx.x;
+      const uint32_t w = k < w1 ? __ldcg(bitmap + k) : 0u;
+      const uint32_t pos = word_positions(w, run, s_warp);
+      if (share > kShareThreads / 2) {
+        emit_words(w, lo + (uint32_t)k * 32u, pos, stage, out);
+        continue;
+      }
+      // a few words: a warp per word, a lane per bit, so that every warp has some
+      s_words[threadIdx.x] = w;
+      s_words[kShareThreads + threadIdx.x] = pos;
+      __syncthreads();
+      for (int i = warp; i < w1 - r0; i += kShareWarps) {
+        const uint32_t v = s_words[i], at = s_words[kShareThreads + i] + __popc(v & ((1u << lane) - 1));
+        if ((v >> lane) & 1u) out[at] = (int32_t)((lo + (uint32_t)(r0 + i) * 32u + (uint32_t)lane) ^ 0x80000000u);
+      }
+      __syncthreads();  // s_words is over
+    }
+  } else {
+    const int segments = (words + kShareThreads - 1) / kShareThreads;
+    last = (int)blockIdx.x == (segments - 1) % ctas;
+    for (int g = blockIdx.x; g < segments; g += ctas) {
+      const int k = g * kShareThreads + threadIdx.x;
+      const uint32_t bits = share_sum(k < words ? __popc(__ldcg(bitmap + k)) : 0u, s_warp);
+      if (threadIdx.x == 0) plan->segment_bits[g] = bits;
+    }
+    if (!grid_barrier(&ctl->barrier[1], ctas, err)) return;
+    {  // segment starts: two counts per thread
+      const int g = 2 * threadIdx.x;
+      const uint32_t c0 = g < segments ? __ldcg(plan->segment_bits + g) : 0u;
+      const uint32_t c1 = g + 1 < segments ? __ldcg(plan->segment_bits + g + 1) : 0u;
+      const uint32_t sum = c0 + c1;
+      uint32_t incl = sum;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += t;
+      }
+      __syncthreads();
+      if (lane == 31) s_warp[warp] = incl;
+      __syncthreads();
+      const uint32_t at = __reduce_add_sync(0xffffffffu, lane < warp ? s_warp[lane] : 0u) + incl - sum;
+      s_words[g] = at;
+      s_words[g + 1] = at + c0;
+      __syncthreads();
+    }
+    for (int g = blockIdx.x; g < segments; g += ctas) {
+      const int k = g * kShareThreads + threadIdx.x;
+      const uint32_t w = k < words ? __ldcg(bitmap + k) : 0u;
+      run = s_words[g];
+      const uint32_t pos = word_positions(w, run, s_warp);
+      emit_words(w, lo + (uint32_t)k * 32u, pos, stage, out);
+    }
+  }
+  if (last && threadIdx.x == 0) {  // run: the bits up to the last word's
+    if (ctl->no_hit) out[run++] = kNoHit;
+    result[0] = (int)run;
+  }
+}
+
+__global__ void __launch_bounds__(kShareThreads) emit_kernel(const uint32_t* bitmap, Control* ctl, Plan* plan,
+                                                             int32_t* out, int* result, int* err) {
+  extern __shared__ __align__(128) uint32_t s_words[];
+  __shared__ uint32_t s_warp[kShareWarps];
+  if (plan->path != kPathPartition) return;
+  emit_bitmap(bitmap, ctl, plan, gridDim.x, s_words, s_warp, out, result, err);
+}
+
+// Sets the keys' bits straight in the bitmap, then writes its values.  Keys
+// that many CTAs of the compaction kept arrive together, and atomics on one
+// word queue (450 thousand keys over 3 thousand words: 120 us): a bitmap of up
+// to 2^20 bits is built in shared memory first, one per CTA, and each CTA adds
+// its words to the global one, starting at a place of its own.  In a wider
+// bitmap each thread looks at a bit before it sets it, one key at a time so
+// that the looks see the bits set before.
+static_assert(kDirectSliceWords * 4 >= kEmitSmemBytes, "the slice's memory serves the writing too");
+__global__ void __launch_bounds__(kShareThreads) direct_bitmap_kernel(const uint32_t* keys, Control* ctl, Plan* plan,
+                                                                      uint32_t* bitmap, int32_t* out, int* result,
+                                                                      int* err) {
+  extern __shared__ __align__(128) uint32_t s_slice[];
+  __shared__ uint32_t s_warp[kShareWarps];
+  if (plan->path != kPathDirect) return;
+  const uint32_t m = (uint32_t)ctl->keys, lo = ~ctl->range[0];
+  const int words = (int)plan->bitmap_words;
+  const uint32_t first = blockIdx.x * kShareThreads + threadIdx.x, step = gridDim.x * kShareThreads;
+  int ctas = gridDim.x;
+  if (words > kDirectSliceWords) {
+    for (uint32_t i = first; i < m; i += step) {
+      const uint32_t bit = __ldg(keys + i) - lo, mask = 1u << (bit & 31);
+      if ((__ldcg(bitmap + (bit >> 5)) & mask) == 0) atomicOr(bitmap + (bit >> 5), mask);
+    }
+  } else {
+    ctas = (int)min((uint32_t)gridDim.x, (m + kShareThreads - 1) / kShareThreads);
+    if ((int)blockIdx.x >= ctas) return;
+    for (int i = threadIdx.x; i < words; i += kShareThreads) s_slice[i] = 0;
+    __syncthreads();
+    for (uint32_t i = first; i < m; i += step * 4) {
+      uint32_t bit[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) bit[r] = i + r * step < m ? __ldg(keys + i + r * step) - lo : 0xffffffffu;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t mask = 1u << (bit[r] & 31);
+        if (bit[r] != 0xffffffffu && (s_slice[bit[r] >> 5] & mask) == 0) atomicOr(s_slice + (bit[r] >> 5), mask);
+      }
+    }
+    __syncthreads();
+    const int turn = (int)((unsigned long long)words * blockIdx.x / ctas);
+    for (int i = threadIdx.x; i < words; i += kShareThreads) {
+      const int k = i + turn < words ? i + turn : i + turn - words;
+      const uint32_t v = s_slice[k];
+      if (v && (__ldcg(bitmap + k) & v) != v) atomicOr(bitmap + k, v);
+    }
+  }
+  if (!grid_barrier(&ctl->barrier[0], ctas, err)) return;
+  emit_bitmap(bitmap, ctl, plan, ctas, s_slice, s_warp, out, result, err);
+}
+
+// Histogram of the range buckets (top 8 bits of key - min) of the kept keys,
+// each lane counting in its own bank (see digit_hist_kernel); the last CTA
+// turns the counts into offsets.
+__global__ void __launch_bounds__(kThreads) range_hist_kernel(const uint32_t* keys, Control* ctl, Plan* plan) {
+  __shared__ uint32_t sh[kBuckets * 32];
+  if (plan->path != kPathPartition) return;
+  const uint32_t m = (uint32_t)ctl->keys, lo = ~ctl->range[0];
+  const int shift = (int)plan->range_shift;
+  for (int i = threadIdx.x; i < kBuckets * 32; i += kThreads) sh[i] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
   for (uint32_t i0 = blockIdx.x * kThreads * 8u; i0 < m; i0 += gridDim.x * kThreads * 8u) {
@@ -792,49 +1405,44 @@ __global__ void __launch_bounds__(kThreads) range_hist_kernel(const uint32_t* ke
       k[r] = i < m ? __ldg(keys + i) : 0u;
     }
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {  // one shared atomic per distinct bucket per warp: frequent keys share one
-      const bool ok = i0 + r * kThreads + threadIdx.x < m;
-      const uint32_t b = ok ? (k[r] - lo) >> shift : 0x100u + (uint32_t)lane;
-      const unsigned peers = __match_any_sync(0xffffffffu, b);
-      if (ok && lane == __ffs(peers) - 1) atomicAdd(&sh[b], (uint32_t)__popc(peers));
-    }
+    for (int r = 0; r < 8; ++r)
+      if (i0 + r * kThreads + threadIdx.x < m) atomicAdd(&sh[((k[r] - lo) >> shift) * 32 + lane], 1u);
   }
   __syncthreads();
-  if (sh[threadIdx.x]) atomicAdd(hist + kRangeCounts + threadIdx.x, sh[threadIdx.x]);
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const uint32_t c = *(volatile uint32_t*)(hist + kRangeCounts + threadIdx.x);
-  sh[threadIdx.x] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t run = 0;
-    for (int d = 0; d < kBuckets; ++d) { const uint32_t v = sh[d]; sh[d] = run; run += v; }
+  {
+    uint32_t sum = 0;
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) sum += sh[threadIdx.x * 32 + ((lane + k) & 31)];
+    if (sum) atomicAdd(&ctl->range_counts[threadIdx.x], sum);
   }
+  if (!last_cta(&ctl->done[1], gridDim.x)) return;
   __syncthreads();
-  hist[kRangeOffsets + threadIdx.x] = sh[threadIdx.x];
-  cursors[threadIdx.x * kCursorStride] = sh[threadIdx.x];
+  sh[threadIdx.x] = *(volatile uint32_t*)&ctl->range_counts[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x < 32) warp_scan_256(sh, sh);
+  __syncthreads();
+  plan->range_offsets[threadIdx.x] = sh[threadIdx.x];
+  plan->cursors[threadIdx.x * kCursorStride] = sh[threadIdx.x];
 }
 
 // Range partition of the bitmap path.  Unstable (the bitmap does not care
 // about order): tiles of 4096 keys, grid-strided; a key's slot in its range
-// bucket comes from a shared per-tile count (one atomic per distinct bucket
-// per warp), the tile claims one range per bucket from the bucket's cursor,
-// and the keys are staged in shared memory in bucket order so each bucket's
-// run goes out contiguously while the next tile's keys load.  No CTA waits on
-// another.
+// bucket comes from a shared per-tile count, the tile claims one range per
+// bucket from the bucket's cursor, and the keys are staged in shared memory in
+// bucket order so each bucket's run goes out contiguously while the next
+// tile's keys load.  A key takes its slot with an atomic of its own, except
+// in the bucket of a lane picked each round, whose lanes share one: feedback's
+// frequent blocks lie in one bucket, where single atomics would queue.  No CTA
+// waits on another.
 __global__ void __launch_bounds__(kThreads, 4) range_partition_kernel(const uint32_t* in, uint32_t* out,
-                                                                   const int* count, const uint32_t* range,
-                                                                   uint32_t* cursors) {
+                                                                   const Control* ctl, Plan* plan) {
   __shared__ uint32_t s_cnt[kBuckets];    // per-tile count, then the tile-local start of each bucket
   __shared__ uint32_t s_base[kBuckets];   // global start of each bucket's run
   __shared__ uint32_t s_keys[kTile];
-  if (range[2] != kBitmapPath) return;
-  const uint32_t m = (uint32_t)*count, lo = ~range[0];
-  const int shift = (int)range[4];
+  if (plan->path != kPathPartition) return;
+  const uint32_t m = (uint32_t)ctl->keys, lo = ~ctl->range[0];
+  const int shift = (int)plan->range_shift;
+  uint32_t* cursors = plan->cursors;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1;
   const uint32_t stride = gridDim.x * (uint32_t)kTile;
@@ -852,13 +1460,17 @@ __global__ void __launch_bounds__(kThreads, 4) range_partition_kernel(const uint
 #pragma unroll
     for (int r = 0; r < kItems; ++r) {
       const bool ok = r * kThreads + threadIdx.x < valid;
-      const uint32_t b = ok ? (k[r] - lo) >> shift : 0x100u + (uint32_t)lane;
-      const unsigned peers = __match_any_sync(0xffffffffu, b);
-      const int leader = __ffs(peers) - 1;
-      uint32_t first = 0;
-      if (ok && lane == leader) first = atomicAdd(&s_cnt[b], (uint32_t)__popc(peers));
-      first = __shfl_sync(0xffffffffu, first, leader);
-      const uint32_t sl = first + __popc(peers & lt);
+      const uint32_t b = ok ? (k[r] - lo) >> shift : 0x100u;
+      const uint32_t shared_b = __shfl_sync(0xffffffffu, b, r);  // lane r's bucket
+      const unsigned peers = __ballot_sync(0xffffffffu, b == shared_b);
+      uint32_t sl = 0;
+      if (ok) {
+        const bool sharing = b == shared_b;
+        const int leader = __ffs(peers) - 1;
+        if (!sharing || lane == leader) sl = atomicAdd(&s_cnt[b], sharing ? (uint32_t)__popc(peers) : 1u);
+      }
+      const uint32_t first = __shfl_sync(0xffffffffu, sl, __ffs(peers) - 1);
+      if (b == shared_b) sl = first + __popc(peers & lt);
       slot[r / 2] = (r & 1) ? slot[r / 2] | (sl << 16) : sl;
     }
     __syncthreads();
@@ -867,20 +1479,7 @@ __global__ void __launch_bounds__(kThreads, 4) range_partition_kernel(const uint
       if (c) s_base[threadIdx.x] = atomicAdd(cursors + threadIdx.x * kCursorStride, c);
     }
     __syncthreads();
-    if (threadIdx.x < 32) {  // tile-local bucket starts: exclusive scan of 256 counts by one warp
-      uint32_t v[8], sum = 0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { v[q] = s_cnt[lane * 8 + q]; sum += v[q]; }
-      uint32_t incl = sum;
-      for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += t;
-      }
-      uint32_t run = incl - sum;
-      __syncwarp();
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { s_cnt[lane * 8 + q] = run; run += v[q]; }
-    }
+    if (threadIdx.x < 32) warp_scan_256(s_cnt, s_cnt);  // tile-local bucket starts
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < kItems; ++r)
@@ -911,49 +1510,33 @@ __global__ void __launch_bounds__(kThreads, 4) range_partition_kernel(const uint
 // Zipf-like) is spread over many CTAs.
 constexpr int kChunk = 16384;
 constexpr int kSliceWords = (1 << (kMaxSpanLog2 - 8)) / 32 + 1;
-__global__ void __launch_bounds__(kThreads) bucket_bitmap_kernel(const uint32_t* keys, const uint32_t* range,
-                                                                 const uint32_t* hist, uint32_t* bitmap,
-                                                                 int* item_counter) {
+__global__ void __launch_bounds__(kThreads) bucket_bitmap_kernel(const uint32_t* keys, Control* ctl, const Plan* plan,
+                                                                 uint32_t* bitmap) {
   __shared__ uint32_t s_bits[kSliceWords];
   __shared__ uint32_t s_first[kBuckets + 1];  // first item of each bucket; [256] = all items
   __shared__ int s_item;
-  if (range[2] != kBitmapPath) return;
-  const uint32_t lo = ~range[0];
-  const int shift = (int)range[4];
-  const int lane = threadIdx.x & 31;
-  {  // items per bucket, scanned by one warp
-    const uint32_t c = hist[kRangeCounts + threadIdx.x];
-    s_first[threadIdx.x] = (c + kChunk - 1) / kChunk;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      uint32_t v[8], sum = 0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) { v[k] = s_first[lane * 8 + k]; sum += v[k]; }
-      uint32_t incl = sum;
-      for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += t;
-      }
-      uint32_t run = incl - sum;
-      __syncwarp();
-#pragma unroll
-      for (int k = 0; k < 8; ++k) { s_first[lane * 8 + k] = run; run += v[k]; }
-      if (lane == 31) s_first[kBuckets] = run;
-    }
-    __syncthreads();
+  if (plan->path != kPathPartition) return;
+  const uint32_t lo = ~ctl->range[0];
+  const int shift = (int)plan->range_shift;
+  s_first[threadIdx.x] = (ctl->range_counts[threadIdx.x] + kChunk - 1) / kChunk;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const uint32_t total = warp_scan_256(s_first, s_first);
+    if (threadIdx.x == 0) s_first[kBuckets] = total;
   }
+  __syncthreads();
   const uint32_t items = s_first[kBuckets];
   for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(item_counter, 1);
+    if (threadIdx.x == 0) s_item = atomicAdd(&ctl->bucket_items, 1);
     __syncthreads();
     const uint32_t item = (uint32_t)s_item;
     if (item >= items) return;
     int b = 0;  // the bucket: last with s_first[b] <= item
     for (int step = kBuckets / 2; step > 0; step >>= 1)
       if (s_first[b + step] <= item) b += step;
-    const uint32_t count = hist[kRangeCounts + b];
-    const uint32_t first = hist[kRangeOffsets + b] + (item - s_first[b]) * kChunk;
-    const uint32_t end = hist[kRangeOffsets + b] + min(count, (item - s_first[b] + 1) * kChunk);
+    const uint32_t count = ctl->range_counts[b];
+    const uint32_t first = plan->range_offsets[b] + (item - s_first[b]) * kChunk;
+    const uint32_t end = plan->range_offsets[b] + min(count, (item - s_first[b] + 1) * kChunk);
     const uint32_t bit0 = (uint32_t)b << shift;  // the bucket's first bit
     const uint32_t w0 = bit0 >> 5;
     const int words = (int)(((bit0 + (1u << shift) - 1) >> 5) - w0 + 1);
@@ -983,210 +1566,286 @@ __global__ void __launch_bounds__(kThreads) bucket_bitmap_kernel(const uint32_t*
   }
 }
 
-// The set bits in order, as signed words: tiles of 1024 bitmap words (4 per
-// thread, one 16-byte load), a CTA scan of the per-thread bit counts and a
-// look-back for the tile's output position.  Persistent like unique_kernel.
-// The last tile writes the count and the NO_HIT sentinel when any word was
-// NO_HIT.
-constexpr int kBitmapTile = kThreads * 4;
-__global__ void __launch_bounds__(kThreads) bitmap_unique_kernel(const uint32_t* bitmap, const int* count,
-                                                                 int n_total, const uint32_t* range, int32_t* out,
-                                                                 unsigned long long* status, int* tile_counter,
-                                                                 int* result) {
-  __shared__ int s_tile;
-  __shared__ uint32_t s_warp[kWarps + 1];
-  __shared__ uint32_t s_excl;
-  if (range[2] != kBitmapPath) return;
-  const uint32_t n_words = range[3], lo = ~range[0];
-  const int m = *count;
-  const uint32_t tag = g_epoch * 8u + 5u;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (;;) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1);
-    __syncthreads();
-    const int tile = s_tile;
-    const size_t base = (size_t)tile * kBitmapTile;
-    if (base >= n_words) return;
-    const size_t first = base + (size_t)threadIdx.x * 4;
-    uint32_t w[4];
-    if (first + 4 <= n_words) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(bitmap + first));
-      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    } else {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) w[r] = first + r < n_words ? __ldg(bitmap + first + r) : 0u;
-    }
-    const uint32_t cnt = __popc(w[0]) + __popc(w[1]) + __popc(w[2]) + __popc(w[3]);
-    uint32_t incl = cnt;
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += t;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-      const uint32_t excl = tile_prefix(s_warp, status, tile, tag);
-      if (lane == 0 && base + kBitmapTile >= n_words) {  // last tile
-        int u = min((int)(excl + s_warp[kWarps]), m);
-        if (m < n_total) out[u++] = kNoHit;
-        *result = u;
-      }
-      if (lane == 0) s_excl = excl;
-    }
-    __syncthreads();
-    uint32_t pos = s_excl + s_warp[warp] + incl - cnt;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      uint32_t v = w[r];
-      const uint32_t key0 = lo + (uint32_t)(first + r) * 32u;
-      while (v) {
-        const int b = __ffs(v) - 1;
-        v &= v - 1;
-        if (pos < (uint32_t)m) out[pos] = (int32_t)((key0 + (uint32_t)b) ^ 0x80000000u);
-        ++pos;
-      }
-    }
-    __syncthreads();  // s_tile / s_warp / s_excl are reused by the next tile
-  }
-}
-
 // ---- inclusive scan (wrapping int32) ---------------------------------------------
-// Tiles of 4096 values claimed in order; a tile's prefix comes from a warp-wide
-// look-back over a status table cleared per call (tag 0: a cleared word is
-// unpublished).  Sums wrap like the reference's int arithmetic.
-__global__ void __launch_bounds__(kThreads) scan_kernel(int32_t* data, int n, unsigned long long* status,
-                                                        int* tile_counter) {
-  __shared__ int s_tile;
-  __shared__ uint32_t s_warp[kWarps + 1];
-  __shared__ uint32_t s_excl;
-  if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1);
-  __syncthreads();
-  const int tile = s_tile;
-  const int base = tile * kTile;
-  if (base >= n) return;
+// One CTA per SM, in rounds: in round k CTA c has tile k * gridDim.x + c, which
+// it holds in shared memory from the one read to the one write.  A round's sums
+// are published by every CTA and read by every CTA, so a CTA knows the sum of
+// all rounds before and needs no walk over its predecessors.  Three buffers
+// let the steps overlap: while tile k + 1 is on its way (one bulk async copy),
+// tile k is summed and its sum published, and then tile k - 1, whose round has
+// had that long to arrive, is scanned and written.  A look-back of tiles in
+// claim order, however wide, took 570 to 840 us on 2^28 values where the reads
+// and writes alone took 400 (a tile's slot waits for the slowest load before
+// it).  The CTAs wait on one another, so the launch is cooperative; each wait
+// is bounded.  Sums wrap like the reference's int arithmetic.
+//
+// The array is taken from the 16-byte boundary at or before it: element i of
+// the tiles is data[i - mis], zero before `mis` and from `end` on.  The copies
+// move the whole 16-byte units inside the array, the threads the elements
+// before and after them.
+constexpr int kScanThreads = 512;
+constexpr int kScanWarps = kScanThreads / 32;
+constexpr int kScanRows = 8;                            // rows of 128 elements per warp, at most
+constexpr int kScanTile = kScanWarps * 128 * kScanRows;  // 16384 elements
+constexpr int kScanBuffers = 3;
+constexpr int kScanBlock = kScanThreads + 32;            // and the warp that collects the rounds' sums
+constexpr int kScanSmemBytes = kScanBuffers * kScanTile * 4;
+
+// Thread 0 starts the copy of the tile's whole units; the others fill in the
+// array's first and last elements and zeros.
+__device__ __forceinline__ void scan_load(uint32_t* buf, const int32_t* base, int first, int rows, int mis, int end,
+                                          unsigned long long* bar) {
+  const int stop = first + rows * (kScanWarps * 128);
+  const int a = max(first, (mis + 3) & ~3), b = max(a, min(stop, end) & ~3);
+  if (threadIdx.x == 0) bulk_load(buf + (a - first), base + a, (uint32_t)(b - a) * 4u, bar);
+  auto edge = [&](int i) { buf[i - first] = i >= mis && i < end ? (uint32_t)base[i] : 0u; };
+  if ((int)threadIdx.x < a - first) edge(first + threadIdx.x);  // the first unit
+  for (int i = b + threadIdx.x; i < stop; i += kScanThreads) edge(i);
+}
+
+// The scanning warps' barrier (the collecting warp does not take part).
+__device__ __forceinline__ void scan_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kScanThreads) : "memory"); }
+
+// The same; true when every one of them passes true.
+__device__ __forceinline__ bool scan_sync_and(bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+      : "=r"(r)
+      : "r"((uint32_t)v), "n"(kScanThreads)
+      : "memory");
+  return r != 0;
+}
+
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+__global__ void __launch_bounds__(kScanBlock, 1) scan_kernel(int32_t* data, int n, int rows,
+                                                             unsigned long long* status, uint32_t tag, int* err) {
+  extern __shared__ __align__(128) uint32_t s_tiles[];
+  __shared__ unsigned long long s_bar[kScanBuffers];        // a tile has landed
+  __shared__ unsigned long long s_collected[2], s_used[2];  // a round's sums are in s_round; they are used
+  __shared__ uint32_t s_warp[kScanBuffers][kScanWarps];
+  // sum of the round's tiles before this CTA's, of all of them, and whether every one arrived
+  __shared__ uint32_t s_round[2][3];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t v[kItems], sum = 0;
-  const int first = base + threadIdx.x * kItems;
-  if (first + kItems <= n && ((reinterpret_cast<uintptr_t>(data + first) & 15) == 0)) {
-#pragma unroll
-    for (int r = 0; r < kItems / 4; ++r) {
-      const int4 q = reinterpret_cast<const int4*>(data + first)[r];
-      v[4 * r] = (uint32_t)q.x; v[4 * r + 1] = (uint32_t)q.y; v[4 * r + 2] = (uint32_t)q.z; v[4 * r + 3] = (uint32_t)q.w;
+  const int mis = (int)((reinterpret_cast<uintptr_t>(data) >> 2) & 3u);
+  int32_t* base = data - mis;
+  const int end = n + mis, tile_size = rows * (kScanWarps * 128);  // n < 2^30
+  const int tiles = (end + tile_size - 1) / tile_size, step = gridDim.x;
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < kScanBuffers; ++b) mbar_init(&s_bar[b]);
+    for (int b = 0; b < 2; ++b) mbar_init(&s_collected[b]), mbar_init(&s_used[b]);
+    mbar_init_fence();
+  }
+  __syncthreads();
+  if (warp == kScanWarps) {  // collects each round's sums
+    for (int k = 0; (int)blockIdx.x + k * step < tiles; ++k) {
+      const int row0 = k * step, count = min(step, tiles - row0);
+      uint32_t before = 0, all = 0;
+      bool ok = true;
+      for (int i = lane; tiles > 1 && i < count; i += 32) {
+        unsigned long long w = ld_volatile64(status + row0 + i);
+        long long spins = 0;
+        const unsigned long long start = lb_ready(w, tag) ? 0 : global_ns();
+        while (!lb_ready(w, tag)) {
+          if (wait_over(spins, start)) {
+            set_error(err);
+            ok = false;
+            break;
+          }
+          __nanosleep(64);
+          w = ld_volatile64(status + row0 + i);
+        }
+        all += (uint32_t)w;
+        if (i < (int)blockIdx.x) before += (uint32_t)w;
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      before = __reduce_add_sync(0xffffffffu, before);
+      all = __reduce_add_sync(0xffffffffu, all);
+      // the slot's sums of two rounds ago are used
+      if (k >= 2 && !mbar_wait(&s_used[k & 1], (uint32_t)(k / 2 - 1) & 1u, err)) ok = false;
+      if (lane == 0) {
+        s_round[k & 1][0] = before;
+        s_round[k & 1][1] = all;
+        s_round[k & 1][2] = ok ? 1u : 0u;
+        mbar_arrive(&s_collected[k & 1]);
+      }
+      if (!__all_sync(0xffffffffu, ok)) return;
     }
-  } else {
-#pragma unroll
-    for (int r = 0; r < kItems; ++r) v[r] = first + r < n ? (uint32_t)data[first + r] : 0u;
+    return;
   }
-#pragma unroll
-  for (int r = 0; r < kItems; ++r) sum += v[r];
-  uint32_t incl = sum;
-  for (int off = 1; off < 32; off <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += t;
+  const int seg = warp * rows * 128 + lane * 4;  // the thread's first element in a tile
+  int issued = kScanBuffers;                     // rounds whose copies were started
+  for (int b = 0; b < kScanBuffers; ++b) {
+    const int t = blockIdx.x + b * step;
+    if (t < tiles) scan_load(s_tiles + b * kScanTile, base, t * tile_size, rows, mis, end, &s_bar[b]);
   }
-  if (lane == 31) s_warp[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    const uint32_t excl = tile_prefix(s_warp, status, tile, 0u);
-    if (lane == 0) s_excl = excl;
-  }
-  __syncthreads();
-  uint32_t run = s_excl + s_warp[warp] + incl - sum;
+  // A wait that ran out (error flag set) ends the CTA once the copies under way
+  // have landed (bounded), so that nothing lands after it has left.
+  auto leave = [&](int k) {
+    if (threadIdx.x == 0)
+      for (int q = k; q <= k + 2; ++q)
+        if ((int)blockIdx.x + q * step < tiles && q < issued)
+          mbar_wait(&s_bar[q % kScanBuffers], (uint32_t)(q / kScanBuffers) & 1u, err);
+  };
+  uint32_t carry = 0;  // sum of all rounds before
+  for (int k = 0;; ++k) {
+    const int t = blockIdx.x + k * step;  // below 2^31: at most 2^30 / 2048 tiles
+    if (t < tiles) {
+      const int b = k % kScanBuffers;
+      const bool landed = mbar_wait(&s_bar[b], (uint32_t)(k / kScanBuffers) & 1u, err);
+      scan_sync();  // the threads' own elements are in place
+      const uint32_t* tile = s_tiles + b * kScanTile;
+      uint32_t sum = 0;
 #pragma unroll
-  for (int r = 0; r < kItems; ++r) {
-    run += v[r];
-    v[r] = run;
-  }
-  if (first + kItems <= n && ((reinterpret_cast<uintptr_t>(data + first) & 15) == 0)) {
+      for (int r = 0; r < kScanRows; ++r)
+        if (r < rows) {
+          const uint4 q = *reinterpret_cast<const uint4*>(tile + seg + r * 128);
+          sum += q.x + q.y + q.z + q.w;
+        }
+      sum = __reduce_add_sync(0xffffffffu, sum);
+      if (lane == 0) s_warp[b][warp] = sum;
+      if (!scan_sync_and(landed)) return leave(k);
+      if (warp == 0 && tiles > 1) {
+        const uint32_t total = __reduce_add_sync(0xffffffffu, lane < kScanWarps ? s_warp[b][lane] : 0u);
+        if (lane == 0) st_volatile64(status + t, lb_word(tag, 2u, total));
+      }
+    }
+    if (k > 0) {  // finish the tile of the round before
+      const int p = t - step, b = (k - 1) % kScanBuffers, slot = (k - 1) & 1;
+      const bool arrived = mbar_wait(&s_collected[slot], (uint32_t)((k - 1) / 2) & 1u, err) && s_round[slot][2] != 0;
+      if (!scan_sync_and(arrived)) return leave(k);
+      uint32_t* tile = s_tiles + b * kScanTile;
+      uint32_t run = carry + s_round[slot][0];
+      run += __reduce_add_sync(0xffffffffu, lane < warp ? s_warp[b][lane] : 0u);  // warp < 16
+      carry += s_round[slot][1];
+      uint32_t v[kScanRows][4];
 #pragma unroll
-    for (int r = 0; r < kItems / 4; ++r)
-      reinterpret_cast<int4*>(data + first)[r] =
-          make_int4((int)v[4 * r], (int)v[4 * r + 1], (int)v[4 * r + 2], (int)v[4 * r + 3]);
-  } else {
+      for (int r = 0; r < kScanRows; ++r) {
+        if (r >= rows) break;
+        const uint4 q = *reinterpret_cast<const uint4*>(tile + seg + r * 128);
+        v[r][0] = q.x;
+        v[r][1] = v[r][0] + q.y;
+        v[r][2] = v[r][1] + q.z;
+        v[r][3] = v[r][2] + q.w;
+      }
+      scan_sync();  // the buffer and the slot are read
+      if (threadIdx.x == 0) mbar_arrive(&s_used[slot]);
+      const int next = p + kScanBuffers * step;
+      if (next < tiles) scan_load(tile, base, next * tile_size, rows, mis, end, &s_bar[b]);
+      issued = k + 3;
 #pragma unroll
-    for (int r = 0; r < kItems; ++r)
-      if (first + r < n) data[first + r] = (int32_t)v[r];
+      for (int r = 0; r < kScanRows; ++r) {
+        if (r >= rows) break;
+        uint32_t incl = v[r][3];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const uint32_t u = __shfl_up_sync(0xffffffffu, incl, off);
+          if (lane >= off) incl += u;
+        }
+        const uint32_t at = run + incl - v[r][3];
+        run += __shfl_sync(0xffffffffu, incl, 31);
+        const int i = p * tile_size + seg + r * 128;
+        if (i >= mis && i + 4 <= end) {
+          *reinterpret_cast<int4*>(base + i) = make_int4((int)(v[r][0] + at), (int)(v[r][1] + at),
+                                                         (int)(v[r][2] + at), (int)(v[r][3] + at));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (i + j >= mis && i + j < end) base[i + j] = (int32_t)(v[r][j] + at);
+        }
+      }
+    }
+    if (t >= tiles) return;
   }
 }
 
-int grid_for(int n) {
-  const int tiles = (n + kTile - 1) / kTile;
-  return tiles > 0 ? tiles : 1;
+// Copy of an array that does not start on a 16-byte boundary (the digit passes
+// bring their tiles in by 16-byte copies).
+__global__ void __launch_bounds__(kThreads) copy_keys_kernel(const uint32_t* in, uint32_t* out, int n) {
+  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < (uint32_t)n; i += gridDim.x * kThreads) out[i] = in[i];
 }
 
-// Resident CTAs of persistent kernel K, at most the tiles of n keys.
+int tiles_of(int n, int tile) { return std::max(1, (int)(((long long)n + tile - 1) / tile)); }
+
+// Resident CTAs of kernel K of `threads` threads, at most `tiles`.
 template <auto K>
-int persistent_grid(int n) {
-  static int resident = 0;
-  if (!resident) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
+int persistent_grid(int tiles, int threads = kThreads, int smem = 0) {
+  static int resident[64] = {};  // by device (the callers hold prims_mutex())
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int& r = resident[dev & 63];
+  if (!r) {
+    int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K, kThreads, 0);
-    resident = sms * (per_sm > 0 ? per_sm : 1);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K, threads, smem);
+    r = sms * (per_sm > 0 ? per_sm : 1);
   }
-  return std::min(resident, grid_for(n));
+  return std::min(r, tiles);
 }
 
-// Resident digit_kernel CTAs (two per SM), at most the tiles of n keys.
-int digit_grid(int n) {
-  static int resident = 0;
-  if (!resident) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(digit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDigitSmemBytes);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, digit_kernel, kDigitThreads, kDigitSmemBytes);
-    resident = sms * (per_sm > 0 ? per_sm : 1);
-  }
-  return std::max(1, std::min(resident, (n + kDigitTile - 1) / kDigitTile));
+// Digit counts, offsets and the plan of the passes over n keys (or *count).
+cudaError_t launch_digit_hist(const uint32_t* keys, int n, const int* count, uint32_t flip, bool in_place,
+                              const SortScratchLayout& l, cudaStream_t s) {
+  const int tiles = tiles_of(n, kHistThreads * 4);
+  if ((reinterpret_cast<uintptr_t>(keys) & 15) == 0)
+    digit_hist_kernel<true><<<persistent_grid<digit_hist_kernel<true>>(tiles, kHistThreads, kHistSmemBytes),
+                              kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, l.control, l.plan);
+  else
+    digit_hist_kernel<false><<<persistent_grid<digit_hist_kernel<false>>(tiles, kHistThreads, kHistSmemBytes),
+                               kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, l.control, l.plan);
+  return cudaGetLastError();
 }
 
-// The four digit passes.  With `range` (feedback unique) they return at once
-// when the bitmap path was chosen.
-cudaError_t run_passes(SortScratchLayout& l, int n, uint32_t*& cur, uint32_t*& other, int32_t* final_out,
-                       const uint32_t* range, cudaStream_t s) {
-  cudaError_t e;
-  const int grid = digit_grid(n);
+// The four digit passes.  `sign_flip`: the keys are signed words (the top
+// digit's upper bit is flipped as it is read).
+cudaError_t launch_digits(const DigitBuffers& bufs, int n, const int* count, bool sign_flip,
+                          const SortScratchLayout& l, unsigned long long* status, uint32_t epoch, int* err,
+                          cudaStream_t s) {
+  const int grid = persistent_grid<digit_kernel>(tiles_of(n, kDigitTile), kDigitThreads, kDigitSmemBytes);
   for (int p = 0; p < kPasses; ++p) {
-    const bool last = p == kPasses - 1;
-    digit_kernel<<<grid, kDigitThreads, kDigitSmemBytes, s>>>(cur, other, l.count, 8 * p, l.hist + p * kBuckets,
-                                                              l.status, l.tile_counter + p, p, last,
-                                                              last ? final_out : nullptr, range);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    std::swap(cur, other);
+    digit_kernel<<<grid, kDigitThreads, kDigitSmemBytes, s>>>(
+        bufs, n, count, p, sign_flip && p == kPasses - 1 ? 0x80u : 0u, l.plan, status, &l.control->tiles[p],
+        epoch * 8u + (uint32_t)p, err);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
-int compact_grid(int n) {
-  static int resident = 0;
-  if (!resident) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, compact_kernel<true, true>, kThreads, 0);
-    resident = sms * (per_sm > 0 ? per_sm : 1);
-  }
-  return std::min(resident, grid_for(n));
+template <int kRounds>
+void launch_small_sort(int32_t* data, int n, cudaStream_t s) {
+  constexpr int bytes = small_smem_bytes<kRounds>();
+  const int grid = persistent_grid<small_sort_kernel<kRounds>>(1, kSmallThreads, bytes);
+  small_sort_kernel<kRounds><<<grid, kSmallThreads, bytes, s>>>(data, n);
+}
+template <int kRounds>
+void launch_small_unique(const int32_t* words, int n, int nib, int32_t* out, int* result, cudaStream_t s) {
+  constexpr int bytes = small_smem_bytes<kRounds>();
+  const int grid = persistent_grid<small_unique_kernel<kRounds>>(1, kSmallThreads, bytes);
+  small_unique_kernel<kRounds><<<grid, kSmallThreads, bytes, s>>>(words, n, nib, make_divider((uint32_t)nib), out,
+                                                                 result);
 }
 
 // Waits, as a look-back does, on a word that nothing publishes: the wait must
 // give up after g_wait_ns, set the error flag and return.
-__global__ void bounded_wait_probe_kernel(const unsigned long long* never) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) look_back(never, 1, 1, 0, 1u);
+__global__ void bounded_wait_probe_kernel(const unsigned long long* never, int* err) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) look_back(never, 1, 1, 0, 1u, err);
 }
 
 }  // namespace
 
-cudaError_t bounded_wait_probe(double limit_s, cudaStream_t s) {
+cudaError_t bounded_wait_probe(double limit_s, int* err, cudaStream_t s) {
   const unsigned long long limit = (unsigned long long)(limit_s * 1e9), normal = 1000000000ull;
   unsigned long long* never = nullptr;
   cudaError_t e = cudaMalloc(&never, 2 * sizeof(unsigned long long));
   if (e != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(never, 0, 2 * sizeof(unsigned long long), s)) == cudaSuccess &&
       (e = cudaMemcpyToSymbolAsync(g_wait_ns, &limit, sizeof(limit), 0, cudaMemcpyHostToDevice, s)) == cudaSuccess) {
-    bounded_wait_probe_kernel<<<1, 32, 0, s>>>(never);
+    bounded_wait_probe_kernel<<<1, 32, 0, s>>>(never, err);
     e = cudaGetLastError();
   }
   cudaError_t e2 = cudaMemcpyToSymbolAsync(g_wait_ns, &normal, sizeof(normal), 0, cudaMemcpyHostToDevice, s);
@@ -1195,84 +1854,107 @@ cudaError_t bounded_wait_probe(double limit_s, cudaStream_t s) {
   return e != cudaSuccess ? e : (e2 != cudaSuccess ? e2 : e3);
 }
 
-int* device_error_flag() {
-  int* p = nullptr;
-  cudaGetSymbolAddress((void**)&p, g_error_flag);
-  return p;
-}
+size_t sort_scratch_bytes(int n) { return n <= kSmall ? 0 : layout(nullptr, n).bytes; }
+size_t feedback_scratch_bytes(int n) { return n <= kSmall ? 0 : layout(nullptr, n).bytes; }
+size_t sort_status_bytes(int n) { return n <= kSmall ? 0 : (size_t)tiles_of(n, kDigitTile) * kBuckets * 8; }
+// the digit passes' words, or the unique kernel's one per tile of sorted keys
+size_t feedback_status_bytes(int n) { return std::max(sort_status_bytes(n), (size_t)tiles_of(n, kTile) * 8); }
+size_t scan_status_bytes(int n) { return ((size_t)tiles_of(n, kScanTile) + 1024) * 8; }
 
-cudaError_t set_lookback_epoch(uint32_t epoch, cudaStream_t s) {
-  // pageable source: the copy reads `epoch` before the call returns
-  return cudaMemcpyToSymbolAsync(g_epoch, &epoch, sizeof(epoch), 0, cudaMemcpyHostToDevice, s);
-}
-
-size_t sort_scratch_bytes(int n) { return layout(nullptr, n).bytes; }
-size_t feedback_scratch_bytes(int n) { return layout(nullptr, n).bytes; }
-size_t scan_scratch_bytes(int n) { return (((size_t)n + kTile - 1) / kTile + 1) * 8 + 256; }
-
-cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t* unique_out, int* counts_dev,
-                                   void* scratch, size_t scratch_bytes, cudaStream_t s) {
-  SortScratchLayout l = layout(scratch, n);
-  if (scratch_bytes < l.bytes) return cudaErrorInvalidValue;
+cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t* unique_out, void* scratch,
+                                   unsigned long long* status, uint32_t epoch, int* result, int* err,
+                                   cudaStream_t s) {
+  if (n <= kSmall) {
+    if (n <= 2 * kSmallThreads) launch_small_unique<2>(words, n, nib, unique_out, result, s);
+    else if (n <= 4 * kSmallThreads) launch_small_unique<4>(words, n, nib, unique_out, result, s);
+    else launch_small_unique<kSmall / kSmallThreads>(words, n, nib, unique_out, result, s);
+    return cudaGetLastError();
+  }
+  const SortScratchLayout l = layout(scratch, n);
   cudaError_t e;
-  if ((e = cudaMemsetAsync(l.hist, 0, kHistRows * kBuckets * 4, s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(l.tile_counter, 0, 16 * 4, s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(l.count, 0, 4 * 4, s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(l.range, 0, 8 * 4, s)) != cudaSuccess) return e;
-  const int grid = compact_grid(n);
-  if ((e = launch_compact<true>(grid, words, n, nib, l.keys_a, l.count, l.hist, l.range, s)) != cudaSuccess)
+  if ((e = cudaMemsetAsync(l.control, 0, sizeof(Control), s)) != cudaSuccess) return e;
+  const int tiles = tiles_of(n, kTile);
+  if ((e = launch_compact(persistent_grid<compact_kernel<true>>(tiles), words, n, nib, l, unique_out, result, s)) !=
+      cudaSuccess)
     return e;
-  hist_offsets_kernel<<<1, kBuckets, 0, s>>>(l.hist, l.count, l.range, l.bitmap_bits);
-  // bitmap path (each kernel returns at once on the radix path): range
-  // partition keys_a -> keys_b, bitmap in keys_a, its set bits in order
-  const int grid_n = std::min(grid, std::max(1, (int)(((size_t)n + 4095) / 4096)));
-  range_hist_kernel<<<grid_n, kThreads, 0, s>>>(l.keys_a, l.count, l.range, l.hist, l.tile_counter + kCtrRangeDone,
-                                                l.cursors);
-  range_partition_kernel<<<grid_n, kThreads, 0, s>>>(l.keys_a, l.keys_b, l.count, l.range, l.cursors);
-  bitmap_clear_kernel<<<grid_n, kThreads, 0, s>>>(l.range, reinterpret_cast<uint4*>(l.keys_a));
-  bucket_bitmap_kernel<<<persistent_grid<bucket_bitmap_kernel>(n), kThreads, 0, s>>>(
-      l.keys_b, l.range, l.hist, l.keys_a, l.tile_counter + kCtrBuckets);
-  bitmap_unique_kernel<<<persistent_grid<bitmap_unique_kernel>(n), kThreads, 0, s>>>(
-      l.keys_a, l.count, n, l.range, unique_out, l.status, l.tile_counter + kCtrBitmapUnique, counts_dev);
+  const uint32_t* keys = l.keys_a;
+  Control* control = l.control;
+  Plan* plan = l.plan;
+  uint32_t* bitmap = l.bitmap;
+  {
+    const int grid =
+        persistent_grid<direct_bitmap_kernel>(tiles_of(n, kShareThreads), kShareThreads, kDirectSliceWords * 4);
+    void* args[] = {&keys, &control, &plan, &bitmap, &unique_out, &result, &err};
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(direct_bitmap_kernel), dim3(grid),
+                                    dim3(kShareThreads), args, kDirectSliceWords * 4, s);
+    if (e != cudaSuccess || n <= kDirectWords) return e;
+  }
+  range_hist_kernel<<<persistent_grid<range_hist_kernel>(tiles), kThreads, 0, s>>>(l.keys_a, l.control, l.plan);
+  range_partition_kernel<<<persistent_grid<range_partition_kernel>(tiles), kThreads, 0, s>>>(l.keys_a, l.keys_b,
+                                                                                            l.control, l.plan);
+  bucket_bitmap_kernel<<<persistent_grid<bucket_bitmap_kernel>(tiles), kThreads, 0, s>>>(l.keys_b, l.control, l.plan,
+                                                                                        l.bitmap);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  // radix path (each kernel returns at once on the bitmap path)
-  uint32_t* cur = l.keys_a;
-  uint32_t* other = l.keys_b;
-  if ((e = run_passes(l, n, cur, other, nullptr, l.range, s)) != cudaSuccess) return e;
-  unique_kernel<<<persistent_grid<unique_kernel>(n), kThreads, 0, s>>>(cur, l.count, n, unique_out, l.status,
-                                                                      l.tile_counter + kCtrUnique, counts_dev,
-                                                                      l.range);
+  const int grid = persistent_grid<emit_kernel>(tiles_of(n, kShareThreads), kShareThreads, kEmitSmemBytes);
+  void* args[] = {&bitmap, &control, &plan, &unique_out, &result, &err};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(emit_kernel), dim3(grid),
+                                     dim3(kShareThreads), args, kEmitSmemBytes, s);
+}
+
+bool feedback_unique_needs_radix(const int* result) { return result[1] == kPathRadix; }
+
+cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scratch, unsigned long long* status,
+                                         uint32_t epoch, int* result, int* err, cudaStream_t s) {
+  const SortScratchLayout l = layout(scratch, n);
+  cudaError_t e;
+  if ((e = launch_digit_hist(l.keys_a, n, &l.control->keys, 0u, false, l, s)) != cudaSuccess) return e;
+  const DigitBuffers bufs = {l.keys_a, l.keys_a, l.keys_b, nullptr};
+  if ((e = launch_digits(bufs, n, &l.control->keys, false, l, status, epoch, err, s)) != cudaSuccess) return e;
+  unique_kernel<<<persistent_grid<unique_kernel>(tiles_of(n, kTile)), kThreads, 0, s>>>(
+      l.keys_a, l.keys_b, l.control, l.plan, unique_out, status, result, epoch * 8u + 4u, err);
   return cudaGetLastError();
 }
 
-cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch, int* err,
+                            cudaStream_t s) {
   if (n <= 1) return cudaSuccess;
-  SortScratchLayout l = layout(scratch, n);
-  if (scratch_bytes < l.bytes) return cudaErrorInvalidValue;
+  if (n <= kSmall) {
+    if (n <= 2 * kSmallThreads) launch_small_sort<2>(data, n, s);
+    else if (n <= 4 * kSmallThreads) launch_small_sort<4>(data, n, s);
+    else launch_small_sort<kSmall / kSmallThreads>(data, n, s);
+    return cudaGetLastError();
+  }
+  const SortScratchLayout l = layout(scratch, n);
   cudaError_t e;
-  if ((e = cudaMemsetAsync(l.hist, 0, kPasses * kBuckets * 4, s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(l.tile_counter, 0, 16 * 4, s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(l.count, 0, 4 * 4, s)) != cudaSuccess) return e;
-  if ((e = launch_fill_i32(l.count, n, 1, s)) != cudaSuccess) return e;  // [0] keys; [2] the compaction's claims
-  const int grid = compact_grid(n);
-  if ((e = launch_compact<false>(grid, data, n, 0, l.keys_a, l.count + 2, l.hist, nullptr, s)) != cudaSuccess)
-    return e;
-  hist_offsets_kernel<<<1, kBuckets, 0, s>>>(l.hist, l.count, nullptr, 0);
-  uint32_t* cur = l.keys_a;
-  uint32_t* other = l.keys_b;
-  return run_passes(l, n, cur, other, data, nullptr, s);
+  if ((e = cudaMemsetAsync(l.control, 0, sizeof(Control), s)) != cudaSuccess) return e;
+  uint32_t* keys = reinterpret_cast<uint32_t*>(data);
+  DigitBuffers bufs = {keys, keys, l.keys_a, l.keys_b};
+  if (reinterpret_cast<uintptr_t>(data) & 15) {  // the passes read a copy (keys_b is written by the second pass)
+    copy_keys_kernel<<<persistent_grid<copy_keys_kernel>(tiles_of(n, kThreads)), kThreads, 0, s>>>(keys, l.keys_b, n);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    bufs.in0 = l.keys_b;
+  }
+  if ((e = launch_digit_hist(bufs.in0, n, nullptr, 0x80000000u, true, l, s)) != cudaSuccess) return e;
+  return launch_digits(bufs, n, nullptr, true, l, status, epoch, err, s);
 }
 
-cudaError_t scan_i32_device(int32_t* data, int n, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+cudaError_t scan_i32_device(int32_t* data, int n, unsigned long long* status, uint32_t epoch, int* err,
+                            cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  if (scratch_bytes < scan_scratch_bytes(n)) return cudaErrorInvalidValue;
-  const size_t tiles = ((size_t)n + kTile - 1) / kTile + 1;
-  unsigned long long* status = static_cast<unsigned long long*>(scratch);
-  int* counter = reinterpret_cast<int*>(static_cast<uint8_t*>(scratch) + tiles * 8);
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(scratch, 0, tiles * 8 + 16, s)) != cudaSuccess) return e;
-  scan_kernel<<<grid_for(n), kThreads, 0, s>>>(data, n, status, counter);
-  return cudaGetLastError();
+  const int end = n + (int)((reinterpret_cast<uintptr_t>(data) >> 2) & 3u);
+  // rows per warp: a full tile per CTA, or what spreads the array over every SM
+  const int sms = persistent_grid<scan_kernel>(1 << 30, kScanBlock, kScanSmemBytes);
+  constexpr int kRow = kScanWarps * 128;
+  int rows = std::min(kScanRows, (int)(((long long)end + (long long)sms * kRow - 1) / ((long long)sms * kRow)));
+  uint32_t tag = epoch * 8u + 6u;
+  const int grid = std::min(sms, tiles_of(end, rows * kRow));
+  if (grid == 1) {
+    scan_kernel<<<1, kScanBlock, kScanSmemBytes, s>>>(data, n, rows, status, tag, err);
+    return cudaGetLastError();
+  }
+  void* args[] = {&data, &n, &rows, &status, &tag, &err};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(scan_kernel), dim3(grid), dim3(kScanBlock), args,
+                                     kScanSmemBytes, s);
 }
 
 }  // namespace rayt

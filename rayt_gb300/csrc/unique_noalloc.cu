@@ -20,7 +20,7 @@
 //    point take the library's primitives lock and return only after their
 //    stream has finished, so calls from several host threads are serialised
 //    like rayt_sort_i32 / rayt_scan_i32 / rayt_feedback_unique, with which
-//    they also share the device error flag and the look-back epoch.  GPU work
+//    they also share the look-back epoch.  GPU work
 //    the caller queued on other streams that reads or writes the array is not
 //    ordered by the library.  The array keeps the previous call's contents;
 //    every part the kernels expect to start at zero is cleared by each call.
@@ -37,21 +37,18 @@ namespace rayt {
 namespace {
 
 constexpr int kMaxWords = RAYT_FEEDBACK_UNIQUE_NOALLOC_MAX_WORDS;
-constexpr size_t kCountsBytes = 256;
 
-// Sort/unique scratch for kMaxWords words plus 256 bytes for the result count.
-// feedback_scratch_bytes() is a host function, so the size is computed from the
-// same layout rules here: two key arrays of (n + 4) words rounded to 256 bytes,
-// 6 x 256 histogram words, one 8-byte look-back word per 256 buckets per
-// 4096-key tile (+1 tile), 16 tile counters, 4 counts, 8 key-range words and
-// 256 partition cursors 128 bytes apart, each rounded to 256 bytes.
+// Scratch of the unique for kMaxWords words (feedback_scratch_bytes() is a host
+// function, so the size is computed from the same layout rules here: two key
+// arrays of (n + 4) words rounded to 256 bytes, and at most 64 KiB of control
+// words and plan), look-back words (256 digits x 8 bytes per 8192-key tile),
+// and a result block: error flag, unique count, path.
 constexpr size_t Up256(size_t v) { return (v + 255) & ~(size_t)255; }
-constexpr size_t kTiles = ((size_t)kMaxWords + 4095) / 4096 + 1;
-constexpr size_t kScratchBytes = 2 * Up256((size_t)kMaxWords * 4 + 16) + Up256(6 * 256 * 4) +
-                                 Up256(kTiles * 256 * 8) + Up256(16 * 4) + Up256(4 * 4) + Up256(8 * 4) +
-                                 Up256(256 * 32 * 4);
+constexpr size_t kScratchBytes = 2 * Up256((size_t)kMaxWords * 4 + 16) + (64 << 10);
+constexpr size_t kStatusBytes = ((size_t)kMaxWords + 8191) / 8192 * 256 * 8;
+constexpr size_t kResultBytes = 256;
 
-static __device__ __align__(256) uint8_t g_noalloc_scratch[kScratchBytes + kCountsBytes];
+static __device__ __align__(256) uint8_t g_noalloc_scratch[kStatusBytes + kScratchBytes + kResultBytes];
 
 void* g_scratch_ptr[64];
 
@@ -66,13 +63,24 @@ int scratch_address(void** out, cudaStream_t s) {
   if (!g_scratch_ptr[dev]) {
     void* p = nullptr;
     RAYT_CUDA_TRY(cudaGetSymbolAddress(&p, g_noalloc_scratch));
-    // the sort's look-back words are epoch-tagged, never cleared: start from zeros
+    // look-back words are epoch-tagged, never cleared: start from zeros
     RAYT_CUDA_TRY(cudaMemsetAsync(p, 0, sizeof(g_noalloc_scratch), s));
-    register_lookback_area(p, sizeof(g_noalloc_scratch));
+    register_lookback_area(p, kStatusBytes);
     g_scratch_ptr[dev] = p;
   }
   *out = g_scratch_ptr[dev];
   return RAYT_OK;
+}
+
+// Waits for the call's work and reads its result block {error flag, unique
+// count, path}.
+int read_result(int* host, int* result_dev, cudaStream_t s) {
+  RAYT_CUDA_TRY(cudaMemcpyAsync(host, result_dev, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  RAYT_CUDA_TRY(cudaStreamSynchronize(s));
+  if (!host[0]) return RAYT_OK;
+  RAYT_CUDA_TRY(cudaMemsetAsync(result_dev, 0, sizeof(int), s));
+  RAYT_CUDA_TRY(cudaStreamSynchronize(s));
+  return fail(RAYT_E_TIMEOUT, "rayt_feedback_unique_noalloc: a bounded device wait gave up");
 }
 
 }  // namespace
@@ -89,27 +97,27 @@ extern "C" int rayt_feedback_unique_noalloc(const int32_t* words, int n, int nod
     *unique_count = 0;
     return RAYT_OK;
   }
-  if (rayt::feedback_scratch_bytes(n) > rayt::kScratchBytes)
+  if (rayt::feedback_scratch_bytes(n) > rayt::kScratchBytes || rayt::feedback_status_bytes(n) > rayt::kStatusBytes)
     return fail(RAYT_E_LIMIT, "rayt_feedback_unique_noalloc: scratch layout larger than the static area");
   std::lock_guard<std::mutex> lock(rayt::prims_mutex());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   void* base = nullptr;
   int rc = rayt::scratch_address(&base, s);
   if (rc != RAYT_OK) return rc;
-  if ((rc = rayt::lookback_epoch_step(s)) != RAYT_OK) return rc;
-  int* counts = reinterpret_cast<int*>(static_cast<uint8_t*>(base) + rayt::kScratchBytes);
-  // the launcher clears the histograms, tile counters and counts it relies on
-  RAYT_CUDA_TRY(rayt::feedback_unique_device(words, n, nodes_in_block, unique, counts, base, rayt::kScratchBytes, s));
-  int host = 0;
-  RAYT_CUDA_TRY(cudaMemcpyAsync(&host, counts, sizeof(int), cudaMemcpyDeviceToHost, s));
-  RAYT_CUDA_TRY(cudaStreamSynchronize(s));
-  int flag = 0;
-  RAYT_CUDA_TRY(cudaMemcpy(&flag, rayt::device_error_flag(), sizeof(int), cudaMemcpyDeviceToHost));
-  if (flag) {
-    const int zero = 0;
-    cudaMemcpy(rayt::device_error_flag(), &zero, sizeof(int), cudaMemcpyHostToDevice);
-    return fail(RAYT_E_TIMEOUT, "rayt_feedback_unique_noalloc: a bounded device wait gave up");
+  uint32_t epoch = 0;
+  if ((rc = rayt::lookback_epoch_step(s, &epoch)) != RAYT_OK) return rc;
+  unsigned long long* status = static_cast<unsigned long long*>(base);
+  uint8_t* scratch = static_cast<uint8_t*>(base) + rayt::kStatusBytes;
+  int* result = reinterpret_cast<int*>(scratch + rayt::kScratchBytes);
+  int host[3] = {0, 0, 0};
+  // the launcher clears the control words it relies on
+  RAYT_CUDA_TRY(rayt::feedback_unique_device(words, n, nodes_in_block, unique, scratch, status, epoch, result + 1,
+                                             result, s));
+  if ((rc = rayt::read_result(host, result, s)) != RAYT_OK) return rc;
+  if (rayt::feedback_unique_needs_radix(host + 1)) {
+    RAYT_CUDA_TRY(rayt::feedback_unique_radix_device(n, unique, scratch, status, epoch, result + 1, result, s));
+    if ((rc = rayt::read_result(host, result, s)) != RAYT_OK) return rc;
   }
-  *unique_count = host;
+  *unique_count = host[1];
   return RAYT_OK;
 }

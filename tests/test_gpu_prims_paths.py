@@ -1,0 +1,121 @@
+"""The feedback primitives at the sizes and key distributions where a call
+changes its path: one CTA or a chain of launches, full and partial tiles,
+digit passes that every key shares, the first pass's unordered ranking, the
+straight and the partitioned bitmap, aligned and unaligned arrays.  Integers:
+compared exactly with numpy."""
+import numpy as np
+import pytest
+
+import rayt_gb300 as R
+from tests.golden.common import NO_HIT, feedback_words
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a, np.int32)).cuda()
+
+
+def _wide(rng, n):
+    return rng.integers(-2**31, 2**31, n, dtype=np.int64).astype(np.int32)
+
+
+KEYS = {
+    "wide": _wide,
+    "narrow": lambda rng, n: rng.integers(-100, 101, n).astype(np.int32),
+    "blocks": lambda rng, n: rng.integers(0, 1 << 24, n).astype(np.int32),
+    "equal": lambda rng, n: np.full(n, -7, np.int32),
+    "one_digit": lambda rng, n: (0x12003400 + (rng.integers(0, 256, n) << 16)).astype(np.int32),
+    "two_digits": lambda rng, n: (rng.integers(0, 256, n) * 0x01000100 - 2**31).astype(np.int64).astype(np.int32),
+    "skewed": lambda rng, n: np.where(rng.random(n) < 0.9, np.int32(5), _wide(rng, n)).astype(np.int32),
+    "sorted": lambda rng, n: np.sort(_wide(rng, n)),
+}
+
+
+@pytest.mark.parametrize("n", [2, 33, 2047, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 8195, 16384, 16385, 24578, 100003])
+@pytest.mark.parametrize("keys", sorted(KEYS))
+@pytest.mark.parametrize("offset", [0, 1])
+def test_sort_paths(built, n, keys, offset):
+    a = KEYS[keys](np.random.default_rng(n), n)
+    x = _dev(np.concatenate([np.full(offset, 9, np.int32), a, np.full(5, 9, np.int32)]))
+    R.GPUSort(x[offset:], n)
+    got = x.cpu().numpy()
+    np.testing.assert_array_equal(got[offset:offset + n], np.sort(a))
+    assert np.all(got[:offset] == 9) and np.all(got[offset + n:] == 9)
+
+
+@pytest.mark.parametrize("n", [1, 3, 127, 128, 1023, 8191, 8192, 8193, 16384, 16387, 1 << 20, (1 << 20) + 1])
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_scan_paths(built, n, offset):
+    a = _wide(np.random.default_rng(n), n)
+    x = _dev(np.concatenate([np.full(offset, 9, np.int32), a, np.full(5, 9, np.int32)]))
+    R.GPUScan(x[offset:], n)
+    got = x.cpu().numpy()
+    ref = np.cumsum(a.astype(np.int64)).astype(np.uint64).astype(np.uint32).view(np.int32)
+    np.testing.assert_array_equal(got[offset:offset + n], ref)
+    assert np.all(got[:offset] == 9) and np.all(got[offset + n:] == 9)
+
+
+def _check_unique(words, nib, offset=0):
+    import torch
+    w = _dev(np.concatenate([np.zeros(offset, np.int32), words]))[offset:]
+    out = torch.full((words.size + 3,), 9, dtype=torch.int32, device="cuda")
+    cnt = R.feedback_unique(w, words.size, nib, out)
+    conv = words.astype(np.int64)
+    hit = (conv > 0) & (conv != NO_HIT)
+    if nib > 0:
+        conv[hit] = ((((conv[hit] >> 1) - 1) // nib + 1) << 1) | (conv[hit] & 1)
+    ref = np.unique(conv).astype(np.int32)
+    got = out.cpu().numpy()
+    np.testing.assert_array_equal(got[:cnt], ref)
+    assert np.all(got[words.size:] == 9)
+    np.testing.assert_array_equal(w.cpu().numpy(), words)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 2047, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 12289, 65536, 262145])
+@pytest.mark.parametrize("kind", ["feedback", "all_no_hit", "wide", "extremes", "no_no_hit", "dense"])
+def test_unique_paths(built, n, kind):
+    rng = np.random.default_rng(n)
+    nib = 512 if kind in ("feedback", "no_no_hit") else 0
+    if kind == "feedback":
+        words = feedback_words(n, n)
+    elif kind == "all_no_hit":
+        words = np.full(n, NO_HIT, np.int32)
+    elif kind == "wide":
+        words = _wide(rng, n)
+        words[rng.random(n) < 0.3] = NO_HIT
+    elif kind == "extremes":
+        words = rng.choice(np.array([-2**31, 2**31 - 2, NO_HIT, -1, 0, 1], np.int64), n).astype(np.int32)
+    elif kind == "no_no_hit":
+        words = feedback_words(n, n, no_hit=False, id_bits=12)
+    else:  # every value of a range: full bitmap words
+        words = (np.arange(n) - n // 2).astype(np.int32)
+        rng.shuffle(words)
+    _check_unique(words, nib, offset=n % 2)
+
+
+@pytest.mark.parametrize("case", ["direct_limit", "over_limit", "few_keys", "more_keys", "small_bitmap", "partition", "partition_one_bucket", "wide_over_direct"])
+def test_unique_large_paths(built, case):
+    """The largest inputs that go straight into the bitmap (2^21 words), kept
+    keys around 2^18 and a wide bitmap, the partitioned bitmap on even and
+    skewed ranges, the radix passes."""
+    rng = np.random.default_rng(11)
+    if case == "direct_limit":
+        words = (rng.permutation((1 << 21) + 64)[:1 << 21] - 5000).astype(np.int32)
+    elif case == "over_limit":
+        words = (rng.permutation((1 << 21) + 64)[:1 << 21] - 5000).astype(np.int32)
+        words = np.concatenate([words, np.full(9, NO_HIT, np.int32)])
+    elif case in ("few_keys", "more_keys"):
+        words = np.full((1 << 21) + 4097, NO_HIT, np.int32)
+        m = (1 << 18) + (case == "more_keys")
+        words[rng.permutation(words.size)[:m]] = rng.permutation(1 << 25)[:m]
+    elif case == "small_bitmap":  # 2^20 values, each several times
+        words = rng.integers(-1000, (1 << 20) - 1000, (1 << 22) + 5).astype(np.int32)
+    elif case == "partition":
+        words = rng.permutation((1 << 22) + 4097).astype(np.int32)
+    elif case == "partition_one_bucket":
+        words = np.concatenate([rng.permutation(3 << 20), [(1 << 26) - 1, NO_HIT]]).astype(np.int32)
+    else:
+        words = _wide(rng, (1 << 22) + 3)
+    _check_unique(words, 0)
