@@ -52,6 +52,13 @@ void pixel_coords(int w, int h, float* out);
 // The per-view origin the same way: (m[2], m[6], m[10], 0) / m[14].
 void view_origin(const float* m, float* origin);
 
+// Counters of a pass: {pad, rays out, pad, pad, work counter per launch group
+// ...}, then the flags for rays without a feedback word, one per 128-byte line
+// (a warp sets the flag of its CTA's number: one flag for all took a launch's
+// warps, ending together, 5 ns each).
+constexpr int kNoWordFlags = 32, kNoWordStride = 32;
+constexpr int kPassBlockInts = 16 + kNoWordFlags * kNoWordStride;
+
 struct TraceParams {
   // cache (the reference's cache format)
   const uint32_t* links;
@@ -94,7 +101,7 @@ struct TraceParams {
   uint32_t* fault_bits;    // one bit per tree block
   int fault_bit_limit;     // number of tree blocks (bits in fault_bits)
   uint32_t* hit_bits;      // bit 2*cache_block + dup
-  int* no_word;            // set to 1 when a ray produced no feedback word this pass
+  int* no_word;            // kNoWordFlags flags, set when a ray produced no feedback word this pass
   unsigned long long* counters;  // optional: rays, link fetches, far fetches, iterations, hits, faults
   // served mode (zero in the per-frame path).  Client slot i owns the pixels
   // [client_base[i], client_base[i + 1]) of the image buffer.
@@ -144,7 +151,7 @@ struct UniqueFromBitsParams {
   int fault_words;
   const uint32_t* hit_bits;
   int hit_words;
-  const int* no_word;    // set: some ray of the pass produced no word
+  const int* no_word;    // kNoWordFlags flags: some ray of the pass produced no word
   const int* n_in;       // later passes: rays traced (the other pixels have no word); null: all of them
   int total_pixels;
   int32_t* unique_out;   // room for fault bits + hit bits + 1

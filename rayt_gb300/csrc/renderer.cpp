@@ -66,7 +66,7 @@ class Renderer {
   cudaStream_t stream() const { return s_; }
 
  private:
-  static constexpr int kBlockInts = 16;  // pass block: {some ray without a word, rays out, pad, pad, work counter per launch group}
+  static constexpr int kBlockInts = kPassBlockInts;
   Cache* cache_ = nullptr;
   int total_pixels_ = 0, padded_pixels_ = 0;
   cudaStream_t s_ = nullptr;
@@ -299,7 +299,7 @@ TraceParams Renderer::Params(int it) const {
   p.fault_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts);
   p.fault_bit_limit = (int)cache_->tree_blocks();
   p.hit_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts + fault_words_);
-  p.no_word = block(k);
+  p.no_word = block(k) + 16;
   p.lanes = 32;
   p.work = block(k) + 4;
   p.refill = refill;
@@ -354,7 +354,7 @@ UniqueFromBitsParams Renderer::UniqueParams(int it) const {
   q.fault_words = fault_words_;
   q.hit_bits = reinterpret_cast<const uint32_t*>(d_state_ + kBlockInts + fault_words_);
   q.hit_words = hit_words_;
-  q.no_word = block(it & 1);
+  q.no_word = block(it & 1) + 16;
   q.n_in = it > 0 ? block(1 - (it & 1)) + 1 : nullptr;
   q.n_rays = block(it & 1) + 1;
   q.total_pixels = total_pixels_;

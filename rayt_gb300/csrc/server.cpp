@@ -61,7 +61,7 @@ class Server {
   LibcRand rand;
 
  private:
-  static constexpr int kBlockInts = 16;  // {some ray without a word, rays out, pad}
+  static constexpr int kBlockInts = kPassBlockInts;
   struct Client {
     bool live = false;
     int w = 0, h = 0;
@@ -338,7 +338,7 @@ TraceParams Server::Params(int k) const {
   p.fault_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts);
   p.fault_bit_limit = (int)cache_->tree_blocks();
   p.hit_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts + fault_words_);
-  p.no_word = block(k);
+  p.no_word = block(k) + 16;
   p.lanes = 32;
   p.refill = 32;
   p.restart = 1;
