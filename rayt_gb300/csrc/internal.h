@@ -52,14 +52,24 @@ void pixel_coords(int w, int h, float* out);
 // The per-view origin the same way: (m[2], m[6], m[10], 0) / m[14].
 void view_origin(const float* m, float* origin);
 
-// Counters of a pass: {pad, rays out, pad, pad, work counter per launch group
-// ...}, then the flags for rays without a feedback word, one per 128-byte line
-// (a warp sets the flag of its CTA's number: one flag for all took a launch's
-// warps, ending together, 5 ns each).
+// Words of a pass: its counters, then the flags for rays without a feedback
+// word, one per 128-byte line (a warp sets the flag of its CTA's number: one
+// flag for all took a launch's warps, ending together, 5 ns each).  A tracing
+// state is two of these and the feedback bitmaps: a pass counts into one of
+// the two and reads the rays of the pass before from the other, and its unique
+// kernel leaves the other and the bitmaps zero for the pass after it.
 constexpr int kNoWordFlags = 32, kNoWordStride = 32;
-constexpr int kPassBlockInts = 16 + kNoWordFlags * kNoWordStride;
+struct PassState {
+  int rays;                // rays appended to the output list
+  int pad;
+  unsigned long long start_ns;  // when the pass's traversal began
+  int work[12];            // persistent kernel: work counter per launch
+  int no_word[kNoWordFlags * kNoWordStride];
+};
+constexpr int kPassInts = sizeof(PassState) / 4;
 
-struct TraceParams {
+// Parameters of a traversal launch but for its views.
+struct TraceCore {
   // cache (the reference's cache format)
   const uint32_t* links;
   const uint32_t* far_ptrs;
@@ -89,7 +99,6 @@ struct TraceParams {
   float4* out_dir;         // xyz direction, w LOD coefficient
   int* out_parent;
   uint32_t* out_ray;
-  int* n_out;
   // optional depth output (all four set, or all null): per pixel the distance
   // along the ray to what it shows and the cache node that shaded it; records
   // carry the distance a faulted ray advanced so far
@@ -101,7 +110,8 @@ struct TraceParams {
   uint32_t* fault_bits;    // one bit per tree block
   int fault_bit_limit;     // number of tree blocks (bits in fault_bits)
   uint32_t* hit_bits;      // bit 2*cache_block + dup
-  int* no_word;            // kNoWordFlags flags, set when a ray produced no feedback word this pass
+  PassState* words;        // of this pass
+  bool stamp;              // the launch notes when the pass began
   unsigned long long* counters;  // optional: rays, link fetches, far fetches, iterations, hits, faults
   // served mode (zero in the per-frame path).  Client slot i owns the pixels
   // [client_base[i], client_base[i + 1]) of the image buffer.
@@ -115,7 +125,14 @@ struct TraceParams {
   int refill;              // idle lanes that let a warp take new rays (< 32)
   int step_budget;         // iterations a warp runs between refill checks
   int lanes;               // rays per warp (a power of two; see trace_lanes)
+};
+struct TraceParams : TraceCore {
   ViewDesc views[kViewsPerLaunch];
+};
+// What a launch of one view (or of no views: later passes) carries: parameters
+// of 9 KB cost the host 3 us more per graph launch than these.
+struct TraceParams1 : TraceCore {
+  ViewDesc views[1];
 };
 
 // Faulted-ray records carried from one pass to the next (device arrays).
@@ -134,32 +151,51 @@ struct RayList {
 // Rays per warp (TraceParams::lanes) for a launch over `rays` rays.
 int trace_lanes(bool first, int rays);
 cudaError_t launch_trace(const TraceParams& p, bool first, bool count, int rays, int grid, cudaStream_t s);
-// The same launch as a kernel node of a CUDA graph (args: room for one pointer;
-// p must stay valid until the node is added or updated).
-cudaError_t trace_node_params(const TraceParams* p, bool first, bool count, int rays, int grid, void** args,
-                              cudaKernelNodeParams* kp);
+// The same launch as a kernel node of a CUDA graph; l must stay valid until the
+// node is added or updated.
+struct TraceLaunch {
+  TraceParams1 one;       // p, when it has at most one view
+  void* args[1];
+  cudaKernelNodeParams kp;
+};
+void trace_node_params(const TraceParams* p, bool first, bool count, int rays, int grid, TraceLaunch* l);
 // Resident CTAs of the persistent traversal kernel on the current device.
 int trace_persistent_grid(bool count);
-cudaError_t launch_finish(const TraceParams& p, int max_rays, cudaStream_t s);
+cudaError_t launch_finish(const TraceCore& p, int max_rays, cudaStream_t s);
 cudaError_t launch_fill_i32(int* p, int32_t v, size_t n, cudaStream_t s);
 // The reference's debug depth view (raytracer.cl) of views[0] into image.
-cudaError_t launch_depth_view(const TraceParams& p, cudaStream_t s);
+cudaError_t launch_depth_view(const TraceParams1& p, cudaStream_t s);
 
-// Feedback bitmaps -> the reference's sorted unique array.
+// Feedback bitmaps -> the reference's sorted unique array, in host-mapped
+// memory; clears the tracing state for the next pass (see PassState) and ends
+// by publishing the pass's number, so that the host need not wait for the
+// stream.
+struct UniqueResult {     // host-mapped
+  int unique, faults;     // unique count (incl. NO_HIT), fault count
+  int rays;               // rays the pass appended to its output list
+  float trace_ms, unique_ms;
+  int client_faults[kMaxClients];
+  unsigned int pass;      // passes done; written last
+};
 struct UniqueFromBitsParams {
-  const uint32_t* fault_bits;
+  uint32_t* fault_bits;
   int fault_words;
-  const uint32_t* hit_bits;
+  uint32_t* hit_bits;
   int hit_words;
-  const int* no_word;    // kNoWordFlags flags: some ray of the pass produced no word
-  const int* n_in;       // later passes: rays traced (the other pixels have no word); null: all of them
+  PassState* words;      // of this pass
+  PassState* previous;   // of the pass before
+  bool later;            // the pass traced the rays of the pass before (pixels without one have no word)
   int total_pixels;
+  int* client_faults;    // served mode: per client, copied and cleared; may be null
+  unsigned int* passes;  // passes done, on the device
   int32_t* unique_out;   // room for fault bits + hit bits + 1
-  const int* n_rays;     // rays the pass appended to its output list
-  int* counts_out;       // [0] unique count (incl. NO_HIT), [1] fault count, [2] *n_rays
+  UniqueResult* result;
 };
 cudaError_t launch_unique_from_bits(const UniqueFromBitsParams& p, cudaStream_t s);
 cudaError_t unique_node_params(const UniqueFromBitsParams* q, void** args, cudaKernelNodeParams* kp);
+// Waits until `pass` is published in *r; everything queued on s before that
+// pass's unique kernel is done then.
+int wait_pass(const UniqueResult* r, unsigned int pass, cudaStream_t s);
 
 // ---- radix sort / scan / unique -------------------------------------------------
 // Memory of a call: `scratch` (any contents), `status` (look-back words, zero or

@@ -66,7 +66,6 @@ class Renderer {
   cudaStream_t stream() const { return s_; }
 
  private:
-  static constexpr int kBlockInts = kPassBlockInts;
   Cache* cache_ = nullptr;
   int total_pixels_ = 0, padded_pixels_ = 0;
   cudaStream_t s_ = nullptr;
@@ -79,16 +78,22 @@ class Renderer {
   float* d_depth_ = nullptr;        // per pixel (same layout as the images): distance to what it shows
   int32_t* d_hit_ = nullptr;        // per pixel: the cache node that shaded it (-1 miss, -2 error)
   RayList lists_[2];
-  // [pass block 0][fault bits][hit bits][pass block 1]: pass k clears its own
-  // block and the bitmaps with one memset and reads the other block's ray
-  // count as its input.
+  // Tracing state: two PassStates, fault bits, hit bits.  A pass counts into
+  // words(par_) and leaves the other and the bits zero (see PassState), so
+  // par_ changes with every pass, over frames too; dirty_ while that does not
+  // hold (a failed frame, passes without their unique kernel).
   int* d_state_ = nullptr;
+  size_t state_ints_ = 0;
+  int par_ = 0;
+  bool dirty_ = false, in_frame_ = false;
   int fault_words_ = 0, hit_words_ = 0;
+  unsigned int* d_passes_ = nullptr;  // passes done
+  unsigned int passes_ = 0;           // passes launched
   unsigned long long* d_fetch_ = nullptr;
   int32_t* h_unique_ = nullptr;      // mapped pinned
   int32_t* d_unique_ = nullptr;
-  int* h_counts_ = nullptr;          // mapped pinned: unique count, fault count, rays faulted
-  int* d_counts_ = nullptr;
+  UniqueResult* h_result_ = nullptr;  // mapped pinned
+  UniqueResult* d_result_ = nullptr;
   int32_t* h_dense_ = nullptr;       // pinned, for recording
   uint8_t* d_flush_ = nullptr;       // L2 flush buffer for TimePass
   // Host delivery of the image (one view): the caller's page-locked buffer,
@@ -98,25 +103,28 @@ class Renderer {
   uchar4* host_img_dev_ = nullptr;
   cudaStream_t copy_s_ = nullptr;
   cudaEvent_t copy_ev_[2] = {};
-  cudaEvent_t ev_[8] = {};
+  cudaEvent_t ev_[2] = {};           // TimePass
   std::vector<std::vector<int32_t>> pass_words_;
   FeedbackDecoder fb_;
 
-  int* block(int k) const { return k ? d_state_ + kBlockInts + fault_words_ + hit_words_ : d_state_; }
+  PassState* words(int par) const { return reinterpret_cast<PassState*>(d_state_) + par; }
+  uint32_t* fault_bits() const { return reinterpret_cast<uint32_t*>(d_state_ + 2 * kPassInts); }
+  uint32_t* hit_bits() const { return fault_bits() + fault_words_; }
   int SetViews(const float* m);
   TraceParams Params(int it) const;
   int Grid(bool count) const;
-  int Prepare(int it);
+  int ClearState();
   int Trace(int it, bool count, int rays);
+  void FirstPassGroup(int g, TraceParams* p) const;
   UniqueFromBitsParams UniqueParams(int it) const;
   int RunPass(int it, int rays, int* launches);
-  int PassGraph(int kind, int it, int rays);
+  int PassGraph(int it, int rays);
   int groups() const { return (int)group_tiles_.size(); }
 
-  // One pass's device work (clear feedback state, traversal, unique) as a
-  // graph: kind 0 = first pass, 1 and 2 = later passes writing list 1 and 0.
-  // The first pass's traversal nodes get the frame's view matrices before
-  // every replay; later passes replay unchanged.
+  // One pass's device work (traversal, unique) as a graph: kind 0 and 1 = first
+  // passes counting into words(0) and words(1), 2 and 3 = later ones.  The
+  // first pass's traversal nodes get the frame's view matrices before every
+  // replay; later passes replay unchanged but for their grid.
   struct Graph {
     cudaGraph_t graph = nullptr;  // kept: node handles refer to it
     cudaGraphExec_t exec = nullptr;
@@ -126,7 +134,7 @@ class Renderer {
     unsigned blocks = 0;  // later passes: the traversal node's grid
     int lanes = 0;        // and rays per warp now
   };
-  Graph graphs_[3];
+  Graph graphs_[4];
   void DropGraphs();
 };
 
@@ -163,9 +171,10 @@ Renderer::~Renderer() {
   cudaFree(d_dense_);
   cudaFree(d_state_);
   cudaFree(d_fetch_);
+  cudaFree(d_passes_);
   cudaFree(d_flush_);
   cudaFreeHost(h_unique_);
-  cudaFreeHost(h_counts_);
+  cudaFreeHost(h_result_);
   cudaFreeHost(h_dense_);
   for (auto& e : ev_)
     if (e) cudaEventDestroy(e);
@@ -204,13 +213,15 @@ int Renderer::Init(Cache* cache, int n_views, const int* widths, const int* heig
   fault_words_ = (int)((cache->tree_blocks() + 31) / 32);
   hit_words_ = (int)(((uint64_t)cache->max_blocks() * 2 + 31) / 32);
   const size_t bit_words = (size_t)fault_words_ + hit_words_;
-  if (cudaMalloc(&d_state_, (bit_words + 2 * kBlockInts) * 4) != cudaSuccess)
+  state_ints_ = 2 * (size_t)kPassInts + bit_words;
+  if (cudaMalloc(&d_state_, state_ints_ * 4) != cudaSuccess || cudaMalloc(&d_passes_, 4) != cudaSuccess)
     return fail(RAYT_E_OOM, "feedback bitmap allocation failed");
   if (cudaHostAlloc(&h_unique_, (bit_words * 32 + 1) * 4, cudaHostAllocMapped) != cudaSuccess ||
-      cudaHostAlloc(&h_counts_, 4 * 4, cudaHostAllocMapped) != cudaSuccess)
+      cudaHostAlloc(&h_result_, sizeof(UniqueResult), cudaHostAllocMapped) != cudaSuccess)
     return fail(RAYT_E_OOM, "pinned host allocation failed");
   RAYT_CUDA_TRY(cudaHostGetDevicePointer((void**)&d_unique_, h_unique_, 0));
-  RAYT_CUDA_TRY(cudaHostGetDevicePointer((void**)&d_counts_, h_counts_, 0));
+  std::memset(h_result_, 0, sizeof(UniqueResult));
+  RAYT_CUDA_TRY(cudaHostGetDevicePointer((void**)&d_result_, h_result_, 0));
   for (auto& e : ev_) RAYT_CUDA_TRY(cudaEventCreate(&e));
   // the views' normalised pixel coordinates (they depend only on the sizes)
   std::vector<size_t> coord_at(n_views);
@@ -225,7 +236,8 @@ int Renderer::Init(Cache* cache, int n_views, const int* widths, const int* heig
   RAYT_CUDA_TRY(cudaMemcpy(d_coords_, coords.data(), coords.size() * sizeof(float), cudaMemcpyHostToDevice));
   for (int v = 0; v < n_views; ++v) views_[v].coords = d_coords_ + coord_at[v];
   RAYT_CUDA_TRY(cudaMemsetAsync(d_images_, 0, (size_t)padded * 4, s_));
-  RAYT_CUDA_TRY(cudaMemsetAsync(d_state_, 0, (bit_words + 2 * kBlockInts) * 4, s_));
+  RAYT_CUDA_TRY(cudaMemsetAsync(d_state_, 0, state_ints_ * 4, s_));
+  RAYT_CUDA_TRY(cudaMemsetAsync(d_passes_, 0, 4, s_));
   RAYT_CUDA_TRY(cudaStreamSynchronize(s_));
   return RAYT_OK;
 }
@@ -257,7 +269,7 @@ int Renderer::SetViews(const float* m) {
 }
 
 TraceParams Renderer::Params(int it) const {
-  const int k = it & 1;
+  const int k = par_;
   TraceParams p;
   std::memset(&p, 0, sizeof(p));
   p.links = cache_->links();
@@ -284,24 +296,24 @@ TraceParams Renderer::Params(int it) const {
   p.in_dir = in.dir;
   p.in_parent = in.parent;
   p.in_ray = in.ray;
-  p.n_in = block(1 - k) + 1;
+  p.n_in = &words(1 - k)->rays;
   p.out_origin = out.origin;
   p.out_dir = out.dir;
   p.out_parent = out.parent;
   p.out_ray = out.ray;
-  p.n_out = block(k) + 1;
   if (depth_out_) {
     p.depth = d_depth_;
     p.hit_node = d_hit_;
     p.in_adv = in.adv;
     p.out_adv = out.adv;
   }
-  p.fault_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts);
+  p.fault_bits = fault_bits();
   p.fault_bit_limit = (int)cache_->tree_blocks();
-  p.hit_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts + fault_words_);
-  p.no_word = block(k) + 16;
+  p.hit_bits = hit_bits();
+  p.words = words(k);
+  p.stamp = true;
   p.lanes = 32;
-  p.work = block(k) + 4;
+  p.work = words(k)->work;
   p.refill = refill;
   p.step_budget = step_budget;
   return p;
@@ -317,11 +329,13 @@ int Renderer::Grid(bool count) const {
 }
 
 
-// Clears pass `it`'s block and the feedback bitmaps (one contiguous range).
-int Renderer::Prepare(int it) {
-  const size_t words = kBlockInts + (size_t)fault_words_ + hit_words_;
-  RAYT_CUDA_TRY(cudaMemsetAsync((it & 1) ? d_state_ + kBlockInts : d_state_, 0, words * 4, s_));
-  if (record) RAYT_CUDA_TRY(launch_fill_i32(d_dense_, kNoHit, (size_t)padded_pixels_, s_));
+// Clears the whole tracing state and starts the passes' numbers again.
+int Renderer::ClearState() {
+  RAYT_CUDA_TRY(cudaStreamSynchronize(s_));  // nothing publishes a number any more
+  RAYT_CUDA_TRY(cudaMemsetAsync(d_state_, 0, state_ints_ * 4, s_));
+  RAYT_CUDA_TRY(cudaMemsetAsync(d_passes_, 0, 4, s_));
+  h_result_->pass = passes_ = 0;
+  dirty_ = false;
   return RAYT_OK;
 }
 
@@ -337,37 +351,44 @@ int Renderer::Trace(int it, bool count, int rays) {
     return RAYT_OK;
   }
   for (int g = 0; g < groups(); ++g) {
-    const int first = g * kViewsPerLaunch, end = std::min(n_views(), first + kViewsPerLaunch);
-    p.n_views = end - first;
-    std::memcpy(p.views, views_.data() + first, (size_t)p.n_views * sizeof(ViewDesc));
-    p.total_tiles = group_tiles_[g];
-    p.work = block(0) + 4 + g;
-    p.lanes = trace_lanes(true, p.total_tiles * 32);
+    FirstPassGroup(g, &p);
     RAYT_CUDA_TRY(launch_trace(p, true, count, group_tiles_[g] * 32, grid, s_));
   }
   return RAYT_OK;
 }
 
+// The first-pass parameters of launch group g: its views and tiles.
+void Renderer::FirstPassGroup(int g, TraceParams* p) const {
+  const int first = g * kViewsPerLaunch, end = std::min(n_views(), first + kViewsPerLaunch);
+  p->n_views = end - first;
+  std::memcpy(p->views, views_.data() + first, (size_t)p->n_views * sizeof(ViewDesc));
+  p->total_tiles = group_tiles_[g];
+  p->work = words(par_)->work + g;
+  p->stamp = g == 0;
+  p->lanes = trace_lanes(true, p->total_tiles * 32);
+}
+
 UniqueFromBitsParams Renderer::UniqueParams(int it) const {
   UniqueFromBitsParams q{};
-  q.fault_bits = reinterpret_cast<const uint32_t*>(d_state_ + kBlockInts);
+  q.fault_bits = fault_bits();
   q.fault_words = fault_words_;
-  q.hit_bits = reinterpret_cast<const uint32_t*>(d_state_ + kBlockInts + fault_words_);
+  q.hit_bits = hit_bits();
   q.hit_words = hit_words_;
-  q.no_word = block(it & 1) + 16;
-  q.n_in = it > 0 ? block(1 - (it & 1)) + 1 : nullptr;
-  q.n_rays = block(it & 1) + 1;
+  q.words = words(par_);
+  q.previous = words(1 - par_);
+  q.later = it > 0;
   q.total_pixels = total_pixels_;
+  q.passes = d_passes_;
   q.unique_out = d_unique_;
-  q.counts_out = d_counts_;
+  q.result = d_result_;
   return q;
 }
 
 // Builds (when missing or when the pass parameters changed) and updates the
-// graph of pass kind `kind`, then launches it.  Events 1 (after traversal)
-// and 2 (after unique) are recorded inside the graph.
-int Renderer::PassGraph(int kind, int it, int rays) {
-  Graph& g = graphs_[kind];
+// graph of pass `it`, then launches it.
+int Renderer::PassGraph(int it, int rays) {
+  const bool first = it == 0;
+  Graph& g = graphs_[(first ? 0 : 2) + par_];
   TraceParams key = Params(it);
   if (g.exec && (std::memcmp(&key, &g.key, sizeof(key)) != 0 || g.ctas != ctas_per_sm)) {
     cudaGraphExecDestroy(g.exec);
@@ -376,57 +397,38 @@ int Renderer::PassGraph(int kind, int it, int rays) {
     g.graph = nullptr;
     g.trace_nodes.clear();
   }
-  const bool first = kind == 0;
-  // per launch group (first pass) or one (later passes): parameters with views
-  std::vector<TraceParams> tp(first ? groups() : 1, key);
-  if (first) {
-    for (int grp = 0; grp < groups(); ++grp) {
-      TraceParams& p = tp[grp];
-      const int v0 = grp * kViewsPerLaunch, v1 = std::min(n_views(), v0 + kViewsPerLaunch);
-      p.n_views = v1 - v0;
-      std::memcpy(p.views, views_.data() + v0, (size_t)p.n_views * sizeof(ViewDesc));
-      p.total_tiles = group_tiles_[grp];
-      p.work = block(0) + 4 + grp;
-      p.lanes = trace_lanes(true, p.total_tiles * 32);
-    }
-  } else {
-    tp[0].lanes = trace_lanes(false, rays);
-  }
   const int grid = refill < 32 ? Grid(false) : 0;
-  void* args[1];
-  cudaKernelNodeParams kp;
-  if (!g.exec) {
-    cudaGraph_t graph;
-    RAYT_CUDA_TRY(cudaGraphCreate(&graph, 0));
-    cudaGraphNode_t prev = nullptr, node = nullptr;
-    cudaMemsetParams mp{};
-    mp.dst = (it & 1) ? d_state_ + kBlockInts : d_state_;
-    mp.value = 0;
-    mp.elementSize = 4;
-    mp.width = kBlockInts + (size_t)fault_words_ + hit_words_;
-    mp.height = 1;
-    cudaError_t e = cudaGraphAddMemsetNode(&node, graph, nullptr, 0, &mp);
-    prev = node;
-    for (size_t i = 0; e == cudaSuccess && i < tp.size(); ++i) {
-      trace_node_params(&tp[i], first, false, first ? group_tiles_[i] * 32 : rays, grid, args, &kp);
-      g.blocks = kp.gridDim.x;
-      g.lanes = tp[i].lanes;
-      e = cudaGraphAddKernelNode(&node, graph, &prev, 1, &kp);
+  TraceLaunch l;
+  cudaGraph_t graph = g.graph;
+  cudaGraphNode_t prev = nullptr, node = nullptr;
+  cudaError_t e = cudaSuccess;
+  const bool build = !g.exec;
+  if (build) e = cudaGraphCreate(&graph, 0);
+  // traversal: one node per launch group (first pass) or one
+  for (int i = 0; e == cudaSuccess && i < (first ? groups() : 1); ++i) {
+    TraceParams p = key;
+    if (first) FirstPassGroup(i, &p);
+    else p.lanes = trace_lanes(false, rays);
+    trace_node_params(&p, first, false, first ? group_tiles_[i] * 32 : rays, grid, &l);
+    if (build) {
+      e = cudaGraphAddKernelNode(&node, graph, prev ? &prev : nullptr, prev ? 1 : 0, &l.kp);
       g.trace_nodes.push_back(node);
       prev = node;
+    } else if (first || l.kp.gridDim.x != g.blocks || p.lanes != g.lanes) {  // a later pass follows its ray count
+      e = cudaGraphExecKernelNodeSetParams(g.exec, g.trace_nodes[i], &l.kp);
     }
-    if (e == cudaSuccess) e = cudaGraphAddEventRecordNode(&node, graph, &prev, 1, ev_[1]);
-    prev = node;
+    g.blocks = l.kp.gridDim.x;
+    g.lanes = p.lanes;
+  }
+  if (build) {
     const UniqueFromBitsParams q = UniqueParams(it);
     if (e == cudaSuccess) {
-      unique_node_params(&q, args, &kp);
-      e = cudaGraphAddKernelNode(&node, graph, &prev, 1, &kp);
-      prev = node;
+      unique_node_params(&q, l.args, &l.kp);
+      e = cudaGraphAddKernelNode(&node, graph, &prev, 1, &l.kp);
     }
-    if (e == cudaSuccess) e = cudaGraphAddEventRecordNode(&node, graph, &prev, 1, ev_[2]);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
     if (e != cudaSuccess) {
-      cudaGraphDestroy(graph);
+      if (graph) cudaGraphDestroy(graph);
       g.exec = nullptr;
       g.trace_nodes.clear();
       return cuda_fail(e, "pass graph construction");
@@ -434,44 +436,27 @@ int Renderer::PassGraph(int kind, int it, int rays) {
     g.graph = graph;
     g.key = key;
     g.ctas = ctas_per_sm;
-  } else if (first) {
-    for (size_t i = 0; i < tp.size(); ++i) {
-      trace_node_params(&tp[i], true, false, group_tiles_[i] * 32, grid, args, &kp);
-      RAYT_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g.exec, g.trace_nodes[i], &kp));
-    }
-  } else {
-    // a later pass's grid and rays per warp follow its ray count
-    trace_node_params(&tp[0], false, false, rays, grid, args, &kp);
-    if (kp.gridDim.x != g.blocks || tp[0].lanes != g.lanes) {
-      RAYT_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g.exec, g.trace_nodes[0], &kp));
-      g.blocks = kp.gridDim.x;
-      g.lanes = tp[0].lanes;
-    }
   }
+  RAYT_CUDA_TRY(e);
   RAYT_CUDA_TRY(cudaGraphLaunch(g.exec, s_));
   return RAYT_OK;
 }
 
 // The device work of pass `it` over `rays` rays (traversal and feedback
-// unique, with events 0..2 around them); adds the kernels it launched.
+// unique); adds the kernels it launched.
 int Renderer::RunPass(int it, int rays, int* launches) {
-  RAYT_CUDA_TRY(cudaEventRecord(ev_[0], s_));
-  if (use_graphs && !record) {
-    int rc = PassGraph(it == 0 ? 0 : ((it & 1) ? 1 : 2), it, rays);
-    if (rc != RAYT_OK) return rc;
-    *launches += (it == 0 ? groups() : 1) + 1;
-    return RAYT_OK;
+  int rc = RAYT_OK;
+  if (dirty_ && (rc = ClearState()) != RAYT_OK) return rc;
+  dirty_ = true;  // until the pass's result is here
+  ++passes_;
+  *launches += (it == 0 ? groups() : 1) + 1;
+  if (use_graphs && !record) return PassGraph(it, rays);
+  if (record) {
+    RAYT_CUDA_TRY(launch_fill_i32(d_dense_, kNoHit, (size_t)padded_pixels_, s_));
+    ++*launches;
   }
-  int rc = Prepare(it);
-  if (rc != RAYT_OK) return rc;
-  if (it == 0 || rays > 0) {
-    if ((rc = Trace(it, false, rays)) != RAYT_OK) return rc;
-    *launches += it == 0 ? groups() : 1;
-  }
-  RAYT_CUDA_TRY(cudaEventRecord(ev_[1], s_));
+  if ((rc = Trace(it, false, rays)) != RAYT_OK) return rc;
   RAYT_CUDA_TRY(launch_unique_from_bits(UniqueParams(it), s_));
-  *launches += 1 + (record ? 1 : 0);
-  RAYT_CUDA_TRY(cudaEventRecord(ev_[2], s_));
   return RAYT_OK;
 }
 
@@ -490,6 +475,8 @@ int Renderer::Frame(const float* m) {
   if (rc != RAYT_OK) return rc;
   rc = cache_->StartSession();
   if (rc != RAYT_OK) return rc;
+  dirty_ = dirty_ || in_frame_;  // the last frame ended with an error
+  in_frame_ = true;
   const int total = total_pixels_;
   int active_prev = total;  // rays traced by the first pass
   float ms_trace = 0, ms_fb = 0, ms_up = 0;
@@ -497,7 +484,9 @@ int Renderer::Frame(const float* m) {
   auto ms_since = [](clock::time_point a) { return std::chrono::duration<double, std::milli>(clock::now() - a).count(); };
   int it;
   bool copy_pending = false;  // the first pass's pixels on their way to the host image
+  int64_t launches_seen = launches0;  // the cache's launches before the last pass
   for (it = 0;; ++it) {
+    if (it > 0) par_ ^= 1;
     if (it > 0 && copy_pending) {  // later passes write host pixels only after the copy
       RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, copy_ev_[1], 0));
       copy_pending = false;
@@ -518,13 +507,13 @@ int Renderer::Frame(const float* m) {
       RAYT_CUDA_TRY(cudaMemcpyAsync(h_dense_, d_dense_, (size_t)padded_pixels_ * 4, cudaMemcpyDeviceToHost, s_));
     }
     const auto tw = clock::now();
-    RAYT_CUDA_TRY(cudaStreamSynchronize(s_));
+    launches_seen = cache_->launches();
+    if (record) RAYT_CUDA_TRY(cudaStreamSynchronize(s_));  // the words' copy too
+    if ((rc = wait_pass(h_result_, passes_, s_)) != RAYT_OK) break;
+    dirty_ = false;
     stats.host_ms_wait += ms_since(tw);
-    float a = 0, b = 0;
-    cudaEventElapsedTime(&a, ev_[0], ev_[1]);
-    cudaEventElapsedTime(&b, ev_[1], ev_[2]);
-    ms_trace += a;
-    ms_fb += b;
+    ms_trace += h_result_->trace_ms;
+    ms_fb += h_result_->unique_ms;
     stats.rays_traced += active_prev;
     if (record) {  // views in order, without the padding between them
       pass_words_.emplace_back();
@@ -532,8 +521,8 @@ int Renderer::Frame(const float* m) {
         pass_words_.back().insert(pass_words_.back().end(), h_dense_ + v.pix_base,
                                   h_dense_ + v.pix_base + (size_t)v.width * v.height);
     }
-    const int active_now = h_counts_[2];
-    d2h += 3 * 4 + (int64_t)h_counts_[0] * 4;  // counts, unique array (mapped reads)
+    const int active_now = h_result_->rays;
+    d2h += 3 * 4 + (int64_t)h_result_->unique * 4;  // counts, unique array (mapped reads)
 
     // the reference always gives the frame one round of loading, then stops
     // on its wall-clock limit (gpu-ray-tracer.cpp:123-125)
@@ -542,7 +531,7 @@ int Renderer::Frame(const float* m) {
     if (max_passes > 0 && it > 0 && it + 1 >= max_passes) { active_prev = active_now; break; }
 
     const auto td = clock::now();
-    fb_.Decode(h_unique_, h_counts_[0], rand);
+    fb_.Decode(h_unique_, h_result_->unique, rand);
     if ((rc = cache_->StartTransaction((int)fb_.faults.size())) != RAYT_OK) break;
     cache_->MarkUsedBatch(fb_.hits, fb_.dup_hits);
     for (int f : fb_.faults) {
@@ -573,20 +562,26 @@ int Renderer::Frame(const float* m) {
   if (src != RAYT_OK) return src;
   // FinishTracingFrame for the rays still faulted, against the cache as it is now
   const TraceParams p = Params(it);
-  TraceParams f = p;
+  TraceCore f = p;
   f.in_origin = p.out_origin;
   f.in_dir = p.out_dir;
   f.in_parent = p.out_parent;
   f.in_ray = p.out_ray;
   f.in_adv = p.out_adv;
-  f.n_in = p.n_out;
+  f.n_in = &p.words->rays;
   f.host_image = host_img_dev_;
-  if (copy_pending) RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, copy_ev_[1], 0));  // also ends with the copy
-  RAYT_CUDA_TRY(launch_finish(f, active_prev, s_));
-  if (active_prev > 0) ++launches;
   const auto tw = clock::now();
-  RAYT_CUDA_TRY(cudaStreamSynchronize(s_));
+  if (active_prev > 0 || cache_->launches() != launches_seen) {
+    if (copy_pending) RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, copy_ev_[1], 0));  // also ends with the copy
+    RAYT_CUDA_TRY(launch_finish(f, active_prev, s_));
+    if (active_prev > 0) ++launches;
+    RAYT_CUDA_TRY(cudaStreamSynchronize(s_));
+  } else if (copy_pending) {  // nothing was queued after the last pass, which is done
+    RAYT_CUDA_TRY(cudaEventSynchronize(copy_ev_[1]));
+  }
   stats.host_ms_wait += ms_since(tw);
+  par_ ^= 1;
+  in_frame_ = false;
   ms_up += cache_->TakeUploadMs();  // every batch the frame's transactions flushed
   stats.gpu_ms_trace = ms_trace;
   stats.gpu_ms_feedback = ms_fb;
@@ -601,8 +596,9 @@ int Renderer::Frame(const float* m) {
 
 int Renderer::CountFetches(const float* m, int64_t* counts) {
   int rc = SetViews(m);
-  if (rc == RAYT_OK) rc = Prepare(0);
+  if (rc == RAYT_OK) rc = ClearState();
   if (rc != RAYT_OK) return rc;
+  dirty_ = true;
   RAYT_CUDA_TRY(cudaMemsetAsync(d_fetch_, 0, 8 * 8, s_));
   if ((rc = Trace(0, true, 0)) != RAYT_OK) return rc;
   unsigned long long h[8];
@@ -622,13 +618,14 @@ int Renderer::TimePass(const float* m, int reps, float* ms) {
   float total = 0;
   for (int r = 0; r < reps; ++r) {
     RAYT_CUDA_TRY(cudaMemsetAsync(d_flush_, r & 255, flush, s_));
-    if ((rc = Prepare(0)) != RAYT_OK) return rc;
-    RAYT_CUDA_TRY(cudaEventRecord(ev_[5], s_));
+    if ((rc = ClearState()) != RAYT_OK) return rc;
+    dirty_ = true;
+    RAYT_CUDA_TRY(cudaEventRecord(ev_[0], s_));
     if ((rc = Trace(0, false, 0)) != RAYT_OK) return rc;
-    RAYT_CUDA_TRY(cudaEventRecord(ev_[6], s_));
-    RAYT_CUDA_TRY(cudaEventSynchronize(ev_[6]));
+    RAYT_CUDA_TRY(cudaEventRecord(ev_[1], s_));
+    RAYT_CUDA_TRY(cudaEventSynchronize(ev_[1]));
     float a = 0;
-    RAYT_CUDA_TRY(cudaEventElapsedTime(&a, ev_[5], ev_[6]));
+    RAYT_CUDA_TRY(cudaEventElapsedTime(&a, ev_[0], ev_[1]));
     total += a;
   }
   *ms = reps > 0 ? total / reps : 0.0f;
@@ -932,7 +929,7 @@ int rayt_cache_depth_view(rayt_cache* cache, const float view_proj_inv[16], floa
   if (width <= 0 || height <= 0 || (int64_t)width * height >= (1ll << 31) || !(lod_voxel_size >= 0))
     return fail(RAYT_E_ARG, "rayt_cache_depth_view: bad size or LOD");
   rayt::Cache* c = reinterpret_cast<rayt::Cache*>(cache);
-  rayt::TraceParams p;
+  rayt::TraceParams1 p;
   std::memset(&p, 0, sizeof(p));
   p.links = c->links();
   p.far_ptrs = c->far_ptrs();

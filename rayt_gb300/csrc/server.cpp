@@ -61,7 +61,6 @@ class Server {
   LibcRand rand;
 
  private:
-  static constexpr int kBlockInts = kPassBlockInts;
   struct Client {
     bool live = false;
     int w = 0, h = 0;
@@ -96,12 +95,19 @@ class Server {
   int64_t image_pixels_ = 0;
   RayList lists_[2];
   int64_t list_cap_ = 0, reserved_ = 0;
-  int* d_state_ = nullptr;  // [block 0][fault bits][hit bits][block 1][client faults]
+  // two PassStates, fault bits, hit bits, client faults; a tick counts into
+  // words(tick_ & 1) and leaves the rest zero (see PassState); dirty_ while that
+  // does not hold (a failed tick)
+  int* d_state_ = nullptr;
+  size_t state_ints_ = 0;
+  bool dirty_ = false;
+  unsigned int* d_passes_ = nullptr;  // passes done
+  unsigned int passes_ = 0;           // passes launched
   int fault_words_ = 0, hit_words_ = 0;
   int32_t* h_unique_ = nullptr;
   int32_t* d_unique_ = nullptr;
-  int* h_counts_ = nullptr;  // mapped: unique count, fault count, rays faulted, client faults [kMaxClients]
-  int* d_counts_ = nullptr;
+  UniqueResult* h_result_ = nullptr;  // mapped
+  UniqueResult* d_result_ = nullptr;
   int* d_client_faults_ = nullptr;
   int tick_ = 0;
   int carried_ = 0;          // faulted rays carried into the next tick
@@ -131,7 +137,9 @@ class Server {
   bool running_ = false, stop_ = false;
   int thread_rc_ = RAYT_OK;
 
-  int* block(int k) const { return k ? d_state_ + kBlockInts + fault_words_ + hit_words_ : d_state_; }
+  PassState* words(int k) const { return reinterpret_cast<PassState*>(d_state_) + k; }
+  uint32_t* fault_bits() const { return reinterpret_cast<uint32_t*>(d_state_ + 2 * kPassInts); }
+  uint32_t* hit_bits() const { return fault_bits() + fault_words_; }
   int Alloc(int64_t pixels, int64_t* base) const;
   TraceParams Params(int k) const;
   void Loop();
@@ -156,16 +164,19 @@ int Server::Init(Cache* cache, const rayt_server_config& cfg) {
       return fail(RAYT_E_OOM, "ray record allocation failed");
   fault_words_ = (int)((cache->tree_blocks() + 31) / 32);
   hit_words_ = (int)(((uint64_t)cache->max_blocks() * 2 + 31) / 32);
-  const size_t words = 2 * kBlockInts + (size_t)fault_words_ + hit_words_ + kMaxClients;
-  if (cudaMalloc(&d_state_, words * 4) != cudaSuccess) return fail(RAYT_E_OOM, "feedback state allocation failed");
-  d_client_faults_ = d_state_ + 2 * kBlockInts + fault_words_ + hit_words_;
+  state_ints_ = 2 * (size_t)kPassInts + (size_t)fault_words_ + hit_words_ + kMaxClients;
+  if (cudaMalloc(&d_state_, state_ints_ * 4) != cudaSuccess || cudaMalloc(&d_passes_, 4) != cudaSuccess)
+    return fail(RAYT_E_OOM, "feedback state allocation failed");
+  d_client_faults_ = d_state_ + state_ints_ - kMaxClients;
   const size_t bit_words = (size_t)fault_words_ + hit_words_;
   if (cudaHostAlloc(&h_unique_, (bit_words * 32 + 1) * 4, cudaHostAllocMapped) != cudaSuccess ||
-      cudaHostAlloc(&h_counts_, (4 + kMaxClients) * 4, cudaHostAllocMapped) != cudaSuccess)
+      cudaHostAlloc(&h_result_, sizeof(UniqueResult), cudaHostAllocMapped) != cudaSuccess)
     return fail(RAYT_E_OOM, "pinned host allocation failed");
   RAYT_CUDA_TRY(cudaHostGetDevicePointer((void**)&d_unique_, h_unique_, 0));
-  RAYT_CUDA_TRY(cudaHostGetDevicePointer((void**)&d_counts_, h_counts_, 0));
-  RAYT_CUDA_TRY(cudaMemsetAsync(d_state_, 0, words * 4, s_));
+  std::memset(h_result_, 0, sizeof(UniqueResult));
+  RAYT_CUDA_TRY(cudaHostGetDevicePointer((void**)&d_result_, h_result_, 0));
+  RAYT_CUDA_TRY(cudaMemsetAsync(d_state_, 0, state_ints_ * 4, s_));
+  RAYT_CUDA_TRY(cudaMemsetAsync(d_passes_, 0, 4, s_));
   RAYT_CUDA_TRY(cudaMemsetAsync(d_images_, 0, image_pixels_ * 4, s_));
   if (cfg.deliver_to_host) {
     RAYT_CUDA_TRY(cudaStreamCreateWithFlags(&copy_s_, cudaStreamNonBlocking));
@@ -193,8 +204,9 @@ Server::~Server() {
     cudaFree(l.ray);
   }
   cudaFree(d_state_);
+  cudaFree(d_passes_);
   cudaFreeHost(h_unique_);
-  cudaFreeHost(h_counts_);
+  cudaFreeHost(h_result_);
   for (auto& c : clients_) {
     if (c.host) cudaFreeHost(c.host);
     cudaFree(c.stage);
@@ -329,16 +341,15 @@ TraceParams Server::Params(int k) const {
   p.in_dir = in.dir;
   p.in_parent = in.parent;
   p.in_ray = in.ray;
-  p.n_in = block(1 - k) + 1;
+  p.n_in = &words(1 - k)->rays;
   p.out_origin = out.origin;
   p.out_dir = out.dir;
   p.out_parent = out.parent;
   p.out_ray = out.ray;
-  p.n_out = block(k) + 1;
-  p.fault_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts);
+  p.fault_bits = fault_bits();
   p.fault_bit_limit = (int)cache_->tree_blocks();
-  p.hit_bits = reinterpret_cast<uint32_t*>(d_state_ + kBlockInts + fault_words_);
-  p.no_word = block(k) + 16;
+  p.hit_bits = hit_bits();
+  p.words = words(k);
   p.lanes = 32;
   p.refill = 32;
   p.restart = 1;
@@ -389,10 +400,14 @@ int Server::Step(int* finished) {
   for (int i = 0; i < p.n_clients; ++i)
     for (int c = 0; c < (int)clients_.size(); ++c)
       if (clients_[c].live && clients_[c].base == p.client_base[i]) slot_of_client[c] = i;
-  // clear this tick's block, the bitmaps and the client fault counters
-  RAYT_CUDA_TRY(cudaMemsetAsync(k ? d_state_ + kBlockInts : d_state_, 0,
-                                (kBlockInts + (size_t)fault_words_ + hit_words_) * 4, s_));
-  RAYT_CUDA_TRY(cudaMemsetAsync(d_client_faults_, 0, kMaxClients * 4, s_));
+  if (dirty_) {  // start clean, and the ticks' numbers again
+    RAYT_CUDA_TRY(cudaStreamSynchronize(s_));
+    RAYT_CUDA_TRY(cudaMemsetAsync(d_state_, 0, state_ints_ * 4, s_));
+    RAYT_CUDA_TRY(cudaMemsetAsync(d_passes_, 0, 4, s_));
+    h_result_->pass = passes_ = 0;
+  }
+  dirty_ = true;  // until the tick's result is here
+  bool stamped = false;  // the tick's first traversal launch notes when it began
   int64_t rays_tick = carried_;
   // first passes of newly admitted requests (one launch per 64 views)
   std::vector<ViewDesc> views;
@@ -423,6 +438,8 @@ int Server::Step(int* finished) {
     }
     q.n_views = n;
     q.total_tiles = (int)tiles;
+    q.stamp = !stamped;
+    stamped = true;
     q.lanes = trace_lanes(true, (int)tiles * 32);
     RAYT_CUDA_TRY(launch_trace(q, true, false, (int)tiles * 32, 0, s_));
     ++stats.kernel_launches;
@@ -433,6 +450,7 @@ int Server::Step(int* finished) {
     for (const Flight& f : flights_)
       if (!f.fresh && f.finishing) q.finish_mask |= 1ull << slot_of_client[f.client];
     q.lanes = trace_lanes(false, carried_);
+    q.stamp = !stamped;
     RAYT_CUDA_TRY(launch_trace(q, false, false, carried_, 0, s_));
     ++stats.kernel_launches;
   }
@@ -441,28 +459,32 @@ int Server::Step(int* finished) {
   u.fault_words = fault_words_;
   u.hit_bits = p.hit_bits;
   u.hit_words = hit_words_;
-  u.no_word = p.no_word;
-  u.n_rays = p.n_out;
+  u.words = words(k);
+  u.previous = words(1 - k);
   u.total_pixels = (int)std::min<int64_t>(rays_tick, 1 << 30);
+  u.client_faults = d_client_faults_;
+  u.passes = d_passes_;
   u.unique_out = d_unique_;
-  u.counts_out = d_counts_;
+  u.result = d_result_;
   RAYT_CUDA_TRY(launch_unique_from_bits(u, s_));
+  ++passes_;
   ++stats.kernel_launches;
-  RAYT_CUDA_TRY(cudaMemcpyAsync(h_counts_ + 4, d_client_faults_, kMaxClients * 4, cudaMemcpyDeviceToHost, s_));
   const double t_sync = now_s();
-  RAYT_CUDA_TRY(cudaStreamSynchronize(s_));
+  const int wrc = wait_pass(h_result_, passes_, s_);
+  if (wrc != RAYT_OK) return wrc;
+  dirty_ = false;
   const double t_pass = now_s();
   stats.host_ms_wait += (t_pass - t_sync) * 1e3;
   stats.gpu_ms_upload += cache_->TakeUploadMs();  // the previous tick's block uploads
   stats.rays_traced += rays_tick;
   ++stats.ticks;
-  carried_ = h_counts_[2];
+  carried_ = h_result_->rays;
 
   // which requests end with this tick
   std::vector<Flight> ended;
   std::vector<Flight> kept;
   for (Flight& f : flights_) {
-    const int faults = h_counts_[4 + slot_of_client[f.client]];
+    const int faults = h_result_->client_faults[slot_of_client[f.client]];
     if (f.finishing) {  // its rays were shaded this tick
       ended.push_back(f);
       continue;
@@ -478,7 +500,7 @@ int Server::Step(int* finished) {
 
   // feedback decode and the cache transaction (shared LRU, block streaming)
   const int64_t uploaded0 = cache_->stats().uploaded_blocks;
-  fb_.Decode(h_unique_, h_counts_[0], rand);
+  fb_.Decode(h_unique_, h_result_->unique, rand);
   int rc = cache_->StartSession();
   if (rc == RAYT_OK) rc = cache_->StartTransaction((int)fb_.faults.size());
   if (rc == RAYT_OK) {
@@ -500,7 +522,10 @@ int Server::Step(int* finished) {
     const int src = cache_->EndSession();
     if (rc == RAYT_OK) rc = src;
   }
-  if (rc != RAYT_OK) return rc;
+  if (rc != RAYT_OK) {
+    dirty_ = true;  // tick_ stays, and this tick has counted into its state
+    return rc;
+  }
   if (filled)  // the cache cannot hold this tick's blocks: stop the requests that still fault
     for (Flight& f : kept) f.finishing = true;
   stats.faults += (int64_t)fb_.faults.size();

@@ -46,6 +46,12 @@ constexpr int kIterLimit = 300;
 constexpr int kBlockThreads = 128;
 constexpr unsigned kFull = 0xffffffffu;
 
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
 __device__ __forceinline__ float dot4(float ax, float ay, float az, float aw, float bx, float by, float bz, float bw) {
   float r = ax * bx;
   r = r + ay * by;
@@ -168,7 +174,7 @@ struct RayEnd {
 // kBias: the ray may have an LOD bias (origins that were advanced, the depth
 // view); first-pass rays start with a bias of zero.
 template <bool kCount, bool kBias>
-__device__ __forceinline__ RayEnd cast_ray(const TraceParams& p, float4 o, float4 d, uint32_t& fetches,
+__device__ __forceinline__ RayEnd cast_ray(const TraceCore& p, float4 o, float4 d, uint32_t& fetches,
                                            uint32_t& far_fetches) {
   RayEnd r;
   r.fault_block = -1;
@@ -335,7 +341,7 @@ __device__ __forceinline__ RayEnd cast_ray(const TraceParams& p, float4 o, float
 // levels reaches (the reference reads and writes past its stack there).  So
 // every stack index stays in [0, 22].
 template <bool kCount, bool kBudget>
-__device__ __forceinline__ int cast_run(Cast& c, int stop, uint2* stack, const TraceParams& p, uint32_t& fetches,
+__device__ __forceinline__ int cast_run(Cast& c, int stop, uint2* stack, const TraceCore& p, uint32_t& fetches,
                                         uint32_t& far_fetches) {
   const float tx_coef = c.tx_coef, ty_coef = c.ty_coef, tz_coef = c.tz_coef;
   const float tx_bias = c.tx_bias, ty_bias = c.ty_bias, tz_bias = c.tz_bias;
@@ -462,7 +468,7 @@ __device__ __forceinline__ float div127(float x) {
 }
 
 // ProcessHit: fixed ambient + three directional lights; returns RGBA8 (A=255).
-__device__ __forceinline__ uchar4 shade(const TraceParams& p, uint32_t node) {
+__device__ __forceinline__ uchar4 shade(const TraceCore& p, uint32_t node) {
   const char4 cn = p.normals[node];
   // the reference's w component is 0 / 127 = +0
   const float nx = div127((float)cn.x), ny = div127((float)cn.y), nz = div127((float)cn.z), nw = 0.0f;
@@ -490,7 +496,7 @@ __device__ __forceinline__ uchar4 shade(const TraceParams& p, uint32_t node) {
 }
 
 // FinishTracingFrame's blend of the accumulated colour over the background.
-__device__ __forceinline__ uchar4 finish(const TraceParams& p, uchar4 c) {
+__device__ __forceinline__ uchar4 finish(const TraceCore& p, uchar4 c) {
   const float w = 255.f - (float)c.w;
   float t[4] = {(float)c.x + p.bg[0] * w + .5f, (float)c.y + p.bg[1] * w + .5f,
                 (float)c.z + p.bg[2] * w + .5f, (float)c.w + p.bg[3] * w + .5f};
@@ -543,14 +549,15 @@ __device__ __forceinline__ void warp_set_bit(uint32_t* bits, int bit) {
 // then ends with NO_HIT).  Only warps with such a ray touch a flag, and only
 // the first of them write it: a count of the words was one atomic per warp on
 // one address.
-__device__ __forceinline__ void mark_no_word(const TraceParams& p, bool none) {
+__device__ __forceinline__ void mark_no_word(const TraceCore& p, bool none) {
   const unsigned m = __ballot_sync(__activemask(), none);
-  int* flag = p.no_word + (blockIdx.x % kNoWordFlags) * kNoWordStride;
+  int* flag = p.words->no_word + (blockIdx.x % kNoWordFlags) * kNoWordStride;
   if (m && (int)(threadIdx.x & 31) == __ffs(m) - 1 && __ldcg(flag) == 0) *flag = 1;
 }
 
 // View of the launch holding tile `tile` (tile_base is ascending).
-__device__ __forceinline__ int view_of_tile(const TraceParams& p, int tile) {
+template <class P>
+__device__ __forceinline__ int view_of_tile(const P& p, int tile) {
   int lo = 0, hi = p.n_views - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -561,7 +568,7 @@ __device__ __forceinline__ int view_of_tile(const TraceParams& p, int tile) {
 }
 
 // Served mode: the client slot owning pixel `ray` (client_base ascending).
-__device__ __forceinline__ int slot_of(const TraceParams& p, uint32_t ray) {
+__device__ __forceinline__ int slot_of(const TraceCore& p, uint32_t ray) {
   int lo = 0, hi = p.n_clients - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -573,9 +580,10 @@ __device__ __forceinline__ int slot_of(const TraceParams& p, uint32_t ray) {
 
 // Pixel (x, y) and view of first-pass ray r (tile r / 32, lane r % 32);
 // false for the lanes of a partial tile that fall outside the view.
-__device__ __forceinline__ bool first_pass_pixel(const TraceParams& p, int r, int& v, int& x, int& y) {
+template <class P>
+__device__ __forceinline__ bool first_pass_pixel(const P& p, int r, int& v, int& x, int& y) {
   const int tile = (int)(r >> 5), k = (int)(r & 31);
-  v = view_of_tile(p, tile);
+  v = sizeof(P) == sizeof(TraceParams1) ? 0 : view_of_tile(p, tile);
   const ViewDesc& vd = p.views[v];
   const int t = tile - vd.tile_base;
   x = ((t % vd.tiles_x) << p.tile_w_log2) + (k & ((1 << p.tile_w_log2) - 1));
@@ -590,8 +598,8 @@ __device__ __forceinline__ bool first_pass_pixel(const TraceParams& p, int r, in
 // record r of the input list): its pixel, origin, direction and (depth
 // output) the distance it advanced in earlier passes; false for the lanes of
 // a partial tile that fall outside their view.
-template <bool kFirst>
-__device__ __forceinline__ bool ray_at(const TraceParams& p, int r, uint32_t& ray, float4& o, float4& d,
+template <bool kFirst, class P>
+__device__ __forceinline__ bool ray_at(const P& p, int r, uint32_t& ray, float4& o, float4& d,
                                        float& adv) {
   adv = 0.0f;
   if (kFirst) {
@@ -613,7 +621,7 @@ __device__ __forceinline__ bool ray_at(const TraceParams& p, int r, uint32_t& ra
 // the pixel shows (earlier passes' advances plus this pass's t, in float, in
 // pass order) and the cache node that shaded it.  Miss: +inf and -1; error
 // (iteration limit, corrupt cache): NaN and -2.
-__device__ __forceinline__ void write_depth(const TraceParams& p, uint32_t ray, float depth, int node) {
+__device__ __forceinline__ void write_depth(const TraceCore& p, uint32_t ray, float depth, int node) {
   p.depth[ray] = depth;
   p.hit_node[ray] = node;
 }
@@ -623,7 +631,7 @@ constexpr uint32_t kDepthInf = 0x7f800000u;
 // A final pixel: into the image, and into the caller's host image when the
 // renderer delivers one (later passes and the finish; the first pass's pixels
 // reach it by one copy).
-__device__ __forceinline__ void put_pixel(const TraceParams& p, uint32_t ray, uchar4 px) {
+__device__ __forceinline__ void put_pixel(const TraceCore& p, uint32_t ray, uchar4 px) {
   p.image[ray] = px;
   if (p.host_image) p.host_image[ray] = px;
 }
@@ -633,7 +641,7 @@ __device__ __forceinline__ void put_pixel(const TraceParams& p, uint32_t ray, uc
 // record of a faulted ray, the feedback bitmaps and counters.  Called by the
 // lanes whose rays ended, together.
 template <bool kCount>
-__device__ __forceinline__ void end_ray(const TraceParams& p, const RayEnd& e, uint32_t ray, float4 o, const float4 d,
+__device__ __forceinline__ void end_ray(const TraceCore& p, const RayEnd& e, uint32_t ray, float4 o, const float4 d,
                                         float adv, uint32_t fetches, uint32_t far_fetches) {
   const int lane = threadIdx.x & 31;
   const bool faulted = !e.error && e.fault_block != -1;
@@ -655,7 +663,7 @@ __device__ __forceinline__ void end_ray(const TraceParams& p, const RayEnd& e, u
     if (p.depth) write_depth(p, ray, adv + e.t, node);
   }
   if (p.words_dense) p.words_dense[ray] = word;
-  const int slot = warp_append(p.n_out, faulted);
+  const int slot = warp_append(&p.words->rays, faulted);
   if (faulted) {
     if (!p.restart) {  // origin moved to the fault (raytracing_pass.cl:37-41)
       o.x = o.x + d.x * e.t;
@@ -689,8 +697,9 @@ __device__ __forceinline__ void end_ray(const TraceParams& p, const RayEnd& e, u
 // that faulted in the pass before.
 // 10 CTAs per SM: at 48 registers; 9 at the 52 it would take are 3% slower on
 // 1919x1079 frames.
-template <bool kFirst, bool kCount>
-__global__ void __launch_bounds__(kBlockThreads, 10) trace_kernel(const __grid_constant__ TraceParams p) {
+template <bool kFirst, bool kCount, class P>
+__global__ void __launch_bounds__(kBlockThreads, 10) trace_kernel(const __grid_constant__ P p) {
+  if (p.stamp && blockIdx.x == 0 && threadIdx.x == 0) p.words->start_ns = global_ns();
   const int total = kFirst ? p.total_tiles * 32 : *p.n_in;
   const int lane = threadIdx.x & 31;
   const int r = (blockIdx.x * (kBlockThreads / 32) + (threadIdx.x >> 5)) * p.lanes + lane;
@@ -720,6 +729,7 @@ __global__ void __launch_bounds__(kBlockThreads, 10) trace_kernel(const __grid_c
 // warp's longest ray.  Once the counter is exhausted the rays run to the end.
 template <bool kFirst, bool kCount>
 __global__ void __launch_bounds__(kBlockThreads) trace_persistent_kernel(const __grid_constant__ TraceParams p) {
+  if (p.stamp && blockIdx.x == 0 && threadIdx.x == 0) p.words->start_ns = global_ns();
   __shared__ float4 s_origin[kBlockThreads], s_dir[kBlockThreads];
   const int lane = threadIdx.x & 31;
   const int total = kFirst ? p.total_tiles * 32 : *p.n_in;  // below 2^31: at most 2^30 pixels
@@ -778,7 +788,7 @@ __global__ void __launch_bounds__(kBlockThreads) trace_persistent_kernel(const _
 // FinishTracingFrame for rays still faulted at the end of the frame: shade
 // with the fault's parent node as the cache holds it now.  Depth output: the
 // distance at which the ray stopped and that parent node.
-__global__ void __launch_bounds__(kBlockThreads) finish_kernel(const __grid_constant__ TraceParams p) {
+__global__ void __launch_bounds__(kBlockThreads) finish_kernel(const __grid_constant__ TraceCore p) {
   const int i = blockIdx.x * kBlockThreads + threadIdx.x;
   if (i >= *p.n_in) return;
   const uchar4 col = (p.normals && p.colors) ? shade(p, (uint32_t)p.in_parent[i]) : make_uchar4(0, 0, 0, 0);
@@ -791,7 +801,7 @@ __global__ void __launch_bounds__(kBlockThreads) finish_kernel(const __grid_cons
 // as it is, no feedback.  Red for a fault or an error, black for a miss, else
 // grey = 255 * (1 - log-depth in [0.01, 5]) clamped to [0, 255] (the
 // reference's float-to-uchar conversion is undefined outside that range).
-__global__ void __launch_bounds__(kBlockThreads) depth_view_kernel(const __grid_constant__ TraceParams p) {
+__global__ void __launch_bounds__(kBlockThreads) depth_view_kernel(const __grid_constant__ TraceParams1 p) {
   const ViewDesc& v = p.views[0];
   const int W = v.width, H = v.height;
   const int i = blockIdx.x * kBlockThreads + threadIdx.x;
@@ -843,21 +853,38 @@ __global__ void fill_kernel(int* p, int32_t v, size_t n) {
 
 // Bitmaps -> [faults by descending block][hits ascending][NO_HIT], the order
 // of the reference's sorted unique array.  One CTA; each thread owns a run of
-// bitmap words in output order.
+// bitmap words in output order, reads them once (up to kUniqKeep of them are
+// kept) and leaves them zero.  It also takes the pass's counters, clears those
+// of the pass before and publishes the result to the host, which is what lets
+// a pass do without a memset before it and event records and a stream
+// synchronisation after it: those took 16 us of a frame's 27 us outside its
+// kernels.
 constexpr int kUniqThreads = 1024;
+constexpr int kUniqKeep = 8;
 __global__ void __launch_bounds__(kUniqThreads) unique_from_bits_kernel(const UniqueFromBitsParams q) {
   __shared__ int warp_sums[32];
   __shared__ int fsum;
-  const bool no_word = __syncthreads_or(threadIdx.x < kNoWordFlags && q.no_word[threadIdx.x * kNoWordStride] != 0);
+  const unsigned long long begin_ns = global_ns();
   const int total = q.fault_words + q.hit_words;
   const int per = (total + kUniqThreads - 1) / kUniqThreads;
   const int begin = min(total, (int)threadIdx.x * per), end = min(total, begin + per);
-  auto word_at = [&](int k) -> uint32_t {
-    return k < q.fault_words ? q.fault_bits[q.fault_words - 1 - k] : q.hit_bits[k - q.fault_words];
+  auto word_ptr = [&](int k) -> uint32_t* {
+    return k < q.fault_words ? q.fault_bits + (q.fault_words - 1 - k) : q.hit_bits + (k - q.fault_words);
   };
+  uint32_t kept[kUniqKeep];
+#pragma unroll
+  for (int i = 0; i < kUniqKeep; ++i) kept[i] = begin + i < end ? *word_ptr(begin + i) : 0u;
+  bool none = threadIdx.x < kNoWordFlags && q.words->no_word[threadIdx.x * kNoWordStride] != 0;
+  if (q.later && threadIdx.x == 0) none = none || q.previous->rays < q.total_pixels;
   int cnt = 0, fcnt = 0;
-  for (int k = begin; k < end; ++k) {
-    const int n = __popc(word_at(k));
+#pragma unroll
+  for (int i = 0; i < kUniqKeep; ++i) {
+    const int n = __popc(kept[i]);
+    cnt += n;
+    if (begin + i < q.fault_words) fcnt += n;
+  }
+  for (int k = begin + kUniqKeep; k < end; ++k) {
+    const int n = __popc(*word_ptr(k));
     cnt += n;
     if (k < q.fault_words) fcnt += n;
   }
@@ -869,20 +896,11 @@ __global__ void __launch_bounds__(kUniqThreads) unique_from_bits_kernel(const Un
   }
   if (lane == 31) warp_sums[warp] = incl;
   if (threadIdx.x == 0) fsum = 0;
-  __syncthreads();
-  if (warp == 0) {
-    int v = warp_sums[lane];
-    int s = v;
-    for (int off = 1; off < 32; off <<= 1) {
-      int u = __shfl_up_sync(kFull, s, off);
-      if (lane >= off) s += u;
-    }
-    warp_sums[lane] = s - v;  // exclusive
-  }
-  __syncthreads();
-  int pos = warp_sums[warp] + incl - cnt;
-  for (int k = begin; k < end; ++k) {
-    uint32_t w = word_at(k);
+  const bool no_word = __syncthreads_or(none);
+  const int sums = warp_sums[lane];
+  int pos = __reduce_add_sync(kFull, lane < warp ? sums : 0) + incl - cnt;
+  const int all = __reduce_add_sync(kFull, sums);
+  auto emit = [&](int k, uint32_t w) {
     if (k < q.fault_words) {
       const int wi = q.fault_words - 1 - k;
       while (w) {  // descending bits
@@ -898,17 +916,42 @@ __global__ void __launch_bounds__(kUniqThreads) unique_from_bits_kernel(const Un
         q.unique_out[pos++] = wi * 32 + b + 2;
       }
     }
+  };
+#pragma unroll
+  for (int i = 0; i < kUniqKeep; ++i)
+    if (kept[i]) {
+      emit(begin + i, kept[i]);
+      *word_ptr(begin + i) = 0u;
+    }
+  for (int k = begin + kUniqKeep; k < end; ++k) {
+    uint32_t* w = word_ptr(k);
+    if (*w) {
+      emit(k, *w);
+      *w = 0u;
+    }
   }
-  int f = fcnt;
-  for (int off = 16; off > 0; off >>= 1) f += __shfl_down_sync(kFull, f, off);
-  if (lane == 0) atomicAdd(&fsum, f);
+  fcnt = __reduce_add_sync(kFull, fcnt);
+  if (lane == 0 && fcnt) atomicAdd(&fsum, fcnt);
+  if (q.client_faults && threadIdx.x < kMaxClients) {
+    q.result->client_faults[threadIdx.x] = q.client_faults[threadIdx.x];
+    q.client_faults[threadIdx.x] = 0;
+  }
+  // the other pass's words; every read of them came before the barrier above
+  for (int i = threadIdx.x; i < kPassInts; i += kUniqThreads) reinterpret_cast<int*>(q.previous)[i] = 0;
+  __threadfence_system();  // the values reach the host before the pass's number
   __syncthreads();
-  if (threadIdx.x == kUniqThreads - 1) {
-    int n = pos;  // the last thread's end position = total set bits
-    if (no_word || (q.n_in && *q.n_in < q.total_pixels)) q.unique_out[n++] = kNoHit;
-    q.counts_out[0] = n;
-    q.counts_out[1] = fsum;
-    q.counts_out[2] = q.n_rays ? *q.n_rays : 0;
+  if (threadIdx.x == 0) {
+    int n = all;
+    if (no_word) q.unique_out[n++] = kNoHit;
+    q.result->unique = n;
+    q.result->faults = fsum;
+    q.result->rays = q.words->rays;
+    q.result->trace_ms = (float)(long long)(begin_ns - q.words->start_ns) * 1e-6f;
+    q.result->unique_ms = (float)(long long)(global_ns() - begin_ns) * 1e-6f;
+    const unsigned int pass = *q.passes + 1;
+    *q.passes = pass;
+    __threadfence_system();
+    *(volatile unsigned int*)&q.result->pass = pass;
   }
 }
 
@@ -927,17 +970,27 @@ int persistent_grid() {
   return grid;
 }
 
-// The traversal launch for pass kind (first, count): function and grid.
+// The traversal launch for pass kind (first, count): function, grid and
+// parameters.
 template <bool kFirst, bool kCount>
-void trace_launch_shape(const TraceParams& p, int rays, int grid, void** func, dim3* blocks) {
-  if (kFirst && p.refill < 32) {
-    *func = reinterpret_cast<void*>(trace_persistent_kernel<true, kCount>);
-    *blocks = dim3(grid > 0 ? grid : persistent_grid<kCount>());
-  } else {
-    *func = reinterpret_cast<void*>(trace_kernel<kFirst, kCount>);
-    const int per = kBlockThreads / 32 * p.lanes;
-    *blocks = dim3(std::max(1, (rays + per - 1) / per));
+void trace_launch_shape(const TraceParams* p, int rays, int grid, TraceLaunch* l) {
+  if (kFirst && p->refill < 32) {
+    l->kp.func = reinterpret_cast<void*>(trace_persistent_kernel<true, kCount>);
+    l->kp.gridDim = dim3(grid > 0 ? grid : persistent_grid<kCount>());
+    l->args[0] = const_cast<TraceParams*>(p);
+    return;
   }
+  const int per = kBlockThreads / 32 * p->lanes;
+  l->kp.gridDim = dim3(std::max(1, (rays + per - 1) / per));
+  if (kFirst && p->n_views > 1) {
+    l->kp.func = reinterpret_cast<void*>(trace_kernel<true, kCount, TraceParams>);
+    l->args[0] = const_cast<TraceParams*>(p);
+    return;
+  }
+  l->kp.func = reinterpret_cast<void*>(trace_kernel<kFirst, kCount, TraceParams1>);
+  static_cast<TraceCore&>(l->one) = *p;
+  l->one.views[0] = p->views[0];
+  l->args[0] = &l->one;
 }
 
 }  // namespace
@@ -969,34 +1022,23 @@ int trace_lanes(bool first, int rays) {
 
 int trace_persistent_grid(bool count) { return count ? persistent_grid<true>() : persistent_grid<false>(); }
 
-cudaError_t trace_node_params(const TraceParams* p, bool first, bool count, int rays, int grid, void** args,
-                              cudaKernelNodeParams* kp) {
-  void* func = nullptr;
-  dim3 blocks;
+void trace_node_params(const TraceParams* p, bool first, bool count, int rays, int grid, TraceLaunch* l) {
+  l->kp = cudaKernelNodeParams{};
   if (first) {
-    if (count) trace_launch_shape<true, true>(*p, rays, grid, &func, &blocks);
-    else trace_launch_shape<true, false>(*p, rays, grid, &func, &blocks);
+    if (count) trace_launch_shape<true, true>(p, rays, grid, l);
+    else trace_launch_shape<true, false>(p, rays, grid, l);
   } else {
-    if (count) trace_launch_shape<false, true>(*p, rays, grid, &func, &blocks);
-    else trace_launch_shape<false, false>(*p, rays, grid, &func, &blocks);
+    if (count) trace_launch_shape<false, true>(p, rays, grid, l);
+    else trace_launch_shape<false, false>(p, rays, grid, l);
   }
-  args[0] = const_cast<TraceParams*>(p);
-  *kp = cudaKernelNodeParams{};
-  kp->func = func;
-  kp->gridDim = blocks;
-  kp->blockDim = dim3(kBlockThreads);
-  kp->sharedMemBytes = 0;
-  kp->kernelParams = args;
-  kp->extra = nullptr;
-  return cudaSuccess;
+  l->kp.blockDim = dim3(kBlockThreads);
+  l->kp.kernelParams = l->args;
 }
 
 cudaError_t launch_trace(const TraceParams& p, bool first, bool count, int rays, int grid, cudaStream_t s) {
-  void* args[1];
-  cudaKernelNodeParams kp;
-  trace_node_params(&p, first, count, rays, grid, args, &kp);
-  if (kp.gridDim.x == 0) return cudaSuccess;
-  return cudaLaunchKernel(kp.func, kp.gridDim, kp.blockDim, kp.kernelParams, 0, s);
+  TraceLaunch l;
+  trace_node_params(&p, first, count, rays, grid, &l);
+  return cudaLaunchKernel(l.kp.func, l.kp.gridDim, l.kp.blockDim, l.kp.kernelParams, 0, s);
 }
 
 cudaError_t unique_node_params(const UniqueFromBitsParams* q, void** args, cudaKernelNodeParams* kp) {
@@ -1009,13 +1051,13 @@ cudaError_t unique_node_params(const UniqueFromBitsParams* q, void** args, cudaK
   return cudaSuccess;
 }
 
-cudaError_t launch_finish(const TraceParams& p, int max_rays, cudaStream_t s) {
+cudaError_t launch_finish(const TraceCore& p, int max_rays, cudaStream_t s) {
   if (max_rays <= 0) return cudaSuccess;
   finish_kernel<<<(max_rays + kBlockThreads - 1) / kBlockThreads, kBlockThreads, 0, s>>>(p);
   return cudaGetLastError();
 }
 
-cudaError_t launch_depth_view(const TraceParams& p, cudaStream_t s) {
+cudaError_t launch_depth_view(const TraceParams1& p, cudaStream_t s) {
   const long long n = (long long)p.views[0].width * p.views[0].height;
   if (n <= 0) return cudaSuccess;
   depth_view_kernel<<<(unsigned)((n + kBlockThreads - 1) / kBlockThreads), kBlockThreads, 0, s>>>(p);
