@@ -35,6 +35,7 @@ struct ViewDesc {
   float m[16];             // view_proj_inv, row-major
   int width, height;
   int tiles_x;             // columns of 32-pixel tiles
+  uint32_t tiles_x_inv;    // reciprocal(tiles_x)
   int tile_base;           // first tile of this view in the launch's tile space
   float lod;               // lod_voxel_size
   int pix_base;            // first pixel of the view in the shared image buffer
@@ -77,9 +78,10 @@ struct TraceCore {
   const uchar4* colors;    // may be null
   uint32_t root;           // node index of the root (cache node indices are unsigned 32-bit)
   int nodes_in_block;
+  int block_shift;         // log2(nodes_in_block), -1 when it is no power of two
   uint32_t node_limit;     // nodes in the cache (max_blocks * nodes_in_block)
   uint32_t far_limit;      // far pointers in the cache (max_blocks * 8)
-  float bg[4];             // background colour (0, 216/255, 1, 1)
+  uchar4 empty_pixel;      // a pixel that shows the background
   // outputs of every view
   uchar4* image;           // RGBA8, row 0 of each view at the bottom
   uchar4* host_image;      // optional: the same pixels also written here (page-locked host memory)
@@ -134,6 +136,14 @@ struct TraceParams : TraceCore {
 struct TraceParams1 : TraceCore {
   ViewDesc views[1];
 };
+
+// ceil(2^32 / d), or the largest word for d = 1 (see first_pass_pixel).
+inline uint32_t reciprocal(int d) { return d > 1 ? (uint32_t)(((1ull << 32) + (uint32_t)d - 1) / (uint32_t)d) : ~0u; }
+inline int log2_or_minus_one(int v) { return v > 0 && (v & (v - 1)) == 0 ? __builtin_ctz((unsigned)v) : -1; }
+// FinishTracingFrame's pixel where nothing was hit, over background bg.
+uchar4 finish_empty(const float* bg);
+// The reference's background (gpu-ray-tracer.cpp:190).
+constexpr float kBackground[4] = {0.0f, (float)(216 / 255.), 1.0f, 1.0f};
 
 // Faulted-ray records carried from one pass to the next (device arrays).
 struct RayList {

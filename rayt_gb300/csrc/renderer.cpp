@@ -256,6 +256,7 @@ int Renderer::SetViews(const float* m) {
       view_origin(d.m, d.origin);
       d.lod = lod_used;
       d.tiles_x = (d.width + tw - 1) / tw;
+      d.tiles_x_inv = reciprocal(d.tiles_x);
       d.tile_base = (int)std::min<int64_t>(tiles, INT32_MAX);
       tiles += (int64_t)d.tiles_x * ((d.height + th - 1) / th);
     }
@@ -278,12 +279,10 @@ TraceParams Renderer::Params(int it) const {
   p.colors = static_cast<const uchar4*>(cache_->channel("colors", 4));
   p.root = cache_->root_node();
   p.nodes_in_block = cache_->nodes_in_block();
+  p.block_shift = log2_or_minus_one(p.nodes_in_block);
   p.node_limit = (uint32_t)cache_->max_blocks() * (uint32_t)cache_->nodes_in_block();
   p.far_limit = (uint32_t)cache_->max_blocks() * 8u;
-  p.bg[0] = 0.0f;
-  p.bg[1] = (float)(216 / 255.);  // the reference's background (gpu-ray-tracer.cpp:190)
-  p.bg[2] = 1.0f;
-  p.bg[3] = 1.0f;
+  p.empty_pixel = finish_empty(kBackground);
   p.image = d_images_;
   // the first pass's pixels reach the host image by one copy; later passes
   // write theirs there too

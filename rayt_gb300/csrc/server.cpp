@@ -327,12 +327,10 @@ TraceParams Server::Params(int k) const {
   p.colors = static_cast<const uchar4*>(cache_->channel("colors", 4));
   p.root = cache_->root_node();
   p.nodes_in_block = cache_->nodes_in_block();
+  p.block_shift = log2_or_minus_one(p.nodes_in_block);
   p.node_limit = (uint32_t)cache_->max_blocks() * (uint32_t)cache_->nodes_in_block();
   p.far_limit = (uint32_t)cache_->max_blocks() * 8u;
-  p.bg[0] = 0.0f;
-  p.bg[1] = (float)(216 / 255.);
-  p.bg[2] = 1.0f;
-  p.bg[3] = 1.0f;
+  p.empty_pixel = finish_empty(kBackground);
   p.image = d_images_;
   p.tile_w_log2 = 2;
   const RayList& in = lists_[1 - k];
@@ -432,6 +430,7 @@ int Server::Step(int* finished) {
     for (int i = 0; i < n; ++i) {
       ViewDesc& v = views[g + i];
       v.tiles_x = (v.width + 3) / 4;
+      v.tiles_x_inv = reciprocal(v.tiles_x);
       v.tile_base = (int)tiles;
       tiles += (int64_t)v.tiles_x * ((v.height + 7) / 8);
       q.views[i] = v;

@@ -495,19 +495,13 @@ __device__ __forceinline__ uchar4 shade(const TraceCore& p, uint32_t node) {
   return make_uchar4((unsigned char)c0, (unsigned char)c1, (unsigned char)c2, 255);
 }
 
-// FinishTracingFrame's blend of the accumulated colour over the background.
-__device__ __forceinline__ uchar4 finish(const TraceCore& p, uchar4 c) {
-  const float w = 255.f - (float)c.w;
-  float t[4] = {(float)c.x + p.bg[0] * w + .5f, (float)c.y + p.bg[1] * w + .5f,
-                (float)c.z + p.bg[2] * w + .5f, (float)c.w + p.bg[3] * w + .5f};
-  unsigned char o[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    float v = t[k] < 255.f ? t[k] : 255.f;
-    v = 0.f < v ? v : 0.f;
-    o[k] = (unsigned char)v;
-  }
-  return make_uchar4(o[0], o[1], o[2], o[3]);
+// FinishTracingFrame's blend of the accumulated colour over the background,
+// for a pixel nothing was accumulated in (alpha 0): the same for every such
+// pixel, so the host computes it (finish_empty).  An opaque pixel (hits,
+// errors) is left as it is: w = 255 - 255 = 0 adds a zero, and c + .5 truncates
+// to c.
+__device__ __forceinline__ uchar4 shaded(const TraceCore& p, uint32_t node) {
+  return p.normals && p.colors ? shade(p, node) : p.empty_pixel;
 }
 
 // Appends `pred` lanes of the active warp to a global list: returns this
@@ -586,8 +580,14 @@ __device__ __forceinline__ bool first_pass_pixel(const P& p, int r, int& v, int&
   v = sizeof(P) == sizeof(TraceParams1) ? 0 : view_of_tile(p, tile);
   const ViewDesc& vd = p.views[v];
   const int t = tile - vd.tile_base;
-  x = ((t % vd.tiles_x) << p.tile_w_log2) + (k & ((1 << p.tile_w_log2) - 1));
-  y = (t / vd.tiles_x) * (32 >> p.tile_w_log2) + (k >> p.tile_w_log2);
+  // t / tiles_x: the product with the reciprocal rounded up is the quotient or
+  // one more (its excess over t / tiles_x is below t / 2^32), with the largest
+  // word for 1 / 1 one less
+  int row = (int)__umulhi((uint32_t)t, vd.tiles_x_inv), col = t - row * vd.tiles_x;
+  if (col < 0) --row, col += vd.tiles_x;
+  if (col >= vd.tiles_x) ++row, col -= vd.tiles_x;
+  x = (col << p.tile_w_log2) + (k & ((1 << p.tile_w_log2) - 1));
+  y = row * (32 >> p.tile_w_log2) + (k >> p.tile_w_log2);
   return x < vd.width && y < vd.height;
 }
 
@@ -649,16 +649,15 @@ __device__ __forceinline__ void end_ray(const TraceCore& p, const RayEnd& e, uin
   const int node = e.node, dup = e.dup, fault_block = e.fault_block;
   int32_t word = kNoHit;
   if (e.error) {
-    put_pixel(p, ray, finish(p, make_uchar4(255, 0, 0, 255)));
+    put_pixel(p, ray, make_uchar4(255, 0, 0, 255));
     if (p.depth) write_depth(p, ray, __uint_as_float(kDepthNaN), -2);
   } else if (faulted) {
     word = -fault_block - 1;
   } else if (!hit) {
-    put_pixel(p, ray, finish(p, make_uchar4(0, 0, 0, 0)));
+    put_pixel(p, ray, p.empty_pixel);
     if (p.depth) write_depth(p, ray, __uint_as_float(kDepthInf), -1);
   } else {
-    const uchar4 col = (p.normals && p.colors) ? shade(p, (uint32_t)node) : make_uchar4(0, 0, 0, 0);
-    put_pixel(p, ray, finish(p, col));
+    put_pixel(p, ray, shaded(p, (uint32_t)node));
     word = (int32_t)(((uint32_t)(node + 1) << 1) | (uint32_t)dup);
     if (p.depth) write_depth(p, ray, adv + e.t, node);
   }
@@ -679,7 +678,8 @@ __device__ __forceinline__ void end_ray(const TraceCore& p, const RayEnd& e, uin
     if (p.out_adv) p.out_adv[slot] = p.restart ? adv : adv + e.t;
   }
   warp_set_bit(p.fault_bits, faulted && fault_block < p.fault_bit_limit ? fault_block : -1);
-  warp_set_bit(p.hit_bits, hit ? (int)(2 * ((uint32_t)node / (uint32_t)p.nodes_in_block)) + dup : -1);
+  const uint32_t block = p.block_shift >= 0 ? (uint32_t)node >> p.block_shift : (uint32_t)node / (uint32_t)p.nodes_in_block;
+  warp_set_bit(p.hit_bits, hit ? (int)(2 * block) + dup : -1);
   mark_no_word(p, word == kNoHit);
   if (kCount) {
     const unsigned v[6] = {1u, fetches, far_fetches, (unsigned)e.iter, hit ? 1u : 0u, faulted ? 1u : 0u};
@@ -711,8 +711,7 @@ __global__ void __launch_bounds__(kBlockThreads, 10) trace_kernel(const __grid_c
   if (!kFirst && p.finish_mask && ((p.finish_mask >> slot_of(p, ray)) & 1ull)) {
     // served mode: the request stops here; FinishTracingFrame's shading with
     // the fault's parent node
-    const uchar4 col = (p.normals && p.colors) ? shade(p, (uint32_t)p.in_parent[r]) : make_uchar4(0, 0, 0, 0);
-    put_pixel(p, ray, finish(p, col));
+    put_pixel(p, ray, shaded(p, (uint32_t)p.in_parent[r]));
     if (p.depth) write_depth(p, ray, adv, p.in_parent[r]);
     mark_no_word(p, true);
     return;
@@ -791,8 +790,7 @@ __global__ void __launch_bounds__(kBlockThreads) trace_persistent_kernel(const _
 __global__ void __launch_bounds__(kBlockThreads) finish_kernel(const __grid_constant__ TraceCore p) {
   const int i = blockIdx.x * kBlockThreads + threadIdx.x;
   if (i >= *p.n_in) return;
-  const uchar4 col = (p.normals && p.colors) ? shade(p, (uint32_t)p.in_parent[i]) : make_uchar4(0, 0, 0, 0);
-  put_pixel(p, p.in_ray[i], finish(p, col));
+  put_pixel(p, p.in_ray[i], shaded(p, (uint32_t)p.in_parent[i]));
   if (p.depth) write_depth(p, p.in_ray[i], p.in_adv[i], p.in_parent[i]);
 }
 
@@ -1049,6 +1047,19 @@ cudaError_t unique_node_params(const UniqueFromBitsParams* q, void** args, cudaK
   kp->blockDim = dim3(kUniqThreads);
   kp->kernelParams = args;
   return cudaSuccess;
+}
+
+uchar4 finish_empty(const float* bg) {
+  unsigned char o[4];
+  for (int k = 0; k < 4; ++k) {
+    const volatile float scaled = bg[k] * 255.f;  // each operation rounds by itself, as on the device
+    const volatile float sum = 0.f + scaled;
+    float v = sum + .5f;
+    v = v < 255.f ? v : 255.f;
+    v = 0.f < v ? v : 0.f;
+    o[k] = (unsigned char)v;
+  }
+  return make_uchar4(o[0], o[1], o[2], o[3]);
 }
 
 cudaError_t launch_finish(const TraceCore& p, int max_rays, cudaStream_t s) {
