@@ -243,6 +243,8 @@ Cache::~Cache() {
   cudaFreeHost(h_slots_);
   cudaFreeHost(h_blocks_);
   cudaFreeHost(h_patches_);
+  cudaFreeHost(h_clock_);
+  cudaFree(d_clock_);
   for (auto& e : stage_free_)
     if (e) cudaEventDestroy(e);
   for (auto& e : patch_free_)
@@ -299,6 +301,12 @@ int Cache::Init(Tree* tree, int max_blocks) {
     if (!mapped_alloc(reinterpret_cast<void**>(&h_blocks_), reinterpret_cast<void**>(&d_blocks_),
                       sizeof(int) * stage_cap_ * 2))
       return fail(RAYT_E_OOM, "staging allocation failed");
+    UploadClock clock{};
+    if (!mapped_alloc(reinterpret_cast<void**>(&h_clock_), reinterpret_cast<void**>(&clock.host), 8) ||
+        cudaMalloc(&d_clock_, sizeof(clock)) != cudaSuccess)
+      return fail(RAYT_E_OOM, "staging allocation failed");
+    *h_clock_ = 0;
+    RAYT_CUDA_TRY(cudaMemcpy(d_clock_, &clock, sizeof(clock), cudaMemcpyHostToDevice));
   } else {
     stage_cap_ = (int)std::max<size_t>(kStageBlocksMin, kStageBytes / area_);
     if (cudaHostAlloc(&h_stage_, area_ * stage_cap_ * 2, cudaHostAllocDefault) != cudaSuccess ||
@@ -441,17 +449,21 @@ void Cache::AddPatch(bool far_buffer, uint32_t index, uint32_t value) {
 int Cache::FlushTo(int end) {
   if (end <= batch_begin_ && patches_.empty()) return RAYT_OK;
   const int h = half_;
-  // device time of the batch: events around its copies and kernels (the
-  // last 256 batches between two TakeUploadMs calls are counted)
-  if (flush_used_ == kFlushEvents) flush_used_ = 0;
-  if (flush_used_ == (int)flush_ev_.size()) {
-    cudaEvent_t a = nullptr, b = nullptr;
-    RAYT_CUDA_TRY(cudaEventCreate(&a));
-    RAYT_CUDA_TRY(cudaEventCreate(&b));
-    flush_ev_.emplace_back(a, b);
+  std::pair<cudaEvent_t, cudaEvent_t> ev{};
+  if (!file_host_) {
+    // device time of the batch: events around its copies and kernels (the
+    // last 256 batches between two TakeUploadMs calls are counted)
+    if (flush_used_ == kFlushEvents) flush_used_ = 0;
+    if (flush_used_ == (int)flush_ev_.size()) {
+      cudaEvent_t a = nullptr, b = nullptr;
+      RAYT_CUDA_TRY(cudaEventCreate(&a));
+      RAYT_CUDA_TRY(cudaEventCreate(&b));
+      flush_ev_.emplace_back(a, b);
+    }
+    ev = flush_ev_[flush_used_++];
+    RAYT_CUDA_TRY(cudaEventRecord(ev.first, stream_));
   }
-  const std::pair<cudaEvent_t, cudaEvent_t> ev = flush_ev_[flush_used_++];
-  RAYT_CUDA_TRY(cudaEventRecord(ev.first, stream_));
+  bool timed = false;  // the upload kernel has started the batch's clock
   if (end > batch_begin_) {
     const size_t first = (size_t)stage_cap_ * h + batch_begin_;
     const int n = end - batch_begin_;
@@ -461,6 +473,8 @@ int Cache::FlushTo(int end) {
       up.file_first = tree_->info.header_bytes + 76;
       up.file_stride = tree_->info.block_stride;
       up.block_ids = d_blocks_ + first;
+      up.clock = d_clock_;
+      timed = true;
     } else {
       uint8_t* hs = h_stage_ + area_ * first;
       uint8_t* ds = d_stage_ + area_ * first;
@@ -476,7 +490,7 @@ int Cache::FlushTo(int end) {
       up.chan_bytes[c] = chan_bytes_[c];
       up.chan[c] = d_chan_[c];
     }
-    RAYT_CUDA_TRY(launch_upload(up, stream_));
+    RAYT_CUDA_TRY(launch_upload(up, h_slots_ + first, h_blocks_ ? h_blocks_ + first : nullptr, stream_));
     ++launches_;
     stats_.bytes_h2d += (int64_t)(file_host_ ? (size_t)tree_->info.content_bytes * n : area_ * n);
   }
@@ -484,21 +498,28 @@ int Cache::FlushTo(int end) {
   for (size_t i = 0; i < patches_.size(); ++i)
     if (!patch_dead_[i]) patches_[live++] = patches_[i];
   patches_.resize(live);
+  uint32_t* links = reinterpret_cast<uint32_t*>(d_chan_[0]);
   size_t done = 0;
-  while (done < patches_.size()) {
+  while (done < patches_.size() || timed) {
     const size_t n = std::min(patches_.size() - done, (size_t)patch_cap_);
-    const int ph = patch_half_;
-    Patch* hp = h_patches_ + (size_t)patch_cap_ * ph;
-    Patch* dp = d_patches_ + (size_t)patch_cap_ * ph;
-    // a pinned patch half is refilled only after the kernel that read it finished
-    RAYT_CUDA_TRY(cudaEventSynchronize(patch_free_[ph]));
-    std::memcpy(hp, patches_.data() + done, n * sizeof(Patch));
-    RAYT_CUDA_TRY(launch_patches(dp, (int)n, reinterpret_cast<uint32_t*>(d_chan_[0]), d_far_, stream_));
-    RAYT_CUDA_TRY(cudaEventRecord(patch_free_[ph], stream_));
-    patch_half_ ^= 1;
+    // the batch's last launch stops its clock
+    UploadClock* clock = timed && done + n == patches_.size() ? d_clock_ : nullptr;
+    if (n <= (size_t)kInlinePatches) {
+      RAYT_CUDA_TRY(launch_patches(patches_.data() + done, (int)n, links, d_far_, clock, stream_));
+    } else {
+      const int ph = patch_half_;
+      Patch* hp = h_patches_ + (size_t)patch_cap_ * ph;
+      // a pinned patch half is refilled only after the kernel that read it finished
+      RAYT_CUDA_TRY(cudaEventSynchronize(patch_free_[ph]));
+      std::memcpy(hp, patches_.data() + done, n * sizeof(Patch));
+      RAYT_CUDA_TRY(launch_patches(d_patches_ + (size_t)patch_cap_ * ph, (int)n, links, d_far_, clock, stream_));
+      RAYT_CUDA_TRY(cudaEventRecord(patch_free_[ph], stream_));
+      patch_half_ ^= 1;
+    }
     ++launches_;
     stats_.bytes_h2d += (int64_t)(n * sizeof(Patch));
     done += n;
+    if (clock) timed = false;
   }
   patches_.clear();
   patch_dead_.clear();
@@ -506,7 +527,7 @@ int Cache::FlushTo(int end) {
   patch_at_.Clear();
   batch_begin_ = std::max(batch_begin_, end);
   ++epoch_;
-  RAYT_CUDA_TRY(cudaEventRecord(ev.second, stream_));
+  if (ev.second) RAYT_CUDA_TRY(cudaEventRecord(ev.second, stream_));
   return RAYT_OK;
 }
 
@@ -519,6 +540,11 @@ float Cache::TakeUploadMs() {
     if (cudaEventElapsedTime(&ms, flush_ev_[i].first, flush_ev_[i].second) == cudaSuccess) total += ms;
   }
   flush_used_ = 0;
+  if (h_clock_) {
+    const unsigned long long ns = __atomic_load_n(h_clock_, __ATOMIC_RELAXED);
+    total += (float)(ns - clock_taken_ns_) * 1e-6f;
+    clock_taken_ns_ = ns;
+  }
   return total;
 }
 

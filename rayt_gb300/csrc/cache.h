@@ -215,6 +215,11 @@ class Cache {
   static constexpr int kFlushEvents = 256;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> flush_ev_;  // per flushed batch, reused
   int flush_used_ = 0;
+  // mapped file: the kernels keep the batches' device time themselves (three
+  // event calls per batch are a third of its host work)
+  unsigned long long* h_clock_ = nullptr;  // pinned: device time of the batches done
+  UploadClock* d_clock_ = nullptr;
+  unsigned long long clock_taken_ns_ = 0;
 
   // MarkUsedBatch's scratch: chain starts in call order, the nodes whose last
   // move falls in each call (walk order), those calls' ranges, seen stamps

@@ -252,6 +252,16 @@ cudaError_t bounded_wait_probe(double limit_s, int* err, cudaStream_t s);
 
 // ---- block upload --------------------------------------------------------------
 constexpr int kMaxChannels = 8;
+// A batch of up to this many blocks, and of patches, carries its slots, block
+// numbers and patch records in the launch parameters.
+constexpr int kInlineBlocks = 128, kInlinePatches = 256;
+// Device time of the batches, in device memory: a batch's last kernel adds the
+// batch's.
+struct UploadClock {
+  unsigned long long start_ns;  // of the batch under way
+  unsigned long long total_ns;  // of the batches done
+  unsigned long long* host;     // total_ns in host-mapped memory
+};
 struct UploadParams {
   const uint8_t* stage;        // block contents, `stride` bytes apart
   size_t stride;               // content bytes rounded up to 16 (keeps every block aligned)
@@ -268,15 +278,24 @@ struct UploadParams {
   uint64_t file_first;         // header bytes + the 76-byte block header
   uint64_t file_stride;
   const int* block_ids;
+  UploadClock* clock;          // mapped reads: the batch's beginning is noted here
   int parts;                   // CTAs per block (mapped reads; set by launch_upload)
+  // mapped reads of blocks whose channel sections are whole words: the word at
+  // which each section begins, and the content's words (0: other blocks)
+  uint32_t section[kMaxChannels + 1];
 };
 struct Patch {
   uint32_t index;  // node-link index (below 2^32) or far-pointer index
   uint32_t value;
   uint32_t far;    // 1: far-pointer buffer, 0: node-link buffer
 };
-cudaError_t launch_upload(const UploadParams& p, cudaStream_t s);
-cudaError_t launch_patches(const Patch* patches, int n, uint32_t* links, uint32_t* far_ptrs, cudaStream_t s);
+// `host_slots` and `host_blocks`: the batch's slots and block numbers in host
+// memory (mapped reads).
+cudaError_t launch_upload(const UploadParams& p, const int* host_slots, const int* host_blocks, cudaStream_t s);
+// n patches, in host memory when there are at most kInlinePatches, else at the
+// device address `patches`.  `clock`: this ends the batch.
+cudaError_t launch_patches(const Patch* patches, int n, uint32_t* links, uint32_t* far_ptrs, UploadClock* clock,
+                           cudaStream_t s);
 
 // ---- glibc-compatible rand() stream -------------------------------------------
 // The additive feedback generator behind glibc's rand()/srand() (TYPE_3:
