@@ -84,10 +84,9 @@ class Cache {
   // GPUOctreeCacheManager protocol
   int InitialFill();
   int StartSession();
-  // expected_requests: the blocks the caller is about to request, when it
-  // knows (a transaction that small reads them on the calling thread, so the
-  // read pool is not woken for it); -1 when it does not.
-  int StartTransaction(int expected_requests = -1);
+  // expected: the blocks the caller is about to request, when it knows; the
+  // read pool is not woken for reads that the calling thread does itself
+  int StartTransaction(const std::vector<int>* expected = nullptr);
   int MarkBlockUsed(int slot);
   int MarkParentUsed(int slot);
   // MarkBlockUsed for every slot of hits, then MarkParentUsed for every slot
@@ -152,6 +151,9 @@ class Cache {
   std::vector<int32_t> block_slot_;    // tree block -> cache slot, -1 absent
   std::vector<int32_t> parent_slot_;   // tree block -> slot of its parent, -1 absent
   std::vector<uint8_t> validated_;     // tree block -> its links passed the check once (the file is read-only)
+  // tree block -> its fault children, once validated: a block that comes back
+  // needs no look at its links (at most one entry per child link of the tree)
+  std::vector<std::vector<uint32_t>> fault_children_;
   std::vector<int> pending_;
   bool in_session_ = false, in_transaction_ = false;
 
@@ -238,6 +240,7 @@ class Cache {
 
   int ReadOne(int pos, int block);
   int Prefetch(const int* blocks, int n);
+  bool ReadInline(const int* blocks, int n) const;
   void StartRead(const int* blocks, int n);
   void FinishRead();
   std::chrono::steady_clock::time_point read_started_;

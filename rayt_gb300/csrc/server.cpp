@@ -501,7 +501,7 @@ int Server::Step(int* finished) {
   const int64_t uploaded0 = cache_->stats().uploaded_blocks;
   fb_.Decode(h_unique_, h_result_->unique, rand);
   int rc = cache_->StartSession();
-  if (rc == RAYT_OK) rc = cache_->StartTransaction((int)fb_.faults.size());
+  if (rc == RAYT_OK) rc = cache_->StartTransaction(&fb_.faults);
   if (rc == RAYT_OK) {
     cache_->MarkUsedBatch(fb_.hits, fb_.dup_hits);
     for (int b : fb_.faults) {
