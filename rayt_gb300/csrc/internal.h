@@ -22,6 +22,11 @@ int cuda_fail(cudaError_t e, const char* what);
 constexpr int32_t kNoHit = 0x7fffffff;
 constexpr uint32_t kRootParent = (1u << 24) - 1;
 
+// Waits until a kernel of stream s has set the host-mapped *word to `value`,
+// which is the last thing it does; everything queued on s before that kernel is
+// done then.
+int wait_word(const unsigned int* word, unsigned int value, cudaStream_t s);
+
 // ---- traversal ----------------------------------------------------------------
 // Views' images (and recorded feedback words) share one buffer; view v starts
 // at pixel pix_base (a multiple of 64).  A ray is identified by its pixel's
@@ -203,9 +208,7 @@ struct UniqueFromBitsParams {
 };
 cudaError_t launch_unique_from_bits(const UniqueFromBitsParams& p, cudaStream_t s);
 cudaError_t unique_node_params(const UniqueFromBitsParams* q, void** args, cudaKernelNodeParams* kp);
-// Waits until `pass` is published in *r; everything queued on s before that
-// pass's unique kernel is done then.
-int wait_pass(const UniqueResult* r, unsigned int pass, cudaStream_t s);
+
 
 // ---- radix sort / scan / unique -------------------------------------------------
 // Memory of a call: `scratch` (any contents), `status` (look-back words, zero or
@@ -213,6 +216,14 @@ int wait_pass(const UniqueResult* r, unsigned int pass, cudaStream_t s);
 // host reads once the stream has finished).  `epoch` (27 bits, from
 // lookback_epoch_step) tags the call's look-back words.  err becomes 1 when a
 // bounded wait gave up.
+// `done`: the call's last kernel sets *flag (host-mapped) to `number` when all its
+// CTAs have ended; what the call wrote is visible then.  *ctas is zero before
+// and after.  flag null: nothing is published.
+struct DoneFlag {
+  int* ctas = nullptr;
+  unsigned int* flag = nullptr;
+  unsigned int number = 0;
+};
 size_t feedback_scratch_bytes(int n);
 size_t feedback_status_bytes(int n);
 // Compaction (drop NO_HIT, NodeToBlock) and sorted unique.  result[0] receives
@@ -220,17 +231,19 @@ size_t feedback_status_bytes(int n);
 // bitmap: feedback_unique_needs_radix(result) says so, and
 // feedback_unique_radix_device, on the same memory, then sorts them.
 cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t* unique_out, void* scratch,
-                                   unsigned long long* status, uint32_t epoch, int* result, int* err, cudaStream_t s);
+                                   unsigned long long* status, uint32_t epoch, int* result, int* err,
+                                   const DoneFlag& done, cudaStream_t s);
 bool feedback_unique_needs_radix(const int* result);
 cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scratch, unsigned long long* status,
-                                         uint32_t epoch, int* result, int* err, cudaStream_t s);
+                                         uint32_t epoch, int* result, int* err, const DoneFlag& done,
+                                         cudaStream_t s);
 size_t sort_scratch_bytes(int n);
 size_t sort_status_bytes(int n);
 cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch, int* err,
-                            cudaStream_t s);
+                            const DoneFlag& done, cudaStream_t s);
 size_t scan_status_bytes(int n);
 cudaError_t scan_i32_device(int32_t* data, int n, unsigned long long* status, uint32_t epoch, int* err,
-                            cudaStream_t s);
+                            const DoneFlag& done, cudaStream_t s);
 
 // ---- stand-alone primitives (prims.cpp) -------------------------------------------
 // Serialises every sort/scan/unique entry point on all devices: they share

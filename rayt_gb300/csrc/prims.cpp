@@ -14,13 +14,15 @@ namespace {
 struct Device {
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
-  unsigned long long* status = nullptr;
+  unsigned long long* status = nullptr;  // look-back words
   size_t status_bytes = 0;
   void* area = nullptr;       // the allocation-free entry point's look-back words
   size_t area_bytes = 0;
   uint32_t epoch = 0;         // of the last call since the tables were cleared
-  int* host = nullptr;        // mapped pinned: [0] error flag, [1..2] result
+  int* host = nullptr;        // mapped pinned: [0] error flag, [1..2] result, [3] number of the last call done
   int* host_dev = nullptr;
+  int* ctas = nullptr;        // device: CTAs of the call's last kernel that have ended
+  unsigned int calls = 0;     // number of the last call
 };
 Device g_devices[64];
 constexpr uint32_t kEpochLimit = (1u << 27) - 1;
@@ -69,6 +71,10 @@ int begin(size_t scratch_bytes, size_t status_bytes, cudaStream_t s, Device** ou
     for (int k = 0; k < 4; ++k) d.host[k] = 0;
     RAYT_CUDA_TRY(cudaHostGetDevicePointer((void**)&d.host_dev, d.host, 0));
   }
+  if (!d.ctas) {
+    if (cudaMalloc(&d.ctas, sizeof(int)) != cudaSuccess) return fail(RAYT_E_OOM, "scratch allocation failed");
+    RAYT_CUDA_TRY(cudaMemsetAsync(d.ctas, 0, sizeof(int), s));
+  }
   if ((rc = grow(&d.scratch, &d.scratch_bytes, scratch_bytes)) != RAYT_OK) return rc;
   if (d.status_bytes < status_bytes) {
     if ((rc = grow(&d.status, &d.status_bytes, status_bytes)) != RAYT_OK) return rc;
@@ -79,15 +85,22 @@ int begin(size_t scratch_bytes, size_t status_bytes, cudaStream_t s, Device** ou
   return lookback_epoch_step(s, epoch);
 }
 
-// Waits for the call's work and reads the error flag.
-int finish(Device& d, cudaStream_t s) {
-  RAYT_CUDA_TRY(cudaStreamSynchronize(s));
+int check_error(Device& d) {
   volatile int* flag = d.host;
-  if (*flag) {
-    *flag = 0;
-    return fail(RAYT_E_TIMEOUT, "a bounded device wait gave up (look-back did not complete)");
-  }
-  return RAYT_OK;
+  if (!*flag) return RAYT_OK;
+  *flag = 0;
+  return fail(RAYT_E_TIMEOUT, "a bounded device wait gave up (look-back did not complete)");
+}
+
+// The flag that the last kernel of the device work to be launched sets.
+DoneFlag next_done(Device& d) {
+  return DoneFlag{d.ctas, reinterpret_cast<unsigned int*>(d.host_dev) + 3, ++d.calls};
+}
+
+// Waits for that and reads the error flag.
+int finish(Device& d, cudaStream_t s) {
+  const int rc = wait_word(reinterpret_cast<const unsigned int*>(d.host) + 3, d.calls, s);
+  return rc != RAYT_OK ? rc : check_error(d);
 }
 }  // namespace
 
@@ -129,7 +142,7 @@ int rayt_sort_i32(int32_t* data, int n, void* stream) {
   uint32_t epoch = 0;
   const int rc = rayt::begin(rayt::sort_scratch_bytes(n), rayt::sort_status_bytes(n), s, &d, &epoch);
   if (rc != RAYT_OK) return rc;
-  RAYT_CUDA_TRY(rayt::sort_i32_device(data, n, d->scratch, d->status, epoch, d->host_dev, s));
+  RAYT_CUDA_TRY(rayt::sort_i32_device(data, n, d->scratch, d->status, epoch, d->host_dev, rayt::next_done(*d), s));
   return rayt::finish(*d, s);
 }
 
@@ -143,7 +156,7 @@ int rayt_scan_i32(int32_t* data, int n, void* stream) {
   uint32_t epoch = 0;
   const int rc = rayt::begin(0, rayt::scan_status_bytes(n), s, &d, &epoch);
   if (rc != RAYT_OK) return rc;
-  RAYT_CUDA_TRY(rayt::scan_i32_device(data, n, d->status, epoch, d->host_dev, s));
+  RAYT_CUDA_TRY(rayt::scan_i32_device(data, n, d->status, epoch, d->host_dev, rayt::next_done(*d), s));
   return rayt::finish(*d, s);
 }
 
@@ -166,8 +179,8 @@ int rayt_selftest_bounded_wait(double limit_s, void* stream) {
   uint32_t epoch = 0;
   int rc = rayt::begin(0, 0, s, &d, &epoch);
   if (rc != RAYT_OK) return rc;
-  RAYT_CUDA_TRY(rayt::bounded_wait_probe(limit_s, d->host_dev, s));
-  rc = rayt::finish(*d, s);
+  RAYT_CUDA_TRY(rayt::bounded_wait_probe(limit_s, d->host_dev, s));  // synchronises the stream
+  rc = rayt::check_error(*d);
   if (rc == RAYT_E_TIMEOUT) return RAYT_OK;  // the wait gave up as it must
   return rc != RAYT_OK ? rc : fail(RAYT_E_STATE, "bounded wait did not give up");
 }
@@ -187,10 +200,10 @@ int rayt_feedback_unique(const int32_t* words, int n, int nib, int32_t* unique, 
   int rc = rayt::begin(rayt::feedback_scratch_bytes(n), rayt::feedback_status_bytes(n), s, &d, &epoch);
   if (rc != RAYT_OK) return rc;
   int *err = d->host_dev, *result = d->host_dev + 1;
-  RAYT_CUDA_TRY(rayt::feedback_unique_device(words, n, nib, unique, d->scratch, d->status, epoch, result, err, s));
+  RAYT_CUDA_TRY(rayt::feedback_unique_device(words, n, nib, unique, d->scratch, d->status, epoch, result, err, rayt::next_done(*d), s));
   if ((rc = rayt::finish(*d, s)) != RAYT_OK) return rc;
   if (rayt::feedback_unique_needs_radix(d->host + 1)) {
-    RAYT_CUDA_TRY(rayt::feedback_unique_radix_device(n, unique, d->scratch, d->status, epoch, result, err, s));
+    RAYT_CUDA_TRY(rayt::feedback_unique_radix_device(n, unique, d->scratch, d->status, epoch, result, err, rayt::next_done(*d), s));
     if ((rc = rayt::finish(*d, s)) != RAYT_OK) return rc;
   }
   *unique_count = d->host[1];

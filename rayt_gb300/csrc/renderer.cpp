@@ -508,7 +508,7 @@ int Renderer::Frame(const float* m) {
     const auto tw = clock::now();
     launches_seen = cache_->launches();
     if (record) RAYT_CUDA_TRY(cudaStreamSynchronize(s_));  // the words' copy too
-    if ((rc = wait_pass(h_result_, passes_, s_)) != RAYT_OK) break;
+    if ((rc = wait_word(&h_result_->pass, passes_, s_)) != RAYT_OK) break;
     dirty_ = false;
     stats.host_ms_wait += ms_since(tw);
     ms_trace += h_result_->trace_ms;

@@ -469,7 +469,7 @@ int Server::Step(int* finished) {
   ++passes_;
   ++stats.kernel_launches;
   const double t_sync = now_s();
-  const int wrc = wait_pass(h_result_, passes_, s_);
+  const int wrc = wait_word(&h_result_->pass, passes_, s_);
   if (wrc != RAYT_OK) return wrc;
   dirty_ = false;
   const double t_pass = now_s();

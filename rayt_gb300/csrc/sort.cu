@@ -84,6 +84,19 @@ __device__ __forceinline__ bool wait_over(long long& spins, unsigned long long s
 // Sets a call's error flag (device or mapped host memory).
 __device__ __forceinline__ void set_error(int* err) { *(volatile int*)err = 1; }
 
+// The end of a call's last kernel: the CTA that ends last publishes the call's
+// number to the host.  Every thread of every CTA comes here.
+__device__ __forceinline__ void publish(const DoneFlag& done) {
+  if (!done.flag) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(done.ctas, 1) == (int)gridDim.x - 1) {
+    *done.ctas = 0;
+    __threadfence_system();
+    *(volatile unsigned int*)done.flag = done.number;
+  }
+}
+
 __device__ __forceinline__ unsigned long long ld_volatile64(const unsigned long long* p) {
   return *(const volatile unsigned long long*)p;
 }
@@ -203,6 +216,7 @@ __device__ uint32_t tile_prefix(uint32_t* s_warp, unsigned long long* status, in
   return excl;
 }
 
+constexpr int kCountValues = 1 << 14;
 // Control words of a call, zeroed by one memset before it.
 struct Control {
   uint32_t hist[kPasses * kBuckets];  // digit counts
@@ -222,6 +236,9 @@ struct Plan {
   int skip[kPasses];      // digit pass not needed
   int unstable[kPasses];  // first pass: equal digits may leave in any order
   int src[kPasses], dst[kPasses], last;  // buffers of the passes, and where the keys end up
+  int counting;           // sort: the keys take this many values from `lowest` on (0: too many), and are counted
+  uint32_t lowest;
+  uint32_t values[kCountValues];         // keys of each value
   uint32_t offsets[kPasses * kBuckets];  // global start of each digit
   uint32_t range_offsets[kBuckets];
   uint32_t cursors[kBuckets * kCursorStride];
@@ -502,7 +519,8 @@ cudaError_t launch_compact(int grid, const int32_t* words, int n, int nib, const
 // of a warp counts in its own bank, 256 x 32 counters per digit, so an atomic
 // is one wavefront whatever the digits are.  One CTA of 1024 threads per SM
 // holds the 128 KB of counters.  The last CTA turns the counts into offsets
-// and lays out the passes: a digit that is the same in every key needs none.
+// and lays out the passes: a digit that is the same in every key needs none,
+// and keys of up to kCountValues different values are not passed over at all.
 constexpr int kHistThreads = 1024;
 constexpr int kHistSmemBytes = kPasses * kBuckets * 32 * 4;
 template <bool kVec>
@@ -511,6 +529,9 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
                                                                     Plan* plan) {
   extern __shared__ __align__(128) uint32_t s_hist[];
   __shared__ uint32_t s_max[kPasses];
+  uint32_t not_min = 0, max_key = 0;
+  for (int i = blockIdx.x * kHistThreads + threadIdx.x; i < kCountValues; i += gridDim.x * kHistThreads)
+    plan->values[i] = 0;
   for (int i = threadIdx.x; i < kPasses * kBuckets * 32; i += kHistThreads) s_hist[i] = 0;
   const uint32_t m = count ? (uint32_t)*count : (uint32_t)n;
   __syncthreads();
@@ -518,6 +539,8 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
   uint32_t* col = s_hist + lane;
   auto add = [&](uint32_t k) {
     k ^= flip;
+    not_min = max(not_min, ~k);
+    max_key = max(max_key, k);
 #pragma unroll
     for (int p = 0; p < kPasses; ++p) atomicAdd(col + (p * kBuckets + ((k >> (8 * p)) & 255u)) * 32, 1u);
   };
@@ -548,6 +571,14 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
     for (int k = 0; k < 32; ++k) sum += s_hist[threadIdx.x * 32 + ((lane + k) & 31)];
     if (sum) atomicAdd(&ctl->hist[threadIdx.x], sum);
   }
+  if (in_place) {
+    not_min = __reduce_max_sync(0xffffffffu, not_min);
+    max_key = __reduce_max_sync(0xffffffffu, max_key);
+    if (lane == 0) {
+      atomicMax(&ctl->range[0], not_min);
+      atomicMax(&ctl->range[1], max_key);
+    }
+  }
   if (!last_cta(&ctl->done[2], gridDim.x)) return;
   uint32_t* counts = s_hist;  // reused
   __syncthreads();
@@ -561,6 +592,10 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
     warp_scan_256(counts + p * kBuckets, plan->offsets + p * kBuckets);
   }
   if (threadIdx.x == 0) {
+    const volatile Control* c = ctl;
+    const uint32_t lo = ~c->range[0], hi = c->range[1];
+    plan->counting = in_place && hi - lo < (uint32_t)kCountValues ? (int)(hi - lo) + 1 : 0;
+    plan->lowest = lo;
     int active = 0;
     bool skip[kPasses];
     for (int p = 0; p < kPasses; ++p) active += !(skip[p] = s_max[p] == m);
@@ -673,6 +708,7 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 constexpr int kDigitThreads = 512;
 constexpr int kDigitWarps = kDigitThreads / 32;
 constexpr int kDigitTile = kDigitThreads * kItems;  // 8192 keys
+static_assert(kCountValues <= 2 * kDigitTile, "the tile buffers hold the value counters");
 // shared memory: two tile buffers, per-warp counts and peer masks, the run
 // starts and offsets, 8 warp totals, two mbarriers and the next tile's index
 constexpr int kDigitSmemBytes = (2 * kDigitTile + 2 * kDigitWarps * kBuckets + 2 * kBuckets + 8) * 4 + 32;
@@ -682,6 +718,93 @@ constexpr int kDigitSmemBytes = (2 * kDigitTile + 2 * kDigitWarps * kBuckets + 2
 __device__ __forceinline__ uint32_t digit_tile_bytes(int t, int m) {
   const int valid = min(kDigitTile, m - t * kDigitTile);
   return (uint32_t)(valid / 4 * 16);
+}
+
+// ---- few values ----------------------------------------------------------------
+// Keys of few different values need no passes: the first pass's launch counts
+// each value and the second's writes the runs (four launches over 2^26 keys of
+// 201 values took 1490 us, as every lane's digit met in two words; counted,
+// 290).  The counters lie in the CTA's shared memory, one per lane and value
+// where there is room for that, so that frequent values do not queue.
+__device__ __forceinline__ void count_values(const uint32_t* keys, int n, uint32_t flip, Plan* plan, uint32_t* smem) {
+  const int values = plan->counting, lane = threadIdx.x & 31;
+  const uint32_t lo = plan->lowest;
+  const bool by_lane = values * 32 <= kCountValues;
+  const int words = by_lane ? values * 32 : values, scale = by_lane ? 32 : 1, col = by_lane ? lane : 0;
+  for (int i = threadIdx.x; i < words; i += kDigitThreads) smem[i] = 0;
+  __syncthreads();
+  const uint32_t step = gridDim.x * kDigitThreads;
+  for (uint32_t i = blockIdx.x * kDigitThreads + threadIdx.x; i < (uint32_t)n; i += 4 * step) {  // n < 2^30
+    uint32_t k[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) k[r] = i + r * step < (uint32_t)n ? (__ldg(keys + i + r * step) ^ flip) - lo : ~0u;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (k[r] != ~0u) atomicAdd(&smem[k[r] * scale + col], 1u);
+  }
+  __syncthreads();
+  for (int v = threadIdx.x; v < values; v += kDigitThreads) {
+    uint32_t sum = 0;
+    if (by_lane) {
+#pragma unroll 8
+      for (int k = 0; k < 32; ++k) sum += smem[v * 32 + ((lane + k) & 31)];
+    } else {
+      sum = smem[v];
+    }
+    if (sum) atomicAdd(&plan->values[v], sum);
+  }
+}
+
+// Every CTA scans the counts and writes its part of the runs.
+__device__ __forceinline__ void write_values(uint32_t* out, int n, uint32_t flip, const Plan* plan, uint32_t* smem) {
+  __shared__ uint32_t s_warp[kDigitWarps];
+  const int values = plan->counting, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lo = plan->lowest;
+  // smem[v]: the first position of value v; thread t scans `per` values
+  constexpr int kPer = kCountValues / kDigitThreads;
+  for (int v = threadIdx.x; v < kCountValues; v += kDigitThreads) smem[v] = v < values ? plan->values[v] : 0u;
+  __syncthreads();
+  uint32_t sum = 0;
+  for (int k = 0; k < kPer; ++k) sum += smem[threadIdx.x * kPer + ((k + lane) & (kPer - 1))];
+  uint32_t incl = sum;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += t;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  uint32_t run = incl - sum + __reduce_add_sync(0xffffffffu, lane < warp ? s_warp[lane] : 0u);  // warp < 16
+  for (int k = 0; k < kPer; ++k) {
+    uint32_t* at = smem + threadIdx.x * kPer + k;
+    const uint32_t c = *at;
+    *at = run;
+    run += c;
+  }
+  __syncthreads();
+  // each thread four neighbouring positions at a time: the value of the first
+  // by bisection (the last value that starts at or before it and has keys),
+  // the others' by stepping on
+  const uint32_t step = gridDim.x * kDigitThreads * 4u;
+  const bool whole = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  for (uint32_t p = (blockIdx.x * kDigitThreads + threadIdx.x) * 4u; p < (uint32_t)n; p += step) {
+    int v = 0;
+    for (int half = kCountValues / 2; half > 0; half >>= 1)
+      if (v + half < values && smem[v + half] <= p) v += half;
+    uint32_t q[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      while (v + 1 < values && smem[v + 1] <= p + r) ++v;
+      q[r] = (lo + (uint32_t)v) ^ flip;
+    }
+    if (whole && p + 4 <= (uint32_t)n) {
+      *reinterpret_cast<uint4*>(out + p) = make_uint4(q[0], q[1], q[2], q[3]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (p + r < (uint32_t)n) out[p + r] = q[r];
+    }
+  }
 }
 
 // Key `li` of a partial tile of `valid` keys: in shared memory, or past the last
@@ -728,10 +851,9 @@ struct DigitBuffers {
   uint32_t *out0, *b1, *b2;
 };
 
-__global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const DigitBuffers bufs, int n, const int* count,
-                                                              int pass, uint32_t flip, const Plan* plan,
-                                                              unsigned long long* status, int* tile_counter,
-                                                              uint32_t tag, int* err) {
+__device__ __forceinline__ void digit_kernel_cta(const DigitBuffers bufs, int n, const int* count, int pass,
+                                                 uint32_t flip, Plan* plan, unsigned long long* status,
+                                                 int* tile_counter, uint32_t tag, int* err) {
   extern __shared__ __align__(128) uint32_t smem[];
   uint32_t* s_warp = smem + 2 * kDigitTile;         // [warp][digit] counts, then offsets
   uint32_t* s_peers = s_warp + kDigitWarps * kBuckets;  // [warp][digit] peer masks of a round
@@ -740,6 +862,11 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const DigitBuff
   uint32_t* s_wsum = s_off + kBuckets;                  // per digit warp: its digits' counts summed
   unsigned long long* s_bar = reinterpret_cast<unsigned long long*>(s_wsum + 8);
   int* s_next = reinterpret_cast<int*>(s_bar + 2);
+  if (plan->counting) {
+    if (pass == 0) count_values(bufs.in0, n, 0x80000000u, plan, smem);
+    if (pass == 1) write_values(bufs.out0, n, 0x80000000u, plan, smem);
+    return;
+  }
   if (plan->skip[pass]) return;
   const int m = count ? *count : n;
   const int shift = 8 * pass;
@@ -798,7 +925,8 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const DigitBuff
     }
     phases ^= 1u << b;
     const int next = *s_next;
-    if (threadIdx.x == 0 && (long long)next * kDigitTile < m)  // the other buffer was drained before the last tile ended
+    // the other buffer was drained before the last tile ended
+    if (threadIdx.x == 0 && (long long)next * kDigitTile < m)
       bulk_load(smem + (b ^ 1) * kDigitTile, in + (size_t)next * kDigitTile, digit_tile_bytes(next, m), &s_bar[b ^ 1]);
     // per digit: exclusive prefix over warps and the tile's count; the count
     // is published at once so later tiles' look-backs can pass this one
@@ -888,6 +1016,12 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const DigitBuff
     b ^= 1;
   }
 }
+__global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const DigitBuffers bufs, int n, const int* count,
+                                  int pass, uint32_t flip, Plan* plan, unsigned long long* status,
+                                  int* tile_counter, uint32_t tag, int* err, const DoneFlag done) {
+  digit_kernel_cta(bufs, n, count, pass, flip, plan, status, tile_counter, tag, err);
+  publish(done);
+}
 
 // ---- one CTA --------------------------------------------------------------------
 // Up to kSmall keys stay in one CTA: a chain of launches costs 40 to 80 us
@@ -971,7 +1105,7 @@ __device__ __forceinline__ void cta_range(uint32_t& lo, uint32_t& hi) {
 }
 
 template <int kRounds>
-__global__ void __launch_bounds__(kSmallThreads, 1) small_sort_kernel(int32_t* data, int n) {
+__device__ __forceinline__ void small_sort_kernel_cta(int32_t* data, int n) {
   extern __shared__ __align__(128) uint32_t smem[];
   uint32_t k[kRounds], lo = 0xffffffffu, hi = 0;
 #pragma unroll
@@ -993,12 +1127,17 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_sort_kernel(int32_t* d
   cta_sort<kRounds>(smem, 32 - __clz((int)(hi - lo)));
   for (int i = threadIdx.x; i < n; i += kSmallThreads) data[i] = (int32_t)((smem[i] + lo) ^ 0x80000000u);
 }
+template <int kRounds>
+__global__ void __launch_bounds__(kSmallThreads, 1) small_sort_kernel(int32_t* data, int n, const DoneFlag done) {
+  small_sort_kernel_cta<kRounds>(data, n);
+  publish(done);
+}
 
 // Feedback unique of up to kSmall words: NO_HIT words (and the places past n)
 // become a key above every other.  result[0] = the unique count.
 template <int kRounds>
-__global__ void __launch_bounds__(kSmallThreads, 1) small_unique_kernel(const int32_t* words, int n, int nib,
-                                                                       Divider div, int32_t* out, int* result) {
+__device__ __forceinline__ void small_unique_kernel_cta(const int32_t* words, int n, int nib, Divider div,
+                                                        int32_t* out, int* result) {
   extern __shared__ __align__(128) uint32_t smem[];
   __shared__ uint32_t s_warp[kSmallWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1056,16 +1195,21 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_unique_kernel(const in
     result[1] = kPathEmpty;
   }
 }
+template <int kRounds>
+__global__ void __launch_bounds__(kSmallThreads, 1) small_unique_kernel(const int32_t* words, int n, int nib,
+                                  Divider div, int32_t* out, int* result, const DoneFlag done) {
+  small_unique_kernel_cta<kRounds>(words, n, nib, div, out, result);
+  publish(done);
+}
 
 // ---- unique of sorted keys -----------------------------------------------------
 // Persistent like digit_kernel, and pipelined the same way: a tile's run-start
 // keys are compacted into shared memory (each warp into its own range), the
 // next tile (claimed at the start of this one) is loaded, and only then does
 // the tile's look-back for its output position run.
-__global__ void __launch_bounds__(kThreads) unique_kernel(const uint32_t* keys_a, const uint32_t* keys_b,
-                                                          Control* ctl, const Plan* plan, int32_t* out,
-                                                          unsigned long long* status, int* result, uint32_t tag,
-                                                          int* err) {
+__device__ __forceinline__ void unique_kernel_cta(const uint32_t* keys_a, const uint32_t* keys_b, Control* ctl,
+                                                  const Plan* plan, int32_t* out, unsigned long long* status,
+                                                  int* result, uint32_t tag, int* err) {
   __shared__ int s_tile;
   __shared__ uint32_t s_warp[kWarps + 1];
   __shared__ uint32_t s_excl;
@@ -1134,6 +1278,12 @@ __global__ void __launch_bounds__(kThreads) unique_kernel(const uint32_t* keys_a
     if (next_base >= m) return;
     tile = next;
   }
+}
+__global__ void __launch_bounds__(kThreads) unique_kernel(const uint32_t* keys_a, const uint32_t* keys_b,
+                                  Control* ctl, const Plan* plan, int32_t* out, unsigned long long* status,
+                                  int* result, uint32_t tag, int* err, const DoneFlag done) {
+  unique_kernel_cta(keys_a, keys_b, ctl, plan, out, status, result, tag, err);
+  publish(done);
 }
 
 // ---- unique by bitmap ------------------------------------------------------------
@@ -1328,12 +1478,17 @@ __device__ __forceinline__ void emit_bitmap(const uint32_t* bitmap, Control* ctl
   }
 }
 
-__global__ void __launch_bounds__(kShareThreads) emit_kernel(const uint32_t* bitmap, Control* ctl, Plan* plan,
-                                                             int32_t* out, int* result, int* err) {
+__device__ __forceinline__ void emit_kernel_cta(const uint32_t* bitmap, Control* ctl, Plan* plan, int32_t* out,
+                                                int* result, int* err) {
   extern __shared__ __align__(128) uint32_t s_words[];
   __shared__ uint32_t s_warp[kShareWarps];
   if (plan->path != kPathPartition) return;
   emit_bitmap(bitmap, ctl, plan, gridDim.x, s_words, s_warp, out, result, err);
+}
+__global__ void __launch_bounds__(kShareThreads) emit_kernel(const uint32_t* bitmap, Control* ctl, Plan* plan,
+                                  int32_t* out, int* result, int* err, const DoneFlag done) {
+  emit_kernel_cta(bitmap, ctl, plan, out, result, err);
+  publish(done);
 }
 
 // Sets the keys' bits straight in the bitmap, then writes its values.  Keys
@@ -1344,9 +1499,8 @@ __global__ void __launch_bounds__(kShareThreads) emit_kernel(const uint32_t* bit
 // bitmap each thread looks at a bit before it sets it, one key at a time so
 // that the looks see the bits set before.
 static_assert(kDirectSliceWords * 4 >= kEmitSmemBytes, "the slice's memory serves the writing too");
-__global__ void __launch_bounds__(kShareThreads) direct_bitmap_kernel(const uint32_t* keys, Control* ctl, Plan* plan,
-                                                                      uint32_t* bitmap, int32_t* out, int* result,
-                                                                      int* err) {
+__device__ __forceinline__ void direct_bitmap_kernel_cta(const uint32_t* keys, Control* ctl, Plan* plan,
+                                                         uint32_t* bitmap, int32_t* out, int* result, int* err) {
   extern __shared__ __align__(128) uint32_t s_slice[];
   __shared__ uint32_t s_warp[kShareWarps];
   if (plan->path != kPathDirect) return;
@@ -1384,6 +1538,11 @@ __global__ void __launch_bounds__(kShareThreads) direct_bitmap_kernel(const uint
   }
   if (!grid_barrier(&ctl->barrier[0], ctas, err)) return;
   emit_bitmap(bitmap, ctl, plan, ctas, s_slice, s_warp, out, result, err);
+}
+__global__ void __launch_bounds__(kShareThreads) direct_bitmap_kernel(const uint32_t* keys, Control* ctl, Plan* plan,
+                                  uint32_t* bitmap, int32_t* out, int* result, int* err, const DoneFlag done) {
+  direct_bitmap_kernel_cta(keys, ctl, plan, bitmap, out, result, err);
+  publish(done);
 }
 
 // Histogram of the range buckets (top 8 bits of key - min) of the kept keys,
@@ -1621,8 +1780,8 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-__global__ void __launch_bounds__(kScanBlock, 1) scan_kernel(int32_t* data, int n, int rows,
-                                                             unsigned long long* status, uint32_t tag, int* err) {
+__device__ __forceinline__ void scan_kernel_cta(int32_t* data, int n, int rows, unsigned long long* status,
+                                                uint32_t tag, int* err) {
   extern __shared__ __align__(128) uint32_t s_tiles[];
   __shared__ unsigned long long s_bar[kScanBuffers];        // a tile has landed
   __shared__ unsigned long long s_collected[2], s_used[2];  // a round's sums are in s_round; they are used
@@ -1761,6 +1920,11 @@ __global__ void __launch_bounds__(kScanBlock, 1) scan_kernel(int32_t* data, int 
     if (t >= tiles) return;
   }
 }
+__global__ void __launch_bounds__(kScanBlock, 1) scan_kernel(int32_t* data, int n, int rows,
+                                  unsigned long long* status, uint32_t tag, int* err, const DoneFlag done) {
+  scan_kernel_cta(data, n, rows, status, tag, err);
+  publish(done);
+}
 
 // Copy of an array that does not start on a 16-byte boundary (the digit passes
 // bring their tiles in by 16-byte copies).
@@ -1804,12 +1968,12 @@ cudaError_t launch_digit_hist(const uint32_t* keys, int n, const int* count, uin
 // digit's upper bit is flipped as it is read).
 cudaError_t launch_digits(const DigitBuffers& bufs, int n, const int* count, bool sign_flip,
                           const SortScratchLayout& l, unsigned long long* status, uint32_t epoch, int* err,
-                          cudaStream_t s) {
+                          const DoneFlag& done, cudaStream_t s) {
   const int grid = persistent_grid<digit_kernel>(tiles_of(n, kDigitTile), kDigitThreads, kDigitSmemBytes);
   for (int p = 0; p < kPasses; ++p) {
     digit_kernel<<<grid, kDigitThreads, kDigitSmemBytes, s>>>(
         bufs, n, count, p, sign_flip && p == kPasses - 1 ? 0x80u : 0u, l.plan, status, &l.control->tiles[p],
-        epoch * 8u + (uint32_t)p, err);
+        epoch * 8u + (uint32_t)p, err, p == kPasses - 1 ? done : DoneFlag{});
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -1817,17 +1981,18 @@ cudaError_t launch_digits(const DigitBuffers& bufs, int n, const int* count, boo
 }
 
 template <int kRounds>
-void launch_small_sort(int32_t* data, int n, cudaStream_t s) {
+void launch_small_sort(int32_t* data, int n, const DoneFlag& done, cudaStream_t s) {
   constexpr int bytes = small_smem_bytes<kRounds>();
   const int grid = persistent_grid<small_sort_kernel<kRounds>>(1, kSmallThreads, bytes);
-  small_sort_kernel<kRounds><<<grid, kSmallThreads, bytes, s>>>(data, n);
+  small_sort_kernel<kRounds><<<grid, kSmallThreads, bytes, s>>>(data, n, done);
 }
 template <int kRounds>
-void launch_small_unique(const int32_t* words, int n, int nib, int32_t* out, int* result, cudaStream_t s) {
+void launch_small_unique(const int32_t* words, int n, int nib, int32_t* out, int* result, const DoneFlag& done,
+                         cudaStream_t s) {
   constexpr int bytes = small_smem_bytes<kRounds>();
   const int grid = persistent_grid<small_unique_kernel<kRounds>>(1, kSmallThreads, bytes);
   small_unique_kernel<kRounds><<<grid, kSmallThreads, bytes, s>>>(words, n, nib, make_divider((uint32_t)nib), out,
-                                                                 result);
+                                                                 result, done);
 }
 
 // Waits, as a look-back does, on a word that nothing publishes: the wait must
@@ -1863,11 +2028,11 @@ size_t scan_status_bytes(int n) { return ((size_t)tiles_of(n, kScanTile) + 1024)
 
 cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t* unique_out, void* scratch,
                                    unsigned long long* status, uint32_t epoch, int* result, int* err,
-                                   cudaStream_t s) {
+                                   const DoneFlag& done, cudaStream_t s) {
   if (n <= kSmall) {
-    if (n <= 2 * kSmallThreads) launch_small_unique<2>(words, n, nib, unique_out, result, s);
-    else if (n <= 4 * kSmallThreads) launch_small_unique<4>(words, n, nib, unique_out, result, s);
-    else launch_small_unique<kSmall / kSmallThreads>(words, n, nib, unique_out, result, s);
+    if (n <= 2 * kSmallThreads) launch_small_unique<2>(words, n, nib, unique_out, result, done, s);
+    else if (n <= 4 * kSmallThreads) launch_small_unique<4>(words, n, nib, unique_out, result, done, s);
+    else launch_small_unique<kSmall / kSmallThreads>(words, n, nib, unique_out, result, done, s);
     return cudaGetLastError();
   }
   const SortScratchLayout l = layout(scratch, n);
@@ -1884,7 +2049,8 @@ cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t
   {
     const int grid =
         persistent_grid<direct_bitmap_kernel>(tiles_of(n, kShareThreads), kShareThreads, kDirectSliceWords * 4);
-    void* args[] = {&keys, &control, &plan, &bitmap, &unique_out, &result, &err};
+    DoneFlag d = n <= kDirectWords ? done : DoneFlag{};
+    void* args[] = {&keys, &control, &plan, &bitmap, &unique_out, &result, &err, &d};
     e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(direct_bitmap_kernel), dim3(grid),
                                     dim3(kShareThreads), args, kDirectSliceWords * 4, s);
     if (e != cudaSuccess || n <= kDirectWords) return e;
@@ -1896,7 +2062,8 @@ cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t
                                                                                         l.bitmap);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const int grid = persistent_grid<emit_kernel>(tiles_of(n, kShareThreads), kShareThreads, kEmitSmemBytes);
-  void* args[] = {&bitmap, &control, &plan, &unique_out, &result, &err};
+  DoneFlag d = done;
+  void* args[] = {&bitmap, &control, &plan, &unique_out, &result, &err, &d};
   return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(emit_kernel), dim3(grid),
                                      dim3(kShareThreads), args, kEmitSmemBytes, s);
 }
@@ -1904,24 +2071,26 @@ cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t
 bool feedback_unique_needs_radix(const int* result) { return result[1] == kPathRadix; }
 
 cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scratch, unsigned long long* status,
-                                         uint32_t epoch, int* result, int* err, cudaStream_t s) {
+                                         uint32_t epoch, int* result, int* err, const DoneFlag& done,
+                                         cudaStream_t s) {
   const SortScratchLayout l = layout(scratch, n);
   cudaError_t e;
   if ((e = launch_digit_hist(l.keys_a, n, &l.control->keys, 0u, false, l, s)) != cudaSuccess) return e;
   const DigitBuffers bufs = {l.keys_a, l.keys_a, l.keys_b, nullptr};
-  if ((e = launch_digits(bufs, n, &l.control->keys, false, l, status, epoch, err, s)) != cudaSuccess) return e;
+  if ((e = launch_digits(bufs, n, &l.control->keys, false, l, status, epoch, err, DoneFlag{}, s)) != cudaSuccess)
+    return e;
   unique_kernel<<<persistent_grid<unique_kernel>(tiles_of(n, kTile)), kThreads, 0, s>>>(
-      l.keys_a, l.keys_b, l.control, l.plan, unique_out, status, result, epoch * 8u + 4u, err);
+      l.keys_a, l.keys_b, l.control, l.plan, unique_out, status, result, epoch * 8u + 4u, err, done);
   return cudaGetLastError();
 }
 
 cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch, int* err,
-                            cudaStream_t s) {
+                            const DoneFlag& done, cudaStream_t s) {
   if (n <= 1) return cudaSuccess;
   if (n <= kSmall) {
-    if (n <= 2 * kSmallThreads) launch_small_sort<2>(data, n, s);
-    else if (n <= 4 * kSmallThreads) launch_small_sort<4>(data, n, s);
-    else launch_small_sort<kSmall / kSmallThreads>(data, n, s);
+    if (n <= 2 * kSmallThreads) launch_small_sort<2>(data, n, done, s);
+    else if (n <= 4 * kSmallThreads) launch_small_sort<4>(data, n, done, s);
+    else launch_small_sort<kSmall / kSmallThreads>(data, n, done, s);
     return cudaGetLastError();
   }
   const SortScratchLayout l = layout(scratch, n);
@@ -1935,11 +2104,11 @@ cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long l
     bufs.in0 = l.keys_b;
   }
   if ((e = launch_digit_hist(bufs.in0, n, nullptr, 0x80000000u, true, l, s)) != cudaSuccess) return e;
-  return launch_digits(bufs, n, nullptr, true, l, status, epoch, err, s);
+  return launch_digits(bufs, n, nullptr, true, l, status, epoch, err, done, s);
 }
 
 cudaError_t scan_i32_device(int32_t* data, int n, unsigned long long* status, uint32_t epoch, int* err,
-                            cudaStream_t s) {
+                            const DoneFlag& done, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const int end = n + (int)((reinterpret_cast<uintptr_t>(data) >> 2) & 3u);
   // rows per warp: a full tile per CTA, or what spreads the array over every SM
@@ -1949,10 +2118,11 @@ cudaError_t scan_i32_device(int32_t* data, int n, unsigned long long* status, ui
   uint32_t tag = epoch * 8u + 6u;
   const int grid = std::min(sms, tiles_of(end, rows * kRow));
   if (grid == 1) {
-    scan_kernel<<<1, kScanBlock, kScanSmemBytes, s>>>(data, n, rows, status, tag, err);
+    scan_kernel<<<1, kScanBlock, kScanSmemBytes, s>>>(data, n, rows, status, tag, err, done);
     return cudaGetLastError();
   }
-  void* args[] = {&data, &n, &rows, &status, &tag, &err};
+  DoneFlag d = done;
+  void* args[] = {&data, &n, &rows, &status, &tag, &err, &d};
   return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(scan_kernel), dim3(grid), dim3(kScanBlock), args,
                                      kScanSmemBytes, s);
 }

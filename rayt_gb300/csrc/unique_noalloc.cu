@@ -40,11 +40,11 @@ constexpr int kMaxWords = RAYT_FEEDBACK_UNIQUE_NOALLOC_MAX_WORDS;
 
 // Scratch of the unique for kMaxWords words (feedback_scratch_bytes() is a host
 // function, so the size is computed from the same layout rules here: two key
-// arrays of (n + 4) words rounded to 256 bytes, and at most 64 KiB of control
+// arrays of (n + 4) words rounded to 256 bytes, and at most 128 KiB of control
 // words and plan), look-back words (256 digits x 8 bytes per 8192-key tile),
 // and a result block: error flag, unique count, path.
 constexpr size_t Up256(size_t v) { return (v + 255) & ~(size_t)255; }
-constexpr size_t kScratchBytes = 2 * Up256((size_t)kMaxWords * 4 + 16) + (64 << 10);
+constexpr size_t kScratchBytes = 2 * Up256((size_t)kMaxWords * 4 + 16) + (128 << 10);
 constexpr size_t kStatusBytes = ((size_t)kMaxWords + 8191) / 8192 * 256 * 8;
 constexpr size_t kResultBytes = 256;
 
@@ -112,10 +112,11 @@ extern "C" int rayt_feedback_unique_noalloc(const int32_t* words, int n, int nod
   int host[3] = {0, 0, 0};
   // the launcher clears the control words it relies on
   RAYT_CUDA_TRY(rayt::feedback_unique_device(words, n, nodes_in_block, unique, scratch, status, epoch, result + 1,
-                                             result, s));
+                                             result, rayt::DoneFlag{}, s));
   if ((rc = rayt::read_result(host, result, s)) != RAYT_OK) return rc;
   if (rayt::feedback_unique_needs_radix(host + 1)) {
-    RAYT_CUDA_TRY(rayt::feedback_unique_radix_device(n, unique, scratch, status, epoch, result + 1, result, s));
+    RAYT_CUDA_TRY(rayt::feedback_unique_radix_device(n, unique, scratch, status, epoch, result + 1, result,
+                                                     rayt::DoneFlag{}, s));
     if ((rc = rayt::read_result(host, result, s)) != RAYT_OK) return rc;
   }
   *unique_count = host[1];

@@ -50,17 +50,17 @@ int LibcRand::Next() {
 // The host looks at the mapped word itself: a kernel's last write arrives some
 // microseconds before the runtime says that the stream has finished.  After
 // two milliseconds it asks the runtime (for an error, and so as not to spin
-// through a long pass).
-int wait_pass(const UniqueResult* r, unsigned int pass, cudaStream_t s) {
+// through long work).
+int wait_word(const unsigned int* word, unsigned int value, cudaStream_t s) {
   using clock = std::chrono::steady_clock;
   const auto until = clock::now() + std::chrono::milliseconds(2);
   do {
     for (int spin = 0; spin < 256; ++spin)
-      if (__atomic_load_n(&r->pass, __ATOMIC_ACQUIRE) == pass) return RAYT_OK;
+      if (__atomic_load_n(word, __ATOMIC_ACQUIRE) == value) return RAYT_OK;
   } while (clock::now() < until);
   RAYT_CUDA_TRY(cudaStreamSynchronize(s));
-  if (__atomic_load_n(&r->pass, __ATOMIC_ACQUIRE) == pass) return RAYT_OK;
-  return fail(RAYT_E_CUDA, "a pass ended without its result");
+  if (__atomic_load_n(word, __ATOMIC_ACQUIRE) == value) return RAYT_OK;
+  return fail(RAYT_E_CUDA, "device work ended without its result");
 }
 
 }  // namespace rayt

@@ -29,6 +29,11 @@ KEYS = {
     "one_digit": lambda rng, n: (0x12003400 + (rng.integers(0, 256, n) << 16)).astype(np.int32),
     "two_digits": lambda rng, n: (rng.integers(0, 256, n) * 0x01000100 - 2**31).astype(np.int64).astype(np.int32),
     "skewed": lambda rng, n: np.where(rng.random(n) < 0.9, np.int32(5), _wide(rng, n)).astype(np.int32),
+    "count_limit": lambda rng, n: (rng.integers(0, 1 << 14, n) - 2**31).astype(np.int64).astype(np.int32),
+    "over_count_limit": lambda rng, n: np.where(np.arange(n) == 1, np.int32(16384 - 77),
+                                                rng.integers(-77, 16384 - 77, n)).astype(np.int32),
+    "by_lane_limit": lambda rng, n: (2**31 - 1 - rng.integers(0, 512, n)).astype(np.int32),
+    "over_by_lane": lambda rng, n: rng.integers(-256, 257, n).astype(np.int32),
     "sorted": lambda rng, n: np.sort(_wide(rng, n)),
 }
 
