@@ -84,6 +84,12 @@ __device__ __forceinline__ bool wait_over(long long& spins, unsigned long long s
 // Sets a call's error flag (device or mapped host memory).
 __device__ __forceinline__ void set_error(int* err) { *(volatile int*)err = 1; }
 
+// Programmatic launches: the kernel after this one may take its place while this
+// one still runs; what it reads of this one's, it reads after its own
+// wait_for_dependency.
+__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_dependency() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // The end of a call's last kernel: the CTA that ends last publishes the call's
 // number to the host.  Every thread of every CTA comes here.
 __device__ __forceinline__ void publish(const DoneFlag& done) {
@@ -530,6 +536,7 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
   extern __shared__ __align__(128) uint32_t s_hist[];
   __shared__ uint32_t s_max[kPasses];
   uint32_t not_min = 0, max_key = 0;
+  dependents_may_start();
   for (int i = blockIdx.x * kHistThreads + threadIdx.x; i < kCountValues; i += gridDim.x * kHistThreads)
     plan->values[i] = 0;
   for (int i = threadIdx.x; i < kPasses * kBuckets * 32; i += kHistThreads) s_hist[i] = 0;
@@ -862,6 +869,15 @@ __device__ __forceinline__ void digit_kernel_cta(const DigitBuffers bufs, int n,
   uint32_t* s_wsum = s_off + kBuckets;                  // per digit warp: its digits' counts summed
   unsigned long long* s_bar = reinterpret_cast<unsigned long long*>(s_wsum + 8);
   int* s_next = reinterpret_cast<int*>(s_bar + 2);
+  // what does not depend on the kernel before runs beside it
+  dependents_may_start();
+  for (int i = threadIdx.x; i < 2 * kDigitWarps * kBuckets; i += kDigitThreads) s_warp[i] = 0;
+  if (threadIdx.x == 0) {
+    mbar_init(&s_bar[0]);
+    mbar_init(&s_bar[1]);
+    mbar_init_fence();
+  }
+  wait_for_dependency();
   if (plan->counting) {
     if (pass == 0) count_values(bufs.in0, n, 0x80000000u, plan, smem);
     if (pass == 1) write_values(bufs.out0, n, 0x80000000u, plan, smem);
@@ -879,11 +895,7 @@ __device__ __forceinline__ void digit_kernel_cta(const DigitBuffers bufs, int n,
   const int w0 = warp * (kItems * 32);  // warp `warp` ranks keys [w0, w0 + 512) of a tile
   const int rows = unstable ? 1 : kDigitWarps;  // rows of counts in use
   uint32_t* s_mine = unstable ? s_warp : s_warp + warp * kBuckets;  // this warp's row
-  for (int i = threadIdx.x; i < 2 * kDigitWarps * kBuckets; i += kDigitThreads) s_warp[i] = 0;
   if (threadIdx.x == 0) {
-    mbar_init(&s_bar[0]);
-    mbar_init(&s_bar[1]);
-    mbar_init_fence();
     const int t = atomicAdd(tile_counter, 1);
     *s_next = t;
     if ((long long)t * kDigitTile < m) bulk_load(smem, in + (size_t)t * kDigitTile, digit_tile_bytes(t, m), &s_bar[0]);
@@ -1971,10 +1983,20 @@ cudaError_t launch_digits(const DigitBuffers& bufs, int n, const int* count, boo
                           const DoneFlag& done, cudaStream_t s) {
   const int grid = persistent_grid<digit_kernel>(tiles_of(n, kDigitTile), kDigitThreads, kDigitSmemBytes);
   for (int p = 0; p < kPasses; ++p) {
-    digit_kernel<<<grid, kDigitThreads, kDigitSmemBytes, s>>>(
-        bufs, n, count, p, sign_flip && p == kPasses - 1 ? 0x80u : 0u, l.plan, status, &l.control->tiles[p],
-        epoch * 8u + (uint32_t)p, err, p == kPasses - 1 ? done : DoneFlag{});
-    const cudaError_t e = cudaGetLastError();
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kDigitThreads);
+    cfg.dynamicSmemBytes = kDigitSmemBytes;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, digit_kernel, bufs, n, count, p,
+                                             sign_flip && p == kPasses - 1 ? 0x80u : 0u, l.plan, status,
+                                             &l.control->tiles[p], epoch * 8u + (uint32_t)p, err,
+                                             p == kPasses - 1 ? done : DoneFlag{});
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
