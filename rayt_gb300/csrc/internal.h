@@ -150,6 +150,20 @@ uchar4 finish_empty(const float* bg);
 // The reference's background (gpu-ray-tracer.cpp:190).
 constexpr float kBackground[4] = {0.0f, (float)(216 / 255.), 1.0f, 1.0f};
 
+// Frames on their way to host memory: image k goes to `host` when no ray of its
+// client faulted (faults[slot] == 0), else nothing happens.
+struct DeliverParams {
+  int images;
+  const int* faults;
+  struct {
+    const uchar4* image;
+    uchar4* host;  // device address of page-locked memory
+    int64_t pixels;
+    int slot;
+  } at[kMaxClients];
+};
+cudaError_t launch_deliver(const DeliverParams& p, cudaStream_t s);
+
 // Faulted-ray records carried from one pass to the next (device arrays).
 struct RayList {
   float4* origin = nullptr;  // xyz advanced to the fault, w LOD bias
@@ -201,7 +215,8 @@ struct UniqueFromBitsParams {
   PassState* previous;   // of the pass before
   bool later;            // the pass traced the rays of the pass before (pixels without one have no word)
   int total_pixels;
-  int* client_faults;    // served mode: per client, copied and cleared; may be null
+  const int* client_faults;  // served mode: per client, copied; may be null
+  int* next_client_faults;   // and the next tick's, cleared
   unsigned int* passes;  // passes done, on the device
   int32_t* unique_out;   // room for fault bits + hit bits + 1
   UniqueResult* result;

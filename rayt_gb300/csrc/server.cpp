@@ -68,6 +68,7 @@ class Server {
     int64_t pixels = 0;      // w * h rounded up to 64
     uint64_t in_flight = 0;  // request being rendered (0: none)
     uchar4* host = nullptr;  // pinned copy of the last finished frame (deliver_to_host)
+    uchar4* host_dev = nullptr;  // its device address
     uchar4* stage = nullptr; // device copy of a finished frame on its way to `host`
     float* coords = nullptr; // pixel_coords(w, h) in device memory
   };
@@ -108,7 +109,7 @@ class Server {
   int32_t* d_unique_ = nullptr;
   UniqueResult* h_result_ = nullptr;  // mapped
   UniqueResult* d_result_ = nullptr;
-  int* d_client_faults_ = nullptr;
+  int* d_client_faults_[2] = {};  // by tick parity; a tick's unique kernel clears the next one's
   int tick_ = 0;
   int carried_ = 0;          // faulted rays carried into the next tick
   // deliver_to_host: finished frames are copied to their client's stage on
@@ -118,6 +119,14 @@ class Server {
   // requests as done once their images are on the host.
   cudaStream_t copy_s_ = nullptr;
   cudaEvent_t staged_ev_ = nullptr, copied_ev_ = nullptr;
+  // A tick whose new requests' rays fill several of these launches traces them
+  // group by group, and the frames of all but the last group are copied to the
+  // host beside the groups after them, those that turn out to be done (no
+  // fault).
+  static constexpr int64_t kGroupRays = 4 << 20;
+  static constexpr int kMaxGroups = 8;
+  cudaEvent_t group_ev_ = nullptr, early_ev_ = nullptr;
+  bool early_pending_ = false;  // early_ev_ marks copies from framebuffers
   bool copy_pending_ = false;  // copied_ev_ marks the last delivery
   struct Delivery {
     Server* server;
@@ -164,10 +173,10 @@ int Server::Init(Cache* cache, const rayt_server_config& cfg) {
       return fail(RAYT_E_OOM, "ray record allocation failed");
   fault_words_ = (int)((cache->tree_blocks() + 31) / 32);
   hit_words_ = (int)(((uint64_t)cache->max_blocks() * 2 + 31) / 32);
-  state_ints_ = 2 * (size_t)kPassInts + (size_t)fault_words_ + hit_words_ + kMaxClients;
+  state_ints_ = 2 * (size_t)kPassInts + (size_t)fault_words_ + hit_words_ + 2 * kMaxClients;
   if (cudaMalloc(&d_state_, state_ints_ * 4) != cudaSuccess || cudaMalloc(&d_passes_, 4) != cudaSuccess)
     return fail(RAYT_E_OOM, "feedback state allocation failed");
-  d_client_faults_ = d_state_ + state_ints_ - kMaxClients;
+  for (int k = 0; k < 2; ++k) d_client_faults_[k] = d_state_ + state_ints_ - (k + 1) * kMaxClients;
   const size_t bit_words = (size_t)fault_words_ + hit_words_;
   if (cudaHostAlloc(&h_unique_, (bit_words * 32 + 1) * 4, cudaHostAllocMapped) != cudaSuccess ||
       cudaHostAlloc(&h_result_, sizeof(UniqueResult), cudaHostAllocMapped) != cudaSuccess)
@@ -182,6 +191,8 @@ int Server::Init(Cache* cache, const rayt_server_config& cfg) {
     RAYT_CUDA_TRY(cudaStreamCreateWithFlags(&copy_s_, cudaStreamNonBlocking));
     RAYT_CUDA_TRY(cudaEventCreateWithFlags(&staged_ev_, cudaEventDisableTiming));
     RAYT_CUDA_TRY(cudaEventCreateWithFlags(&copied_ev_, cudaEventDisableTiming));
+    RAYT_CUDA_TRY(cudaEventCreateWithFlags(&group_ev_, cudaEventDisableTiming));
+    RAYT_CUDA_TRY(cudaEventCreateWithFlags(&early_ev_, cudaEventDisableTiming));
   }
   RAYT_CUDA_TRY(cudaStreamSynchronize(s_));
   return RAYT_OK;
@@ -196,6 +207,8 @@ Server::~Server() {
   }
   if (staged_ev_) cudaEventDestroy(staged_ev_);
   if (copied_ev_) cudaEventDestroy(copied_ev_);
+  if (group_ev_) cudaEventDestroy(group_ev_);
+  if (early_ev_) cudaEventDestroy(early_ev_);
   cudaFree(d_images_);
   for (auto& l : lists_) {
     cudaFree(l.origin);
@@ -259,7 +272,8 @@ int Server::AddClient(int w, int h, int* id) {
   if (Alloc(pixels, &base) != RAYT_OK) return fail(RAYT_E_LIMIT, "not admitted: no free framebuffer memory");
   Client& c = clients_[slot];
   if (cfg_.deliver_to_host && !c.host &&
-      cudaHostAlloc(&c.host, (size_t)w * h * 4, cudaHostAllocDefault) != cudaSuccess)
+      (cudaHostAlloc(&c.host, (size_t)w * h * 4, cudaHostAllocMapped) != cudaSuccess ||
+       cudaHostGetDevicePointer((void**)&c.host_dev, c.host, 0) != cudaSuccess))
     return fail(RAYT_E_OOM, "pinned host image allocation failed");
   if (cfg_.deliver_to_host) {
     if (copy_s_) RAYT_CUDA_TRY(cudaStreamSynchronize(copy_s_));  // an earlier client's stage may still be read
@@ -351,7 +365,7 @@ TraceParams Server::Params(int k) const {
   p.lanes = 32;
   p.refill = 32;
   p.restart = 1;
-  p.client_faults = d_client_faults_;
+  p.client_faults = d_client_faults_[k];
   // client slots by framebuffer base (free slots get an empty range at the end)
   std::vector<std::pair<int64_t, int>> order;
   for (int i = 0; i < (int)clients_.size(); ++i)
@@ -409,6 +423,7 @@ int Server::Step(int* finished) {
   int64_t rays_tick = carried_;
   // first passes of newly admitted requests (one launch per 64 views)
   std::vector<ViewDesc> views;
+  std::vector<int> view_client;
   for (Flight& f : flights_)
     if (f.fresh) {
       const Client& c = clients_[f.client];
@@ -421,19 +436,30 @@ int Server::Step(int* finished) {
       v.lod = cfg_.lod_voxel_size;
       v.pix_base = (int)c.base;
       views.push_back(v);
+      view_client.push_back(f.client);
       rays_tick += (int64_t)c.w * c.h;
     }
-  for (size_t g = 0; g < views.size(); g += kViewsPerLaunch) {
+  // the framebuffers the tick writes are not read by the last tick's copies
+  // any more (they ran beside its traversal)
+  if (early_pending_) RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, early_ev_, 0));
+  early_pending_ = false;
+  int64_t fresh_rays = 0;
+  for (const ViewDesc& v : views) fresh_rays += (int64_t)v.width * v.height;
+  const int64_t groups = cfg_.deliver_to_host ? std::min<int64_t>(kMaxGroups, fresh_rays / kGroupRays) : 1;
+  const int64_t group_rays = groups > 1 ? (fresh_rays + groups - 1) / groups : fresh_rays;
+  std::vector<char> early(clients_.size(), 0);  // clients whose frames were sent on their way below
+  for (size_t g = 0; g < views.size();) {
     TraceParams q = p;
-    const int n = (int)std::min<size_t>(kViewsPerLaunch, views.size() - g);
-    int64_t tiles = 0;
-    for (int i = 0; i < n; ++i) {
-      ViewDesc& v = views[g + i];
+    int n = 0;
+    int64_t tiles = 0, rays = 0;
+    for (; g + n < views.size() && n < kViewsPerLaunch && (n == 0 || rays < group_rays); ++n) {
+      ViewDesc& v = views[g + n];
       v.tiles_x = (v.width + 3) / 4;
       v.tiles_x_inv = reciprocal(v.tiles_x);
       v.tile_base = (int)tiles;
       tiles += (int64_t)v.tiles_x * ((v.height + 7) / 8);
-      q.views[i] = v;
+      rays += (int64_t)v.width * v.height;
+      q.views[n] = v;
     }
     q.n_views = n;
     q.total_tiles = (int)tiles;
@@ -442,6 +468,26 @@ int Server::Step(int* finished) {
     q.lanes = trace_lanes(true, (int)tiles * 32);
     RAYT_CUDA_TRY(launch_trace(q, true, false, (int)tiles * 32, 0, s_));
     ++stats.kernel_launches;
+    if (groups > 1 && g + n < views.size()) {
+      DeliverParams d{};
+      d.faults = d_client_faults_[k];
+      for (int i = 0; i < n; ++i) {
+        const int id = view_client[g + i];
+        const Client& c = clients_[id];
+        d.at[d.images].image = d_images_ + c.base;
+        d.at[d.images].host = c.host_dev;
+        d.at[d.images].pixels = (int64_t)c.w * c.h;
+        d.at[d.images++].slot = slot_of_client[id];
+        early[id] = 1;
+      }
+      RAYT_CUDA_TRY(cudaEventRecord(group_ev_, s_));
+      RAYT_CUDA_TRY(cudaStreamWaitEvent(copy_s_, group_ev_, 0));
+      RAYT_CUDA_TRY(launch_deliver(d, copy_s_));
+      RAYT_CUDA_TRY(cudaEventRecord(early_ev_, copy_s_));
+      early_pending_ = true;
+      ++stats.kernel_launches;
+    }
+    g += n;
   }
   // faulted rays of older requests (finished instead for finishing ones)
   if (carried_ > 0) {
@@ -461,7 +507,8 @@ int Server::Step(int* finished) {
   u.words = words(k);
   u.previous = words(1 - k);
   u.total_pixels = (int)std::min<int64_t>(rays_tick, 1 << 30);
-  u.client_faults = d_client_faults_;
+  u.client_faults = d_client_faults_[k];
+  u.next_client_faults = d_client_faults_[1 - k];
   u.passes = d_passes_;
   u.unique_out = d_unique_;
   u.result = d_result_;
@@ -542,13 +589,15 @@ int Server::Step(int* finished) {
       if (copy_pending_) RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, copied_ev_, 0));
       for (const Flight& f : ended) {
         const Client& c = clients_[f.client];
-        RAYT_CUDA_TRY(cudaMemcpyAsync(c.stage, d_images_ + c.base, (size_t)c.w * c.h * 4, cudaMemcpyDeviceToDevice, s_));
+        if (!early[f.client])
+          RAYT_CUDA_TRY(cudaMemcpyAsync(c.stage, d_images_ + c.base, (size_t)c.w * c.h * 4, cudaMemcpyDeviceToDevice, s_));
       }
       RAYT_CUDA_TRY(cudaEventRecord(staged_ev_, s_));
       RAYT_CUDA_TRY(cudaStreamWaitEvent(copy_s_, staged_ev_, 0));
       for (const Flight& f : ended) {
         const Client& c = clients_[f.client];
-        RAYT_CUDA_TRY(cudaMemcpyAsync(c.host, c.stage, (size_t)c.w * c.h * 4, cudaMemcpyDeviceToHost, copy_s_));
+        if (!early[f.client])
+          RAYT_CUDA_TRY(cudaMemcpyAsync(c.host, c.stage, (size_t)c.w * c.h * 4, cudaMemcpyDeviceToHost, copy_s_));
         stats.bytes_d2h += (int64_t)c.w * c.h * 4;
       }
       RAYT_CUDA_TRY(cudaEventRecord(copied_ev_, copy_s_));

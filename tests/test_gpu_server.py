@@ -134,6 +134,27 @@ def test_served_delivery_through_client_changes(trees):
     srv.close()
 
 
+@pytest.mark.parametrize("max_blocks", [0, 640])
+def test_served_delivery_in_groups(trees, max_blocks):
+    """A tick large enough to be traced group by group (three frames of a little
+    over 2^22 pixels): the frames of all but the last group go to the host
+    beside the groups after them, unless a ray of theirs faulted; every
+    delivered image equals the resident oracle frame."""
+    w, h, frames = 2304, 1824, 3
+    pixels = 3 * w * h
+    ld, cm, srv = _server(trees, max_blocks=max_blocks, deliver_to_host=True, framebuffer_bytes=4 * pixels,
+                          max_rays_in_flight=pixels)
+    ids = [srv.add_client(w, h) for _ in range(3)]
+    for f in range(frames):
+        mats = [_matrix(_cam(70.0 * v + 15.0 * (f % 2), v), w, h) for v in range(3)]
+        reqs = [srv.submit(c, m) for c, m in zip(ids, mats)]
+        for r in reqs:
+            assert not srv.wait(r)["truncated"]
+        for v, (c, m) in enumerate(zip(ids, mats)):
+            np.testing.assert_array_equal(srv.host_image(c), _resident(trees, w, h, m), err_msg="%d %d" % (v, f))
+    srv.close()
+
+
 def test_served_admission_limits(trees):
     # framebuffer memory admits clients: 2 frames of 128x128 fit, a third does not
     ld, cm, srv = _server(trees, framebuffer_bytes=2 * 128 * 128 * 4)
