@@ -137,7 +137,7 @@ def test_served_delivery_through_client_changes(trees):
 @pytest.mark.parametrize("max_blocks", [0, 640])
 def test_served_delivery_in_groups(trees, max_blocks):
     """A tick large enough to be traced group by group (three frames of a little
-    over 2^22 pixels): the frames of all but the last group go to the host
+    over 2^22 pixels each): the frames of all but the last group go to the host
     beside the groups after them, unless a ray of theirs faulted; every
     delivered image equals the resident oracle frame."""
     w, h, frames = 2304, 1824, 3
