@@ -254,8 +254,14 @@ cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scrat
                                          cudaStream_t s);
 size_t sort_scratch_bytes(int n);
 size_t sort_status_bytes(int n);
-cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch, int* err,
-                            const DoneFlag& done, cudaStream_t s);
+// Sorts in place; or, where *again (mapped host memory, cleared by the caller) is
+// set, sort_needs_passes(again), leaves some order of the same keys, which
+// sort_passes_device, on the same memory, then sorts.
+cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch,
+                            int* again, int* err, const DoneFlag& done, cudaStream_t s);
+bool sort_needs_passes(const int* again);
+cudaError_t sort_passes_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch,
+                               int* err, const DoneFlag& done, cudaStream_t s);
 size_t scan_status_bytes(int n);
 cudaError_t scan_i32_device(int32_t* data, int n, unsigned long long* status, uint32_t epoch, int* err,
                             const DoneFlag& done, cudaStream_t s);

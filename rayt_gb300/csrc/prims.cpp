@@ -140,9 +140,15 @@ int rayt_sort_i32(int32_t* data, int n, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   rayt::Device* d = nullptr;
   uint32_t epoch = 0;
-  const int rc = rayt::begin(rayt::sort_scratch_bytes(n), rayt::sort_status_bytes(n), s, &d, &epoch);
+  int rc = rayt::begin(rayt::sort_scratch_bytes(n), rayt::sort_status_bytes(n), s, &d, &epoch);
   if (rc != RAYT_OK) return rc;
-  RAYT_CUDA_TRY(rayt::sort_i32_device(data, n, d->scratch, d->status, epoch, d->host_dev, rayt::next_done(*d), s));
+  int *err = d->host_dev, *again = d->host_dev + 1;
+  d->host[1] = 0;
+  RAYT_CUDA_TRY(
+      rayt::sort_i32_device(data, n, d->scratch, d->status, epoch, again, err, rayt::next_done(*d), s));
+  if ((rc = rayt::finish(*d, s)) != RAYT_OK) return rc;
+  if (!rayt::sort_needs_passes(d->host + 1)) return RAYT_OK;
+  RAYT_CUDA_TRY(rayt::sort_passes_device(data, n, d->scratch, d->status, epoch, err, rayt::next_done(*d), s));
   return rayt::finish(*d, s);
 }
 

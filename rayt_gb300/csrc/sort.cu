@@ -23,10 +23,16 @@
 //   radix            (wider ranges; launched once the host has read the
 //                    choice) digit_hist, the digit passes, unique_kernel.
 // Sort, up to kSmall keys: small_sort_kernel, one CTA.  Above: digit_hist (the
-// four digits' counts in one read) and four digit_kernel passes (persistent
-// CTAs, tiles of 8192 keys brought into shared memory by bulk async copies a
-// tile ahead, per-digit decoupled look-back, scatter staged through shared
-// memory); a pass whose digit is the same in every key is skipped.
+// four digits' counts in one read, and the range), and then
+//   few values       counted by split_kernel, written by split_sort_kernel;
+//   evenly spread    split_kernel moves the keys to up to 4608 parts of their
+//                    range, split_sort_kernel sorts each in shared memory;
+//   other keys, or more than 70 million: four digit_kernel passes (persistent
+//                    CTAs, tiles of 8192 keys brought into shared memory by
+//                    bulk async copies a tile ahead, per-digit decoupled
+//                    look-back, scatter staged through shared memory); a pass
+//                    whose digit is the same in every key is skipped.
+//                    Launched once the host has read that they are needed.
 //
 // Scan: scan_kernel.
 //
@@ -37,6 +43,7 @@
 // and are tagged with a per-call epoch and the pass, so the table is never
 // cleared.  Every wait is bounded and sets an error flag instead of hanging.
 #include <algorithm>
+#include <cmath>
 
 #include "internal.h"
 
@@ -230,10 +237,11 @@ struct Control {
   uint32_t range[2];                  // max of ~key (so the minimum), max key
   int keys;                           // compacted keys
   int no_hit;                         // 1: some input word was NO_HIT
-  int done[3];                        // CTAs finished: compaction, range histogram, digit histogram
+  int done[4];                        // CTAs finished: compaction, range histogram, digit histogram, split
   int barrier[3];                     // CTAs at the barriers of the bitmap's cooperative kernels
   int tiles[kPasses];                 // tile counters: digit passes
   int unique_tiles, bucket_items;
+  int split_over;                     // 1: a range of the split got more keys than it holds
 };
 // Words one kernel of a call leaves for the next; not cleared.
 struct Plan {
@@ -244,7 +252,8 @@ struct Plan {
   int src[kPasses], dst[kPasses], last;  // buffers of the passes, and where the keys end up
   int counting;           // sort: the keys take this many values from `lowest` on (0: too many), and are counted
   uint32_t lowest;
-  uint32_t values[kCountValues];         // keys of each value
+  uint32_t split;         // sort: factor of the split's linear map (0: the keys take the digit passes)
+  uint32_t values[kCountValues];         // keys of each value; or of each range of the split, and their starts
   uint32_t offsets[kPasses * kBuckets];  // global start of each digit
   uint32_t range_offsets[kBuckets];
   uint32_t cursors[kBuckets * kCursorStride];
@@ -255,6 +264,7 @@ constexpr int kPathEmpty = 0, kPathDirect = 1, kPathPartition = 2, kPathRadix = 
 struct SortScratchLayout {
   uint32_t* keys_a;
   uint32_t* keys_b;
+  size_t key_words;  // of both together
   uint32_t* bitmap;
   Control* control;
   Plan* plan;
@@ -271,6 +281,7 @@ SortScratchLayout layout(void* base, int n) {
   l.plan = reinterpret_cast<Plan*>(b + off); off += up(sizeof(Plan));
   l.keys_a = reinterpret_cast<uint32_t*>(b + off); off += up((size_t)n * 4 + 16);
   l.keys_b = reinterpret_cast<uint32_t*>(b + off); off += up((size_t)n * 4 + 16);
+  l.key_words = (size_t)(b + off - reinterpret_cast<uint8_t*>(l.keys_a)) / 4;
   l.bitmap_bits = std::min<size_t>((((size_t)n * 4 + 16) / 16) * 16 * 8, (size_t)1 << kMaxSpanLog2);
   // the direct path leaves keys_b free; larger inputs may be partitioned into it
   if (n <= kDirectWords) l.bitmap = l.keys_b;
@@ -528,11 +539,24 @@ cudaError_t launch_compact(int grid, const int32_t* words, int n, int nib, const
 // and lays out the passes: a digit that is the same in every key needs none,
 // and keys of up to kCountValues different values are not passed over at all.
 constexpr int kHistThreads = 1024;
+// True if digit p has the value v in about as many of m keys as it would have
+// if the keys were spread evenly over [lo, hi]: within what a range of the
+// split holds beyond its even share.
+__device__ __forceinline__ bool even_digit(uint32_t count, int p, uint32_t v, uint32_t lo, uint32_t hi, uint32_t m) {
+  const uint32_t unit = 1u << (8 * p);
+  auto below = [&](unsigned long long x) {  // numbers below x whose digit p is v
+    const unsigned long long whole = x >> (8 * p + 8);
+    const long long rest = (long long)(x - (whole << (8 * p + 8))) - (long long)v * unit;
+    return whole * unit + (unsigned long long)(rest < 0 ? 0 : rest > (long long)unit ? (long long)unit : rest);
+  };
+  const float share = (float)(below((unsigned long long)hi + 1) - below(lo)) * (float)m / ((float)(hi - lo) + 1.f);
+  return (float)count <= share * 1.0625f + 8.f * sqrtf(share) + 8.f;
+}
 constexpr int kHistSmemBytes = kPasses * kBuckets * 32 * 4;
 template <bool kVec>
 __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint32_t* keys, int n, const int* count,
-                                                                    uint32_t flip, bool in_place, Control* ctl,
-                                                                    Plan* plan) {
+                                                                    uint32_t flip, bool in_place, int split_ranges,
+                                                                    Control* ctl, Plan* plan) {
   extern __shared__ __align__(128) uint32_t s_hist[];
   __shared__ uint32_t s_max[kPasses];
   uint32_t not_min = 0, max_key = 0;
@@ -598,9 +622,13 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
     const int p = threadIdx.x >> 5;
     warp_scan_256(counts + p * kBuckets, plan->offsets + p * kBuckets);
   }
+  const uint32_t lo = ~*(volatile uint32_t*)&ctl->range[0], hi = *(volatile uint32_t*)&ctl->range[1];
+  const bool uneven = __syncthreads_or(
+      split_ranges && !even_digit(counts[threadIdx.x], threadIdx.x >> 8, threadIdx.x & 255u, lo, hi, m));
   if (threadIdx.x == 0) {
-    const volatile Control* c = ctl;
-    const uint32_t lo = ~c->range[0], hi = c->range[1];
+    plan->split = split_ranges && !uneven && hi - lo >= (uint32_t)kCountValues
+                      ? (uint32_t)(((unsigned long long)split_ranges << 32) / ((unsigned long long)(hi - lo) + 1))
+                      : 0u;
     plan->counting = in_place && hi - lo < (uint32_t)kCountValues ? (int)(hi - lo) + 1 : 0;
     plan->lowest = lo;
     int active = 0;
@@ -738,10 +766,10 @@ __device__ __forceinline__ void count_values(const uint32_t* keys, int n, uint32
   const uint32_t lo = plan->lowest;
   const bool by_lane = values * 32 <= kCountValues;
   const int words = by_lane ? values * 32 : values, scale = by_lane ? 32 : 1, col = by_lane ? lane : 0;
-  for (int i = threadIdx.x; i < words; i += kDigitThreads) smem[i] = 0;
+  for (uint32_t i = threadIdx.x; i < (uint32_t)words; i += blockDim.x) smem[i] = 0;
   __syncthreads();
-  const uint32_t step = gridDim.x * kDigitThreads;
-  for (uint32_t i = blockIdx.x * kDigitThreads + threadIdx.x; i < (uint32_t)n; i += 4 * step) {  // n < 2^30
+  const uint32_t step = gridDim.x * blockDim.x;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (uint32_t)n; i += 4 * step) {  // n < 2^30
     uint32_t k[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) k[r] = i + r * step < (uint32_t)n ? (__ldg(keys + i + r * step) ^ flip) - lo : ~0u;
@@ -750,7 +778,7 @@ __device__ __forceinline__ void count_values(const uint32_t* keys, int n, uint32
       if (k[r] != ~0u) atomicAdd(&smem[k[r] * scale + col], 1u);
   }
   __syncthreads();
-  for (int v = threadIdx.x; v < values; v += kDigitThreads) {
+  for (uint32_t v = threadIdx.x; v < (uint32_t)values; v += blockDim.x) {
     uint32_t sum = 0;
     if (by_lane) {
 #pragma unroll 8
@@ -1032,6 +1060,394 @@ __global__ void __launch_bounds__(kDigitThreads, 2) digit_kernel(const DigitBuff
                                   int pass, uint32_t flip, Plan* plan, unsigned long long* status,
                                   int* tile_counter, uint32_t tag, int* err, const DoneFlag done) {
   digit_kernel_cta(bufs, n, count, pass, flip, plan, status, tile_counter, tag, err);
+  publish(done);
+}
+
+// ---- evenly spread keys ----------------------------------------------------------
+// A sort of keys alone may put equal keys in any order, and keys that are
+// spread about evenly over their range need no digit passes: a linear map of
+// the range, product = (key - lowest) * factor, has the number of one of up to
+// kSplitRanges equal parts of the range in its upper word.
+// split_kernel moves each key into its part's region of scratch (regions have
+// room for a part's even share and some more, so nothing has to be counted
+// first: a tile claims its places with one atomic per part), and
+// split_sort_kernel sorts each region in shared memory and writes it where it
+// belongs.  Keys are read and written twice instead of four times and no tile
+// waits on another (2^26 random keys: four digit passes 1040 us; here 256 +
+// 261; 10^6 keys, whole call: 84 us, here 48).
+// The histogram kernel before them chooses by the digits' counts (even_digit).
+// Keys that pass that test and still overfill a region, or crowd one of
+// split_sort_kernel's bins, leave the array a permutation of itself, and the
+// host launches the digit passes over it.
+constexpr int kMoveThreads = 1024;   // split_kernel
+constexpr int kMoveTile = 32768;     // keys of a tile, at most
+constexpr int kMoveGroups = kMoveTile / (4 * kMoveThreads);  // 16-byte units per thread
+constexpr int kSplitThreads = 512;   // split_sort_kernel
+constexpr int kSplitRoom = 16384;    // keys of a region, at most
+constexpr int kSplitRanges = 4608;
+constexpr int kSplitFill = 15360;    // keys a region gets on average, at most
+constexpr int kSplitGroups = kSplitRoom / (4 * kSplitThreads);
+constexpr int kSplitSmemBytes = (kMoveTile + 2 * kSplitRanges) * 4;
+constexpr int kSplitPer = (kSplitRanges + kMoveThreads - 1) / kMoveThreads;
+constexpr int kSortBins = 12288;     // at most; a multiple of kSortBinsUnit, four per thread
+constexpr int kSortBinsUnit = 4 * kSplitThreads;
+constexpr int kSortSmemBytes = (kSplitRoom + kSortBins) * 4;
+constexpr uint32_t kSortRun = 16;    // keys that a thread sorts in registers
+constexpr uint32_t kCrowded = 64;    // keys of a bin that are ranked against one another
+static_assert(kCountValues <= kMoveTile && kCountValues <= kSplitRoom && kSplitThreads == kDigitThreads,
+              "the value counters lie in the tile, and in the region");
+static_assert(2 * kSplitRanges + 1 <= kCountValues, "the ranges' counts and starts lie in the plan's value counts");
+
+struct SplitShape {
+  int ranges;      // 0: no split
+  uint32_t room;   // keys of a region
+  int tile;        // keys of a tile, a multiple of 4
+  int bins;        // of a region
+};
+
+// Brings keys [begin, end) into L2 (begin a multiple of 4, the keys on a 16-byte
+// boundary; up to three at the end may be left out).
+__device__ __forceinline__ void fetch_keys(const uint32_t* keys, uint32_t begin, uint32_t end) {
+  if (begin / 4 < end / 4)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(keys + begin), "r"((end / 4 - begin / 4) * 16)
+                 : "memory");
+}
+// Four keys from position 4 * u on; past the end of n keys whatever.
+template <bool kVec>
+__device__ __forceinline__ uint4 load_unit(const uint32_t* keys, uint32_t u, uint32_t n) {
+  if (kVec && u * 4 + 4 <= n) return __ldg(reinterpret_cast<const uint4*>(keys) + u);
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (u * 4 < n) v.x = __ldg(keys + u * 4);
+  if (u * 4 + 1 < n) v.y = __ldg(keys + u * 4 + 1);
+  if (u * 4 + 2 < n) v.z = __ldg(keys + u * 4 + 2);
+  if (u * 4 + 3 < n) v.w = __ldg(keys + u * 4 + 3);
+  return v;
+}
+
+// Exclusive scan over the CTA of one value per thread.
+__device__ __forceinline__ uint32_t cta_exclusive(uint32_t v, uint32_t* s_wsum) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += t;
+  }
+  if (lane == 31) s_wsum[warp] = incl;
+  __syncthreads();
+  return incl - v + __reduce_add_sync(0xffffffffu, lane < warp ? s_wsum[lane] : 0u);  // warp < 32
+}
+
+// The longer a range's run in a tile, the fewer lines a warp's stores meet:
+// tiles of 32768 keys (7 keys a run at 4560 ranges), one per SM, took 250 us
+// for 2^26 keys where two per SM of 16384 took 310, 97 of them for the stores
+// being scattered.  A tile's keys are read again (from L2) to be staged, as
+// registers hold their ranks.  Each CTA has its next tile fetched into L2.
+template <bool kVec>
+__device__ __forceinline__ void split_cta(const uint32_t* keys, uint32_t n, uint32_t* regions, const SplitShape shape,
+                                          Control* ctl, Plan* plan, uint32_t* smem) {
+  __shared__ uint32_t s_wsum[kMoveThreads / 32];
+  uint32_t* s_tile = smem;
+  uint32_t* s_count = smem + kMoveTile;      // keys of the tile per range, then their starts in the tile
+  uint32_t* s_off = s_count + kSplitRanges;   // position in the regions - position in the tile
+  uint32_t* claimed = plan->values;
+  const uint32_t lo = plan->lowest, factor = plan->split, ranges = (uint32_t)shape.ranges, room = shape.room;
+  const uint32_t tile = (uint32_t)shape.tile;
+  const uint32_t per = ((ranges + kMoveThreads - 1) / kMoveThreads) | 1u;  // odd: a thread's ranges lie in all banks
+  const uint32_t tiles = (n + tile - 1) / tile;
+  for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const uint32_t begin = t * tile, end = min(n, begin + tile);  // n < 2^27
+    for (uint32_t i = threadIdx.x; i < per * kMoveThreads && i < (uint32_t)kSplitRanges; i += kMoveThreads)
+      s_count[i] = 0;
+    const bool over = *(volatile int*)&ctl->split_over != 0;
+    if (__syncthreads_or(over)) return;
+    if (kVec && threadIdx.x == 0 && t + gridDim.x < tiles) {  // this CTA's next tile
+      const uint32_t next = (t + gridDim.x) * tile;
+      fetch_keys(keys, next, min(n, next + tile));
+    }
+    uint32_t ranks[kMoveGroups * 2];
+    auto range_of = [&](uint32_t x) { return __umulhi(x, factor); };
+#pragma unroll
+    for (int h = 0; h < kMoveGroups; h += 4) {
+      uint4 v[4];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const uint32_t at = begin + ((h + g) * kMoveThreads + threadIdx.x) * 4;
+        const uint32_t k[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
+        uint32_t r[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (at + e < end) r[e] = atomicAdd(&s_count[range_of((k[e] ^ 0x80000000u) - lo)], 1u);
+        ranks[(h + g) * 2] = r[0] | (r[1] << 16);
+        ranks[(h + g) * 2 + 1] = r[2] | (r[3] << 16);
+      }
+    }
+    __syncthreads();
+    // every claim in flight beside the scan
+    uint32_t count[kSplitPer], got[kSplitPer];
+#pragma unroll
+    for (int j = 0; j < kSplitPer; ++j) {
+      const uint32_t d = threadIdx.x + j * kMoveThreads;
+      count[j] = d < ranges ? s_count[d] : 0u;
+      got[j] = count[j] ? atomicAdd(&claimed[d], count[j]) : 0u;
+    }
+    __syncthreads();
+    {
+      const uint32_t first = threadIdx.x * per;
+      uint32_t sum = 0;
+#pragma unroll
+      for (int j = 0; j < kSplitPer; ++j)
+        if (j < per && first + j < ranges) sum += s_count[first + j];
+      uint32_t run = cta_exclusive(sum, s_wsum);
+#pragma unroll
+      for (int j = 0; j < kSplitPer; ++j)
+        if (j < per && first + j < ranges) {
+          const uint32_t c = s_count[first + j];
+          s_count[first + j] = run;
+          run += c;
+        }
+    }
+    __syncthreads();
+    bool full = false;
+#pragma unroll
+    for (int j = 0; j < kSplitPer; ++j) {
+      const uint32_t d = threadIdx.x + j * kMoveThreads;
+      full |= got[j] + count[j] > room;
+      if (d < ranges) s_off[d] = d * room + got[j] - s_count[d];
+    }
+    if (full) *(volatile int*)&ctl->split_over = 1;
+#pragma unroll
+    for (int h = 0; h < kMoveGroups; h += 4) {
+      uint4 v[4];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const uint32_t at = begin + ((h + g) * kMoveThreads + threadIdx.x) * 4;
+        const uint32_t k[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
+        const uint32_t r[2] = {ranks[(h + g) * 2], ranks[(h + g) * 2 + 1]};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t x = (k[e] ^ 0x80000000u) - lo;
+          if (at + e < end) s_tile[s_count[range_of(x)] + ((r[e >> 1] >> (16 * (e & 1))) & 0xffffu)] = x;
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (uint32_t i = threadIdx.x; i < end - begin; i += kMoveThreads) {
+      const uint32_t x = s_tile[i], d = range_of(x);
+      const uint32_t pos = s_off[d] + i;
+      if (pos - d * room < room) regions[pos] = x;  // else split_over is set
+    }
+    __syncthreads();
+  }
+}
+template <bool kVec>
+__global__ void __launch_bounds__(kMoveThreads, 1) split_kernel(const uint32_t* keys, int n, uint32_t* regions,
+                                                                 const SplitShape shape, Control* ctl, Plan* plan) {
+  extern __shared__ __align__(128) uint32_t smem[];
+  __shared__ uint32_t s_wsum[kMoveThreads / 32];
+  dependents_may_start();
+  wait_for_dependency();
+  if (plan->counting) {
+    count_values(keys, n, 0x80000000u, plan, smem);
+    return;
+  }
+  if (!plan->split) return;
+  split_cta<kVec>(keys, (uint32_t)n, regions, shape, ctl, plan, smem);
+  if (!last_cta(&ctl->done[3], gridDim.x)) return;
+  // where each range's keys begin in the array
+  const uint32_t ranges = (uint32_t)shape.ranges, per = (ranges + kMoveThreads - 1) / kMoveThreads;
+  const volatile uint32_t* claimed = plan->values;
+  uint32_t sum = 0, c[kSplitPer];
+#pragma unroll
+  for (uint32_t j = 0; j < kSplitPer; ++j) {
+    c[j] = j < per && threadIdx.x * per + j < ranges ? claimed[threadIdx.x * per + j] : 0u;
+    sum += c[j];
+  }
+  uint32_t run = cta_exclusive(sum, s_wsum);
+#pragma unroll
+  for (uint32_t j = 0; j < kSplitPer; ++j) {
+    if (j < per && threadIdx.x * per + j < ranges) plan->values[kSplitRanges + threadIdx.x * per + j] = run;
+    run += c[j];
+  }
+}
+
+// One region per CTA and turn.  The lower word of the product is the key's place
+// within its range, and that times the number of bins its bin, about one key
+// each: a key's rank among its bin's keys is what the atomic that counts it
+// returns, the bins' starts are scanned, and the keys go to their bins in
+// shared memory.  What is left is to order the few keys of each bin: a thread
+// sorts 16 neighbouring keys in registers, and then merges the halves of two
+// such runs that meet, which puts every bin of up to 9 keys in order, as it
+// lies in two runs at most.  (Ranking each key against the others of its bin
+// took 365 us for 2^26 keys, at 157 instructions per 32 of them; this takes 261
+// at 79 and is bound by shared memory, 67% of its wavefronts' rate.)  Where
+// a bin has more keys they are ranked so; no order is missing where a bin is a
+// single value.
+__device__ __forceinline__ void order(uint32_t& a, uint32_t& b) {
+  const uint32_t lo = min(a, b);
+  b = max(a, b);
+  a = lo;
+}
+// The steps of Batcher's odd-even merge sort of 16 keys that merge sorted runs
+// of kP keys, from kP = kFrom on.
+template <int kFrom>
+__device__ __forceinline__ void merge_runs(uint32_t (&k)[kSortRun]) {
+#pragma unroll
+  for (int p = kFrom; p < (int)kSortRun; p *= 2) {
+#pragma unroll
+    for (int q = p; q >= 1; q /= 2) {
+#pragma unroll
+      for (int j = 0; j < (int)kSortRun; ++j)
+        if (j >= q % p && (j - q % p) % (2 * q) < q && j + q < (int)kSortRun && j / (2 * p) == (j + q) / (2 * p))
+          order(k[j], k[j + q]);
+    }
+  }
+}
+// Where position i of a region lies in shared memory: 16-byte units of
+// neighbouring runs lie in different banks.
+__device__ __forceinline__ uint32_t run_place(uint32_t i) { return i ^ ((i >> 3) & 12u); }
+template <int kFrom>
+__device__ __forceinline__ void sort_run(uint32_t* s_keys, uint32_t at) {
+  uint32_t k[kSortRun];
+#pragma unroll
+  for (uint32_t u = 0; u < kSortRun; u += 4) {
+    const uint4 v = *reinterpret_cast<const uint4*>(s_keys + run_place(at + u));
+    k[u] = v.x, k[u + 1] = v.y, k[u + 2] = v.z, k[u + 3] = v.w;
+  }
+  merge_runs<kFrom>(k);
+#pragma unroll
+  for (uint32_t u = 0; u < kSortRun; u += 4)
+    *reinterpret_cast<uint4*>(s_keys + run_place(at + u)) = make_uint4(k[u], k[u + 1], k[u + 2], k[u + 3]);
+}
+
+__device__ __forceinline__ bool split_sort_cta(uint32_t* out, const uint32_t* regions, const SplitShape shape,
+                                               const Plan* plan, uint32_t* smem) {
+  __shared__ uint32_t s_wsum[kSplitThreads / 32];
+  uint32_t* s_keys = smem;
+  uint32_t* s_bin = smem + kSplitRoom;  // count, then start | count << 16
+  const uint32_t lo = plan->lowest, factor = plan->split, bins = (uint32_t)shape.bins;
+  // neighbouring keys are at least a bin apart
+  const bool single = (unsigned long long)factor * bins >> 32 != 0;
+  auto bin_of = [&](uint32_t x) { return __umulhi(x * factor, bins); };
+  bool any_crowded = false;
+  for (int q = blockIdx.x; q < shape.ranges; q += gridDim.x) {
+    const uint32_t count = plan->values[q], base = plan->values[kSplitRanges + q];
+    const uint32_t* keys = regions + (size_t)q * shape.room;
+    if (threadIdx.x == 0 && q + (int)gridDim.x < shape.ranges)  // this CTA's next region
+      fetch_keys(keys + (size_t)gridDim.x * shape.room, 0, plan->values[q + gridDim.x]);
+    for (uint32_t i = threadIdx.x * 4; i < bins; i += kSortBinsUnit)
+      *reinterpret_cast<uint4*>(s_bin + i) = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    uint32_t ranks[kSplitGroups * 2];
+#pragma unroll
+    for (int h = 0; h < kSplitGroups; h += 4) {
+      if (h * kSplitThreads * 4 >= count) break;
+      uint4 v[4];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) v[g] = load_unit<true>(keys, (h + g) * kSplitThreads + threadIdx.x, count);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const uint32_t at = ((h + g) * kSplitThreads + threadIdx.x) * 4;
+        const uint32_t k[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
+        uint32_t r[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (at + e < count) r[e] = atomicAdd(&s_bin[bin_of(k[e])], 1u);
+        ranks[(h + g) * 2] = r[0] | (r[1] << 16);
+        ranks[(h + g) * 2 + 1] = r[2] | (r[3] << 16);
+      }
+    }
+    __syncthreads();
+    uint32_t most = 0;
+    {
+      const uint32_t per = bins / kSplitThreads, first = threadIdx.x * per;
+      uint32_t sum = 0;
+      for (uint32_t j = 0; j < per; j += 4) {
+        const uint4 v = *reinterpret_cast<const uint4*>(s_bin + first + j);
+        sum += v.x + v.y + v.z + v.w;
+        most = max(max(most, max(v.x, v.y)), max(v.z, v.w));
+      }
+      uint32_t run = cta_exclusive(sum, s_wsum);
+      for (uint32_t j = 0; j < per; j += 4) {
+        uint4* at = reinterpret_cast<uint4*>(s_bin + first + j);
+        const uint4 v = *at;
+        const uint32_t y = run + v.x, z = y + v.y, w = z + v.z;
+        *at = make_uint4(run | (v.x << 16), y | (v.y << 16), z | (v.z << 16), w | (v.w << 16));
+        run = w + v.w;
+      }
+    }
+    const bool ranked = __syncthreads_or(most > kSortRun / 2 + 1) && !single;
+    const bool crowded = __syncthreads_or(most > kCrowded) && !single;
+    any_crowded |= crowded;
+#pragma unroll
+    for (int h = 0; h < kSplitGroups; h += 4) {
+      if (h * kSplitThreads * 4 >= count) break;
+      uint4 v[4];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) v[g] = load_unit<true>(keys, (h + g) * kSplitThreads + threadIdx.x, count);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const uint32_t at = ((h + g) * kSplitThreads + threadIdx.x) * 4;
+        const uint32_t k[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
+        const uint32_t r[2] = {ranks[(h + g) * 2], ranks[(h + g) * 2 + 1]};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (at + e < count) {
+            const uint32_t rank = (r[e >> 1] >> (16 * (e & 1))) & 0xffffu;
+            s_keys[run_place((s_bin[bin_of(k[e])] & 0xffffu) + rank)] = k[e];
+          }
+      }
+    }
+    const uint32_t runs = (count + kSortRun - 1) / kSortRun;  // runs * 16 <= kSplitRoom
+    if (count + threadIdx.x < runs * kSortRun) s_keys[run_place(count + threadIdx.x)] = ~0u;
+    __syncthreads();
+    if (!single && !ranked) {
+      for (uint32_t r = threadIdx.x; r < runs; r += kSplitThreads) sort_run<1>(s_keys, r * kSortRun);
+      __syncthreads();
+      for (uint32_t r = threadIdx.x; r + 1 < runs; r += kSplitThreads)
+        sort_run<kSortRun / 2>(s_keys, r * kSortRun + kSortRun / 2);
+      __syncthreads();
+    }
+    if (ranked && !crowded) {
+      for (uint32_t i = threadIdx.x; i < count; i += kSplitThreads) {
+        const uint32_t x = s_keys[run_place(i)];
+        const uint32_t w = s_bin[bin_of(x)], first = w & 0xffffu, last = first + (w >> 16);
+        uint32_t to = first;
+        for (uint32_t j = first; j < last; ++j) {
+          const uint32_t y = s_keys[run_place(j)];
+          to += y < x || (y == x && j < i);
+        }
+        out[base + to] = (x + lo) ^ 0x80000000u;
+      }
+    } else {
+#pragma unroll 4
+      for (uint32_t i = threadIdx.x; i < count; i += kSplitThreads)
+        out[base + i] = (s_keys[run_place(i)] + lo) ^ 0x80000000u;
+    }
+    __syncthreads();
+  }
+  return any_crowded;
+}
+// `again` (mapped host memory): 1 if the keys must take the digit passes.
+__global__ void __launch_bounds__(kSplitThreads, 2) split_sort_kernel(uint32_t* out, int n, const uint32_t* regions,
+                                                                      const SplitShape shape, Control* ctl,
+                                                                      const Plan* plan, int* again,
+                                                                      const DoneFlag done) {
+  extern __shared__ __align__(128) uint32_t smem[];
+  wait_for_dependency();
+  bool digits = false;
+  if (plan->counting)
+    write_values(out, n, 0x80000000u, plan, smem);
+  else if (!plan->split || *(volatile int*)&ctl->split_over)
+    digits = true;
+  else
+    digits = split_sort_cta(out, regions, shape, plan, smem);
+  if (digits && threadIdx.x == 0) *(volatile int*)again = 1;
   publish(done);
 }
 
@@ -1965,14 +2381,16 @@ int persistent_grid(int tiles, int threads = kThreads, int smem = 0) {
 
 // Digit counts, offsets and the plan of the passes over n keys (or *count).
 cudaError_t launch_digit_hist(const uint32_t* keys, int n, const int* count, uint32_t flip, bool in_place,
-                              const SortScratchLayout& l, cudaStream_t s) {
+                              int split_ranges, const SortScratchLayout& l, cudaStream_t s) {
   const int tiles = tiles_of(n, kHistThreads * 4);
   if ((reinterpret_cast<uintptr_t>(keys) & 15) == 0)
     digit_hist_kernel<true><<<persistent_grid<digit_hist_kernel<true>>(tiles, kHistThreads, kHistSmemBytes),
-                              kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, l.control, l.plan);
+                              kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, split_ranges,
+                                                             l.control, l.plan);
   else
     digit_hist_kernel<false><<<persistent_grid<digit_hist_kernel<false>>(tiles, kHistThreads, kHistSmemBytes),
-                               kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, l.control, l.plan);
+                               kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, split_ranges,
+                                                             l.control, l.plan);
   return cudaGetLastError();
 }
 
@@ -2000,6 +2418,55 @@ cudaError_t launch_digits(const DigitBuffers& bufs, int n, const int* count, boo
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+// The split of n keys.  Two regions per SM or more, so that every SM sorts, and
+// of more keys a multiple of that, so that every CTA sorts as many; regions of
+// 512 keys on average or more.
+SplitShape split_shape(int n, const SortScratchLayout& l) {
+  SplitShape sh{};
+  const int resident = persistent_grid<split_sort_kernel>(1 << 30, kSplitThreads, kSortSmemBytes);
+  const long long full = ((long long)n + (long long)resident * kSplitFill - 1) / ((long long)resident * kSplitFill);
+  const long long ranges = std::min<long long>(resident * full, n / 512);
+  if (ranges < 1 || ranges > kSplitRanges) return sh;
+  const double share = (double)n / (double)ranges;
+  const double room = share * 1.0625 + 8 * std::sqrt(share) + 64;
+  sh.room = (uint32_t)std::min<long long>(kSplitRoom, ((long long)room + 3) / 4 * 4);
+  if ((size_t)ranges * sh.room > l.key_words) return sh;
+  sh.ranges = (int)ranges;
+  const int moving = persistent_grid<split_kernel<true>>(1 << 30, kMoveThreads, kSplitSmemBytes);
+  // tiles: as many for every resident CTA
+  const long long turns = ((long long)n + (long long)moving * kMoveTile - 1) / ((long long)moving * kMoveTile);
+  const long long tile = ((long long)n + moving * turns - 1) / (moving * turns);
+  sh.tile = (int)std::max<long long>(4 * kMoveThreads, (tile + 3) / 4 * 4);
+  // about a bin per key, as shared memory allows
+  sh.bins = std::min(kSortBins, ((int)sh.room + kSortBinsUnit - 1) / kSortBinsUnit * kSortBinsUnit);
+  return sh;
+}
+
+cudaError_t launch_split(uint32_t* keys, int n, const SplitShape& shape, const SortScratchLayout& l, int* again,
+                         const DoneFlag& done, cudaStream_t s) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kMoveThreads);
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const int tiles = tiles_of(n, shape.tile);
+  const bool whole = (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
+  cfg.gridDim = dim3(whole ? persistent_grid<split_kernel<true>>(tiles, kMoveThreads, kSplitSmemBytes)
+                           : persistent_grid<split_kernel<false>>(tiles, kMoveThreads, kSplitSmemBytes));
+  cfg.dynamicSmemBytes = kSplitSmemBytes;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, whole ? split_kernel<true> : split_kernel<false>,
+                                           (const uint32_t*)keys, n, l.keys_a, shape, l.control, l.plan);
+  if (e != cudaSuccess) return e;
+  cfg.blockDim = dim3(kSplitThreads);
+  cfg.gridDim = dim3(persistent_grid<split_sort_kernel>(shape.ranges, kSplitThreads, kSortSmemBytes));
+  cfg.dynamicSmemBytes = kSortSmemBytes;
+  return cudaLaunchKernelEx(&cfg, split_sort_kernel, keys, n, (const uint32_t*)l.keys_a, shape, l.control,
+                            (const Plan*)l.plan, again, done);
 }
 
 template <int kRounds>
@@ -2097,7 +2564,7 @@ cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scrat
                                          cudaStream_t s) {
   const SortScratchLayout l = layout(scratch, n);
   cudaError_t e;
-  if ((e = launch_digit_hist(l.keys_a, n, &l.control->keys, 0u, false, l, s)) != cudaSuccess) return e;
+  if ((e = launch_digit_hist(l.keys_a, n, &l.control->keys, 0u, false, 0, l, s)) != cudaSuccess) return e;
   const DigitBuffers bufs = {l.keys_a, l.keys_a, l.keys_b, nullptr};
   if ((e = launch_digits(bufs, n, &l.control->keys, false, l, status, epoch, err, DoneFlag{}, s)) != cudaSuccess)
     return e;
@@ -2106,8 +2573,10 @@ cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scrat
   return cudaGetLastError();
 }
 
-cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch, int* err,
-                            const DoneFlag& done, cudaStream_t s) {
+bool sort_needs_passes(const int* again) { return *again != 0; }
+
+cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch,
+                            int* again, int* err, const DoneFlag& done, cudaStream_t s) {
   if (n <= 1) return cudaSuccess;
   if (n <= kSmall) {
     if (n <= 2 * kSmallThreads) launch_small_sort<2>(data, n, done, s);
@@ -2116,16 +2585,26 @@ cudaError_t sort_i32_device(int32_t* data, int n, void* scratch, unsigned long l
     return cudaGetLastError();
   }
   const SortScratchLayout l = layout(scratch, n);
+  const SplitShape shape = split_shape(n, l);
   cudaError_t e;
   if ((e = cudaMemsetAsync(l.control, 0, sizeof(Control), s)) != cudaSuccess) return e;
+  uint32_t* keys = reinterpret_cast<uint32_t*>(data);
+  if ((e = launch_digit_hist(keys, n, nullptr, 0x80000000u, true, shape.ranges, l, s)) != cudaSuccess) return e;
+  if (shape.ranges) return launch_split(keys, n, shape, l, again, done, s);
+  return sort_passes_device(data, n, scratch, status, epoch, err, done, s);
+}
+
+cudaError_t sort_passes_device(int32_t* data, int n, void* scratch, unsigned long long* status, uint32_t epoch,
+                               int* err, const DoneFlag& done, cudaStream_t s) {
+  const SortScratchLayout l = layout(scratch, n);
   uint32_t* keys = reinterpret_cast<uint32_t*>(data);
   DigitBuffers bufs = {keys, keys, l.keys_a, l.keys_b};
   if (reinterpret_cast<uintptr_t>(data) & 15) {  // the passes read a copy (keys_b is written by the second pass)
     copy_keys_kernel<<<persistent_grid<copy_keys_kernel>(tiles_of(n, kThreads)), kThreads, 0, s>>>(keys, l.keys_b, n);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
     bufs.in0 = l.keys_b;
   }
-  if ((e = launch_digit_hist(bufs.in0, n, nullptr, 0x80000000u, true, l, s)) != cudaSuccess) return e;
   return launch_digits(bufs, n, nullptr, true, l, status, epoch, err, done, s);
 }
 

@@ -50,6 +50,39 @@ def test_sort_paths(built, n, keys, offset):
     assert np.all(got[:offset] == 9) and np.all(got[offset + n:] == 9)
 
 
+def _digits(rng, n, *pick):
+    """Keys of four digits: a number draws the digit as the numbers before it drew
+    theirs, so every digit is spread evenly but the keys are not."""
+    d = [rng.integers(0, 256, n) for _ in range(4)]
+    return (sum(d[p] << (24 - 8 * k) for k, p in enumerate(pick)) - 2**31).astype(np.int32)
+
+
+SPLIT_KEYS = {
+    "wide": _wide,
+    "blocks": KEYS["blocks"],
+    "odd_range": lambda rng, n: rng.integers(-77, 3 << 22, n).astype(np.int32),
+    "over_count_limit": KEYS["over_count_limit"],
+    "sorted": KEYS["sorted"],
+    "overfull": lambda rng, n: _digits(rng, n, 0, 0, 1, 2),
+    "repeats": lambda rng, n: _digits(rng, n, 0, 1, 0, 1),
+}
+
+
+# one region for each resident CTA at most, whole turns of regions, partial and
+# several tiles; the digits of "overfull" and "repeats" look even, but a region
+# gets more keys than it holds, and bins get repeats by the dozen
+@pytest.mark.parametrize("n", [8193, 155648, 155649, 622593, 1 << 20, 4669441, 5000003, 1 << 23])
+@pytest.mark.parametrize("keys", sorted(SPLIT_KEYS))
+@pytest.mark.parametrize("offset", [0, 3])
+def test_sort_split(built, n, keys, offset):
+    a = SPLIT_KEYS[keys](np.random.default_rng(n), n)
+    x = _dev(np.concatenate([np.full(offset, 9, np.int32), a, np.full(5, 9, np.int32)]))
+    R.GPUSort(x[offset:], n)
+    got = x.cpu().numpy()
+    np.testing.assert_array_equal(got[offset:offset + n], np.sort(a))
+    assert np.all(got[:offset] == 9) and np.all(got[offset + n:] == 9)
+
+
 @pytest.mark.parametrize("n", [1, 3, 127, 128, 1023, 8191, 8192, 8193, 16384, 16387, 1 << 20, (1 << 20) + 1])
 @pytest.mark.parametrize("offset", [0, 1, 2])
 def test_scan_paths(built, n, offset):
