@@ -12,8 +12,7 @@
 //                    to an unsigned key (x ^ 0x80000000 keeps signed order),
 //                    drops most repeats through a per-CTA filter, finds the
 //                    key range; its last CTA chooses the path:
-//   bitmap           (the keys span at most 32 values per input word and at
-//                    most 2^26) a bitmap over [min, max], whose set bits read
+//   bitmap           (the keys span at most 2^26 values) a bitmap over [min, max], whose set bits read
 //                    in order are the sorted unique set: set straight into
 //                    the global bitmap and written out (direct_bitmap: few
 //                    keys or a small bitmap), or range by range: range_hist and range_partition
@@ -64,14 +63,23 @@ constexpr int kCursorStride = 32;
 constexpr int kMaxSpanLog2 = 26;
 // Inputs of up to kDirectWords words put their keys straight into the bitmap
 // (the launches of the partition would cost more than they give).  Of larger
-// ones, those that kept up to kDirectKeys keys, or whose bitmap is built in
-// shared memory: scattered atomics on a wide one take 10 to 100 us per million
-// keys (30 million words, 1.5 million kept, 50 million bits: 196 us straight,
-// 160 us partitioned).
+// ones, those that kept up to kDirectKeys keys, or whose bitmap is one slice,
+// or a few slices and not many keys for each CTA to read: scattered atomics on
+// a wide one take 10 to 100 us per million keys (30 million words, 1.5 million
+// kept, 50 million bits: 196 us straight, 160 us partitioned), and every slice
+// is another read of the keys (30 million words, 24 million kept, 1.1 million
+// bits, two slices: 168 us partitioned, 144 straight).
 constexpr int kDirectWords = 1 << 21;
 constexpr int kDirectKeys = 1 << 18;
-// A bitmap of up to this many words is built in shared memory.
+constexpr unsigned long long kDirectFewSlices = 4, kDirectReads = 1ull << 26;
+// The straight bitmap is built in shared memory, in slices of up to this many
+// words, each by its share of the CTAs (at least kDirectSliceCtas): 1.9 million
+// words, 1.6 million kept over 1.1 million bits: 110 us with atomics on the
+// bitmap in memory, 58 in two slices.  Fewer than kDirectSliceKeys keys set
+// their bits in memory when they span more than one slice.
 constexpr int kDirectSliceWords = 1 << 15;
+constexpr uint32_t kDirectSliceKeys = 1 << 15;
+constexpr int kDirectSliceCtas = 2;
 constexpr long long kSpinLimit = 1ll << 26;  // polls, a backstop to the time limit
 
 // Time limit of every wait on another CTA's result (ns): a correct wait ends in
@@ -94,7 +102,9 @@ __device__ __forceinline__ void set_error(int* err) { *(volatile int*)err = 1; }
 // Programmatic launches: the kernel after this one may take its place while this
 // one still runs; what it reads of this one's, it reads after its own
 // wait_for_dependency.
-__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dependents_may_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void wait_for_dependency() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // The end of a call's last kernel: the CTA that ends last publishes the call's
@@ -247,6 +257,7 @@ struct Control {
 struct Plan {
   int path;               // feedback unique: kPath...
   uint32_t bitmap_words, range_shift;
+  int clear;              // the bitmap is wider than what the compaction cleared
   int skip[kPasses];      // digit pass not needed
   int unstable[kPasses];  // first pass: equal digits may leave in any order
   int src[kPasses], dst[kPasses], last;  // buffers of the passes, and where the keys end up
@@ -268,11 +279,12 @@ struct SortScratchLayout {
   uint32_t* bitmap;
   Control* control;
   Plan* plan;
-  size_t bitmap_bits;  // unique-by-bitmap capacity
+  size_t bitmap_bits;  // of the bitmap that the compaction clears
+  size_t bitmap_cap;   // and that there is room for
   size_t bytes;
 };
 
-SortScratchLayout layout(void* base, int n) {
+SortScratchLayout layout(void* base, int n, bool unique = false) {
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
   SortScratchLayout l{};
   size_t off = 0;
@@ -280,9 +292,12 @@ SortScratchLayout layout(void* base, int n) {
   l.control = reinterpret_cast<Control*>(b + off); off += up(sizeof(Control));
   l.plan = reinterpret_cast<Plan*>(b + off); off += up(sizeof(Plan));
   l.keys_a = reinterpret_cast<uint32_t*>(b + off); off += up((size_t)n * 4 + 16);
-  l.keys_b = reinterpret_cast<uint32_t*>(b + off); off += up((size_t)n * 4 + 16);
+  l.keys_b = reinterpret_cast<uint32_t*>(b + off);
+  const size_t widest = unique && n <= kDirectWords ? ((size_t)1 << kMaxSpanLog2) / 8 : 0;
+  off += up(std::max((size_t)n * 4 + 16, widest));
   l.key_words = (size_t)(b + off - reinterpret_cast<uint8_t*>(l.keys_a)) / 4;
   l.bitmap_bits = std::min<size_t>((((size_t)n * 4 + 16) / 16) * 16 * 8, (size_t)1 << kMaxSpanLog2);
+  l.bitmap_cap = std::max(l.bitmap_bits, widest * 8);
   // the direct path leaves keys_b free; larger inputs may be partitioned into it
   if (n <= kDirectWords) l.bitmap = l.keys_b;
   else l.bitmap = reinterpret_cast<uint32_t*>(b + off), off += up(l.bitmap_bits / 8);
@@ -389,7 +404,7 @@ __device__ __forceinline__ void load_words(int32_t (&w)[kItems], const int32_t* 
 template <bool kVec>
 __global__ void __launch_bounds__(kThreads) compact_kernel(const int32_t* words, int n_words, int nib, Divider div,
                                                            uint32_t* keys, Control* ctl, Plan* plan, uint4* bitmap,
-                                                           uint32_t bitmap_units, unsigned long long bitmap_bits,
+                                                           uint32_t bitmap_units, unsigned long long bitmap_cap,
                                                            int32_t* out, int* result) {
   __shared__ uint32_t s_range[2];  // max of ~key (so the minimum), max key
   __shared__ uint32_t s_keys[kWarps * kRegion];
@@ -501,10 +516,14 @@ __global__ void __launch_bounds__(kThreads) compact_kernel(const int32_t* words,
   const int m = c->keys;
   const uint32_t lo = ~c->range[0], hi = c->range[1];
   const unsigned long long span = (unsigned long long)hi - (unsigned long long)lo + 1ull;
-  const bool direct = n_words <= kDirectWords || m <= kDirectKeys || span <= kDirectSliceWords * 32ull;
-  const int path = m == 0 ? kPathEmpty : span > bitmap_bits ? kPathRadix : direct ? kPathDirect : kPathPartition;
+  constexpr unsigned long long kSlice = kDirectSliceWords * 32ull;
+  const unsigned long long slices = (span + kSlice - 1) / kSlice;
+  const bool direct = n_words <= kDirectWords || m <= kDirectKeys || slices == 1 ||
+                      (slices <= kDirectFewSlices && m * slices <= kDirectReads);
+  const int path = m == 0 ? kPathEmpty : span > bitmap_cap ? kPathRadix : direct ? kPathDirect : kPathPartition;
   plan->path = path;
   plan->bitmap_words = (uint32_t)((span + 31) / 32);
+  plan->clear = path == kPathDirect && span > bitmap_units * 128ull;
   const int bits = span > 1 ? 64 - __clzll((long long)(span - 1)) : 0;  // bits of the largest key - min
   plan->range_shift = bits > 8 ? (uint32_t)(bits - 8) : 0u;
   if (path == kPathEmpty) {
@@ -522,10 +541,10 @@ cudaError_t launch_compact(int grid, const int32_t* words, int n, int nib, const
   const uint32_t units = (uint32_t)(l.bitmap_bits / 128);
   if ((reinterpret_cast<uintptr_t>(words) & 15) == 0)
     compact_kernel<true><<<grid, kThreads, 0, s>>>(words, n, nib, div, l.keys_a, l.control, l.plan, bitmap, units,
-                                                  l.bitmap_bits, out, result);
+                                                  l.bitmap_cap, out, result);
   else
     compact_kernel<false><<<grid, kThreads, 0, s>>>(words, n, nib, div, l.keys_a, l.control, l.plan, bitmap, units,
-                                                   l.bitmap_bits, out, result);
+                                                   l.bitmap_cap, out, result);
   return cudaGetLastError();
 }
 
@@ -1921,11 +1940,15 @@ __global__ void __launch_bounds__(kShareThreads) emit_kernel(const uint32_t* bit
 
 // Sets the keys' bits straight in the bitmap, then writes its values.  Keys
 // that many CTAs of the compaction kept arrive together, and atomics on one
-// word queue (450 thousand keys over 3 thousand words: 120 us): a bitmap of up
-// to 2^20 bits is built in shared memory first, one per CTA, and each CTA adds
-// its words to the global one, starting at a place of its own.  In a wider
-// bitmap each thread looks at a bit before it sets it, one key at a time so
-// that the looks see the bits set before.
+// word queue (450 thousand keys over 3 thousand words: 120 us): each CTA takes
+// a slice of up to 2^20 bits and a share of the keys, builds the slice in
+// shared memory from those of them that fall in it, and adds its words to the
+// global bitmap, starting at a place of its own.  Where few keys span several
+// slices each thread looks at a bit in memory before it sets it, one key at a
+// time so that the looks see the bits set before.  A range wider than the
+// bitmap that the compaction cleared is cleared here first (until ranges of up
+// to 2^26 values had a bitmap at every size, 8 thousand to 2 million words
+// took the six launches of the radix passes: 73 to 94 us, now 37 to 72).
 static_assert(kDirectSliceWords * 4 >= kEmitSmemBytes, "the slice's memory serves the writing too");
 __device__ __forceinline__ void direct_bitmap_kernel_cta(const uint32_t* keys, Control* ctl, Plan* plan,
                                                          uint32_t* bitmap, int32_t* out, int* result, int* err) {
@@ -1934,34 +1957,46 @@ __device__ __forceinline__ void direct_bitmap_kernel_cta(const uint32_t* keys, C
   if (plan->path != kPathDirect) return;
   const uint32_t m = (uint32_t)ctl->keys, lo = ~ctl->range[0];
   const int words = (int)plan->bitmap_words;
-  const uint32_t first = blockIdx.x * kShareThreads + threadIdx.x, step = gridDim.x * kShareThreads;
   int ctas = gridDim.x;
-  if (words > kDirectSliceWords) {
-    for (uint32_t i = first; i < m; i += step) {
+  if (plan->clear) {
+    uint4* units = reinterpret_cast<uint4*>(bitmap);
+    for (int i = blockIdx.x * kShareThreads + threadIdx.x; i < (words + 3) / 4; i += gridDim.x * kShareThreads)
+      units[i] = make_uint4(0, 0, 0, 0);
+    if (!grid_barrier(&ctl->barrier[2], ctas, err)) return;
+  }
+  const int slices = (words + kDirectSliceWords - 1) / kDirectSliceWords;
+  if (slices > 1 && (m < kDirectSliceKeys || slices > ctas / kDirectSliceCtas)) {
+    for (uint32_t i = blockIdx.x * kShareThreads + threadIdx.x; i < m; i += gridDim.x * kShareThreads) {
       const uint32_t bit = __ldg(keys + i) - lo, mask = 1u << (bit & 31);
       if ((__ldcg(bitmap + (bit >> 5)) & mask) == 0) atomicOr(bitmap + (bit >> 5), mask);
     }
   } else {
-    ctas = (int)min((uint32_t)gridDim.x, (m + kShareThreads - 1) / kShareThreads);
+    if (slices == 1) ctas = (int)min((uint32_t)gridDim.x, (m + kShareThreads - 1) / kShareThreads);
     if ((int)blockIdx.x >= ctas) return;
-    for (int i = threadIdx.x; i < words; i += kShareThreads) s_slice[i] = 0;
+    const int slice = (int)blockIdx.x % slices, part = (int)blockIdx.x / slices;
+    const int parts = (ctas - 1 - slice) / slices + 1;
+    uint32_t* slice_words = bitmap + slice * kDirectSliceWords;
+    const int n = min(kDirectSliceWords, words - slice * kDirectSliceWords);
+    for (int i = threadIdx.x; i < n; i += kShareThreads) s_slice[i] = 0;
     __syncthreads();
-    for (uint32_t i = first; i < m; i += step * 4) {
+    const uint32_t low = lo + (uint32_t)slice * (kDirectSliceWords * 32u), bits = (uint32_t)n * 32u;
+    const uint32_t step = (uint32_t)parts * kShareThreads;
+    for (uint32_t i = part * kShareThreads + threadIdx.x; i < m; i += step * 4) {
       uint32_t bit[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) bit[r] = i + r * step < m ? __ldg(keys + i + r * step) - lo : 0xffffffffu;
+      for (int r = 0; r < 4; ++r) bit[r] = i + r * step < m ? __ldg(keys + i + r * step) - low : 0xffffffffu;
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const uint32_t mask = 1u << (bit[r] & 31);
-        if (bit[r] != 0xffffffffu && (s_slice[bit[r] >> 5] & mask) == 0) atomicOr(s_slice + (bit[r] >> 5), mask);
+        if (bit[r] < bits && (s_slice[bit[r] >> 5] & mask) == 0) atomicOr(s_slice + (bit[r] >> 5), mask);
       }
     }
     __syncthreads();
-    const int turn = (int)((unsigned long long)words * blockIdx.x / ctas);
-    for (int i = threadIdx.x; i < words; i += kShareThreads) {
-      const int k = i + turn < words ? i + turn : i + turn - words;
+    const int turn = (int)((unsigned long long)n * part / parts);
+    for (int i = threadIdx.x; i < n; i += kShareThreads) {
+      const int k = i + turn < n ? i + turn : i + turn - n;
       const uint32_t v = s_slice[k];
-      if (v && (__ldcg(bitmap + k) & v) != v) atomicOr(bitmap + k, v);
+      if (v && (__ldcg(slice_words + k) & v) != v) atomicOr(slice_words + k, v);
     }
   }
   if (!grid_barrier(&ctl->barrier[0], ctas, err)) return;
@@ -2509,7 +2544,7 @@ cudaError_t bounded_wait_probe(double limit_s, int* err, cudaStream_t s) {
 }
 
 size_t sort_scratch_bytes(int n) { return n <= kSmall ? 0 : layout(nullptr, n).bytes; }
-size_t feedback_scratch_bytes(int n) { return n <= kSmall ? 0 : layout(nullptr, n).bytes; }
+size_t feedback_scratch_bytes(int n) { return n <= kSmall ? 0 : layout(nullptr, n, true).bytes; }
 size_t sort_status_bytes(int n) { return n <= kSmall ? 0 : (size_t)tiles_of(n, kDigitTile) * kBuckets * 8; }
 // the digit passes' words, or the unique kernel's one per tile of sorted keys
 size_t feedback_status_bytes(int n) { return std::max(sort_status_bytes(n), (size_t)tiles_of(n, kTile) * 8); }
@@ -2524,7 +2559,7 @@ cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t
     else launch_small_unique<kSmall / kSmallThreads>(words, n, nib, unique_out, result, done, s);
     return cudaGetLastError();
   }
-  const SortScratchLayout l = layout(scratch, n);
+  const SortScratchLayout l = layout(scratch, n, true);
   cudaError_t e;
   if ((e = cudaMemsetAsync(l.control, 0, sizeof(Control), s)) != cudaSuccess) return e;
   const int tiles = tiles_of(n, kTile);
@@ -2537,7 +2572,7 @@ cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t
   uint32_t* bitmap = l.bitmap;
   {
     const int grid =
-        persistent_grid<direct_bitmap_kernel>(tiles_of(n, kShareThreads), kShareThreads, kDirectSliceWords * 4);
+        persistent_grid<direct_bitmap_kernel>(1 << 30, kShareThreads, kDirectSliceWords * 4);
     DoneFlag d = n <= kDirectWords ? done : DoneFlag{};
     void* args[] = {&keys, &control, &plan, &bitmap, &unique_out, &result, &err, &d};
     e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(direct_bitmap_kernel), dim3(grid),
@@ -2562,7 +2597,7 @@ bool feedback_unique_needs_radix(const int* result) { return result[1] == kPathR
 cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scratch, unsigned long long* status,
                                          uint32_t epoch, int* result, int* err, const DoneFlag& done,
                                          cudaStream_t s) {
-  const SortScratchLayout l = layout(scratch, n);
+  const SortScratchLayout l = layout(scratch, n, true);
   cudaError_t e;
   if ((e = launch_digit_hist(l.keys_a, n, &l.control->keys, 0u, false, 0, l, s)) != cudaSuccess) return e;
   const DigitBuffers bufs = {l.keys_a, l.keys_a, l.keys_b, nullptr};

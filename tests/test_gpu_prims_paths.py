@@ -157,3 +157,19 @@ def test_unique_large_paths(built, case):
     else:
         words = _wide(rng, (1 << 22) + 3)
     _check_unique(words, 0)
+
+
+@pytest.mark.parametrize("n", [8193, 70001, 1 << 19, (1 << 21) - 3, (1 << 21) + 1])
+@pytest.mark.parametrize("bits", [15, 20, 21, 22, 25, 26])
+@pytest.mark.parametrize("kept", [0.03, 0.9])
+def test_unique_bitmap_slices(built, n, bits, kept):
+    """Bitmaps of one slice, of several (few keys and many), wider than 32 bits
+    per input word, of the widest range that has one, and one value wider."""
+    rng = np.random.default_rng(n + bits)
+    for span in {15: [31 << 15], 20: [1 << 20, (1 << 20) + 1], 26: [1 << 26, (1 << 26) + 1]}.get(bits, [1 << bits]):
+        words = np.full(n, NO_HIT, np.int32)
+        at = rng.permutation(n)[:max(2, int(n * kept))]
+        keys = np.where(rng.random(at.size) < 0.5, rng.integers(0, span, at.size), rng.integers(0, 1 + span // 64, at.size))
+        keys[:2] = 0, span - 1
+        words[at] = (keys - span // 3).astype(np.int32)
+        _check_unique(words, 0, offset=n % 2)
