@@ -123,9 +123,10 @@ class Server {
   // group by group, and the frames of all but the last group are copied to the
   // host beside the groups after them, those that turn out to be done (no
   // fault).  A launch's tail of long rays costs 30 us a group, so there are at
-  // most four: 17.5 million rays take 1439 us in 4 groups, 1480 in 8, 1715 in
-  // one; 9.2 million 725 in 4, 770 in 2.
-  static constexpr int64_t kGroupRays = 2 << 20;
+  // most four: 17.5 million rays of 8 clients take 1439 us in 4 groups, 1480 in
+  // 8, 1715 in one; 7.8 million of 3 clients 541 in 3, 595 in 2 (groups of 2
+  // million rays or more); 3.9 million of 3 353 in 3, 386 in one.
+  static constexpr int64_t kGroupRays = 1 << 20;
   static constexpr int kMaxGroups = 4;
   cudaEvent_t group_ev_ = nullptr, early_ev_ = nullptr;
   bool early_pending_ = false;  // early_ev_ marks copies from framebuffers
