@@ -119,13 +119,16 @@ class Server {
   // requests as done once their images are on the host.
   cudaStream_t copy_s_ = nullptr;
   cudaEvent_t staged_ev_ = nullptr, copied_ev_ = nullptr;
-  // A tick whose new requests' rays fill several of these launches traces them
-  // group by group, and the frames of all but the last group are copied to the
-  // host beside the groups after them, those that turn out to be done (no
-  // fault).  A launch's tail of long rays costs 30 us a group, so there are at
-  // most four: 17.5 million rays of 8 clients take 1439 us in 4 groups, 1480 in
-  // 8, 1715 in one; 7.8 million of 3 clients 541 in 3, 595 in 2 (groups of 2
-  // million rays or more); 3.9 million of 3 353 in 3, 386 in one.
+  // A tick that no request waits behind sends its new requests' frames, those
+  // that turn out to be done (no fault), straight from the framebuffers, and
+  // where their rays fill several of these launches it traces them group by
+  // group, each group's frames on their way beside the groups after it.  A
+  // launch's tail of long rays costs 30 us a group, so there are at most four:
+  // 17.5 million rays of 8 clients take 1439 us in 4 groups, 1480 in 8, 1715 in
+  // one; 7.8 million of 3 541 in 3, 595 in 2; 3.9 million of 3 353 in 3, 386 in
+  // one.  Under a backlog the copies run beside the next tick, which would
+  // have to wait for those from framebuffers: 16 clients in a closed loop
+  // deliver 6330 frames/s so, 5850 group by group.
   static constexpr int64_t kGroupRays = 1 << 20;
   static constexpr int kMaxGroups = 4;
   cudaEvent_t group_ev_ = nullptr, early_ev_ = nullptr;
@@ -383,6 +386,7 @@ TraceParams Server::Params(int k) const {
 // One tick: admit, one pass over everything in flight, feedback, transaction.
 int Server::Step(int* finished) {
   if (finished) *finished = 0;
+  bool waiting = false;  // requests that the next tick may admit
   {
     std::lock_guard<std::mutex> lock(mu_);
     // under the lock: every request admitted here was submitted before
@@ -406,6 +410,7 @@ int Server::Step(int* finished) {
       flights_.push_back(f);
       it = queue_.erase(it);
     }
+    waiting = !queue_.empty();
   }
   if (flights_.empty()) return RAYT_OK;
 
@@ -444,11 +449,14 @@ int Server::Step(int* finished) {
     }
   // the framebuffers the tick writes are not read by the last tick's copies
   // any more (they ran beside its traversal)
-  if (early_pending_) RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, early_ev_, 0));
-  early_pending_ = false;
+  if (early_pending_ && !views.empty()) {
+    RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, early_ev_, 0));
+    early_pending_ = false;
+  }
   int64_t fresh_rays = 0;
   for (const ViewDesc& v : views) fresh_rays += (int64_t)v.width * v.height;
-  const int64_t groups = cfg_.deliver_to_host ? std::min<int64_t>(kMaxGroups, fresh_rays / kGroupRays) : 1;
+  const bool straight = cfg_.deliver_to_host && !waiting;
+  const int64_t groups = straight ? std::min<int64_t>(kMaxGroups, fresh_rays / kGroupRays) : 1;
   const int64_t group_rays = groups > 1 ? (fresh_rays + groups - 1) / groups : fresh_rays;
   std::vector<char> early(clients_.size(), 0);  // clients whose frames were sent on their way below
   for (size_t g = 0; g < views.size();) {
@@ -471,7 +479,7 @@ int Server::Step(int* finished) {
     q.lanes = trace_lanes(true, (int)tiles * 32);
     RAYT_CUDA_TRY(launch_trace(q, true, false, (int)tiles * 32, 0, s_));
     ++stats.kernel_launches;
-    if (groups > 1 && g + n < views.size()) {
+    if (straight) {
       DeliverParams d{};
       d.faults = d_client_faults_[k];
       for (int i = 0; i < n; ++i) {

@@ -155,6 +155,26 @@ def test_served_delivery_in_groups(trees, max_blocks):
     srv.close()
 
 
+@pytest.mark.parametrize("requests", [1, 2, 3])
+def test_served_delivery_under_backlog(trees, requests):
+    """Requests that wait behind a tick (frames then go through the stages beside
+    the next tick) and none (frames go straight from the framebuffers, in groups
+    where there are many rays): each client's last image is the resident oracle's."""
+    sizes = [(1280, 720), (96, 64), (1024, 1024)]
+    pixels = sum(w * h + 64 for w, h in sizes)
+    ld, cm, srv = _server(trees, max_blocks=0, deliver_to_host=True, framebuffer_bytes=4 * pixels,
+                          max_rays_in_flight=pixels)
+    ids = [srv.add_client(w, h) for w, h in sizes]
+    for f in range(2):
+        mats = [[_matrix(_cam(70.0 * v + 25.0 * k + 40.0 * f, v), w, h) for k in range(requests)]
+                for v, (w, h) in enumerate(sizes)]
+        for r in [srv.submit(c, m) for k in range(requests) for c, m in zip(ids, (x[k] for x in mats))]:
+            assert not srv.wait(r)["truncated"]
+        for v, (c, (w, h)) in enumerate(zip(ids, sizes)):
+            np.testing.assert_array_equal(srv.host_image(c), _resident(trees, w, h, mats[v][-1]), err_msg="%d %d" % (v, f))
+    srv.close()
+
+
 def test_served_admission_limits(trees):
     # framebuffer memory admits clients: 2 frames of 128x128 fit, a third does not
     ld, cm, srv = _server(trees, framebuffer_bytes=2 * 128 * 128 * 4)
