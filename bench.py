@@ -1087,15 +1087,14 @@ def zipf_words(n, seed=5, blocks=1 << 24, s=1.1):
 def c2_path(words, nib):
     """(kept words, bitmap path taken, key span) of one feedback-unique call:
     the library takes the bitmap path when the kept keys (after NodeToBlock)
-    span at most 32 values per input word and at most 2^26."""
+    span at most 2^26 values."""
     w = words[words != 0x7FFFFFFF].astype(np.int64)
     hit = w > 0
     w[hit] = ((((w[hit] >> 1) - 1) // nib + 1) << 1) | (w[hit] & 1)
     if w.size == 0:
         return 0, False, 0
     span = int(w.max() - w.min() + 1)
-    cap = ((words.size * 4 + 16) // 16) * 16 * 8
-    return int(w.size), span <= cap and span <= (1 << 26), span
+    return int(w.size), span <= 1 << 26, span
 
 
 def time_primitives(R, n, steps):
@@ -1184,10 +1183,10 @@ def bench_c2(args, rank, world, local):
     t_e2e = max_over_ranks(time.perf_counter() - t, world)
     clk = clocks.stop()
     m, bitmap, span = c2_path(words, 4096)
-    if bitmap:  # compaction, range histogram, partition, bucket bitmaps, bitmap clear/write/read, unique out
-        alg = 4 * n + 4 * m + 4 * m + 8 * m + 4 * m + 3 * ((span + 31) // 32) * 4 + 4 * cnt
-    else:  # compaction, four digit passes, unique
-        alg = 4 * n + 4 * m + 32 * m + 4 * m + 4 * cnt
+    # what any method reads and writes: the words and the unique array (the
+    # compaction drops most repeats, so the passes after it are over keys that
+    # the host does not count)
+    alg = 4 * n + 4 * cnt
     achieved = alg / (t_dev / steps) / 1e9
     peak, kind = hbm_peak()
     if rank != 0:
@@ -1220,9 +1219,9 @@ def bench_c2(args, rank, world, local):
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "traffic": traffic, "traffic_rule": traffic_rule,
                          "peak_source": kind,
-                         "kernel": ("compaction + range partition + bucket bitmaps + bitmap unique (one call)" if bitmap
+                         "kernel": ("compaction + range partition + bucket bitmaps + emit (one call)" if bitmap
                                     else "compaction + 4 digit passes + unique (one call)")},
-            "cpu_baseline": cpu, "gpu_launches": steps * 12, "clocks": clk, "primitives": prims}
+            "cpu_baseline": cpu, "gpu_launches": steps * (2 if n <= 1 << 21 else 6 if bitmap else 12), "clocks": clk, "primitives": prims}
 
 
 def main():
