@@ -204,7 +204,7 @@ int rayt_renderer_set_max_passes(rayt_renderer* r, int max_passes);
  * srand(seed), which the reference's feedback extractor draws from
  * (ray-tracing-feedback-extractor.cpp:147). */
 int rayt_renderer_seed(rayt_renderer* r, uint32_t seed);
-/* Replay each pass's device work (feedback reset, traversal, feedback unique)
+/* Replay each pass's device work (traversal, feedback unique)
  * from a CUDA graph built once per pass kind (default on; recording passes
  * uses plain launches).  Results do not depend on it. */
 int rayt_renderer_use_graphs(rayt_renderer* r, int on);
@@ -390,7 +390,9 @@ int rayt_server_stats_get(const rayt_server* s, rayt_server_stats* out);
 /* Feedback primitives on device arrays of int32. */
 
 /* GPUSort::Sort (rayt/GPU algorithms/gpu-sort.cpp:16-49): ascending signed
- * sort in place (LSD radix sort, 8-bit digits, decoupled look-back). */
+ * sort in place (one CTA for few keys; evenly spread keys are moved to parts of
+ * their range and sorted there; others by an LSD radix sort of 8-bit digits).
+ * Returns when the array is sorted. */
 int rayt_sort_i32(int32_t* device_data, int n, void* stream);
 /* GPUScan::Scan (rayt/GPU algorithms/gpu-scan.cpp:15-43): inclusive prefix
  * sum in place, wrapping int32 arithmetic. */
@@ -399,12 +401,10 @@ int rayt_scan_i32(int32_t* device_data, int n, void* stream);
  * NodeToBlock (when nodes_in_block > 0), then the sorted unique values
  * (signed ascending, RAYT_NO_HIT last when present) into device_unique (n
  * entries of room); *unique_count (host) receives the count.  Computed as
- * stream compaction, then, when the kept values span at most 32 per input
- * word and at most 2^26, a bitmap over their range read in order; otherwise
- * an LSD radix sort and unique.  The scratch memory is a device buffer the
- * library keeps per device and grows on demand.  The device work is captured
- * once as a CUDA graph and replayed while the pointers, n and nodes_in_block
- * repeat (one graph per device is kept).  device_words is not modified. */
+ * stream compaction, then, when the kept values span at most 2^26, a bitmap
+ * over their range read in order; otherwise an LSD radix sort and unique.  The
+ * scratch memory is a device buffer the library keeps per device and grows on
+ * demand.  Returns when the values are written; device_words is not modified. */
 int rayt_feedback_unique(const int32_t* device_words, int n, int nodes_in_block,
                          int32_t* device_unique, int* unique_count, void* stream);
 
@@ -418,7 +418,7 @@ int rayt_feedback_unique(const int32_t* device_words, int n, int nodes_in_block,
  * All calls on a device share that array: calls whose GPU work overlaps race.
  * The library serialises its own calls: this entry point, rayt_sort_i32,
  * rayt_scan_i32 and rayt_feedback_unique take one lock and return after their
- * stream finished (they share the look-back epoch).  The
+ * kernels finished (they share the look-back epoch).  The
  * first call on a device looks up the array's address and zeroes the array on
  * `stream`; make it before any stream capture.
  * Returns after the result is on the device and *unique_count is set. */
@@ -428,7 +428,7 @@ int rayt_feedback_unique_noalloc(const int32_t* device_words, int n, int nodes_i
 
 /* No counterpart in the reference.  Failure detection self-test: every wait
  * of a kernel on another CTA's result (the sort's look-back) gives up after a
- * time limit (1 s), sets a device error flag and returns, and the call reports
+ * time limit (1 s), sets an error flag and returns, and the call reports
  * RAYT_E_TIMEOUT with the context still usable.  This runs one such wait on a
  * word nothing ever publishes, with a limit of limit_s seconds, and returns
  * RAYT_OK when the wait gave up and was reported as it must. */
