@@ -360,7 +360,9 @@ __device__ __forceinline__ uint32_t divide(uint32_t x, Divider v) {
 // (scalar loads otherwise, and for the last, partial tile).  The next tile's
 // loads are issued before the current tile is processed, so memory latency
 // overlaps the work.  The per-word loop only drops NO_HIT words: each warp
-// appends the words it keeps to its own region of shared memory.
+// appends the words it keeps to its own region of shared memory, each thread's
+// together (a ballot and two counts per row of 32 words instead: 349 us for the
+// unique of 2^28 words, so 341).
 // NodeToBlock, the key mapping and the filter run when the regions are
 // flushed, on the kept words with every lane busy (at 10% kept words, doing
 // them per word cost three quarters of the instructions of an issue-bound
@@ -432,12 +434,21 @@ __global__ void __launch_bounds__(kThreads) compact_kernel(const int32_t* words,
     const uint32_t next = base + stride;
     load_words<kVec>(nxt, words, n, next + mine);
     const uint32_t before = fill;
+    {  // each thread's kept words together: one scan for the tile's 16 words
+      uint32_t count = 0;
 #pragma unroll
-    for (int q = 0; q < kItems; ++q) {
-      const bool keep = cur[q] != kNoHit;  // words past the end were loaded as NO_HIT
-      const unsigned mask = __ballot_sync(0xffffffffu, keep);
-      if (keep) region[fill + __popc(mask & lt)] = (uint32_t)cur[q];
-      fill += __popc(mask);
+      for (int q = 0; q < kItems; ++q) count += cur[q] != kNoHit;  // words past the end were loaded as NO_HIT
+      uint32_t incl = count;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += t;
+      }
+      uint32_t* at = region + fill + (incl - count);
+      fill += __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+      for (int q = 0; q < kItems; ++q)
+        if (cur[q] != kNoHit) *at++ = (uint32_t)cur[q];
     }
     {
       const uint32_t first = base + warp * (kItems * 32);
