@@ -122,13 +122,16 @@ class Server {
   // A tick that no request waits behind sends its new requests' frames, those
   // that turn out to be done (no fault), straight from the framebuffers, and
   // where their rays fill several of these launches it traces them group by
-  // group, each group's frames on their way beside the groups after it.  A
-  // launch's tail of long rays costs 30 us a group, so there are at most four:
-  // 17.5 million rays of 8 clients take 1439 us in 4 groups, 1480 in 8, 1715 in
-  // one; 7.8 million of 3 541 in 3, 595 in 2; 3.9 million of 3 353 in 3, 386 in
-  // one.  Under a backlog the copies run beside the next tick, which would
-  // have to wait for those from framebuffers: 16 clients in a closed loop
-  // deliver 6330 frames/s so, 5850 group by group.
+  // group, each group's frames on their way beside the groups after it.  The
+  // copies' stream has the higher priority: a group's CTAs leave no SM room for
+  // the copy's until its last wave (8 clients, 17.5 million rays 1513 -> 1376
+  // us; 9.2 million 769 -> 685).  A launch's tail of long rays costs 30 us a
+  // group, so there are at most four: 8 clients take 1376 us in 4 groups, 1425
+  // in 6, 1440 in 8, 1483 in 3 (before the priority 1715 in one); 3.9 million
+  // rays of 3 clients 329 in 3, 386 in one.  Under a backlog the copies run
+  // beside the next tick, which would have to wait for those from
+  // framebuffers: 16 clients in a closed loop deliver 6330 frames/s so, 5850
+  // group by group.
   static constexpr int64_t kGroupRays = 1 << 20;
   static constexpr int kMaxGroups = 4;
   cudaEvent_t group_ev_ = nullptr, early_ev_ = nullptr;
@@ -194,7 +197,9 @@ int Server::Init(Cache* cache, const rayt_server_config& cfg) {
   RAYT_CUDA_TRY(cudaMemsetAsync(d_passes_, 0, 4, s_));
   RAYT_CUDA_TRY(cudaMemsetAsync(d_images_, 0, image_pixels_ * 4, s_));
   if (cfg.deliver_to_host) {
-    RAYT_CUDA_TRY(cudaStreamCreateWithFlags(&copy_s_, cudaStreamNonBlocking));
+    int least = 0, greatest = 0;
+    RAYT_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    RAYT_CUDA_TRY(cudaStreamCreateWithPriority(&copy_s_, cudaStreamNonBlocking, greatest));
     RAYT_CUDA_TRY(cudaEventCreateWithFlags(&staged_ev_, cudaEventDisableTiming));
     RAYT_CUDA_TRY(cudaEventCreateWithFlags(&copied_ev_, cudaEventDisableTiming));
     RAYT_CUDA_TRY(cudaEventCreateWithFlags(&group_ev_, cudaEventDisableTiming));
