@@ -789,7 +789,7 @@ __device__ __forceinline__ uint32_t digit_tile_bytes(int t, int m) {
 // Keys of few different values need no passes: the first pass's launch counts
 // each value and the second's writes the runs (four launches over 2^26 keys of
 // 201 values took 1490 us, as every lane's digit met in two words; counted,
-// 290).  The counters lie in the CTA's shared memory, one per lane and value
+// 252).  The counters lie in the CTA's shared memory, one per lane and value
 // where there is room for that, so that frequent values do not queue.
 __device__ __forceinline__ void count_values(const uint32_t* keys, int n, uint32_t flip, Plan* plan, uint32_t* smem) {
   const int values = plan->counting, lane = threadIdx.x & 31;
@@ -820,14 +820,18 @@ __device__ __forceinline__ void count_values(const uint32_t* keys, int n, uint32
   }
 }
 
-// Every CTA scans the counts and writes its part of the runs.
-__device__ __forceinline__ void write_values(uint32_t* out, int n, uint32_t flip, const Plan* plan, uint32_t* smem) {
+// Every CTA scans the counts and writes its part of the runs, kValues of them at
+// most (the scan and the bisection are unrolled over that many: 300 thousand
+// keys of 201 values 47 us with 16384 always, 35 with 512; loops over the values
+// there are were 25% slower for 16000).
+template <int kValues>
+__device__ __forceinline__ void write_values_of(uint32_t* out, int n, uint32_t flip, const Plan* plan, uint32_t* smem) {
   __shared__ uint32_t s_warp[kDigitWarps];
   const int values = plan->counting, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lo = plan->lowest;
   // smem[v]: the first position of value v; thread t scans `per` values
-  constexpr int kPer = kCountValues / kDigitThreads;
-  for (int v = threadIdx.x; v < kCountValues; v += kDigitThreads) smem[v] = v < values ? plan->values[v] : 0u;
+  constexpr int kPer = kValues / kDigitThreads;
+  for (int v = threadIdx.x; v < kValues; v += kDigitThreads) smem[v] = v < values ? plan->values[v] : 0u;
   __syncthreads();
   uint32_t sum = 0;
   for (int k = 0; k < kPer; ++k) sum += smem[threadIdx.x * kPer + ((k + lane) & (kPer - 1))];
@@ -854,7 +858,8 @@ __device__ __forceinline__ void write_values(uint32_t* out, int n, uint32_t flip
   const bool whole = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   for (uint32_t p = (blockIdx.x * kDigitThreads + threadIdx.x) * 4u; p < (uint32_t)n; p += step) {
     int v = 0;
-    for (int half = kCountValues / 2; half > 0; half >>= 1)
+#pragma unroll
+    for (int half = kValues / 2; half > 0; half >>= 1)
       if (v + half < values && smem[v + half] <= p) v += half;
     uint32_t q[4];
 #pragma unroll
@@ -870,6 +875,11 @@ __device__ __forceinline__ void write_values(uint32_t* out, int n, uint32_t flip
         if (p + r < (uint32_t)n) out[p + r] = q[r];
     }
   }
+}
+
+__device__ __forceinline__ void write_values(uint32_t* out, int n, uint32_t flip, const Plan* plan, uint32_t* smem) {
+  if (plan->counting <= kDigitThreads) write_values_of<kDigitThreads>(out, n, flip, plan, smem);
+  else write_values_of<kCountValues>(out, n, flip, plan, smem);
 }
 
 // Key `li` of a partial tile of `valid` keys: in shared memory, or past the last
