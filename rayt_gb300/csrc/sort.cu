@@ -1183,7 +1183,7 @@ __device__ __forceinline__ uint32_t cta_exclusive(uint32_t v, uint32_t* s_wsum) 
 // for 2^26 keys where two per SM of 16384 took 310, 97 of them for the stores
 // being scattered.  A tile's keys are read again (from L2) to be staged, as
 // registers hold their ranks.  Each CTA has its next tile fetched into L2.
-template <bool kVec>
+template <bool kVec, int kGroups>
 __device__ __forceinline__ void split_cta(const uint32_t* keys, uint32_t n, uint32_t* regions, const SplitShape shape,
                                           Control* ctl, Plan* plan, uint32_t* smem) {
   __shared__ uint32_t s_wsum[kMoveThreads / 32];
@@ -1205,15 +1205,16 @@ __device__ __forceinline__ void split_cta(const uint32_t* keys, uint32_t n, uint
       const uint32_t next = (t + gridDim.x) * tile;
       fetch_keys(keys, next, min(n, next + tile));
     }
-    uint32_t ranks[kMoveGroups * 2];
+    constexpr int kBatch = kGroups < 4 ? kGroups : 4;
+    uint32_t ranks[kGroups * 2];
     auto range_of = [&](uint32_t x) { return __umulhi(x, factor); };
 #pragma unroll
-    for (int h = 0; h < kMoveGroups; h += 4) {
-      uint4 v[4];
+    for (int h = 0; h < kGroups; h += kBatch) {
+      uint4 v[kBatch];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
+      for (int g = 0; g < kBatch; ++g) v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
+      for (int g = 0; g < kBatch; ++g) {
         const uint32_t at = begin + ((h + g) * kMoveThreads + threadIdx.x) * 4;
         const uint32_t k[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
         uint32_t r[4] = {0, 0, 0, 0};
@@ -1259,12 +1260,12 @@ __device__ __forceinline__ void split_cta(const uint32_t* keys, uint32_t n, uint
     }
     if (full) *(volatile int*)&ctl->split_over = 1;
 #pragma unroll
-    for (int h = 0; h < kMoveGroups; h += 4) {
-      uint4 v[4];
+    for (int h = 0; h < kGroups; h += kBatch) {
+      uint4 v[kBatch];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
+      for (int g = 0; g < kBatch; ++g) v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
+      for (int g = 0; g < kBatch; ++g) {
         const uint32_t at = begin + ((h + g) * kMoveThreads + threadIdx.x) * 4;
         const uint32_t k[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
         const uint32_t r[2] = {ranks[(h + g) * 2], ranks[(h + g) * 2 + 1]};
@@ -1285,7 +1286,7 @@ __device__ __forceinline__ void split_cta(const uint32_t* keys, uint32_t n, uint
     __syncthreads();
   }
 }
-template <bool kVec>
+template <bool kVec, int kGroups>
 __global__ void __launch_bounds__(kMoveThreads, 1) split_kernel(const uint32_t* keys, int n, uint32_t* regions,
                                                                  const SplitShape shape, Control* ctl, Plan* plan) {
   extern __shared__ __align__(128) uint32_t smem[];
@@ -1297,7 +1298,7 @@ __global__ void __launch_bounds__(kMoveThreads, 1) split_kernel(const uint32_t* 
     return;
   }
   if (!plan->split) return;
-  split_cta<kVec>(keys, (uint32_t)n, regions, shape, ctl, plan, smem);
+  split_cta<kVec, kGroups>(keys, (uint32_t)n, regions, shape, ctl, plan, smem);
   if (!last_cta(&ctl->done[3], gridDim.x)) return;
   // where each range's keys begin in the array
   const uint32_t ranges = (uint32_t)shape.ranges, per = (ranges + kMoveThreads - 1) / kMoveThreads;
@@ -1365,6 +1366,7 @@ __device__ __forceinline__ void sort_run(uint32_t* s_keys, uint32_t at) {
     *reinterpret_cast<uint4*>(s_keys + run_place(at + u)) = make_uint4(k[u], k[u + 1], k[u + 2], k[u + 3]);
 }
 
+template <int kGroups>
 __device__ __forceinline__ bool split_sort_cta(uint32_t* out, const uint32_t* regions, const SplitShape shape,
                                                const Plan* plan, uint32_t* smem) {
   __shared__ uint32_t s_wsum[kSplitThreads / 32];
@@ -1383,15 +1385,16 @@ __device__ __forceinline__ bool split_sort_cta(uint32_t* out, const uint32_t* re
     for (uint32_t i = threadIdx.x * 4; i < bins; i += kSortBinsUnit)
       *reinterpret_cast<uint4*>(s_bin + i) = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    uint32_t ranks[kSplitGroups * 2];
+    constexpr int kBatch = kGroups < 4 ? kGroups : 4;
+    uint32_t ranks[kGroups * 2];
 #pragma unroll
-    for (int h = 0; h < kSplitGroups; h += 4) {
+    for (int h = 0; h < kGroups; h += kBatch) {
       if (h * kSplitThreads * 4 >= count) break;
-      uint4 v[4];
+      uint4 v[kBatch];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) v[g] = load_unit<true>(keys, (h + g) * kSplitThreads + threadIdx.x, count);
+      for (int g = 0; g < kBatch; ++g) v[g] = load_unit<true>(keys, (h + g) * kSplitThreads + threadIdx.x, count);
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
+      for (int g = 0; g < kBatch; ++g) {
         const uint32_t at = ((h + g) * kSplitThreads + threadIdx.x) * 4;
         const uint32_t k[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
         uint32_t r[4] = {0, 0, 0, 0};
@@ -1425,13 +1428,13 @@ __device__ __forceinline__ bool split_sort_cta(uint32_t* out, const uint32_t* re
     const bool crowded = __syncthreads_or(most > kCrowded) && !single;
     any_crowded |= crowded;
 #pragma unroll
-    for (int h = 0; h < kSplitGroups; h += 4) {
+    for (int h = 0; h < kGroups; h += kBatch) {
       if (h * kSplitThreads * 4 >= count) break;
-      uint4 v[4];
+      uint4 v[kBatch];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) v[g] = load_unit<true>(keys, (h + g) * kSplitThreads + threadIdx.x, count);
+      for (int g = 0; g < kBatch; ++g) v[g] = load_unit<true>(keys, (h + g) * kSplitThreads + threadIdx.x, count);
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
+      for (int g = 0; g < kBatch; ++g) {
         const uint32_t at = ((h + g) * kSplitThreads + threadIdx.x) * 4;
         const uint32_t k[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
         const uint32_t r[2] = {ranks[(h + g) * 2], ranks[(h + g) * 2 + 1]};
@@ -1474,6 +1477,7 @@ __device__ __forceinline__ bool split_sort_cta(uint32_t* out, const uint32_t* re
   return any_crowded;
 }
 // `again` (mapped host memory): 1 if the keys must take the digit passes.
+template <int kGroups>
 __global__ void __launch_bounds__(kSplitThreads, 2) split_sort_kernel(uint32_t* out, int n, const uint32_t* regions,
                                                                       const SplitShape shape, Control* ctl,
                                                                       const Plan* plan, int* again,
@@ -1486,7 +1490,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) split_sort_kernel(uint32_t* 
   else if (!plan->split || *(volatile int*)&ctl->split_over)
     digits = true;
   else
-    digits = split_sort_cta(out, regions, shape, plan, smem);
+    digits = split_sort_cta<kGroups>(out, regions, shape, plan, smem);
   if (digits && threadIdx.x == 0) *(volatile int*)again = 1;
   publish(done);
 }
@@ -2497,7 +2501,7 @@ cudaError_t launch_digits(const DigitBuffers& bufs, int n, const int* count, boo
 // 512 keys on average or more.
 SplitShape split_shape(int n, const SortScratchLayout& l) {
   SplitShape sh{};
-  const int resident = persistent_grid<split_sort_kernel>(1 << 30, kSplitThreads, kSortSmemBytes);
+  const int resident = persistent_grid<split_sort_kernel<kSplitGroups>>(1 << 30, kSplitThreads, kSortSmemBytes);
   const long long full = ((long long)n + (long long)resident * kSplitFill - 1) / ((long long)resident * kSplitFill);
   const long long ranges = std::min<long long>(resident * full, n / 512);
   if (ranges < 1 || ranges > kSplitRanges) return sh;
@@ -2506,7 +2510,7 @@ SplitShape split_shape(int n, const SortScratchLayout& l) {
   sh.room = (uint32_t)std::min<long long>(kSplitRoom, ((long long)room + 3) / 4 * 4);
   if ((size_t)ranges * sh.room > l.key_words) return sh;
   sh.ranges = (int)ranges;
-  const int moving = persistent_grid<split_kernel<true>>(1 << 30, kMoveThreads, kSplitSmemBytes);
+  const int moving = persistent_grid<split_kernel<true, kMoveGroups>>(1 << 30, kMoveThreads, kSplitSmemBytes);
   // tiles: as many for every resident CTA
   const long long turns = ((long long)n + (long long)moving * kMoveTile - 1) / ((long long)moving * kMoveTile);
   const long long tile = ((long long)n + moving * turns - 1) / (moving * turns);
@@ -2516,29 +2520,52 @@ SplitShape split_shape(int n, const SortScratchLayout& l) {
   return sh;
 }
 
-cudaError_t launch_split(uint32_t* keys, int n, const SplitShape& shape, const SortScratchLayout& l, int* again,
-                         const DoneFlag& done, cudaStream_t s) {
+// Kernel K behind the one before it on the stream, grid CTAs of `threads`.
+template <auto K, class... Args>
+cudaError_t launch_behind(int tiles, int threads, int smem, cudaStream_t s, Args... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.blockDim = dim3(kMoveThreads);
+  cfg.gridDim = dim3(persistent_grid<K>(tiles, threads, smem));
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, K, args...);
+}
+
+template <auto K>
+struct Kernel {
+  static constexpr auto value = K;
+};
+
+// Tiles of one 16-byte unit per thread, and regions of one, have kernels that
+// are not unrolled over eight (300 thousand keys: 38.8 us a call with eight
+// always, 34.9 so).
+cudaError_t launch_split(uint32_t* keys, int n, const SplitShape& shape, const SortScratchLayout& l, int* again,
+                         const DoneFlag& done, cudaStream_t s) {
   const int tiles = tiles_of(n, shape.tile);
-  const bool whole = (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
-  cfg.gridDim = dim3(whole ? persistent_grid<split_kernel<true>>(tiles, kMoveThreads, kSplitSmemBytes)
-                           : persistent_grid<split_kernel<false>>(tiles, kMoveThreads, kSplitSmemBytes));
-  cfg.dynamicSmemBytes = kSplitSmemBytes;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, whole ? split_kernel<true> : split_kernel<false>,
-                                           (const uint32_t*)keys, n, l.keys_a, shape, l.control, l.plan);
+  const bool whole = (reinterpret_cast<uintptr_t>(keys) & 15) == 0, one = shape.tile <= 4 * kMoveThreads;
+  const uint32_t* in = keys;
+  auto move = [&](auto kernel) {
+    return launch_behind<decltype(kernel)::value>(tiles, kMoveThreads, kSplitSmemBytes, s, in, n, l.keys_a, shape,
+                                                  l.control, l.plan);
+  };
+  cudaError_t e;
+  if (whole && one) e = move(Kernel<split_kernel<true, 1>>());
+  else if (whole) e = move(Kernel<split_kernel<true, kMoveGroups>>());
+  else if (one) e = move(Kernel<split_kernel<false, 1>>());
+  else e = move(Kernel<split_kernel<false, kMoveGroups>>());
   if (e != cudaSuccess) return e;
-  cfg.blockDim = dim3(kSplitThreads);
-  cfg.gridDim = dim3(persistent_grid<split_sort_kernel>(shape.ranges, kSplitThreads, kSortSmemBytes));
-  cfg.dynamicSmemBytes = kSortSmemBytes;
-  return cudaLaunchKernelEx(&cfg, split_sort_kernel, keys, n, (const uint32_t*)l.keys_a, shape, l.control,
-                            (const Plan*)l.plan, again, done);
+  const uint32_t* regions = l.keys_a;
+  const Plan* plan = l.plan;
+  if (shape.room <= 4 * kSplitThreads)
+    return launch_behind<split_sort_kernel<1>>(shape.ranges, kSplitThreads, kSortSmemBytes, s, keys, n, regions, shape,
+                                               l.control, plan, again, done);
+  return launch_behind<split_sort_kernel<kSplitGroups>>(shape.ranges, kSplitThreads, kSortSmemBytes, s, keys, n, regions,
+                                                        shape, l.control, plan, again, done);
 }
 
 template <int kRounds>
