@@ -593,7 +593,8 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
   dependents_may_start();
   for (int i = blockIdx.x * kHistThreads + threadIdx.x; i < kCountValues; i += gridDim.x * kHistThreads)
     plan->values[i] = 0;
-  for (int i = threadIdx.x; i < kPasses * kBuckets * 32; i += kHistThreads) s_hist[i] = 0;
+  for (int i = threadIdx.x; i < kPasses * kBuckets * 8; i += kHistThreads)
+    reinterpret_cast<uint4*>(s_hist)[i] = make_uint4(0, 0, 0, 0);
   const uint32_t m = count ? (uint32_t)*count : (uint32_t)n;
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -626,10 +627,13 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
       add(__ldg(keys + i));
   }
   __syncthreads();
-  {  // thread t: digit value t of the 4 x 256, its 32 columns from its own bank on
+  {  // thread t: digit value t of the 4 x 256, its 32 columns from its own banks on
     uint32_t sum = 0;
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) sum += s_hist[threadIdx.x * 32 + ((lane + k) & 31)];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint4 v = reinterpret_cast<const uint4*>(s_hist)[threadIdx.x * 8 + ((lane + k) & 7)];
+      sum += v.x + v.y + v.z + v.w;
+    }
     if (sum) atomicAdd(&ctl->hist[threadIdx.x], sum);
   }
   if (in_place) {
@@ -646,7 +650,10 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
   counts[threadIdx.x] = *(volatile uint32_t*)&ctl->hist[threadIdx.x];
   if (threadIdx.x < kPasses) s_max[threadIdx.x] = 0;
   __syncthreads();
-  atomicMax(&s_max[threadIdx.x >> 8], counts[threadIdx.x]);
+  {
+    const uint32_t most = __reduce_max_sync(0xffffffffu, counts[threadIdx.x]);
+    if (lane == 0) atomicMax(&s_max[threadIdx.x >> 8], most);
+  }
   __syncthreads();
   if (threadIdx.x < 32 * kPasses) {
     const int p = threadIdx.x >> 5;
@@ -1212,7 +1219,8 @@ __device__ __forceinline__ void split_cta(const uint32_t* keys, uint32_t n, uint
     for (int h = 0; h < kGroups; h += kBatch) {
       uint4 v[kBatch];
 #pragma unroll
-      for (int g = 0; g < kBatch; ++g) v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
+      for (int g = 0; g < kBatch; ++g)
+        v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
 #pragma unroll
       for (int g = 0; g < kBatch; ++g) {
         const uint32_t at = begin + ((h + g) * kMoveThreads + threadIdx.x) * 4;
@@ -1263,7 +1271,8 @@ __device__ __forceinline__ void split_cta(const uint32_t* keys, uint32_t n, uint
     for (int h = 0; h < kGroups; h += kBatch) {
       uint4 v[kBatch];
 #pragma unroll
-      for (int g = 0; g < kBatch; ++g) v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
+      for (int g = 0; g < kBatch; ++g)
+        v[g] = load_unit<kVec>(keys, begin / 4 + (h + g) * kMoveThreads + threadIdx.x, end);
 #pragma unroll
       for (int g = 0; g < kBatch; ++g) {
         const uint32_t at = begin + ((h + g) * kMoveThreads + threadIdx.x) * 4;
@@ -2564,8 +2573,8 @@ cudaError_t launch_split(uint32_t* keys, int n, const SplitShape& shape, const S
   if (shape.room <= 4 * kSplitThreads)
     return launch_behind<split_sort_kernel<1>>(shape.ranges, kSplitThreads, kSortSmemBytes, s, keys, n, regions, shape,
                                                l.control, plan, again, done);
-  return launch_behind<split_sort_kernel<kSplitGroups>>(shape.ranges, kSplitThreads, kSortSmemBytes, s, keys, n, regions,
-                                                        shape, l.control, plan, again, done);
+  return launch_behind<split_sort_kernel<kSplitGroups>>(shape.ranges, kSplitThreads, kSortSmemBytes, s, keys, n,
+                                                        regions, shape, l.control, plan, again, done);
 }
 
 template <int kRounds>
