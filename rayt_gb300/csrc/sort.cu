@@ -2005,48 +2005,56 @@ __device__ __forceinline__ void direct_bitmap_kernel_cta(const uint32_t* keys, C
       if ((__ldcg(bitmap + (bit >> 5)) & mask) == 0) atomicOr(bitmap + (bit >> 5), mask);
     }
   } else {
-    if (slices == 1) ctas = (int)min((uint32_t)gridDim.x, (m + kShareThreads - 1) / kShareThreads);
-    if ((int)blockIdx.x >= ctas) return;
+    // one slice: a CTA per 1024 keys builds, and per 1024 words at least writes
+    // (8193 words, 820 keys over a million bits: 62 us with one CTA for both, 40 so)
+    int builders = ctas;
+    if (slices == 1) {
+      builders = (int)min((uint32_t)ctas, (m + kShareThreads - 1) / kShareThreads);
+      ctas = min(ctas, max(builders, (words + kShareThreads - 1) / kShareThreads));
+      if ((int)blockIdx.x >= ctas) return;
+    }
     const int slice = (int)blockIdx.x % slices, part = (int)blockIdx.x / slices;
-    const int parts = (ctas - 1 - slice) / slices + 1;
-    uint32_t* slice_words = bitmap + slice * kDirectSliceWords;
-    const int n = min(kDirectSliceWords, words - slice * kDirectSliceWords);
-    for (int i = threadIdx.x; i < n; i += kShareThreads) s_slice[i] = 0;
-    __syncthreads();
-    const uint32_t low = lo + (uint32_t)slice * (kDirectSliceWords * 32u), bits = (uint32_t)n * 32u;
-    const uint32_t step = (uint32_t)parts * kShareThreads;
-    auto set = [&](uint32_t key) {
-      const uint32_t bit = key - low, mask = 1u << (bit & 31);
-      if (bit < bits && (s_slice[bit >> 5] & mask) == 0) atomicOr(s_slice + (bit >> 5), mask);
-    };
-    // eight keys in flight per thread by 16-byte loads, four by scalar ones where
-    // there are too few for that (30 million words, 15 million kept, three
-    // slices: the call took 168 us with four scalar ones, 158 so; 16 keys as many)
-    const uint32_t units = m / (step * 4) * step;  // 16-byte units that give every thread as many
-    const uint4* keys4 = reinterpret_cast<const uint4*>(keys);
-    for (uint32_t u = part * kShareThreads + threadIdx.x; u < units; u += step * 2) {
-      uint4 v[2];
+    const int parts = (builders - 1 - slice) / slices + 1;
+    if ((int)blockIdx.x < builders) {
+      uint32_t* slice_words = bitmap + slice * kDirectSliceWords;
+      const int n = min(kDirectSliceWords, words - slice * kDirectSliceWords);
+      for (int i = threadIdx.x; i < n; i += kShareThreads) s_slice[i] = 0;
+      __syncthreads();
+      const uint32_t low = lo + (uint32_t)slice * (kDirectSliceWords * 32u), bits = (uint32_t)n * 32u;
+      const uint32_t step = (uint32_t)parts * kShareThreads;
+      auto set = [&](uint32_t key) {
+        const uint32_t bit = key - low, mask = 1u << (bit & 31);
+        if (bit < bits && (s_slice[bit >> 5] & mask) == 0) atomicOr(s_slice + (bit >> 5), mask);
+      };
+      // eight keys in flight per thread by 16-byte loads, four by scalar ones where
+      // there are too few for that (30 million words, 15 million kept, three
+      // slices: the call took 168 us with four scalar ones, 158 so; 16 keys as many)
+      const uint32_t units = m / (step * 4) * step;  // 16-byte units that give every thread as many
+      const uint4* keys4 = reinterpret_cast<const uint4*>(keys);
+      for (uint32_t u = part * kShareThreads + threadIdx.x; u < units; u += step * 2) {
+        uint4 v[2];
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const uint32_t none = low - 1u;  // in no slice
-        v[r] = u + r * step < units ? __ldg(keys4 + u + r * step) : make_uint4(none, none, none, none);
+        for (int r = 0; r < 2; ++r) {
+          const uint32_t none = low - 1u;  // in no slice
+          v[r] = u + r * step < units ? __ldg(keys4 + u + r * step) : make_uint4(none, none, none, none);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) set(v[r].x), set(v[r].y), set(v[r].z), set(v[r].w);
       }
+      for (uint32_t i = units * 4 + part * kShareThreads + threadIdx.x; i < m; i += step * 4) {
+        uint32_t key[4];
 #pragma unroll
-      for (int r = 0; r < 2; ++r) set(v[r].x), set(v[r].y), set(v[r].z), set(v[r].w);
-    }
-    for (uint32_t i = units * 4 + part * kShareThreads + threadIdx.x; i < m; i += step * 4) {
-      uint32_t key[4];
+        for (int r = 0; r < 4; ++r) key[r] = i + r * step < m ? __ldg(keys + i + r * step) : low - 1u;
 #pragma unroll
-      for (int r = 0; r < 4; ++r) key[r] = i + r * step < m ? __ldg(keys + i + r * step) : low - 1u;
-#pragma unroll
-      for (int r = 0; r < 4; ++r) set(key[r]);
-    }
-    __syncthreads();
-    const int turn = (int)((unsigned long long)n * part / parts);
-    for (int i = threadIdx.x; i < n; i += kShareThreads) {
-      const int k = i + turn < n ? i + turn : i + turn - n;
-      const uint32_t v = s_slice[k];
-      if (v && (__ldcg(slice_words + k) & v) != v) atomicOr(slice_words + k, v);
+        for (int r = 0; r < 4; ++r) set(key[r]);
+      }
+      __syncthreads();
+      const int turn = (int)((unsigned long long)n * part / parts);
+      for (int i = threadIdx.x; i < n; i += kShareThreads) {
+        const int k = i + turn < n ? i + turn : i + turn - n;
+        const uint32_t v = s_slice[k];
+        if (v && (__ldcg(slice_words + k) & v) != v) atomicOr(slice_words + k, v);
+      }
     }
   }
   if (!grid_barrier(&ctl->barrier[0], ctas, err)) return;
