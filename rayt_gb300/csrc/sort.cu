@@ -43,6 +43,7 @@
 // cleared.  Every wait is bounded and sets an error flag instead of hanging.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "internal.h"
 
@@ -2553,36 +2554,38 @@ cudaError_t launch_behind(int tiles, int threads, int smem, cudaStream_t s, Args
   return cudaLaunchKernelEx(&cfg, K, args...);
 }
 
-template <auto K>
-struct Kernel {
-  static constexpr auto value = K;
-};
+// f of the smallest of 1, 2, 4 and 8 units per thread with which `threads`
+// threads hold `keys`: small tiles and regions have kernels that are not unrolled
+// over eight (a call with eight always and so: 300 thousand keys 38.8 and 34.9 us,
+// a million 45.5 and 41.4).
+template <class F>
+cudaError_t by_units(uint32_t keys, uint32_t threads, const F& f) {
+  if (keys <= 4 * threads) return f(std::integral_constant<int, 1>());
+  if (keys <= 8 * threads) return f(std::integral_constant<int, 2>());
+  if (keys <= 16 * threads) return f(std::integral_constant<int, 4>());
+  return f(std::integral_constant<int, 8>());
+}
 
-// Tiles of one 16-byte unit per thread, and regions of one, have kernels that
-// are not unrolled over eight (300 thousand keys: 38.8 us a call with eight
-// always, 34.9 so).
 cudaError_t launch_split(uint32_t* keys, int n, const SplitShape& shape, const SortScratchLayout& l, int* again,
                          const DoneFlag& done, cudaStream_t s) {
+  static_assert(kMoveGroups == 8 && kSplitGroups == 8, "by_units ends there");
   const int tiles = tiles_of(n, shape.tile);
-  const bool whole = (reinterpret_cast<uintptr_t>(keys) & 15) == 0, one = shape.tile <= 4 * kMoveThreads;
-  const uint32_t* in = keys;
-  auto move = [&](auto kernel) {
-    return launch_behind<decltype(kernel)::value>(tiles, kMoveThreads, kSplitSmemBytes, s, in, n, l.keys_a, shape,
-                                                  l.control, l.plan);
-  };
-  cudaError_t e;
-  if (whole && one) e = move(Kernel<split_kernel<true, 1>>());
-  else if (whole) e = move(Kernel<split_kernel<true, kMoveGroups>>());
-  else if (one) e = move(Kernel<split_kernel<false, 1>>());
-  else e = move(Kernel<split_kernel<false, kMoveGroups>>());
-  if (e != cudaSuccess) return e;
-  const uint32_t* regions = l.keys_a;
+  const bool whole = (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
+  const uint32_t *in = keys, *regions = l.keys_a;
   const Plan* plan = l.plan;
-  if (shape.room <= 4 * kSplitThreads)
-    return launch_behind<split_sort_kernel<1>>(shape.ranges, kSplitThreads, kSortSmemBytes, s, keys, n, regions, shape,
-                                               l.control, plan, again, done);
-  return launch_behind<split_sort_kernel<kSplitGroups>>(shape.ranges, kSplitThreads, kSortSmemBytes, s, keys, n,
-                                                        regions, shape, l.control, plan, again, done);
+  const cudaError_t e = by_units((uint32_t)shape.tile, kMoveThreads, [&](auto units) {
+    constexpr int kGroups = decltype(units)::value;
+    return whole ? launch_behind<split_kernel<true, kGroups>>(tiles, kMoveThreads, kSplitSmemBytes, s, in, n, l.keys_a,
+                                                              shape, l.control, l.plan)
+                 : launch_behind<split_kernel<false, kGroups>>(tiles, kMoveThreads, kSplitSmemBytes, s, in, n,
+                                                               l.keys_a, shape, l.control, l.plan);
+  });
+  if (e != cudaSuccess) return e;
+  return by_units(shape.room, kSplitThreads, [&](auto units) {
+    constexpr int kGroups = decltype(units)::value;
+    return launch_behind<split_sort_kernel<kGroups>>(shape.ranges, kSplitThreads, kSortSmemBytes, s, keys, n, regions,
+                                                     shape, l.control, plan, again, done);
+  });
 }
 
 template <int kRounds>

@@ -71,7 +71,7 @@ SPLIT_KEYS = {
 # one region for each resident CTA at most, whole turns of regions, partial and
 # several tiles; the digits of "overfull" and "repeats" look even, but a region
 # gets more keys than it holds, and bins get repeats by the dozen
-@pytest.mark.parametrize("n", [8193, 155648, 155649, 622593, 1 << 20, 4669441, 5000003, 1 << 23])
+@pytest.mark.parametrize("n", [8193, 155648, 155649, 622593, 1 << 20, 2000003, 4669441, 5000003, 1 << 23])
 @pytest.mark.parametrize("keys", sorted(SPLIT_KEYS))
 @pytest.mark.parametrize("offset", [0, 3])
 def test_sort_split(built, n, keys, offset):
