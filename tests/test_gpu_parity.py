@@ -274,3 +274,76 @@ def test_depth_output_resident_full_hd(trees):
     rt.set_depth_output(False)
     rt.RenderFrame(m)
     np.testing.assert_array_equal(rt.read_image(), ref)
+
+
+def _edge_matrices(w, h):
+    """View matrices whose rays have no direction (an origin at infinity, where
+    m[14] is 0, or a NaN), beside two with infinite and huge entries."""
+    plain = _matrix(C1_CAMERA, w, h).reshape(16)
+    ortho = np.array([.5, 0, 0, .1, 0, .5, 0, .2, 0, 0, -1, .3, 0, 0, 0, 1], np.float32)
+    out = {"identity": np.eye(4, dtype=np.float32).reshape(16), "ortho": ortho, "zero": np.zeros(16, np.float32)}
+    for name, at, v in [("nan", 5, np.nan), ("inf", 0, np.inf), ("huge", 3, 1e38), ("infinite origin", 2, -np.inf)]:
+        out[name] = plain.copy()
+        out[name][at] = v
+    return out
+
+
+@pytest.mark.parametrize("name", sorted(_edge_matrices(8, 8)))
+@pytest.mark.parametrize("blocks", [0, 250])
+def test_rays_without_direction_vs_oracle(trees, name, blocks):
+    """A ray that can neither enter nor leave a child ends at the iteration limit
+    as an error pixel: images, words and depth of such a view, alone and
+    beside an ordinary one, and an ordinary frame after it."""
+    from oracle import oracle as O
+    sizes = [(70, 33), (64, 48)]
+    plain = [_matrix(C1_CAMERA, w, h).reshape(16) for w, h in sizes]
+    edge = _edge_matrices(*sizes[0])[name]
+    frames = [[edge, plain[1]], plain]
+    for views in (sizes[:1], sizes):
+        sc = O.OracleScene(trees["terrain8s"], blocks, views=views)
+        sc.record(True)
+        libc_srand(5)
+        ld = R.StoredOctreeLoader(trees["terrain8s"])
+        cm = R.GPUOctreeCacheManager(blocks, ld)
+        cm.InitialFillCache()
+        rt = R.GPURayTracer.views(cm, views)
+        rt.set_lod_voxel_size(1.0)
+        rt.set_frame_time_limit(1e30)
+        rt.seed(5)
+        rt.record_passes(True)
+        rt.set_depth_output(True)
+        for mats in frames:
+            mats = mats[:len(views)]
+            passes, imgs = sc.render_views(mats)
+            ref = sc.depth()
+            rt.RenderViews(mats)
+            assert rt.stats()["passes"] == passes
+            for p in range(passes):
+                np.testing.assert_array_equal(rt.pass_words(p), sc.pass_words(p), err_msg="pass %d" % p)
+            for v in range(len(views)):
+                np.testing.assert_array_equal(rt.read_image(view=v), imgs[v], err_msg="view %d" % v)
+                d, nodes = rt.read_depth(view=v)
+                np.testing.assert_array_equal(nodes, ref[v][1])
+                np.testing.assert_array_equal(d.view(np.uint32), ref[v][0].view(np.uint32))
+        sc.close()
+        # without recording: the pass's graph
+        rt.record_passes(False)
+        rt.RenderViews(frames[0][:len(views)])
+        red = (rt.read_image(view=0) == (255, 0, 0, 255)).all(-1)
+        if name in ("identity", "ortho", "zero", "nan"):
+            assert red.all()
+
+
+def test_served_rays_without_direction(trees):
+    """One client's such view ends as error pixels and holds up nobody."""
+    ld = R.StoredOctreeLoader(trees["terrain8s"])
+    cm = R.GPUOctreeCacheManager(0, ld)
+    cm.InitialFillCache()
+    srv = R.RenderServer(cm, max_clients=2, framebuffer_bytes=1 << 20, max_rays_in_flight=1 << 18)
+    a, b = srv.add_client(70, 33), srv.add_client(64, 48)
+    ra, rb = srv.submit(a, np.eye(4, dtype=np.float32)), srv.submit(b, _matrix(C1_CAMERA, 64, 48))
+    assert not srv.wait(ra)["truncated"] and not srv.wait(rb)["truncated"]
+    assert (srv.read_image(a) == (255, 0, 0, 255)).all()
+    (ref,), _ = _oracle_frame(trees["terrain8s"], 0, 64, 48, [_matrix(C1_CAMERA, 64, 48)])
+    np.testing.assert_array_equal(srv.read_image(b), ref[1])
+    srv.close()
