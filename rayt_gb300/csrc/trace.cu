@@ -618,12 +618,16 @@ __device__ __forceinline__ int slot_of(const TraceCore& p, uint32_t ray) {
 
 // Pixel (x, y) and view of first-pass ray r (tile r / 32, lane r % 32);
 // false for the lanes of a partial tile that fall outside the view.
-template <class P>
+// kOneTile: the warp's rays lie in one tile, and so in one view; the reduction's
+// result is one for the warp, so that the view is read through uniform loads
+// (12 views 2% faster).  Work stealing hands a warp rays from any offset on,
+// of two tiles and two views.
+template <bool kOneTile, class P>
 __device__ __forceinline__ bool first_pass_pixel(const P& p, int r, int& v, int& x, int& y) {
   const int tile = (int)(r >> 5), k = (int)(r & 31);
-  // a warp's rays lie in one tile; the reduction's result is one for the warp,
-  // so that the view is read through uniform loads (12 views 2% faster)
-  v = sizeof(P) == sizeof(TraceParams1) ? 0 : (int)__reduce_max_sync(__activemask(), (unsigned)view_of_tile(p, tile));
+  if (sizeof(P) == sizeof(TraceParams1)) v = 0;
+  else if (kOneTile) v = (int)__reduce_max_sync(__activemask(), (unsigned)view_of_tile(p, tile));
+  else v = view_of_tile(p, tile);
   const ViewDesc& vd = p.views[v];
   const int t = tile - vd.tile_base;
   // t / tiles_x: the product with the reciprocal rounded up is the quotient or
@@ -644,12 +648,12 @@ __device__ __forceinline__ bool first_pass_pixel(const P& p, int r, int& v, int&
 // record r of the input list): its pixel, origin, direction and (depth
 // output) the distance it advanced in earlier passes; false for the lanes of
 // a partial tile that fall outside their view.
-template <bool kFirst, bool kLazy = false, class P>
+template <bool kFirst, bool kLazy, bool kOneTile, class P>
 __device__ __forceinline__ bool ray_at(const P& p, int r, uint32_t& ray, float4& o, float4& d,
                                        float& adv, int& v, int& x, int& y) {
   adv = 0.0f;
   if (kFirst) {
-    if (!first_pass_pixel(p, r, v, x, y)) return false;
+    if (!first_pass_pixel<kOneTile>(p, r, v, x, y)) return false;
     const ViewDesc& vd = p.views[v];
     if (kLazy) init_direction(vd, x, y, o, d);
     else init_ray(vd, x, y, o, d);
@@ -763,7 +767,7 @@ __global__ void __launch_bounds__(kBlockThreads, 10) trace_kernel(const __grid_c
   float adv;
   int v = 0, x = 0, y = 0;
   constexpr bool kLazy = kFirst && !kCount;
-  if (!ray_at<kFirst, kLazy>(p, r, ray, o, d, adv, v, x, y)) return;
+  if (!ray_at<kFirst, kLazy, true>(p, r, ray, o, d, adv, v, x, y)) return;
   if (!kFirst && p.finish_mask && ((p.finish_mask >> slot_of(p, ray)) & 1ull)) {
     // served mode: the request stops here; FinishTracingFrame's shading with
     // the fault's parent node
@@ -811,7 +815,7 @@ __global__ void __launch_bounds__(kBlockThreads) trace_persistent_kernel(const _
         const int r = base + __popc(idle & ((1u << lane) - 1));
         float4 o, d;
         int v, x, y;
-        if (r < total && ray_at<kFirst>(p, r, ray, o, d, adv, v, x, y)) {
+        if (r < total && ray_at<kFirst, false, false>(p, r, ray, o, d, adv, v, x, y)) {
           s_origin[threadIdx.x] = o;  // kept for the ray's fault record
           s_dir[threadIdx.x] = d;
           cast_begin(c, p.root, o, d);

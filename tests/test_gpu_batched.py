@@ -184,3 +184,29 @@ def test_batched_depth_output_vs_oracle(trees):
                                           err_msg="frame %d view %d" % (f, v))
             np.testing.assert_array_equal(rt.read_image(view=v), imgs[v], err_msg="frame %d view %d" % (f, v))
     sc.close()
+
+
+@pytest.mark.parametrize("shape", [(2, 1, 0, 1), (2, 8, 0, 32), (2, 16, 0, 16), (3, 24, 4, 16), (5, 8, 1, 7), (0, 16, 0, 64)])
+@pytest.mark.parametrize("blocks", [0, 250])
+def test_work_stealing_over_views_vs_oracle(trees, shape, blocks):
+    """Work stealing hands a warp rays of two tiles, and at a view's end of two
+    views: ragged views, some a tile or two wide, of a camera that moves,
+    recorded and by graphs, against the oracle's batched frame."""
+    from oracle import oracle as O
+    sizes = SIZES + [(3, 40), (7, 90), (61, 2)]
+    frames = [[_matrix(c, w, h) for c, (w, h) in zip(_cams(len(sizes), 35.0 * f), sizes)] for f in range(4)]
+    libc_srand(29)
+    sc = O.OracleScene(trees["terrain8s"], blocks, views=sizes)
+    sc.record(True)
+    ld, cm, rt = _gpu_views(trees["terrain8s"], blocks, sizes, seed=29)
+    rt.set_launch_shape(*shape)
+    for f, mats in enumerate(frames):
+        n, imgs = sc.render_views(mats)
+        rt.record_passes(f % 2 == 0)
+        rt.RenderViews(mats)
+        assert rt.stats()["passes"] == n, "frame %d" % f
+        for p in range(n if f % 2 == 0 else 0):
+            np.testing.assert_array_equal(rt.pass_words(p), sc.pass_words(p), err_msg="frame %d pass %d" % (f, p))
+        for v in range(len(sizes)):
+            np.testing.assert_array_equal(rt.read_image(view=v), imgs[v], err_msg="frame %d view %d" % (f, v))
+    sc.close()
