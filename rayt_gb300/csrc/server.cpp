@@ -109,7 +109,13 @@ class Server {
   int32_t* d_unique_ = nullptr;
   UniqueResult* h_result_ = nullptr;  // mapped
   UniqueResult* d_result_ = nullptr;
-  int* d_client_faults_[2] = {};  // by tick parity; a tick's unique kernel clears the next one's
+  // Client faults: a tick counts into one array and its unique kernel clears the
+  // next tick's, which is neither that one nor the one that copies from
+  // framebuffers, perhaps still waiting for their turn, decide by.
+  static constexpr int kFaultArrays = 3;
+  int* d_client_faults_[kFaultArrays] = {};
+  int faults_now_ = 0;   // counted into by this tick, zero before it
+  int faults_sent_ = 0;  // read by the copies that early_ev_ marks
   int tick_ = 0;
   int carried_ = 0;          // faulted rays carried into the next tick
   // deliver_to_host: finished frames are copied to their client's stage on
@@ -182,10 +188,10 @@ int Server::Init(Cache* cache, const rayt_server_config& cfg) {
       return fail(RAYT_E_OOM, "ray record allocation failed");
   fault_words_ = (int)((cache->tree_blocks() + 31) / 32);
   hit_words_ = (int)(((uint64_t)cache->max_blocks() * 2 + 31) / 32);
-  state_ints_ = 2 * (size_t)kPassInts + (size_t)fault_words_ + hit_words_ + 2 * kMaxClients;
+  state_ints_ = 2 * (size_t)kPassInts + (size_t)fault_words_ + hit_words_ + kFaultArrays * kMaxClients;
   if (cudaMalloc(&d_state_, state_ints_ * 4) != cudaSuccess || cudaMalloc(&d_passes_, 4) != cudaSuccess)
     return fail(RAYT_E_OOM, "feedback state allocation failed");
-  for (int k = 0; k < 2; ++k) d_client_faults_[k] = d_state_ + state_ints_ - (k + 1) * kMaxClients;
+  for (int k = 0; k < kFaultArrays; ++k) d_client_faults_[k] = d_state_ + state_ints_ - (k + 1) * kMaxClients;
   const size_t bit_words = (size_t)fault_words_ + hit_words_;
   if (cudaHostAlloc(&h_unique_, (bit_words * 32 + 1) * 4, cudaHostAllocMapped) != cudaSuccess ||
       cudaHostAlloc(&h_result_, sizeof(UniqueResult), cudaHostAllocMapped) != cudaSuccess)
@@ -376,7 +382,7 @@ TraceParams Server::Params(int k) const {
   p.lanes = 32;
   p.refill = 32;
   p.restart = 1;
-  p.client_faults = d_client_faults_[k];
+  p.client_faults = d_client_faults_[faults_now_];
   // client slots by framebuffer base (free slots get an empty range at the end)
   std::vector<std::pair<int64_t, int>> order;
   for (int i = 0; i < (int)clients_.size(); ++i)
@@ -427,6 +433,7 @@ int Server::Step(int* finished) {
       if (clients_[c].live && clients_[c].base == p.client_base[i]) slot_of_client[c] = i;
   if (dirty_) {  // start clean, and the ticks' numbers again
     RAYT_CUDA_TRY(cudaStreamSynchronize(s_));
+    if (early_pending_) RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, early_ev_, 0));  // they read the client faults
     RAYT_CUDA_TRY(cudaMemsetAsync(d_state_, 0, state_ints_ * 4, s_));
     RAYT_CUDA_TRY(cudaMemsetAsync(d_passes_, 0, 4, s_));
     h_result_->pass = passes_ = 0;
@@ -486,7 +493,7 @@ int Server::Step(int* finished) {
     ++stats.kernel_launches;
     if (straight) {
       DeliverParams d{};
-      d.faults = d_client_faults_[k];
+      d.faults = d_client_faults_[faults_now_];
       for (int i = 0; i < n; ++i) {
         const int id = view_client[g + i];
         const Client& c = clients_[id];
@@ -501,6 +508,7 @@ int Server::Step(int* finished) {
       RAYT_CUDA_TRY(launch_deliver(d, copy_s_));
       RAYT_CUDA_TRY(cudaEventRecord(early_ev_, copy_s_));
       early_pending_ = true;
+      faults_sent_ = faults_now_;
       ++stats.kernel_launches;
     }
     g += n;
@@ -515,6 +523,8 @@ int Server::Step(int* finished) {
     RAYT_CUDA_TRY(launch_trace(q, false, false, carried_, 0, s_));
     ++stats.kernel_launches;
   }
+  int faults_next = 0;
+  while (faults_next == faults_now_ || (early_pending_ && faults_next == faults_sent_)) ++faults_next;
   UniqueFromBitsParams u{};
   u.fault_bits = p.fault_bits;
   u.fault_words = fault_words_;
@@ -523,8 +533,8 @@ int Server::Step(int* finished) {
   u.words = words(k);
   u.previous = words(1 - k);
   u.total_pixels = (int)std::min<int64_t>(rays_tick, 1 << 30);
-  u.client_faults = d_client_faults_[k];
-  u.next_client_faults = d_client_faults_[1 - k];
+  u.client_faults = d_client_faults_[faults_now_];
+  u.next_client_faults = d_client_faults_[faults_next];
   u.passes = d_passes_;
   u.unique_out = d_unique_;
   u.result = d_result_;
@@ -535,6 +545,7 @@ int Server::Step(int* finished) {
   const int wrc = wait_word(&h_result_->pass, passes_, s_);
   if (wrc != RAYT_OK) return wrc;
   dirty_ = false;
+  faults_now_ = faults_next;
   const double t_pass = now_s();
   stats.host_ms_wait += (t_pass - t_sync) * 1e3;
   stats.gpu_ms_upload += cache_->TakeUploadMs();  // the previous tick's block uploads

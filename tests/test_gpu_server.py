@@ -261,3 +261,29 @@ def test_served_mix_under_eviction_equals_alone(trees):
         if compared >= 2 and uploaded > max_blocks:
             return
     raise AssertionError("no cache size both evicted and kept two requests untruncated: %s" % seen)
+
+
+def test_served_image_stays_the_last_finished_frame(trees):
+    """Two clients in one tick: the first looks past the scene and is done, and
+    its large frame is on its way to the host through the ticks after it; the
+    second's copy is queued behind it and its rays fault for some ticks.  The
+    second's host image stays its last finished frame until the request is
+    done, whatever those ticks have done to the counts by then."""
+    import torch
+    big, w, h = 8192, 160, 90
+    ld, cm, srv = _server(trees, max_blocks=400, max_clients=2, deliver_to_host=True,
+                          framebuffer_bytes=4 * (big * big + w * h + 64), max_rays_in_flight=big * big + w * h)
+    a, b = srv.add_client(big, big), srv.add_client(w, h)
+    away = R.Camera(0.0, 80.0, 0.0, (0.5, 3.0, 0.5), 40.0, 1.0).view_proj_inv()
+    before, after = _matrix(_cam(0.0), w, h), _matrix(_cam(80.0), w, h)
+    assert not srv.wait(srv.submit(b, before))["truncated"]
+    np.testing.assert_array_equal(srv.host_image(b), _resident(trees, w, h, before))
+    ra, rb = srv.submit(a, away), srv.submit(b, after)
+    assert srv.step() == 1  # a
+    assert srv.step() == 0  # only carries b's rays
+    torch.cuda.synchronize()  # every copy queued so far
+    np.testing.assert_array_equal(srv.host_image(b), _resident(trees, w, h, before))
+    assert not srv.wait(rb)["truncated"] and not srv.wait(ra)["truncated"]
+    np.testing.assert_array_equal(srv.host_image(b), _resident(trees, w, h, after))
+    assert (srv.host_image(a) == (0, 216, 255, 255)).all()
+    srv.close()
