@@ -370,7 +370,9 @@ int rayt_server_remove_client(rayt_server* s, int client);
 int rayt_server_seed(rayt_server* s, uint32_t seed);
 /* Queues a frame of `client` (thread-safe). */
 int rayt_server_submit(rayt_server* s, int client, const float view_proj_inv[16], uint64_t* request);
-/* One scheduling tick on the calling thread; *finished = requests it ended. */
+/* One scheduling tick on the calling thread; *finished = requests it ended.
+ * After a tick that failed (a block that cannot be read), the next one starts
+ * the requests in flight again from their cameras. */
 int rayt_server_step(rayt_server* s, int* finished);
 /* Scheduler thread running ticks while requests are queued or in flight. */
 int rayt_server_start(rayt_server* s);

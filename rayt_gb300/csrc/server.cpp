@@ -432,6 +432,14 @@ int Server::Step(int* finished) {
     for (int c = 0; c < (int)clients_.size(); ++c)
       if (clients_[c].live && clients_[c].base == p.client_base[i]) slot_of_client[c] = i;
   if (dirty_) {  // start clean, and the ticks' numbers again
+    // The rays that the failed tick traced or carried are gone with its state:
+    // every request starts again from its camera.
+    for (Flight& f : flights_) {
+      f.fresh = true;
+      f.finishing = false;
+      f.passes = 0;
+    }
+    carried_ = 0;
     RAYT_CUDA_TRY(cudaStreamSynchronize(s_));
     if (early_pending_) RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, early_ev_, 0));  // they read the client faults
     RAYT_CUDA_TRY(cudaMemsetAsync(d_state_, 0, state_ints_ * 4, s_));
@@ -596,7 +604,7 @@ int Server::Step(int* finished) {
     if (rc == RAYT_OK) rc = src;
   }
   if (rc != RAYT_OK) {
-    dirty_ = true;  // tick_ stays, and this tick has counted into its state
+    dirty_ = true;  // the requests start again (see above)
     return rc;
   }
   if (filled)  // the cache cannot hold this tick's blocks: stop the requests that still fault

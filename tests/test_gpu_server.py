@@ -287,3 +287,58 @@ def test_served_image_stays_the_last_finished_frame(trees):
     np.testing.assert_array_equal(srv.host_image(b), _resident(trees, w, h, after))
     assert (srv.host_image(a) == (0, 216, 255, 255)).all()
     srv.close()
+
+
+def _late_blocks(loader, resident):
+    """Blocks below a child of the root block that the initial fill of a cache of
+    `resident` blocks does not load: none of them is requested before its parent
+    was."""
+    info = loader.info
+    links = loader.LoadBlock(info.root_block_index)[1][:4 * info.nodes_in_block].view(np.uint32)
+    named = [int(l) >> 11 for l in links if (int(l) & 0x1FF) > 0x100]
+    loaded = set(list(dict.fromkeys(named))[:resident - 1])
+    parents = [loader.LoadBlock(b)[0].parent_block_index for b in range(info.blocks_count)]
+    below_root = {b for b, p in enumerate(parents) if p == info.root_block_index}
+    return [b for b, p in enumerate(parents) if p in below_root - loaded]
+
+
+@pytest.mark.parametrize("mode", ["mapped", "read"])
+def test_served_request_survives_a_failed_tick(trees, tmp_path, monkeypatch, mode):
+    """A block that cannot be read fails the tick that asks for it, in the middle
+    of two requests, some of whose rays are carried over; once the file is whole
+    again both end with the image of a run in which nothing failed."""
+    monkeypatch.setenv("RAYT_BLOCK_IO", mode)
+    path, resident = str(tmp_path / "scene.tree"), 250
+    with open(trees["terrain8s"], "rb") as f:
+        whole = f.read()
+    with open(path, "wb") as f:
+        f.write(whole)
+    ld = R.StoredOctreeLoader(path)
+    info = ld.info
+    late = _late_blocks(ld, resident)
+    cm = R.GPUOctreeCacheManager(resident, ld)
+    cm.InitialFillCache()
+    assert cm.stats()["mapped"] == (mode == "mapped")
+    srv = R.RenderServer(cm, max_clients=2, framebuffer_bytes=1 << 20, max_rays_in_flight=1 << 18, max_passes=32)
+    sizes = [(160, 90), (33, 17)]
+    ids = [srv.add_client(w, h) for w, h in sizes]
+    mats = [_matrix(_cam(0.0 + 40 * v), w, h) for v, (w, h) in enumerate(sizes)]
+    reqs = [srv.submit(c, m) for c, m in zip(ids, mats)]
+    with open(path, "r+b", buffering=0) as f:
+        for b in late:  # a root count of zero: the record is refused
+            f.seek(info.header_bytes + info.block_stride * b + 8)
+            f.write(b"\0\0\0\0")
+    steps = 0
+    with pytest.raises(R.RaytError):
+        while steps < 32:
+            steps += srv.step() >= 0
+    assert steps >= 1 and srv.stats()["completed"] < 2
+    with pytest.raises(R.RaytError):  # and again
+        srv.step()
+    with open(path, "r+b", buffering=0) as f:
+        f.write(whole)
+    for v, ((w, h), c, r, m) in enumerate(zip(sizes, ids, reqs, mats)):
+        assert not srv.wait(r)["truncated"]
+        np.testing.assert_array_equal(srv.read_image(c), _resident(trees, w, h, m), err_msg="client %d" % v)
+    assert srv.stats()["completed"] == 2
+    srv.close()
