@@ -142,7 +142,7 @@ class Server {
   static constexpr int kMaxGroups = 4;
   cudaEvent_t group_ev_ = nullptr, early_ev_ = nullptr;
   bool early_pending_ = false;  // early_ev_ marks copies from framebuffers
-  bool copy_pending_ = false;  // copied_ev_ marks the last delivery
+  bool copy_pending_ = false;  // copied_ev_ marks the last copies from stages
   struct Delivery {
     Server* server;
     std::vector<rayt_request_info> done;
@@ -617,26 +617,28 @@ int Server::Step(int* finished) {
   if (!ended.empty()) {
     std::unique_ptr<Delivery> delivery;
     if (cfg_.deliver_to_host) {
-      // frames to their stages (after the previous delivery has read them),
-      // then to the host on the copy stream; the framebuffers are free for the
-      // clients' next requests in stream order
+      // frames to their stages (after the last copies from stages), then to the
+      // host on the copy stream; the framebuffers are free for the clients' next
+      // requests in stream order.  Frames sent straight from the framebuffers
+      // are on their way and wait for nothing here.
       delivery.reset(new Delivery{this, {}});
-      if (copy_pending_) RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, copied_ev_, 0));
+      std::vector<const Client*> staged;
       for (const Flight& f : ended) {
         const Client& c = clients_[f.client];
-        if (!early[f.client])
-          RAYT_CUDA_TRY(cudaMemcpyAsync(c.stage, d_images_ + c.base, (size_t)c.w * c.h * 4, cudaMemcpyDeviceToDevice, s_));
-      }
-      RAYT_CUDA_TRY(cudaEventRecord(staged_ev_, s_));
-      RAYT_CUDA_TRY(cudaStreamWaitEvent(copy_s_, staged_ev_, 0));
-      for (const Flight& f : ended) {
-        const Client& c = clients_[f.client];
-        if (!early[f.client])
-          RAYT_CUDA_TRY(cudaMemcpyAsync(c.host, c.stage, (size_t)c.w * c.h * 4, cudaMemcpyDeviceToHost, copy_s_));
+        if (!early[f.client]) staged.push_back(&c);
         stats.bytes_d2h += (int64_t)c.w * c.h * 4;
       }
-      RAYT_CUDA_TRY(cudaEventRecord(copied_ev_, copy_s_));
-      copy_pending_ = true;
+      if (!staged.empty()) {
+        if (copy_pending_) RAYT_CUDA_TRY(cudaStreamWaitEvent(s_, copied_ev_, 0));
+        for (const Client* c : staged)
+          RAYT_CUDA_TRY(cudaMemcpyAsync(c->stage, d_images_ + c->base, (size_t)c->w * c->h * 4, cudaMemcpyDeviceToDevice, s_));
+        RAYT_CUDA_TRY(cudaEventRecord(staged_ev_, s_));
+        RAYT_CUDA_TRY(cudaStreamWaitEvent(copy_s_, staged_ev_, 0));
+        for (const Client* c : staged)
+          RAYT_CUDA_TRY(cudaMemcpyAsync(c->host, c->stage, (size_t)c->w * c->h * 4, cudaMemcpyDeviceToHost, copy_s_));
+        RAYT_CUDA_TRY(cudaEventRecord(copied_ev_, copy_s_));
+        copy_pending_ = true;
+      }
     }
     const double t_done = now_s();
     std::lock_guard<std::mutex> lock(mu_);

@@ -4,6 +4,7 @@ from the camera, so every request that ends without truncation must equal the
 one-view oracle frame of its camera over a fully resident cache, alone or in
 any mix."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -341,4 +342,40 @@ def test_served_request_survives_a_failed_tick(trees, tmp_path, monkeypatch, mod
         assert not srv.wait(r)["truncated"]
         np.testing.assert_array_equal(srv.read_image(c), _resident(trees, w, h, m), err_msg="client %d" % v)
     assert srv.stats()["completed"] == 2
+    srv.close()
+
+
+def test_served_tick_does_not_wait_for_copies_from_framebuffers(trees):
+    """A large frame goes to the host straight from its framebuffer, which reads
+    no stage: a smaller frame that ends in a later tick goes to its stage, and
+    the tick after that, which carries the rays of others, ends while the large
+    copy (3 ms) is under way: one of a few such ticks at least takes less than
+    1 ms (they take 0.1)."""
+    bw, bh, w, h, small = 16384, 8192, 160, 90, 3
+    pixels = bw * bh + small * (w * h + 64)
+    ld, cm, srv = _server(trees, max_blocks=640, deliver_to_host=True, framebuffer_bytes=4 * pixels,
+                          max_rays_in_flight=pixels)
+    a, ids = srv.add_client(bw, bh), [srv.add_client(w, h) for _ in range(small)]
+    away = R.Camera(0.0, 80.0, 0.0, (0.5, 3.0, 0.5), 40.0, 1.0).view_proj_inv()
+    ticks = []
+    for f in range(6):
+        mats = [_matrix(_cam(80.0 * f + 55.0 * v, v), w, h) for v in range(small)]
+        done = srv.stats()["completed"]
+        reqs = [srv.submit(a, away)] + [srv.submit(c, m) for c, m in zip(ids, mats)]
+        left = small + 1 - srv.step()
+        staged = False
+        while left > 0:
+            t0 = time.perf_counter()
+            n = srv.step()
+            if srv.stats()["completed"] != done:
+                break
+            if staged:
+                ticks.append(time.perf_counter() - t0)
+            staged = n > 0
+            left -= n
+        srv.wait(reqs[0])
+        for c, r, m in zip(ids, reqs[1:], mats):
+            if not srv.wait(r)["truncated"]:
+                np.testing.assert_array_equal(srv.host_image(c), _resident(trees, w, h, m), err_msg="frame %d" % f)
+    assert min(ticks) < 1e-3
     srv.close()
