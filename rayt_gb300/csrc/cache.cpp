@@ -345,8 +345,8 @@ int Cache::Init(Tree* tree, int max_blocks) {
   slots_.resize((size_t)max_blocks_);
   block_slot_.assign(tree->info.blocks_count, -1);
   parent_slot_.assign(tree->info.blocks_count, -1);
-  validated_.assign(tree->info.blocks_count, 0);
-  fault_children_.resize(tree->info.blocks_count);
+  children_at_.assign(tree->info.blocks_count, 0);
+  children_.assign(1, 0);
   written_.assign((size_t)max_blocks_, 0);
   written_pos_.assign((size_t)max_blocks_, -1);
   patched_.assign((size_t)max_blocks_, 0);
@@ -654,8 +654,9 @@ int Cache::ReadOne(int pos, int block) {
       if ((l & 0x1FFu) > 0x100u && seen.Insert(l >> 11)) m.faults.push_back(l >> 11);
     }
   };
-  if (validated_[block]) {  // links checked on an earlier load, and their fault children kept
-    m.faults = fault_children_[block];
+  if (const uint32_t at = children_at_[block]) {  // links checked on an earlier load, and their fault children kept
+    const uint32_t* kept = children_.data() + at;
+    m.faults.assign(kept + 1, kept + 1 + kept[0]);
     return RAYT_OK;
   }
   // Every used link must stay in range: a child link's children inside the
@@ -687,8 +688,7 @@ int Cache::ReadOne(int pos, int block) {
   }
   if (child_bad) return bad("child link points past the end of its block");
   if (fault_bad) return bad("fault link points past the last block");
-  fault_children_[block] = m.faults;
-  validated_[block] = 1;  // one byte per block: threads reading other blocks touch other bytes
+  m.checked = true;
   return RAYT_OK;
 }
 
@@ -705,7 +705,7 @@ int Cache::Prefetch(const int* blocks, int n) {
 bool Cache::ReadInline(const int* blocks, int n) const {
   if (n > kInlineReadBlocks) return false;
   int64_t links = 0;
-  for (int i = 0; i < n; ++i) links += file_host_ && validated_[blocks[i]] ? 0 : nib_;
+  for (int i = 0; i < n; ++i) links += file_host_ && children_at_[blocks[i]] ? 0 : nib_;
   return links <= kInlineReadLinks;
 }
 
@@ -716,8 +716,11 @@ void Cache::StartRead(const int* blocks, int n) {
   const int first = staged_;
   const size_t base = (size_t)stage_cap_ * half_ + first;
   read_started_ = std::chrono::steady_clock::now();
+  read_at_ = base;
+  read_n_ = n;
   for (int i = 0; i < n; ++i) {
     h_slots_[base + i] = -1;
+    meta_[base + i].checked = false;
     if (h_blocks_) h_blocks_[base + i] = blocks[i];
     ready_[base + i].store(0, std::memory_order_relaxed);
   }
@@ -734,6 +737,17 @@ void Cache::StartRead(const int* blocks, int n) {
 }
 void Cache::FinishRead() {
   pool_->Wait();
+  // keep the fault children of the blocks it checked (a block may have been
+  // requested, and read, more than once)
+  const size_t most = 2 * (size_t)tree_->info.blocks_count + 1;
+  for (size_t p = read_at_; p < read_at_ + read_n_; ++p) {
+    const Staged& m = meta_[p];
+    if (!m.checked || children_at_[m.block] || children_.size() + 1 + m.faults.size() > most) continue;
+    children_at_[m.block] = (uint32_t)children_.size();
+    children_.push_back((uint32_t)m.faults.size());
+    children_.insert(children_.end(), m.faults.begin(), m.faults.end());
+  }
+  read_n_ = 0;
   stats_.io_seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - read_started_).count();
 }
 

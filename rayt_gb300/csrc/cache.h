@@ -150,10 +150,13 @@ class Cache {
   std::vector<Slot> slots_;
   std::vector<int32_t> block_slot_;    // tree block -> cache slot, -1 absent
   std::vector<int32_t> parent_slot_;   // tree block -> slot of its parent, -1 absent
-  std::vector<uint8_t> validated_;     // tree block -> its links passed the check once (the file is read-only)
-  // tree block -> its fault children, once validated: a block that comes back
-  // needs no look at its links (at most one entry per child link of the tree)
-  std::vector<std::vector<uint32_t>> fault_children_;
+  // A block that comes back needs no look at its links (the file is read-only):
+  // once they passed the check, its fault children lie in children_, after their
+  // number, at children_at_[tree block] (0: not there).  In a tree, where a block
+  // has one parent, all that is a word per block and one per child; what a file
+  // names beyond that is not kept, and checked at every load.  The reading
+  // threads only read both.
+  std::vector<uint32_t> children_at_, children_;
   std::vector<int> pending_;
   bool in_session_ = false, in_transaction_ = false;
 
@@ -178,6 +181,7 @@ class Cache {
     std::string err;
     rayt_block_header hdr{};
     std::vector<uint32_t> faults;  // fault-link targets, in node order
+    bool checked = false;          // this read checked the links
   };
   uint8_t* h_stage_ = nullptr;
   uint8_t* d_stage_ = nullptr;
@@ -244,6 +248,8 @@ class Cache {
   void StartRead(const int* blocks, int n);
   void FinishRead();
   std::chrono::steady_clock::time_point read_started_;
+  size_t read_at_ = 0;  // positions of the read under way (both halves counted)
+  int read_n_ = 0;
   int Place(int pos, std::vector<int>* queue);
   int Unload();
   void AddPatch(bool far_buffer, uint32_t index, uint32_t value);

@@ -141,3 +141,40 @@ def test_batched_feedback_marks_equal_one_by_one(trees, seed, frac):
         assert np.array_equal(x, y)
     if 0 < frac < 1:
         assert a[2] > 0  # requests loaded blocks, each evicting the LRU front
+
+
+@pytest.mark.parametrize("mode", ["mapped", "read"])
+def test_blocks_requested_more_than_once(trees, monkeypatch, mode):
+    """A block requested several times in one transaction is read as often,
+    by several threads at once, and loaded once: same cache bytes as with one
+    request each, over transactions that evict blocks and load them again."""
+    monkeypatch.setenv("RAYT_BLOCK_IO", mode)
+    monkeypatch.setenv("RAYT_IO_THREADS", "8")
+    ld = R.StoredOctreeLoader(trees["terrain8s"])
+    rng = np.random.default_rng(7)
+    orders = [rng.permutation(ld.info.blocks_count) for _ in range(12)]
+    runs = []
+    for times in (1, 4):
+        c = R.GPUOctreeCacheManager(300, ld)  # of 793 blocks
+        c.InitialFillCache()
+        out = []
+        for order in orders:
+            c.StartRequestSession()
+            c.StartRequestTransaction()
+            for b in order:
+                for _ in range(times):
+                    try:
+                        c.RequestBlock(int(b))
+                    except R.RaytError:  # its parent is not resident
+                        break
+            c.EndRequestTransaction()
+            c.EndRequestSession()
+            out.append([c.stats()["uploaded_blocks"]] +
+                       [c.read_buffer(n).copy() for n in ("node links", "normals", "colors", "far pointers")])
+        assert out[-1][0] > 600  # blocks were evicted and came back
+        c.close()
+        runs.append(out)
+    for i, (a, b) in enumerate(zip(*runs)):
+        assert a[0] == b[0], "transaction %d" % i
+        for x, y in zip(a[1:], b[1:]):
+            np.testing.assert_array_equal(x, y, err_msg="transaction %d" % i)
