@@ -173,3 +173,33 @@ def test_unique_bitmap_slices(built, n, bits, kept):
         keys[:2] = 0, span - 1
         words[at] = (keys - span // 3).astype(np.int32)
         _check_unique(words, 0, offset=n % 2)
+
+
+# a round is 16384 elements per SM (152): one, two and three rounds and the
+# element after them, and rounds enough that every buffer and slot is used again
+@pytest.mark.parametrize("n", [2490368, 2490369, 4980736, 4980739, 7471104, 7471107, 17432581, 40000003])
+@pytest.mark.parametrize("offset", [0, 1, 3])
+def test_scan_rounds(built, n, offset):
+    a = _wide(np.random.default_rng(n), n)
+    x = _dev(np.concatenate([np.full(offset, 9, np.int32), a, np.full(5, 9, np.int32)]))
+    R.GPUScan(x[offset:], n)
+    got = x.cpu().numpy()
+    ref = np.cumsum(a.astype(np.int64)).astype(np.uint64).astype(np.uint32).view(np.int32)
+    np.testing.assert_array_equal(got[offset:offset + n], ref)
+    assert np.all(got[:offset] == 9) and np.all(got[offset + n:] == 9)
+
+
+# the split's largest size (15 turns of 304 regions of 15360 keys) and the
+# smallest that takes the digit passes, or the counting in them, at once
+@pytest.mark.parametrize("n,keys,offset", [(70041600, "wide", 0), (70041600, "narrow", 0), (70041601, "wide", 0),
+                                           (70041601, "narrow", 0), (70041601, "count_limit", 3),
+                                           (70041601, "over_count_limit", 0), (70041601, "one_digit", 1),
+                                           (70041601, "equal", 0)])
+def test_sort_beyond_the_split(built, n, keys, offset):
+    a = KEYS[keys](np.random.default_rng(n), n)
+    x = _dev(np.concatenate([np.full(offset, 9, np.int32), a, np.full(5, 9, np.int32)]))
+    R.GPUSort(x[offset:], n)
+    got = x.cpu().numpy()
+    a.sort()
+    np.testing.assert_array_equal(got[offset:offset + n], a)
+    assert np.all(got[:offset] == 9) and np.all(got[offset + n:] == 9)
