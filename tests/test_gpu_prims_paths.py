@@ -203,3 +203,15 @@ def test_sort_beyond_the_split(built, n, keys, offset):
     a.sort()
     np.testing.assert_array_equal(got[offset:offset + n], a)
     assert np.all(got[:offset] == 9) and np.all(got[offset + n:] == 9)
+
+
+@pytest.mark.parametrize("n", [8193, 40000, (1 << 21) + 5, 7000001])
+@pytest.mark.parametrize("span", [199, 1 << 22, 1 << 30])
+def test_unique_full_and_sparse_stretches(built, n, span):
+    """Stretches of 512 words of which all, most, some or none are kept follow
+    one another, so a warp's region of kept words meets every fill before a
+    stretch that is kept whole."""
+    rng = np.random.default_rng(n + span)
+    share = rng.choice([0.0, 0.02, 0.1, 0.24, 0.9, 1.0, 1.0], n // 512 + 1).repeat(512)[:n]
+    words = np.where(rng.random(n) < share, rng.integers(-span, span, n), NO_HIT).astype(np.int32)
+    _check_unique(words, 0, offset=n % 2)
