@@ -24,8 +24,9 @@ constexpr uint32_t kRootParent = (1u << 24) - 1;
 
 // Waits until a kernel of stream s has set the host-mapped *word to `value`,
 // which is the last thing it does; everything queued on s before that kernel is
-// done then.
-int wait_word(const unsigned int* word, unsigned int value, cudaStream_t s);
+// done then.  Or, given `early`, until early(arg).
+int wait_word(const unsigned int* word, unsigned int value, cudaStream_t s, bool (*early)(const int*) = nullptr,
+              const int* arg = nullptr);
 
 // ---- traversal ----------------------------------------------------------------
 // Views' images (and recorded feedback words) share one buffer; view v starts
@@ -244,7 +245,9 @@ size_t feedback_status_bytes(int n);
 // Compaction (drop NO_HIT, NodeToBlock) and sorted unique.  result[0] receives
 // the unique count (incl. NO_HIT), unless the keys span too wide a range for a
 // bitmap: feedback_unique_needs_radix(result) says so, and
-// feedback_unique_radix_device, on the same memory, then sorts them.
+// feedback_unique_radix_device, on the same memory, then sorts them.  In mapped
+// host memory, where the caller has cleared it, result says so as soon as that
+// is known, and the second may be launched behind the rest of the first.
 cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t* unique_out, void* scratch,
                                    unsigned long long* status, uint32_t epoch, int* result, int* err,
                                    const DoneFlag& done, cudaStream_t s);

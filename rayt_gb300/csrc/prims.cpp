@@ -97,9 +97,9 @@ DoneFlag next_done(Device& d) {
   return DoneFlag{d.ctas, reinterpret_cast<unsigned int*>(d.host_dev) + 3, ++d.calls};
 }
 
-// Waits for that and reads the error flag.
-int finish(Device& d, cudaStream_t s) {
-  const int rc = wait_word(reinterpret_cast<const unsigned int*>(d.host) + 3, d.calls, s);
+// Waits for that, or until early(result), and reads the error flag.
+int finish(Device& d, cudaStream_t s, bool (*early)(const int*) = nullptr) {
+  const int rc = wait_word(reinterpret_cast<const unsigned int*>(d.host) + 3, d.calls, s, early, d.host + 1);
   return rc != RAYT_OK ? rc : check_error(d);
 }
 }  // namespace
@@ -206,10 +206,14 @@ int rayt_feedback_unique(const int32_t* words, int n, int nib, int32_t* unique, 
   int rc = rayt::begin(rayt::feedback_scratch_bytes(n), rayt::feedback_status_bytes(n), s, &d, &epoch);
   if (rc != RAYT_OK) return rc;
   int *err = d->host_dev, *result = d->host_dev + 1;
+  d->host[1] = d->host[2] = 0;
   RAYT_CUDA_TRY(rayt::feedback_unique_device(words, n, nib, unique, d->scratch, d->status, epoch, result, err, rayt::next_done(*d), s));
-  if ((rc = rayt::finish(*d, s)) != RAYT_OK) return rc;
+  if ((rc = rayt::finish(*d, s, rayt::feedback_unique_needs_radix)) != RAYT_OK) return rc;
   if (rayt::feedback_unique_needs_radix(d->host + 1)) {
-    RAYT_CUDA_TRY(rayt::feedback_unique_radix_device(n, unique, d->scratch, d->status, epoch, result, err, rayt::next_done(*d), s));
+    const cudaError_t e =
+        rayt::feedback_unique_radix_device(n, unique, d->scratch, d->status, epoch, result, err, rayt::next_done(*d), s);
+    if (e != cudaSuccess) cudaStreamSynchronize(s);  // the kernels before may still be using the scratch memory
+    RAYT_CUDA_TRY(e);
     if ((rc = rayt::finish(*d, s)) != RAYT_OK) return rc;
   }
   *unique_count = d->host[1];

@@ -550,7 +550,8 @@ __global__ void __launch_bounds__(kThreads) compact_kernel(const int32_t* words,
     if (c->no_hit) out[0] = kNoHit;
     result[0] = c->no_hit ? 1 : 0;
   }
-  result[1] = path;
+  // the host may be waiting for this to launch the radix passes
+  *(volatile int*)&result[1] = path;
 }
 
 // Compaction launch: 16-byte loads when `words` allows them.
@@ -2684,7 +2685,9 @@ cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t
                                      dim3(kShareThreads), args, kEmitSmemBytes, s);
 }
 
-bool feedback_unique_needs_radix(const int* result) { return result[1] == kPathRadix; }
+bool feedback_unique_needs_radix(const int* result) {
+  return __atomic_load_n(result + 1, __ATOMIC_ACQUIRE) == kPathRadix;
+}
 
 cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scratch, unsigned long long* status,
                                          uint32_t epoch, int* result, int* err, const DoneFlag& done,

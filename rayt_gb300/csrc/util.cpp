@@ -51,12 +51,13 @@ int LibcRand::Next() {
 // microseconds before the runtime says that the stream has finished.  After
 // two milliseconds it asks the runtime (for an error, and so as not to spin
 // through long work).
-int wait_word(const unsigned int* word, unsigned int value, cudaStream_t s) {
+int wait_word(const unsigned int* word, unsigned int value, cudaStream_t s, bool (*early)(const int*),
+              const int* arg) {
   using clock = std::chrono::steady_clock;
   const auto until = clock::now() + std::chrono::milliseconds(2);
   do {
     for (int spin = 0; spin < 256; ++spin)
-      if (__atomic_load_n(word, __ATOMIC_ACQUIRE) == value) return RAYT_OK;
+      if (__atomic_load_n(word, __ATOMIC_ACQUIRE) == value || (early && early(arg))) return RAYT_OK;
   } while (clock::now() < until);
   RAYT_CUDA_TRY(cudaStreamSynchronize(s));
   if (__atomic_load_n(word, __ATOMIC_ACQUIRE) == value) return RAYT_OK;
