@@ -191,7 +191,14 @@ struct RayEnd {
 // root never do (all the rays of half the warps of a frame that looks past
 // the scene's edge: 1919x1079 pixels with nothing in sight 42.5 -> 28.2 us,
 // 512x512 60.6 -> 58.9, a frame full of the scene 321.4 -> 324.2).
-template <bool kCount, bool kBias, bool kLazy, class F>
+//
+// kMeet: the lanes meet where they have found their child of the root.  Where
+// the view is one of several the compiler left them apart there, and a warp
+// then went through the traversal in parts, by the steps its lanes had taken
+// (500 views of 32x32 pixels 203 us without, 156 so; 12 of 1280x720 full of the
+// scene 1591 and 1545).  With one view it does not, and the meeting costs
+// (512x512 59.0 and 60.2 us).
+template <bool kCount, bool kBias, bool kLazy, bool kMeet, class F>
 __device__ __forceinline__ RayEnd cast_ray(const TraceCore& p, float4 o, float4& d, uint32_t& fetches,
                                            uint32_t& far_fetches, const F& late_coef) {
   RayEnd r;
@@ -253,6 +260,8 @@ __device__ __forceinline__ RayEnd cast_ray(const TraceCore& p, float4 o, float4&
   const int mirror = 31 ^ octant;
   int child = mirror ^ idx;
   if (kLazy) {  // the loop below, as long as no child of the root is entered
+    const unsigned here = __activemask();
+    bool missed = false;
     while (!((int)(desc << child) < 0 && t_min <= t_max)) {
       const float tx_corner = px * tx_coef - tx_bias;
       const float ty_corner = py * ty_coef - ty_bias;
@@ -271,10 +280,15 @@ __device__ __forceinline__ RayEnd cast_ray(const TraceCore& p, float4 o, float4&
       // error.  (That test here instead: a full frame 324 us, so 331.)
       if (child == before) break;
       if (((child ^ mirror) & (child ^ before)) != 0) {  // out of the octree: a miss
-        r.node = -1;
-        r.iter = iter;
-        return r;
+        missed = true;
+        break;
       }
+    }
+    if (kMeet) __syncwarp(here);
+    if (missed) {
+      r.node = -1;
+      r.iter = iter;
+      return r;
     }
     d.w = coef = late_coef();
   }
@@ -777,7 +791,7 @@ __global__ void __launch_bounds__(kBlockThreads, 10) trace_kernel(const __grid_c
     return;
   }
   uint32_t fetches = 0, far_fetches = 0;
-  const RayEnd e = cast_ray<kCount, !kFirst, kLazy>(p, o, d, fetches, far_fetches, [&] {
+  const RayEnd e = cast_ray<kCount, !kFirst, kLazy, sizeof(P) != sizeof(TraceParams1)>(p, o, d, fetches, far_fetches, [&] {
     return init_coef(p.views[v], x, y);
   });
   end_ray<kCount>(p, e, ray, o, d, adv, fetches, far_fetches);
@@ -908,7 +922,7 @@ __global__ void __launch_bounds__(kBlockThreads) depth_view_kernel(const __grid_
   const float coef = bias < 1e-10f ? 0.0f : __fdiv_rn(v.lod * (dist(p1f, p2f) - dist(p1n, p2n)), dist(p1n, p1f));
   uint32_t fetches = 0, far_fetches = 0;
   float4 dir = make_float4(dx, dy, dz, coef);
-  const RayEnd e = cast_ray<false, true, false>(p, make_float4(o[0], o[1], o[2], bias), dir, fetches, far_fetches,
+  const RayEnd e = cast_ray<false, true, false, false>(p, make_float4(o[0], o[1], o[2], bias), dir, fetches, far_fetches,
                                                 [] { return 0.0f; });
   uchar4 c;
   if (e.error || e.fault_block != -1) {
