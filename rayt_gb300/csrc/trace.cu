@@ -192,13 +192,13 @@ struct RayEnd {
 // the scene's edge: 1919x1079 pixels with nothing in sight 42.5 -> 28.2 us,
 // 512x512 60.6 -> 58.9, a frame full of the scene 321.4 -> 324.2).
 //
-// kMeet: the lanes meet where they have found their child of the root.  Where
-// the view is one of several the compiler left them apart there, and a warp
-// then went through the traversal in parts, by the steps its lanes had taken
-// (500 views of 32x32 pixels 203 us without, 156 so; 12 of 1280x720 full of the
-// scene 1591 and 1545).  With one view it does not, and the meeting costs
-// (512x512 59.0 and 60.2 us).
-template <bool kCount, bool kBias, bool kLazy, bool kMeet, class F>
+// The lanes meet again where they have found their child of the root: left to
+// the compiler, those that found it after as many steps stayed together, and
+// a warp went through the traversal in such parts.  That hardly cost cameras
+// whose root children are met in the same step (512x512 59.0 us, 59.1 with the
+// meeting; the most it costs one is 2%), and others a quarter (512x512 85.5 and
+// 69.2 us, 1919x1079 199 and 175, 500 views of 32x32 203 and 156).
+template <bool kCount, bool kBias, bool kLazy, class F>
 __device__ __forceinline__ RayEnd cast_ray(const TraceCore& p, float4 o, float4& d, uint32_t& fetches,
                                            uint32_t& far_fetches, const F& late_coef) {
   RayEnd r;
@@ -284,7 +284,7 @@ __device__ __forceinline__ RayEnd cast_ray(const TraceCore& p, float4 o, float4&
         break;
       }
     }
-    if (kMeet) __syncwarp(here);
+    __syncwarp(here);
     if (missed) {
       r.node = -1;
       r.iter = iter;
@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(kBlockThreads, 10) trace_kernel(const __grid_c
     return;
   }
   uint32_t fetches = 0, far_fetches = 0;
-  const RayEnd e = cast_ray<kCount, !kFirst, kLazy, sizeof(P) != sizeof(TraceParams1)>(p, o, d, fetches, far_fetches, [&] {
+  const RayEnd e = cast_ray<kCount, !kFirst, kLazy>(p, o, d, fetches, far_fetches, [&] {
     return init_coef(p.views[v], x, y);
   });
   end_ray<kCount>(p, e, ray, o, d, adv, fetches, far_fetches);
@@ -922,7 +922,7 @@ __global__ void __launch_bounds__(kBlockThreads) depth_view_kernel(const __grid_
   const float coef = bias < 1e-10f ? 0.0f : __fdiv_rn(v.lod * (dist(p1f, p2f) - dist(p1n, p2n)), dist(p1n, p1f));
   uint32_t fetches = 0, far_fetches = 0;
   float4 dir = make_float4(dx, dy, dz, coef);
-  const RayEnd e = cast_ray<false, true, false, false>(p, make_float4(o[0], o[1], o[2], bias), dir, fetches, far_fetches,
+  const RayEnd e = cast_ray<false, true, false>(p, make_float4(o[0], o[1], o[2], bias), dir, fetches, far_fetches,
                                                 [] { return 0.0f; });
   uchar4 c;
   if (e.error || e.fault_block != -1) {
