@@ -593,7 +593,6 @@ __device__ __forceinline__ bool even_digit(uint32_t count, int p, uint32_t v, ui
   return (float)count <= share * 1.0625f + 8.f * sqrtf(share) + 8.f;
 }
 constexpr int kHistSmemBytes = kPasses * kBuckets * 32 * 4;
-template <bool kVec>
 __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint32_t* keys, int n, const int* count,
                                                                     uint32_t flip, bool in_place, int split_ranges,
                                                                     Control* ctl, Plan* plan) {
@@ -616,9 +615,10 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
 #pragma unroll
     for (int p = 0; p < kPasses; ++p) atomicAdd(col + (p * kBuckets + ((k >> (8 * p)) & 255u)) * 32, 1u);
   };
-  if (kVec) {  // 16-byte units, four in flight per thread
-    const uint32_t units = m / 4, step = gridDim.x * kHistThreads;
-    const uint4* k4 = reinterpret_cast<const uint4*>(keys);
+  {  // 16-byte units from the first boundary on, four in flight per thread, and the keys beside them
+    const uint32_t head = min(m, (uint32_t)(-(reinterpret_cast<uintptr_t>(keys) >> 2) & 3u));
+    const uint32_t units = (m - head) / 4, step = gridDim.x * kHistThreads;
+    const uint4* k4 = reinterpret_cast<const uint4*>(keys + head);
     uint32_t i = blockIdx.x * kHistThreads + threadIdx.x;
     for (; i + 3 * step < units; i += 4 * step) {  // below 2^28 + 4 * step
       uint4 v[4];
@@ -631,10 +631,10 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
       const uint4 v = __ldg(k4 + i);
       add(v.x), add(v.y), add(v.z), add(v.w);
     }
-    if (blockIdx.x == 0 && threadIdx.x < (m & 3u)) add(keys[units * 4 + threadIdx.x]);
-  } else {
-    for (uint32_t i = blockIdx.x * kHistThreads + threadIdx.x; i < m; i += gridDim.x * kHistThreads)
-      add(__ldg(keys + i));
+    if (blockIdx.x == 0) {
+      if (threadIdx.x < head) add(__ldg(keys + threadIdx.x));
+      if (threadIdx.x < m - head - units * 4) add(__ldg(keys + head + units * 4 + threadIdx.x));
+    }
   }
   __syncthreads();
   {  // thread t: digit value t of the 4 x 256, its 32 columns from its own banks on
@@ -2458,9 +2458,17 @@ __global__ void __launch_bounds__(kScanBlock, 1) scan_kernel(int32_t* data, int 
 }
 
 // Copy of an array that does not start on a 16-byte boundary (the digit passes
-// bring their tiles in by 16-byte copies).
+// bring their tiles in by 16-byte copies), kItems loads in flight per thread.
 __global__ void __launch_bounds__(kThreads) copy_keys_kernel(const uint32_t* in, uint32_t* out, int n) {
-  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < (uint32_t)n; i += gridDim.x * kThreads) out[i] = in[i];
+  for (uint32_t i0 = blockIdx.x * kTile + threadIdx.x; i0 < (uint32_t)n; i0 += gridDim.x * kTile) {
+    uint32_t k[kItems];
+#pragma unroll
+    for (int r = 0; r < kItems; ++r)
+      if (i0 + r * kThreads < (uint32_t)n) k[r] = __ldcs(in + i0 + r * kThreads);
+#pragma unroll
+    for (int r = 0; r < kItems; ++r)
+      if (i0 + r * kThreads < (uint32_t)n) out[i0 + r * kThreads] = k[r];
+  }
 }
 
 int tiles_of(int n, int tile) { return std::max(1, (int)(((long long)n + tile - 1) / tile)); }
@@ -2485,15 +2493,9 @@ int persistent_grid(int tiles, int threads = kThreads, int smem = 0) {
 // Digit counts, offsets and the plan of the passes over n keys (or *count).
 cudaError_t launch_digit_hist(const uint32_t* keys, int n, const int* count, uint32_t flip, bool in_place,
                               int split_ranges, const SortScratchLayout& l, cudaStream_t s) {
-  const int tiles = tiles_of(n, kHistThreads * 4);
-  if ((reinterpret_cast<uintptr_t>(keys) & 15) == 0)
-    digit_hist_kernel<true><<<persistent_grid<digit_hist_kernel<true>>(tiles, kHistThreads, kHistSmemBytes),
-                              kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, split_ranges,
-                                                             l.control, l.plan);
-  else
-    digit_hist_kernel<false><<<persistent_grid<digit_hist_kernel<false>>(tiles, kHistThreads, kHistSmemBytes),
-                               kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, split_ranges,
-                                                             l.control, l.plan);
+  const int grid = persistent_grid<digit_hist_kernel>(tiles_of(n, kHistThreads * 4), kHistThreads, kHistSmemBytes);
+  digit_hist_kernel<<<grid, kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, split_ranges, l.control,
+                                                            l.plan);
   return cudaGetLastError();
 }
 
@@ -2730,7 +2732,7 @@ cudaError_t sort_passes_device(int32_t* data, int n, void* scratch, unsigned lon
   uint32_t* keys = reinterpret_cast<uint32_t*>(data);
   DigitBuffers bufs = {keys, keys, l.keys_a, l.keys_b};
   if (reinterpret_cast<uintptr_t>(data) & 15) {  // the passes read a copy (keys_b is written by the second pass)
-    copy_keys_kernel<<<persistent_grid<copy_keys_kernel>(tiles_of(n, kThreads)), kThreads, 0, s>>>(keys, l.keys_b, n);
+    copy_keys_kernel<<<persistent_grid<copy_keys_kernel>(tiles_of(n, kTile)), kThreads, 0, s>>>(keys, l.keys_b, n);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     bufs.in0 = l.keys_b;
