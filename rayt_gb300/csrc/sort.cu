@@ -600,10 +600,11 @@ __global__ void __launch_bounds__(kHistThreads, 1) digit_hist_kernel(const uint3
   __shared__ uint32_t s_max[kPasses];
   uint32_t not_min = 0, max_key = 0;
   dependents_may_start();
-  for (int i = blockIdx.x * kHistThreads + threadIdx.x; i < kCountValues; i += gridDim.x * kHistThreads)
-    plan->values[i] = 0;
   for (int i = threadIdx.x; i < kPasses * kBuckets * 8; i += kHistThreads)
     reinterpret_cast<uint4*>(s_hist)[i] = make_uint4(0, 0, 0, 0);
+  wait_for_dependency();
+  for (int i = blockIdx.x * kHistThreads + threadIdx.x; i < kCountValues; i += gridDim.x * kHistThreads)
+    plan->values[i] = 0;
   const uint32_t m = count ? (uint32_t)*count : (uint32_t)n;
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -1773,6 +1774,7 @@ __device__ __forceinline__ void unique_kernel_cta(const uint32_t* keys_a, const 
 __global__ void __launch_bounds__(kThreads) unique_kernel(const uint32_t* keys_a, const uint32_t* keys_b,
                                   Control* ctl, const Plan* plan, int32_t* out, unsigned long long* status,
                                   int* result, uint32_t tag, int* err, const DoneFlag done) {
+  wait_for_dependency();
   unique_kernel_cta(keys_a, keys_b, ctl, plan, out, status, result, tag, err);
   publish(done);
 }
@@ -2081,6 +2083,7 @@ __global__ void __launch_bounds__(kShareThreads) direct_bitmap_kernel(const uint
 // turns the counts into offsets.
 __global__ void __launch_bounds__(kThreads) range_hist_kernel(const uint32_t* keys, Control* ctl, Plan* plan) {
   __shared__ uint32_t sh[kBuckets * 32];
+  wait_for_dependency();
   if (plan->path != kPathPartition) return;
   const uint32_t m = (uint32_t)ctl->keys, lo = ~ctl->range[0];
   const int shift = (int)plan->range_shift;
@@ -2129,6 +2132,7 @@ __global__ void __launch_bounds__(kThreads, 4) range_partition_kernel(const uint
   __shared__ uint32_t s_cnt[kBuckets];    // per-tile count, then the tile-local start of each bucket
   __shared__ uint32_t s_base[kBuckets];   // global start of each bucket's run
   __shared__ uint32_t s_keys[kTile];
+  wait_for_dependency();
   if (plan->path != kPathPartition) return;
   const uint32_t m = (uint32_t)ctl->keys, lo = ~ctl->range[0];
   const int shift = (int)plan->range_shift;
@@ -2205,6 +2209,7 @@ __global__ void __launch_bounds__(kThreads) bucket_bitmap_kernel(const uint32_t*
   __shared__ uint32_t s_bits[kSliceWords];
   __shared__ uint32_t s_first[kBuckets + 1];  // first item of each bucket; [256] = all items
   __shared__ int s_item;
+  wait_for_dependency();
   if (plan->path != kPathPartition) return;
   const uint32_t lo = ~ctl->range[0];
   const int shift = (int)plan->range_shift;
@@ -2490,13 +2495,27 @@ int persistent_grid(int tiles, int threads = kThreads, int smem = 0) {
   return std::min(r, tiles);
 }
 
+// Kernel K behind the one before it on the stream, grid CTAs of `threads`.
+template <auto K, class... Args>
+cudaError_t launch_behind(int tiles, int threads, int smem, cudaStream_t s, Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(persistent_grid<K>(tiles, threads, smem));
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, K, args...);
+}
+
 // Digit counts, offsets and the plan of the passes over n keys (or *count).
 cudaError_t launch_digit_hist(const uint32_t* keys, int n, const int* count, uint32_t flip, bool in_place,
                               int split_ranges, const SortScratchLayout& l, cudaStream_t s) {
-  const int grid = persistent_grid<digit_hist_kernel>(tiles_of(n, kHistThreads * 4), kHistThreads, kHistSmemBytes);
-  digit_hist_kernel<<<grid, kHistThreads, kHistSmemBytes, s>>>(keys, n, count, flip, in_place, split_ranges, l.control,
-                                                            l.plan);
-  return cudaGetLastError();
+  return launch_behind<digit_hist_kernel>(tiles_of(n, kHistThreads * 4), kHistThreads, kHistSmemBytes, s, keys, n, count,
+                                          flip, in_place, split_ranges, l.control, l.plan);
 }
 
 // The four digit passes.  `sign_flip`: the keys are signed words (the top
@@ -2547,22 +2566,6 @@ SplitShape split_shape(int n, const SortScratchLayout& l) {
   // about a bin per key, as shared memory allows
   sh.bins = std::min(kSortBins, ((int)sh.room + kSortBinsUnit - 1) / kSortBinsUnit * kSortBinsUnit);
   return sh;
-}
-
-// Kernel K behind the one before it on the stream, grid CTAs of `threads`.
-template <auto K, class... Args>
-cudaError_t launch_behind(int tiles, int threads, int smem, cudaStream_t s, Args... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(persistent_grid<K>(tiles, threads, smem));
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, K, args...);
 }
 
 // f of the smallest of 1, 2, 4 and 8 units per thread with which `threads`
@@ -2674,12 +2677,14 @@ cudaError_t feedback_unique_device(const int32_t* words, int n, int nib, int32_t
                                     dim3(kShareThreads), args, kDirectSliceWords * 4, s);
     if (e != cudaSuccess || n <= kDirectWords) return e;
   }
-  range_hist_kernel<<<persistent_grid<range_hist_kernel>(tiles), kThreads, 0, s>>>(l.keys_a, l.control, l.plan);
-  range_partition_kernel<<<persistent_grid<range_partition_kernel>(tiles), kThreads, 0, s>>>(l.keys_a, l.keys_b,
-                                                                                            l.control, l.plan);
-  bucket_bitmap_kernel<<<persistent_grid<bucket_bitmap_kernel>(tiles), kThreads, 0, s>>>(l.keys_b, l.control, l.plan,
-                                                                                        l.bitmap);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  const uint32_t* sorted = l.keys_b;
+  const Control* counts = l.control;
+  const Plan* chosen = l.plan;
+  if ((e = launch_behind<range_hist_kernel>(tiles, kThreads, 0, s, keys, control, plan)) != cudaSuccess) return e;
+  if ((e = launch_behind<range_partition_kernel>(tiles, kThreads, 0, s, keys, l.keys_b, counts, plan)) != cudaSuccess)
+    return e;
+  if ((e = launch_behind<bucket_bitmap_kernel>(tiles, kThreads, 0, s, sorted, control, chosen, bitmap)) != cudaSuccess)
+    return e;
   const int grid = persistent_grid<emit_kernel>(tiles_of(n, kShareThreads), kShareThreads, kEmitSmemBytes);
   DoneFlag d = done;
   void* args[] = {&bitmap, &control, &plan, &unique_out, &result, &err, &d};
@@ -2700,9 +2705,10 @@ cudaError_t feedback_unique_radix_device(int n, int32_t* unique_out, void* scrat
   const DigitBuffers bufs = {l.keys_a, l.keys_a, l.keys_b, nullptr};
   if ((e = launch_digits(bufs, n, &l.control->keys, false, l, status, epoch, err, DoneFlag{}, s)) != cudaSuccess)
     return e;
-  unique_kernel<<<persistent_grid<unique_kernel>(tiles_of(n, kTile)), kThreads, 0, s>>>(
-      l.keys_a, l.keys_b, l.control, l.plan, unique_out, status, result, epoch * 8u + 4u, err, done);
-  return cudaGetLastError();
+  const uint32_t *keys_a = l.keys_a, *keys_b = l.keys_b;
+  const Plan* plan = l.plan;
+  return launch_behind<unique_kernel>(tiles_of(n, kTile), kThreads, 0, s, keys_a, keys_b, l.control, plan, unique_out,
+                                      status, result, epoch * 8u + 4u, err, done);
 }
 
 bool sort_needs_passes(const int* again) { return *again != 0; }
